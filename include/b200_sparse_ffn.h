@@ -69,24 +69,19 @@ int b200_twell_pack(const void* x, const void* w, const float* bias, void* packe
 
 /*
  * Same as b200_twell_pack with the kernel family chosen by the caller:
- *   kernel 0 = automatic (M == 1: kernel 6 where it serves; M <= 16: split-k cluster kernel on mma.sync;
- *              33..256: kernel 8 / 9 while one wave; 17..32: tcgen05
- *              split-k cluster kernel; M > 32: tcgen05 / TMEM / TMA tile kernel),
+ *   kernel 0 = automatic (M == 1: kernel 6 where it serves; M <= 16: kernel 1; 17..32: kernel 3
+ *              or 5; 33..128: kernel 8 while its grid is one wave; beyond: kernel 7),
  *   kernel 1 = mma.sync split-k cluster kernel (any M),
- *   kernel 2 = tcgen05 tile kernel (64 tokens per CTA tile up to 64 tokens, kernel 7 above;
- *              with B200_PACK_TILE=128: 128-token tiles, two co-resident CTAs per SM from
- *              1024 tokens on),
  *   kernel 3 = tcgen05 split-k cluster kernel (32 tokens per tile, D split 4 ways),
- *   kernel 4 = tcgen05 tile kernel, two co-resident 128-token CTAs per SM at any M,
  *   kernel 5 = tcgen05 split-k cluster kernel with D split 8 ways (D % 512 == 0; chosen
  *              automatically for 17..32 tokens when H <= 2048, e.g. a narrow d_ff shard),
  *   kernel 6 = one-token GEMV kernel (M == 1, D 2048 or 4096): each warp reduces whole
  *              weight rows against the token held in registers, no split-k exchange; chosen
  *              automatically for such calls unless B200_ONE_TOKEN=0,
- *   kernel 7 = tcgen05 tile kernel with 256-token tiles, one CTA per SM and sixteen epilogue
- *              warps (what kernels 0 and 2 run above 64 tokens unless B200_PACK_TILE=128),
+ *   kernel 7 = persistent tcgen05 kernel on pairs of SMs, 256 tokens x 256 neurons per pair, two
+ *              accumulators (2 and 4 are other names of it),
  *   kernel 8 / 9 = tcgen05 split-k cluster kernel with 128-token tiles, D split 4 / 2 ways
- *              (chosen automatically for 33..256 tokens while its grid is a single wave).
+ *              (8 is chosen automatically for 33..128 tokens while its grid is a single wave).
  * All produce identical slab bytes on exact-arithmetic inputs.  No reference
  * counterpart (the reference has one WGMMA kernel, matmul_d2t.cu:287-709).
  */
@@ -133,6 +128,30 @@ int b200_twell_gated_mlp(const void* x, const void* gate, const float* gate_bias
                          const void* up, const void* down, void* packed, void* out,
                          int64_t M, int64_t D, int64_t H, int cf, uint32_t flags,
                          void* workspace, size_t workspace_bytes, void* stream);
+
+/*
+ * The same two functions with room for the hidden matrix: a call of more than a few dozen tokens
+ * then runs as three tensor-core GEMMs (gate + pack, up times the slab pattern, down) instead of
+ * pack + per-entry gathers.  Same slab words; the products of the mixed mode are not rounded to
+ * bf16 one by one (fp32 sums of exact products), the high-precision mode keeps its hidden values
+ * to 24 bits as three bf16 terms.
+ *   scratch: b200_twell_mlp_scratch_bytes(M, D, H, gated, flags) bytes (0 = such a call has no
+ *     use for it), 16-byte aligned, uninitialised.  NULL or too small: the functions above.
+ *   workspace: as above; its zero-filled counters are also used to finish the last wave of
+ *     tiles in ranges of k (without a workspace that wave runs unsplit).
+ */
+size_t b200_twell_mlp_scratch_bytes(int64_t M, int64_t D, int64_t H, int gated, uint32_t flags);
+
+int b200_twell_gated_mlp_scratch(const void* x, const void* gate, const float* gate_bias,
+                                 const void* up, const void* down, void* packed, void* out,
+                                 int64_t M, int64_t D, int64_t H, int cf, uint32_t flags,
+                                 void* workspace, size_t workspace_bytes, void* scratch,
+                                 size_t scratch_bytes, void* stream);
+
+int b200_twell_mlp_scratch(const void* x, const void* up, const void* down, void* packed, void* out,
+                           int64_t M, int64_t D, int64_t H, int cf, int num_splits,
+                           void* workspace, size_t workspace_bytes, void* scratch,
+                           size_t scratch_bytes, void* stream);
 
 /*
  * The fused gated MLP as ONE kernel for decode-sized calls (1 <= M <= 32): a thread-block

@@ -26,25 +26,20 @@ int fail(int code, const char* fmt, ...) {
 
 int twell_pack_small(const void* x, const void* w, const float* bias, void* packed, int64_t M,
                      int64_t D, int64_t H, int cf, cudaStream_t stream);
-int twell_pack_tc(const void* x, const void* w, const float* bias, void* packed, int64_t M,
-                  int64_t D, int64_t H, int cf, cudaStream_t stream);
 int twell_pack_tc_splitk(const void* x, const void* w, const float* bias, void* packed, int64_t M,
                          int64_t D, int64_t H, int cf, cudaStream_t stream);
-int twell_pack_tc_pair(const void* x, const void* w, const float* bias, void* packed, int64_t M,
-                       int64_t D, int64_t H, int cf, cudaStream_t stream);
 int twell_pack_tc_splitk8(const void* x, const void* w, const float* bias, void* packed,
                           int64_t M, int64_t D, int64_t H, int cf, cudaStream_t stream);
 int twell_pack_tc_splitk_mid(const void* x, const void* w, const float* bias, void* packed,
                              int64_t M, int64_t D, int64_t H, int cf, int split,
                              cudaStream_t stream);
 int twell_pack_mid_split(int64_t M, int64_t H, int sm_count);
-int twell_pack_tc_wide(const void* x, const void* w, const float* bias, void* packed, int64_t M,
-                       int64_t D, int64_t H, int cf, cudaStream_t stream);
 int twell_pack_tc_status();
 int twell_t2d_launch(bool gated, bool hp, const void* x, const void* packed, const void* up,
                      const void* down, void* out, int64_t M, int64_t D, int64_t H, int cf,
                      void* workspace, size_t workspace_bytes, int sm_count, cudaStream_t stream,
-                     const unsigned char* skip_rows = nullptr, const FusedAr* fused_ar = nullptr);
+                     const unsigned char* skip_rows = nullptr, const FusedAr* fused_ar = nullptr,
+                     const RunIf& run_if = {nullptr, 0u});
 
 size_t twell_decode_workspace_bytes(int64_t M, int64_t D, int64_t H);
 int twell_decode_launch(bool gated, bool hp, const void* x, const void* gate, const float* bias,
@@ -67,6 +62,15 @@ int twell_gemv_layer(bool gated, bool hp, const void* x, const void* w, const fl
                      const void* up, const void* down, void* packed, void* out, int64_t D,
                      int64_t H, int cf, void* workspace, size_t workspace_bytes,
                      cudaStream_t stream);
+int pair_pack(const void* x, const void* w, const float* bias, void* packed, void* dense, int64_t M,
+              int64_t D, int64_t H, int cf, unsigned int* entries, float* part,
+              unsigned int* counters, cudaStream_t stream);
+bool pair_mlp_serves(int64_t M, int64_t D, int64_t H, bool gated, bool hp);
+size_t pair_mlp_scratch_bytes(int64_t M, int64_t D, int64_t H, bool gated, bool hp);
+int pair_mlp(bool gated, bool hp, const void* x, const void* gate, const float* bias,
+             const void* up, const void* down, void* packed, void* out, int64_t M, int64_t D,
+             int64_t H, int cf, void* workspace, size_t workspace_bytes, void* scratch,
+             cudaStream_t stream);
 int twell_decode_status();
 #ifdef B200_TRACE
 void twell_decode_trace(unsigned long long* out16);
@@ -183,9 +187,7 @@ int b200_twell_pack_select(const void* x, const void* w, const float* bias, void
   if (bias != nullptr && (reinterpret_cast<uintptr_t>(bias) & 3u))
     return fail(B200_EALIGN, "%s: bias is not 4-byte aligned", fn);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  // Up to one 32-token tile the weight stream is read once and the split-k kernels are
-  // HBM-bound; 33..256 tokens take 128-token tiles, still split over a cluster while that grid
-  // is one wave; beyond that the tcgen05 tile kernel reuses each weight tile for 256 tokens.
+  // Up to one 32-token tile the weight stream is read once and the split-k kernels are HBM-bound.
   // Measured on B200 (D 2048, H 8192): up to 16 tokens the mma.sync cluster kernel is
   // fastest (9.6-9.9 us vs 11.7-12.4); at 17..32 tokens its mma work per CTA grows and the
   // tcgen05 split-k kernel wins (12.5 vs 13.9 us).
@@ -201,19 +203,20 @@ int b200_twell_pack_select(const void* x, const void* w, const float* bias, void
     return twell_pack_tc_splitk8(x, w, bias, packed, M, D, H, cf, st);
   if (kernel == 3 || (kernel == 0 && M > 16 && M <= 32))
     return twell_pack_tc_splitk(x, w, bias, packed, M, D, H, cf, st);
-  if (kernel == 4) return twell_pack_tc_pair(x, w, bias, packed, M, D, H, cf, st);
   if (kernel == 5) return twell_pack_tc_splitk8(x, w, bias, packed, M, D, H, cf, st);
-  if (kernel == 7) return twell_pack_tc_wide(x, w, bias, packed, M, D, H, cf, st);
   if (kernel == 8) return twell_pack_tc_splitk_mid(x, w, bias, packed, M, D, H, cf, 4, st);
   if (kernel == 9) return twell_pack_tc_splitk_mid(x, w, bias, packed, M, D, H, cf, 2, st);
-  // 33..256 tokens: 128-token tiles with d_model split over a cluster while that grid is one wave.
-  if (kernel == 0 && M > 32 && M <= 256) {
-    const int split = twell_pack_mid_split(M, H, sm_count());
-    if (split != 0) return twell_pack_tc_splitk_mid(x, w, bias, packed, M, D, H, cf, split, st);
-  }
-  const bool use_tc = kernel == 2 || (kernel == 0 && M > 32);
-  return use_tc ? twell_pack_tc(x, w, bias, packed, M, D, H, cf, st)
-                : twell_pack_small(x, w, bias, packed, M, D, H, cf, st);
+  // 33..128 tokens: 128-token tiles with d_model split four ways over a cluster while that grid is
+  // one wave; beyond, 256-token tiles on pairs of SMs.  Measured on B200, us, split-k / pairs:
+  // D 2048, H 8192: 128 tokens 16.0 / 19.9, 256 tokens 25.7 (two-way split) / 20.5; D 4096,
+  // H 16384, 64 tokens: 40.4 (no split fits one wave) / 35.5; D 1024, H 4096, 256 tokens:
+  // 13.2 / 13.7.  Against one-SM tiles of 256 tokens from 257 tokens on: D 2048, H 8192:
+  // 512 tokens 34.6 / 21.5, 2048 tokens 67 / 58, 16384 tokens 576 / 397.
+  if (kernel == 0 && M > 32 && M <= 128 && twell_pack_mid_split(M, H, sm_count()) == 4)
+    return twell_pack_tc_splitk_mid(x, w, bias, packed, M, D, H, cf, 4, st);
+  if (kernel == 2 || kernel == 4 || kernel == 7 || (kernel == 0 && M > 32))
+    return pair_pack(x, w, bias, packed, nullptr, M, D, H, cf, nullptr, nullptr, nullptr, st);
+  return twell_pack_small(x, w, bias, packed, M, D, H, cf, st);
 }
 
 int b200_twell_pack(const void* x, const void* w, const float* bias, void* packed, int64_t M,
@@ -389,6 +392,38 @@ int b200_twell_gated_mlp(const void* x, const void* gate, const float* gate_bias
                               workspace_bytes, stream);
 }
 
+namespace {
+// Whether a fused-MLP call runs on the paired tensor-core GEMM with the given scratch.
+bool pair_wanted(int64_t M, int64_t D, int64_t H, bool gated, bool hp, const void* scratch,
+                 size_t scratch_bytes) {
+  if (scratch == nullptr || M < 1 || D % 256 || H % 256 || D < 256 || D > 4096) return false;
+  const size_t need = pair_mlp_scratch_bytes(M, D, H, gated, hp);
+  return need != 0 && scratch_bytes >= need;
+}
+}  // namespace
+
+size_t b200_twell_mlp_scratch_bytes(int64_t M, int64_t D, int64_t H, int gated, uint32_t flags) {
+  if (M <= 0 || D < 256 || D > 4096 || D % 256 || H < 256 || H > 65536 || H % 256) return 0;
+  return pair_mlp_scratch_bytes(M, D, H, gated != 0, (flags & B200_FLAG_HIGH_PRECISION) != 0);
+}
+
+int b200_twell_gated_mlp_scratch(const void* x, const void* gate, const float* gate_bias,
+                                 const void* up, const void* down, void* packed, void* out,
+                                 int64_t M, int64_t D, int64_t H, int cf, uint32_t flags,
+                                 void* workspace, size_t workspace_bytes, void* scratch,
+                                 size_t scratch_bytes, void* stream) {
+  const bool hp = (flags & B200_FLAG_HIGH_PRECISION) != 0;
+  if (pair_wanted(M, D, H, true, hp, scratch, scratch_bytes)) {
+    B200_TRY(check_decode_args("b200_twell_gated_mlp", x, gate, gate_bias, up, down, packed, out,
+                               M, D, H, cf, flags, workspace, true));
+    B200_TRY(check_ptr("b200_twell_gated_mlp", "scratch", scratch));
+    return pair_mlp(true, hp, x, gate, gate_bias, up, down, packed, out, M, D, H, cf,
+                    workspace, workspace_bytes, scratch, static_cast<cudaStream_t>(stream));
+  }
+  return b200_twell_gated_mlp(x, gate, gate_bias, up, down, packed, out, M, D, H, cf, flags,
+                              workspace, workspace_bytes, stream);
+}
+
 size_t b200_fused_allreduce_block_bytes(int64_t max_tokens, int64_t D) {
   if (max_tokens <= 0 || D <= 0) return 0;
   const size_t slot = ((size_t)max_tokens * (size_t)D * 4 + 255) & ~(size_t)255;
@@ -477,6 +512,22 @@ int b200_twell_mlp(const void* x, const void* up, const void* down, void* packed
   B200_TRY(b200_twell_pack(x, up, nullptr, packed, M, D, H, cf, stream));
   return b200_twell_t2d(packed, down, out, M, D, H, cf, num_splits, workspace, workspace_bytes,
                         stream);
+}
+
+int b200_twell_mlp_scratch(const void* x, const void* up, const void* down, void* packed, void* out,
+                           int64_t M, int64_t D, int64_t H, int cf, int num_splits,
+                           void* workspace, size_t workspace_bytes, void* scratch,
+                           size_t scratch_bytes, void* stream) {
+  if ((num_splits == 1 || num_splits == 2 || num_splits == 4 || num_splits == 8) &&
+      pair_wanted(M, D, H, false, false, scratch, scratch_bytes)) {
+    B200_TRY(check_decode_args("b200_twell_mlp", x, up, nullptr, nullptr, down, packed, out, M, D,
+                               H, cf, 0, workspace, false));
+    B200_TRY(check_ptr("b200_twell_mlp", "scratch", scratch));
+    return pair_mlp(false, false, x, up, nullptr, nullptr, down, packed, out, M, D, H, cf,
+                    workspace, workspace_bytes, scratch, static_cast<cudaStream_t>(stream));
+  }
+  return b200_twell_mlp(x, up, down, packed, out, M, D, H, cf, num_splits, workspace,
+                        workspace_bytes, stream);
 }
 
 }  // extern "C"

@@ -107,6 +107,14 @@ constexpr int kFarErrorWord = 2;            // set when a wait for a peer gave u
 constexpr size_t kFarControlBytes = 1024;   // control words, padding; the inbox follows
 constexpr int kFarMaxTokens = 256;
 
+// A choice between two forms of one product that the device makes itself: the gather form runs
+// when *entries <= limit (stored gate entries of the call), the dense form when it is larger.
+// The form that does not run returns at once.  entries == nullptr: the launched form runs.
+struct RunIf {
+  const unsigned int* entries;
+  unsigned int limit;
+};
+
 __device__ __forceinline__ uint32_t bf16_bits(float v) {
   return (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(v));
 }

@@ -32,8 +32,18 @@ namespace b200 {
 int twell_t2d_launch(bool gated, bool hp, const void* x, const void* packed, const void* up,
                      const void* down, void* out, int64_t M, int64_t D, int64_t H, int cf,
                      void* workspace, size_t workspace_bytes, int sm_count, cudaStream_t stream,
-                     const unsigned char* skip_rows, const FusedAr* fused_ar);
+                     const unsigned char* skip_rows, const FusedAr* fused_ar,
+                     const RunIf& run_if = {nullptr, 0u});
 int sm_count();
+int pair_gemm_status();
+bool pair_mlp_serves(int64_t M, int64_t D, int64_t H, bool gated, bool hp);
+size_t pair_part_bytes(int64_t M, int64_t D, int64_t H);
+int pair_gate_up(bool hp, const void* x, const void* gate, const float* bias, const void* up,
+                 void* packed, void* hidden, int64_t M, int64_t D, int64_t H, int cf,
+                 bool keep_all, cudaStream_t stream);
+int pair_down(const void* hidden, int terms, const void* down, void* out, int64_t M, int64_t D,
+              int64_t H, const RunIf& run_if, float* part, unsigned int* counters,
+              cudaStream_t stream);
 
 namespace {
 
@@ -136,6 +146,25 @@ route_compact_kernel(unsigned char* __restrict__ flags, int M, int cap, int* __r
   if (lossy) atomicAdd(&lossy_s, lossy);
   __syncthreads();
   if (tid == 0) counters[1] = lossy_s;
+}
+
+// Overflowed rows that stay lossy (the capacity of the dense route is exhausted): their hidden values
+// past the last stored column of an overflowed tile are cleared.  One warp per row.
+__global__ void __launch_bounds__(256)
+truncate_rows_kernel(const uint32_t* __restrict__ packed, const unsigned char* __restrict__ flags,
+                     const int* __restrict__ counters, int M, int tiles, int slab_w,
+                     __nv_bfloat16* __restrict__ hidden) {
+  if (counters[1] == 0) return;
+  const int row = blockIdx.x * 8 + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (row >= M || flags[row] != 0) return;  // flags of rows beyond the capacity are cleared
+  const uint32_t* prow = packed + (size_t)row * tiles * slab_w;
+  for (int t = 0; t < tiles; ++t) {
+    if ((int)prow[(size_t)t * slab_w] < slab_w) continue;
+    const int last = (int)(prow[(size_t)t * slab_w + slab_w - 1] & 255u);
+    for (int c = last + 1 + lane; c < kTileN; c += 32)
+      hidden[(size_t)row * tiles * kTileN + t * kTileN + c] = __float2bfloat16(0.f);
+  }
 }
 
 __global__ void __launch_bounds__(256)
@@ -845,6 +874,8 @@ struct DenseWs {
   int* counters;         // [4]
   __nv_bfloat16* xd;     // [cap_pad, D]
   __nv_bfloat16* hd;     // [cap_pad, H]
+  __nv_bfloat16* h_all;  // [M, H]: every row's hidden values (the form of b200_twell_gated_mlp_hybrid
+  float* part;           //   on paired tensor-core tiles) and its split-tile sums, over xd / hd
   size_t total;
 };
 
@@ -866,6 +897,14 @@ DenseWs dense_ws_layout(void* base, int64_t M, int64_t D, int64_t H, int64_t cap
   w.hd = reinterpret_cast<__nv_bfloat16*>(p + off);
   off += align256((size_t)cap_pad * H * 2);
   w.total = off;
+  if (pair_mlp_serves(M, D, H, true, false)) {
+    off = (size_t)(reinterpret_cast<unsigned char*>(w.xd) - p);
+    w.h_all = w.xd;
+    off += align256((size_t)M * H * 2);
+    w.part = reinterpret_cast<float*>(p + off);
+    off += align256(pair_part_bytes(M, D, H));
+    if (off > w.total) w.total = off;
+  }
   return w;
 }
 
@@ -1227,6 +1266,42 @@ int b200_twell_gated_mlp_hybrid(const void* x, const void* gate, const float* ga
                                 uint32_t flags, int64_t nnz_threshold, int64_t dense_cap,
                                 void* hybrid_ws, size_t hybrid_ws_bytes, void* workspace,
                                 size_t workspace_bytes, void* stream) {
+  const char* fn = "b200_twell_gated_mlp_hybrid";
+  if (M > 0 && flags == 0 && D <= 4096 && pair_mlp_serves(M, D, H, true, false) && dense_cap > 0 &&
+      nnz_threshold >= 0 && M <= (int64_t)1 << 20 && hybrid_ws != nullptr && x && gate && up &&
+      down && down_t && packed && out) {
+    // Large calls: every row on the paired tensor-core tiles.  The hidden values of a routed row
+    // are those of the dense formula as long as no positive is dropped, so routing only decides
+    // which overflowed rows stay lossy (beyond dense_cap); nothing is computed twice.
+    if (int rc = check_dims(fn, M, D, H, cf)) return rc;
+    const void* ptrs[8] = {x, packed, gate, up, down, down_t, out, hybrid_ws};
+    const char* names[8] = {"x", "packed", "gate", "up", "down", "down_t", "out", "hybrid_ws"};
+    for (int i = 0; i < 8; ++i)
+      if (!aligned16(ptrs[i])) return fail(B200_EALIGN, "%s: %s is not 16-byte aligned", fn, names[i]);
+    if (reinterpret_cast<uintptr_t>(hybrid_ws) & 255u)
+      return fail(B200_EALIGN, "%s: hybrid_ws is not 256-byte aligned", fn);
+    if (dense_cap > M) dense_cap = M;
+    DenseWs w = dense_ws_layout(hybrid_ws, M, D, H, dense_cap);
+    if (hybrid_ws_bytes < w.total)
+      return fail(B200_EWORKSPACE, "%s: hybrid_ws holds %zu bytes, %zu needed", fn, hybrid_ws_bytes,
+                  w.total);
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const int tiles = (int)(H / kTileN), slab_w = kTileN / cf;
+    if (int rc = pair_gate_up(false, x, gate, gate_bias, up, packed, w.h_all, M, D, H, cf, true, st))
+      return rc;
+    const unsigned row_blocks = (unsigned)((M + 7) / 8);
+    route_flags_kernel<<<row_blocks, 256, 0, st>>>(
+        static_cast<const uint32_t*>(packed), (int)M, tiles, slab_w,
+        (int)(nnz_threshold > 0x7fffffff ? 0x7fffffff : nnz_threshold), w.flags);
+    route_compact_kernel<<<1, 1024, 0, st>>>(w.flags, (int)M, (int)dense_cap, w.rows, w.counters);
+    if (dense_cap < M)
+      truncate_rows_kernel<<<row_blocks, 256, 0, st>>>(static_cast<const uint32_t*>(packed), w.flags,
+                                                      w.counters, (int)M, tiles, slab_w, w.h_all);
+    if (int rc = check_launch(fn)) return rc;
+    return pair_down(w.h_all, 1, down, out, M, D, H, {nullptr, 0u}, w.part,
+                     workspace != nullptr && workspace_bytes >= 16384
+                         ? static_cast<unsigned int*>(workspace) : nullptr, st);
+  }
   if (int rc = b200_twell_pack(x, gate, gate_bias, packed, M, D, H, cf, stream)) return rc;
   return b200_twell_gated_t2d_hybrid(x, packed, gate, gate_bias, up, down, down_t, out, M, D, H,
                                      cf, flags, nnz_threshold, dense_cap, hybrid_ws,
@@ -1276,7 +1351,8 @@ int b200_twell_hybrid_status(void) {
   int v = 0, zero = 0;
   if (cudaMemcpyFromSymbol(&v, g_dense_error, sizeof(int)) != cudaSuccess) return -1;
   if (v != 0) cudaMemcpyToSymbol(g_dense_error, &zero, sizeof(int));
-  return v;
+  const int pair = pair_gemm_status();
+  return v != 0 ? v : pair;
 }
 
 }  // extern "C"

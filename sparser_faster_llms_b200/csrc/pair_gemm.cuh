@@ -1,0 +1,951 @@
+// Persistent tcgen05 GEMM on pairs of SMs (cta_group::2) with the sparse-FFN epilogues.
+//
+//   acc[m, n] = sum_k A[m, k] B[n, k]      bf16 operands, fp32 accumulators in TMEM
+//
+// A pair of CTAs (cluster of 2) computes 256 rows x 256 columns; CTA r holds rows
+// [128 r, +128) of A, columns [128 r, +128) of B and the accumulator of its rows (TMEM lane =
+// row, TMEM column = column).  A 64-k stage is 16 KB + 16 KB per CTA, i.e. 128 flop per staged
+// byte: the rate of the 256 x 256 one-CTA tile, at half its TMEM, so that two accumulators fit and
+// the epilogue of tile i runs under the MMAs of tile i + 1.
+//
+// Either operand may be K-major (rows of k-values) or MN-major (stored [k][m]): products with a
+// transposed operand read the matrix where it lies, no transpose pass.  B can change after
+// seg_ksteps k-steps (one accumulator over [A0 | A1] [B0; B1]) and both operands at row tile
+// second_mt (several products in one launch).
+//
+// Work items: the first full_tiles tiles are one item each; each later tile (the last wave, or
+// all tiles of a product too small to fill the GPU) is cut into `splits` ranges of k.  The warp
+// that arrives last at a (tile, 32-row, column-half) block adds the ranges' fp32 sums in order
+// and runs the epilogue on them, so the result does not depend on the arrival order.
+//
+// Roles per CTA (320 threads): warp 0 TMA producer, warp 1 MMA issuer (leader CTA only), warps
+// 2..9 epilogue, two per TMEM lane quarter.  Barriers:
+//   full[s]   leader:  both CTAs' copies of stage s have landed (the peer's copies signal it too)
+//   empty[s]  each CTA: the MMAs have read stage s (multicast commit)
+//   tfull[b]  each CTA: accumulator b is complete (multicast commit)
+//   tempty[b] leader:  every epilogue warp of both CTAs has read accumulator b
+// Every wait is bounded; a wait that gives up sets the error word, and the CTA pair leaves
+// through the common cluster barrier, which frees TMEM.
+#pragma once
+
+#include <cooperative_groups.h>
+
+#include "tc_common.cuh"
+
+namespace b200 {
+namespace {
+
+namespace pg {
+
+constexpr int kThreads = 320;
+constexpr int kTile = 256;                   // rows and columns per pair
+constexpr int kOperandBytes = 128 * 128;     // one CTA's half of A or B per 64-k stage
+constexpr int kStageBytes = 2 * kOperandBytes;
+constexpr int kBufBytes = 8 * 32 * 256;       // pattern buffers: 32 rows x 256 bytes per epilogue warp
+
+enum Epilogue {
+  kStore = 0,    // out[row, col] = bf16(acc)
+  kPack = 1,     // TwELL slabs of relu(acc + bias)
+  kPackDense = 6,  // the same, and the stored values as a dense matrix
+  kGateUp = 7,   // kPack on a first accumulator (B0) and kMul with its values on a second (B1)
+  kGateUpHp = 8, // kPack and kMulHp likewise
+  kMul = 2,      // out = bf16(g * bf16(acc)) on the slab pattern, 0 elsewhere
+  kMulHp = 3,    // g * acc in fp32, as three bf16 terms side by side (out row = [hi | mid | lo])
+  kFwd = 4,      // training forward: R = bf16(acc) and T = R * P as slabs, T dense, l1 partial sums
+  kBwd = 5       // training backward: dense [dR | dU] and T from acc = dT
+};
+
+struct Args {
+  int rows;                  // rows of the product (device count in rows_ptr when not null)
+  const int* rows_ptr;
+  int n_tiles, ksteps, seg_ksteps, second_mt, group;
+  int full_tiles, splits;    // see above; splits == 1: no split (full_tiles unused)
+  float* sums;               // kStore, every tile split: fp32 sums [splits][rows][256 n_tiles]
+  float* part;               // [items of split tiles][2][8 warps][128 columns][32 rows]
+  unsigned int* counters;    // [split tiles][2][8], zero at rest
+  __nv_bfloat16* out;        // dense result, row stride ld
+  long long ld;
+  int wide;                  // out rows are 32-byte aligned
+  const float* bias;         // packs; bias16: 16-byte aligned
+  int bias16;
+  // slab operands [rows][row_words], slab_w words per 256 columns
+  uint32_t* slab_p;          // pattern and values (kPack: output)
+  uint32_t* slab_r;          // kFwd: output, kBwd: input
+  uint32_t* slab_t;          // kFwd: output
+  int slab_w, row_words;
+  // rows taken out of the slabs: row_slot[row] >= 0 is the row of tail_p / tail_r
+  const int* row_slot;
+  const __nv_bfloat16* tail_p;
+  const __nv_bfloat16* tail_r;
+  __nv_bfloat16* dense_t;    // kBwd: T, row stride ld_t
+  long long ld_t;
+  float* l1_part;            // kFwd: [2 n_tiles][rows] sums of |T|
+  const float* l1_grad;      // kBwd: device scalar or null
+  float inv_m;
+  int keep_all;              // kGateUp: values past a slab's capacity still count in the product
+  unsigned int* entries;     // packs: stored entries are added here (may be null)
+  RunIf run_if;
+};
+
+__device__ int g_error = 0;
+
+__device__ __forceinline__ void tma_load(uint32_t dst, const CUtensorMap* map, int c0, int c1,
+                                         uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
+      "[%0], [%1, {%2, %3}], [%4];"
+      ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(bar)
+      : "memory");
+}
+
+__device__ __forceinline__ void mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc,
+                                    uint32_t accumulate) {
+  asm volatile(
+      "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}"
+      ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
+// Arrives at the barrier of the same offset in both CTAs once all MMAs issued so far are done.
+__device__ __forceinline__ void commit(uint64_t* bar) {
+  asm volatile(
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 "
+      "[%0], %1;"
+      ::"r"(smem_u32(bar)), "h"((uint16_t)3)
+      : "memory");
+}
+
+__device__ __forceinline__ void arrive_leader(uint64_t* bar) {
+  asm volatile(
+      "{\n.reg .b32 a;\nmapa.shared::cluster.u32 a, %0, 0;\n"
+      "mbarrier.arrive.release.cluster.shared::cluster.b64 _, [a];\n}"
+      ::"r"(smem_u32(bar))
+      : "memory");
+}
+
+// MN-major operand, 128-byte swizzle: 64 x 64 boxes of 8 KB, 8-k groups 1024 B apart.
+__device__ __forceinline__ uint64_t desc_mn(uint32_t saddr) {
+  uint64_t d = 0;
+  d |= (uint64_t)((saddr & 0x3FFFFu) >> 4);
+  d |= (uint64_t)(8192 >> 4) << 16;           // next 64 rows / columns
+  d |= (uint64_t)(1024 >> 4) << 32;           // next 8 k
+  d |= (uint64_t)1 << 46;
+  d |= (uint64_t)2 << 61;
+  return d;
+}
+
+// Item t -> tile and range of k-steps; the split tile's index and the item's place in part[].
+struct Item {
+  int tile, k0, k1, split_tile, split;
+};
+__device__ __forceinline__ Item item_of(int t, const Args& a) {
+  Item it = {t, 0, a.ksteps, -1, 0};
+  if (a.splits > 1 && t >= a.full_tiles) {
+    const int j = t - a.full_tiles;
+    it.split_tile = j / a.splits;
+    it.split = j - it.split_tile * a.splits;
+    it.tile = a.full_tiles + it.split_tile;
+    it.k0 = it.split * a.ksteps / a.splits;
+    it.k1 = (it.split + 1) * a.ksteps / a.splits;
+  }
+  return it;
+}
+
+__device__ __forceinline__ void tile_of(int t, int m_tiles, const Args& a, int& mt, int& nt) {
+  const int per = a.group * a.n_tiles;
+  const int g = t / per, first = g * a.group, in = t - g * per;
+  const int rows = min(a.group, m_tiles - first);
+  mt = first + in % rows;
+  nt = in / rows;
+}
+
+__device__ __forceinline__ uint32_t pack2(float a, float b) {
+  __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<uint32_t*>(&v);
+}
+__device__ __forceinline__ uint32_t mul2(uint32_t a, uint32_t b) {
+  __nv_bfloat162 v = __hmul2(*reinterpret_cast<__nv_bfloat162*>(&a),
+                             *reinterpret_cast<__nv_bfloat162*>(&b));
+  return *reinterpret_cast<uint32_t*>(&v);
+}
+// 0xFFFF per half whose value is not +-0.
+__device__ __forceinline__ uint32_t nonzero2(uint32_t a) {
+  const __nv_bfloat162 z = __floats2bfloat162_rn(0.f, 0.f);
+  return __hne2_mask(*reinterpret_cast<__nv_bfloat162*>(&a), z);
+}
+__device__ __forceinline__ float lo_f(uint32_t w) { return __uint_as_float(w << 16); }
+__device__ __forceinline__ float hi_f(uint32_t w) { return __uint_as_float(w & 0xFFFF0000u); }
+
+// 64 consecutive bytes (32 bf16) of one row per lane; `wide`: the row is 32-byte aligned, so a
+// lane fills whole sectors with 256-bit stores.
+__device__ __forceinline__ void store64(__nv_bfloat16* p, const uint32_t (&w)[16], int wide) {
+  if (wide) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+      asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                   ::"l"(p + i * 16), "r"(w[8 * i]), "r"(w[8 * i + 1]), "r"(w[8 * i + 2]),
+                     "r"(w[8 * i + 3]), "r"(w[8 * i + 4]), "r"(w[8 * i + 5]), "r"(w[8 * i + 6]),
+                     "r"(w[8 * i + 7])
+                   : "memory");
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      reinterpret_cast<uint4*>(p)[i] = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
+  }
+}
+
+// Byte `off` of row `row` in a warp's pattern buffer: 256 bytes per row, 16-byte pieces swizzled so
+// that 32 lanes reading the same piece of their own rows hit all banks.
+__device__ __forceinline__ unsigned char* at(unsigned char* buf, int row, int off) {
+  return buf + row * 256 + ((off & ~15) ^ ((row & 7) << 4)) + (off & 15);
+}
+
+// Pattern buffer of one warp: 32 rows x 128 columns of bf16 values (zero where nothing is stored),
+// filled from the slabs of tile `nt`, columns [128 half, +128); rows with a tail slot get their
+// dense values.
+__device__ __forceinline__ void load_values(const Args& a, unsigned char* buf, int row0, int rows,
+                                            int nt, int half, int lane) {
+#pragma unroll
+  for (int i = 0; i < 16; ++i)
+    *reinterpret_cast<uint4*>(buf + lane * 256 + i * 16) = make_uint4(0u, 0u, 0u, 0u);
+  __syncwarp();
+  const uint32_t* base = a.slab_p + (size_t)nt * a.slab_w;
+  for (int t0 = 0; t0 < 32; t0 += 8) {
+    if (row0 + t0 >= rows) break;
+    int cnt[8], most = 0;
+    for (int w0 = 0; w0 < a.slab_w; w0 += 32) {
+      uint32_t w[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int row = row0 + t0 + j;
+        w[j] = row < rows ? base[(size_t)row * a.row_words + w0 + lane] : 0u;
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        if (w0 == 0) {
+          cnt[j] = min(max((int)__shfl_sync(0xffffffffu, w[j], 0), 0), a.slab_w - 1);
+          most = max(most, cnt[j]);
+        }
+        const int slot = w0 + lane, col = (int)(w[j] & 255u);
+        if (slot >= 1 && slot <= cnt[j] && (col >> 7) == half)
+          *reinterpret_cast<uint16_t*>(at(buf, t0 + j, (col & 127) * 2)) =
+              (uint16_t)(w[j] >> 16);
+      }
+      if (most < w0 + 32) break;
+    }
+  }
+  if (a.row_slot != nullptr) {
+    const int mine = row0 + lane < rows ? a.row_slot[row0 + lane] : -1;
+    uint32_t todo = __ballot_sync(0xffffffffu, mine >= 0);
+    __syncwarp();
+    while (todo != 0u) {
+      const int t = __ffs(todo) - 1;
+      todo &= todo - 1;
+      const int slot = __shfl_sync(0xffffffffu, mine, t);
+      const __nv_bfloat16* src =
+          a.tail_p + (size_t)slot * a.n_tiles * kTile + nt * kTile + half * 128 + lane * 4;
+      *reinterpret_cast<uint2*>(at(buf, t, lane * 8)) =
+          *reinterpret_cast<const uint2*>(src);
+    }
+  }
+  __syncwarp();
+}
+
+// The same with P and R interleaved (u32 = P | R << 16) for columns [64 quarter, +64) of the tile.
+__device__ __forceinline__ void load_pairs(const Args& a, unsigned char* buf, int row0, int rows,
+                                           int nt, int quarter, int lane) {
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 16; ++i)
+    *reinterpret_cast<uint4*>(buf + lane * 256 + i * 16) = make_uint4(0u, 0u, 0u, 0u);
+  __syncwarp();
+  const size_t tile_off = (size_t)nt * a.slab_w;
+  for (int t0 = 0; t0 < 32; t0 += 8) {
+    if (row0 + t0 >= rows) break;
+    int cnt[8], most = 0;
+    for (int w0 = 0; w0 < a.slab_w; w0 += 32) {
+      uint32_t w[8], r[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int row = row0 + t0 + j;
+        const size_t off = (size_t)row * a.row_words + tile_off + w0 + lane;
+        w[j] = row < rows ? a.slab_p[off] : 0u;
+        r[j] = row < rows ? a.slab_r[off] : 0u;
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        if (w0 == 0) {
+          cnt[j] = min(max((int)__shfl_sync(0xffffffffu, w[j], 0), 0), a.slab_w - 1);
+          most = max(most, cnt[j]);
+        }
+        const int slot = w0 + lane, col = (int)(w[j] & 255u);
+        if (slot >= 1 && slot <= cnt[j] && (col >> 6) == quarter)
+          *reinterpret_cast<uint32_t*>(at(buf, t0 + j, (col & 63) * 4)) =
+              __byte_perm(w[j], r[j], 0x7632);
+      }
+      if (most < w0 + 32) break;
+    }
+  }
+  if (a.row_slot != nullptr) {
+    const int mine = row0 + lane < rows ? a.row_slot[row0 + lane] : -1;
+    uint32_t todo = __ballot_sync(0xffffffffu, mine >= 0);
+    __syncwarp();
+    while (todo != 0u) {
+      const int t = __ffs(todo) - 1;
+      todo &= todo - 1;
+      const int slot = __shfl_sync(0xffffffffu, mine, t);
+      const size_t off = (size_t)slot * a.n_tiles * kTile + nt * kTile + quarter * 64 + lane * 2;
+      const uint32_t p2 = *reinterpret_cast<const uint32_t*>(a.tail_p + off);
+      const uint32_t r2 = *reinterpret_cast<const uint32_t*>(a.tail_r + off);
+      *reinterpret_cast<uint2*>(at(buf, t, lane * 8)) =
+          make_uint2(__byte_perm(p2, r2, 0x5410), __byte_perm(p2, r2, 0x7632));
+    }
+  }
+  __syncwarp();
+}
+
+// The 32 sums of a lane's row in the 32 columns at `col` of the warp's block: from TMEM, or, for a
+// split tile, the ranges' sums added in order.
+struct Source {
+  uint32_t acc;         // TMEM address of the block's first column
+  const float* part;    // null: TMEM
+  int splits;
+};
+constexpr size_t kItemFloats = (size_t)kTile * kTile;
+
+__device__ __forceinline__ void fetch32(const Source& src, int cb, float (&v)[32]) {
+  if (src.part == nullptr) {
+    tmem_ld32(src.acc + (uint32_t)(cb * 32), v);
+    return;
+  }
+#pragma unroll
+  for (int c = 0; c < 32; ++c) v[c] = 0.f;
+  for (int sp = 0; sp < src.splits; sp += 2) {  // two ranges in flight at a time
+    const float* p = src.part + (size_t)sp * kItemFloats + cb * 1024;
+    const bool two = sp + 1 < src.splits;
+    float u[32], w[32];
+#pragma unroll
+    for (int c = 0; c < 32; ++c) {
+      u[c] = __ldcg(p + c * 32);
+      w[c] = two ? __ldcg(p + kItemFloats + c * 32) : 0.f;
+    }
+#pragma unroll
+    for (int c = 0; c < 32; ++c) v[c] = (v[c] + u[c]) + w[c];
+  }
+}
+
+// h = g * u of 32 columns as three bf16 terms (24 bits of h), zero where g is.
+__device__ __forceinline__ void mul_hp(const uint4* g4, const float (&v)[32], uint32_t (&w0)[16],
+                                       uint32_t (&w1)[16], uint32_t (&w2)[16]) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const uint32_t g[4] = {g4[j].x, g4[j].y, g4[j].z, g4[j].w};
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+      const int c = 8 * j + 2 * p, o = 4 * j + p;
+      const float g0 = lo_f(g[p]), g1 = hi_f(g[p]);
+      float h0 = g0 != 0.f ? g0 * v[c] : 0.f, h1 = g1 != 0.f ? g1 * v[c + 1] : 0.f;
+      w0[o] = pack2(h0, h1);
+      h0 -= lo_f(w0[o]);
+      h1 -= hi_f(w0[o]);
+      w1[o] = pack2(h0, h1);
+      h0 -= lo_f(w1[o]);
+      h1 -= hi_f(w1[o]);
+      w2[o] = pack2(h0, h1);
+    }
+  }
+}
+
+template <int EPI, bool A_MN, bool B_MN, int STAGES>
+__global__ void __launch_bounds__(kThreads, 1)
+pair_gemm_kernel(const __grid_constant__ CUtensorMap map_a0,
+                 const __grid_constant__ CUtensorMap map_a1,
+                 const __grid_constant__ CUtensorMap map_b0,
+                 const __grid_constant__ CUtensorMap map_b1, const __grid_constant__ Args a) {
+  constexpr uint32_t kIdesc = umma_idesc(256, 256) | (A_MN ? 1u << 15 : 0u) | (B_MN ? 1u << 16 : 0u);
+  constexpr bool kGate2 = EPI == kGateUp || EPI == kGateUpHp;
+  constexpr bool kIsPack = EPI == kPack || EPI == kPackDense || kGate2;
+  constexpr int kPhases = kGate2 ? 2 : 1;  // accumulators per item
+
+  // Without a device-side choice or row count the set-up below runs while the predecessor drains.
+  const bool early_wait = a.run_if.entries != nullptr || a.rows_ptr != nullptr;
+  if (early_wait) pdl_wait();
+  if (a.run_if.entries != nullptr && *a.run_if.entries <= a.run_if.limit) return;
+  const int rows = a.rows_ptr != nullptr ? *a.rows_ptr : a.rows;
+  const int m_tiles = (rows + kTile - 1) / kTile;
+  const int tiles = m_tiles * a.n_tiles;
+  const int total = a.splits > 1 ? a.full_tiles + (tiles - a.full_tiles) * a.splits : tiles;
+  const int pair = (int)blockIdx.x >> 1, pairs = (int)gridDim.x >> 1;
+  if (pair >= total) return;  // the same for both CTAs: nothing allocated, no barrier used yet
+
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>(
+      (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  __shared__ __align__(8) uint64_t full_bar[STAGES], empty_bar[STAGES], tfull_bar[2], tempty_bar[2];
+  __shared__ uint32_t tmem_slot;
+  __shared__ volatile int abort_s;
+  __shared__ int half_count[kIsPack ? 2 : 1][kIsPack ? 128 : 1];
+  __shared__ volatile int last_s[4];
+
+  cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  const int crank = (int)blockIdx.x & 1;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(&full_bar[s], 1);
+      mbar_init(&empty_bar[s], 1);
+    }
+#pragma unroll
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&tfull_bar[b], 1);
+      mbar_init(&tempty_bar[b], 16);
+    }
+    abort_s = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a0) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_b0) : "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;"
+                 ::"r"(smem_u32(&tmem_slot)), "r"(512)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  cluster.sync();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem_base = tmem_slot;
+  if (!early_wait) pdl_wait();
+
+  if (warp == 0) {
+    // ---- TMA producer ----
+    if (lane == 0) {
+      uint32_t it = 0;
+      for (int t = pair; t < total && !abort_s; t += pairs) {
+        const Item im = item_of(t, a);
+        int mt, nt;
+        tile_of(im.tile, m_tiles, a, mt, nt);
+        const bool second = mt >= a.second_mt;
+        const CUtensorMap* ma = second ? &map_a1 : &map_a0;
+        const int ra = (second ? mt - a.second_mt : mt) * kTile + crank * 128;
+        const int rb = nt * kTile + crank * 128;
+#pragma unroll 1
+        for (int ph = 0; ph < kPhases && !abort_s; ++ph) {
+          int kb = im.k0 % a.seg_ksteps;
+          const CUtensorMap* mb =
+              ph == 1 || second || im.k0 >= a.seg_ksteps ? &map_b1 : &map_b0;
+          for (int k = im.k0; k < im.k1; ++k, ++it) {
+            if (kb == a.seg_ksteps) {
+              kb = 0;
+              mb = &map_b1;
+            }
+            const int s = (int)(it % STAGES);
+            if (!mbar_wait(&empty_bar[s], ((it / STAGES) & 1u) ^ 1u)) {
+              abort_s = 1;
+              atomicExch(&g_error, 1);
+              break;
+            }
+            // both CTAs' copies are counted at the leader's barrier (bit 24 of a shared-window
+            // address is the CTA's rank in the pair)
+            const uint32_t bar = smem_u32(&full_bar[s]) & 0xFEFFFFFFu;
+            if (crank == 0) mbar_expect_tx(&full_bar[s], 2 * kStageBytes);
+            const uint32_t st = smem_u32(smem + (size_t)s * kStageBytes);
+            if (A_MN) {
+              tma_load(st, ma, ra, k * kStageK, bar);
+              tma_load(st + 8192, ma, ra + 64, k * kStageK, bar);
+            } else {
+              tma_load(st, ma, k * kStageK, ra, bar);
+            }
+            if (B_MN) {
+              tma_load(st + kOperandBytes, mb, rb, kb * kStageK, bar);
+              tma_load(st + kOperandBytes + 8192, mb, rb + 64, kb * kStageK, bar);
+            } else {
+              tma_load(st + kOperandBytes, mb, kb * kStageK, rb, bar);
+            }
+            ++kb;
+          }
+        }
+      }
+      // the commits of the last stages must have arrived before this CTA may leave
+      for (uint32_t i = 0; i < (uint32_t)STAGES && !abort_s; ++i, ++it) {
+        if (!mbar_wait(&empty_bar[it % STAGES], ((it / STAGES) & 1u) ^ 1u)) {
+          abort_s = 1;
+          atomicExch(&g_error, 5);
+        }
+      }
+    }
+  } else if (warp == 1) {
+    // ---- MMA issuer ----
+    if (lane == 0 && crank == 0) {
+      uint32_t it = 0;
+      int i = 0;
+      for (int t = pair; t < total && !abort_s; t += pairs) {
+        const Item im = item_of(t, a);
+#pragma unroll 1
+        for (int ph = 0; ph < kPhases; ++ph, ++i) {
+          const int b = i & 1;
+          if (!mbar_wait(&tempty_bar[b], ((uint32_t)(i >> 1) & 1u) ^ 1u)) {
+            abort_s = 1;
+            atomicExch(&g_error, 4);
+            break;
+          }
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t acc = tmem_base + (uint32_t)(b * 256);
+          for (int k = im.k0; k < im.k1; ++k, ++it) {
+            const int s = (int)(it % STAGES);
+            if (!mbar_wait(&full_bar[s], (it / STAGES) & 1u)) {
+              abort_s = 1;
+              atomicExch(&g_error, 2);
+              break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t sa = smem_u32(smem + (size_t)s * kStageBytes);
+            const uint64_t da = A_MN ? desc_mn(sa) : umma_desc(sa);
+            const uint64_t db = B_MN ? desc_mn(sa + kOperandBytes) : umma_desc(sa + kOperandBytes);
+#pragma unroll
+            for (int kk = 0; kk < kStageK / 16; ++kk)
+              mma(acc, da + (A_MN ? 128 : 2) * kk, db + (B_MN ? 128 : 2) * kk, kIdesc,
+                  (k > im.k0 || kk > 0) ? 1u : 0u);
+            commit(&empty_bar[s]);
+          }
+          if (abort_s) break;
+          commit(&tfull_bar[b]);
+        }
+      }
+    }
+  } else {
+    // ---- epilogue: warp = (lane quarter, column half) ----
+    const int q = warp & 3, half = (warp - 2) >> 2;
+    unsigned char* buf = smem + (size_t)STAGES * kStageBytes + (size_t)(warp - 2) * 32 * 256;
+    const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(half * 128);
+    float shift = 0.f;
+    if (EPI == kBwd && a.l1_grad != nullptr) shift = __ldg(a.l1_grad) * a.inv_m;
+    int i = 0;  // accumulators taken so far
+    auto take = [&]() -> bool {  // waits for accumulator i
+      bool ok = mbar_wait(&tfull_bar[i & 1], (uint32_t)(i >> 1) & 1u);
+      ok = __all_sync(0xffffffffu, ok);
+      // the two warps of a pack's rows meet at barriers: they go on or give up together
+      if (kIsPack) ok = named_barrier_and(1 + q, 64, ok);
+      if (!ok) {
+        abort_s = 1;
+        atomicExch(&g_error, 3);
+        return false;
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      return true;
+    };
+    auto release = [&]() {  // this warp has read accumulator i
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) arrive_leader(&tempty_bar[i & 1]);
+      ++i;
+    };
+    int parity = 0;
+    for (int t = pair; t < total; t += pairs) {
+      const Item im = item_of(t, a);
+      int mt, nt;
+      tile_of(im.tile, m_tiles, a, mt, nt);
+      const int row0 = mt * kTile + crank * 128 + q * 32;
+      const int row = row0 + lane;
+      const bool live = row < rows;
+      __nv_bfloat16* out = a.out + (size_t)row * a.ld + nt * kTile + half * 128;
+      auto load_pattern = [&]() {
+        if (EPI == kMul || EPI == kMulHp || EPI == kFwd)
+          load_values(a, buf, row0, rows, nt, half, lane);
+        if (EPI == kBwd) load_pairs(a, buf, row0, rows, nt, 2 * half, lane);
+      };
+      // the pattern is fetched under the MMAs of this tile (a split tile's only by the warp that
+      // finishes it)
+      if (im.split_tile < 0) load_pattern();
+      if (!take()) break;
+      Source src = {lane_addr + (uint32_t)((i & 1) * 256), nullptr, a.splits};
+
+      if (EPI == kStore && a.sums != nullptr) {
+        float* dst = a.sums + ((size_t)im.split * rows + row) * a.n_tiles * kTile + nt * kTile + half * 128;
+#pragma unroll 1
+        for (int cb = 0; cb < 4 && row0 < rows; ++cb) {
+          float v[32];
+          tmem_ld32(src.acc + (uint32_t)(cb * 32), v);
+          if (!live) continue;
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            uint32_t w[16];
+#pragma unroll
+            for (int p = 0; p < 16; ++p) w[p] = __float_as_uint(v[16 * c + p]);
+            store64(reinterpret_cast<__nv_bfloat16*>(dst + cb * 32 + c * 16), w, 1);
+          }
+        }
+        release();
+        continue;
+      }
+      if (!kGate2 && im.split_tile >= 0) {
+        const size_t blk = ((size_t)crank * 8 + q * 2 + half) * (128 * 32) + lane;
+        float* mine = a.part + (size_t)(im.split_tile * a.splits + im.split) * kItemFloats + blk;
+#pragma unroll 1
+        for (int cb = 0; cb < 4 && row0 < rows; ++cb) {
+          float v[32];
+          tmem_ld32(src.acc + (uint32_t)(cb * 32), v);
+#pragma unroll
+          for (int c = 0; c < 32; ++c) __stcg(mine + cb * 1024 + c * 32, v[c]);
+        }
+        __threadfence();
+        release();
+        unsigned int* ctr = a.counters + (im.split_tile * 2 + crank) * 8 + q * 2 + half;
+        bool last;
+        if (kIsPack) {  // both halves of a row decide together: the slots of the second half follow
+          named_barrier(1 + q, 64);
+          if (half == 0 && lane == 0) {
+            const unsigned int old = atomicAdd(ctr, 1u);
+            if (old == (unsigned int)a.splits - 1u) *ctr = 0u;
+            last_s[q] = old == (unsigned int)a.splits - 1u;
+          }
+          named_barrier(1 + q, 64);
+          last = last_s[q] != 0;
+        } else {
+          unsigned int old = 0;
+          if (lane == 0) {
+            old = atomicAdd(ctr, 1u);
+            if (old == (unsigned int)a.splits - 1u) *ctr = 0u;
+          }
+          last = __shfl_sync(0xffffffffu, old, 0) == (unsigned int)a.splits - 1u;
+        }
+        if (!last) continue;
+        __threadfence();
+        src.part = a.part + (size_t)im.split_tile * a.splits * kItemFloats + blk;
+        load_pattern();
+      }
+
+      if (kIsPack) {
+        // pass 1: positives of each 32-column block as a mask, bf16 values into the buffer
+        uint32_t mask[4];
+        int cnt = 0;
+#pragma unroll
+        for (int cb = 0; cb < 4; ++cb) {
+          float v[32];
+          fetch32(src, cb, v);
+          if (a.bias != nullptr) {
+            const float* bp = a.bias + nt * kTile + half * 128 + cb * 32;
+            if (a.bias16) {
+#pragma unroll
+              for (int c = 0; c < 8; ++c) {
+                const float4 bv = __ldg(reinterpret_cast<const float4*>(bp) + c);
+                v[4 * c] += bv.x;
+                v[4 * c + 1] += bv.y;
+                v[4 * c + 2] += bv.z;
+                v[4 * c + 3] += bv.w;
+              }
+            } else {
+#pragma unroll
+              for (int c = 0; c < 32; ++c) v[c] += __ldg(bp + c);
+            }
+          }
+          uint32_t m = 0;
+#pragma unroll
+          for (int c = 0; c < 32; ++c) m |= v[c] > 0.f ? 1u << c : 0u;
+          mask[cb] = live ? m : 0u;
+          cnt += __popc(mask[cb]);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            uint32_t w[4];
+#pragma unroll
+            for (int p = 0; p < 4; ++p)
+              w[p] = pack2(fmaxf(v[8 * j + 2 * p], 0.f), fmaxf(v[8 * j + 2 * p + 1], 0.f));
+            *reinterpret_cast<uint4*>(at(buf, lane, cb * 64 + j * 16)) =
+                make_uint4(w[0], w[1], w[2], w[3]);
+          }
+        }
+        if (src.part == nullptr) release();
+        // the second half's slots follow the first half's
+        int slot = 0;
+        if (half == 0) half_count[parity][q * 32 + lane] = cnt;
+        named_barrier(1 + q, 64);
+        if (half == 1) slot = half_count[parity][q * 32 + lane];
+        parity ^= 1;
+        const int cap = a.slab_w - 1;
+        uint32_t* slab = a.slab_p + (size_t)row * a.row_words + (size_t)nt * a.slab_w;
+        if (half == 1 && live) slab[0] = (uint32_t)(slot + cnt);
+        if (a.entries != nullptr) {
+          const int kept = max(min(slot + cnt, cap) - slot, 0);
+          const int sum = __reduce_add_sync(0xffffffffu, kept);
+          if (lane == 0 && sum > 0) atomicAdd(a.entries, (unsigned int)sum);
+        }
+        // pass 2: entries; a value past the slab's capacity leaves the buffer too (unless keep_all)
+#pragma unroll
+        for (int cb = 0; cb < 4; ++cb) {
+          uint32_t m = mask[cb];
+          const uint32_t col0 = (uint32_t)(nt * kTile + half * 128 + cb * 32);
+          while (m != 0u) {
+            const int c = __ffs(m) - 1;
+            m &= m - 1;
+            uint16_t* p = reinterpret_cast<uint16_t*>(at(buf, lane, cb * 64 + c * 2));
+            if (slot < cap) slab[1 + slot] = (col0 + c) | ((uint32_t)*p << 16);
+            else if (EPI != kPack && !a.keep_all) *p = 0;
+            ++slot;
+          }
+        }
+        __syncwarp();
+        if (EPI == kPackDense) {  // what the slab stores, as a dense row
+#pragma unroll
+          for (int cb = 0; cb < 4; ++cb) {
+            uint32_t w[16];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const uint4 g4 = *reinterpret_cast<const uint4*>(at(buf, lane, cb * 64 + j * 16));
+              w[4 * j] = g4.x;
+              w[4 * j + 1] = g4.y;
+              w[4 * j + 2] = g4.z;
+              w[4 * j + 3] = g4.w;
+            }
+            if (live) store64(out + cb * 32, w, a.wide);
+          }
+        }
+        if (!kGate2) continue;
+        if (!take()) break;  // the up product of the same tile
+        src = Source{lane_addr + (uint32_t)((i & 1) * 256), nullptr, 1};
+      }
+
+      if (!kIsPack || kGate2) {
+        float l1 = 0.f;
+#pragma unroll 1
+        for (int cb = 0; cb < 4; ++cb) {
+          if (EPI == kBwd && cb == 2) load_pairs(a, buf, row0, rows, nt, 2 * half + 1, lane);
+          float v[32];
+          fetch32(src, cb, v);
+          if (EPI == kStore) {
+            uint32_t w[16];
+#pragma unroll
+            for (int p = 0; p < 16; ++p) w[p] = pack2(v[2 * p], v[2 * p + 1]);
+            if (live) store64(out + cb * 32, w, a.wide);
+          } else if (EPI == kMul || EPI == kGateUp || EPI == kFwd) {
+            uint32_t w[16];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              uint4* gp = reinterpret_cast<uint4*>(at(buf, lane, cb * 64 + j * 16));
+              const uint4 g4 = *gp;
+              const uint32_t g[4] = {g4.x, g4.y, g4.z, g4.w};
+              uint32_t r[4];
+#pragma unroll
+              for (int p = 0; p < 4; ++p) {
+                const int c = 8 * j + 2 * p;
+                const uint32_t m = nonzero2(g[p]);
+                r[p] = pack2(v[c], v[c + 1]) & m;      // never touch u where nothing is stored
+                w[4 * j + p] = mul2(g[p], r[p]) & m;
+                if (EPI == kFwd) {
+                  l1 += fabsf(lo_f(w[4 * j + p]));
+                  l1 += fabsf(hi_f(w[4 * j + p]));
+                }
+              }
+              if (EPI == kFwd) *gp = make_uint4(r[0], r[1], r[2], r[3]);
+            }
+            if (live) store64(out + cb * 32, w, a.wide);
+          } else if (EPI == kMulHp || EPI == kGateUpHp) {
+            uint4 g4[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              g4[j] = *reinterpret_cast<const uint4*>(at(buf, lane, cb * 64 + j * 16));
+            uint32_t w0[16], w1[16], w2[16];
+            mul_hp(g4, v, w0, w1, w2);
+            if (live) {
+              const size_t h = (size_t)a.n_tiles * kTile;
+              store64(out + cb * 32, w0, a.wide);
+              store64(out + h + cb * 32, w1, a.wide);
+              store64(out + 2 * h + cb * 32, w2, a.wide);
+            }
+          } else if (EPI == kBwd) {
+            uint32_t dr[16], du[16], tt[16];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              const uint4 g4 =
+                  *reinterpret_cast<const uint4*>(at(buf, lane, (cb & 1) * 128 + j * 16));
+#pragma unroll
+              for (int p = 0; p < 2; ++p) {
+                const uint32_t x0 = p == 0 ? g4.x : g4.z, x1 = p == 0 ? g4.y : g4.w;
+                const int c = 4 * j + 2 * p, o = 2 * j + p;
+                const uint32_t p2 = __byte_perm(x0, x1, 0x5410), r2 = __byte_perm(x0, x1, 0x7632);
+                const uint32_t m = nonzero2(p2);
+                uint32_t dt = pack2(v[c], v[c + 1]);
+                if (shift != 0.f) {
+                  const float r0 = lo_f(r2), r1 = hi_f(r2);
+                  const float s0 = r0 > 0.f ? shift : (r0 < 0.f ? -shift : 0.f);
+                  const float s1 = r1 > 0.f ? shift : (r1 < 0.f ? -shift : 0.f);
+                  dt = pack2(lo_f(dt) + s0, hi_f(dt) + s1);
+                }
+                dt &= m;
+                dr[o] = mul2(dt, p2) & m;
+                du[o] = mul2(dt, r2) & m;
+                tt[o] = mul2(r2, p2) & m;
+              }
+            }
+            if (live) {
+              store64(out + cb * 32, dr, a.wide);
+              store64(out + (size_t)a.n_tiles * kTile + cb * 32, du, a.wide);
+              store64(a.dense_t + (size_t)row * a.ld_t + nt * kTile + half * 128 + cb * 32, tt, a.wide);
+            }
+          }
+        }
+        if (EPI == kFwd && live) a.l1_part[(size_t)(nt * 2 + half) * rows + row] = l1;
+        if (src.part == nullptr) release();
+        __syncwarp();
+      }
+      if (EPI == kFwd) {
+        // R and T in the slots of P, from the R values left in the pattern buffer
+        const size_t tile_off = (size_t)nt * a.slab_w;
+        for (int tk = 0; tk < 32; ++tk) {
+          const int r = row0 + tk;
+          if (r >= rows) break;
+          int cnt = 0;
+          for (int w0 = 0; w0 < a.slab_w; w0 += 32) {
+            const size_t off = (size_t)r * a.row_words + tile_off + w0 + lane;
+            const uint32_t w = a.slab_p[off];
+            if (w0 == 0) {
+              cnt = min(max((int)__shfl_sync(0xffffffffu, w, 0), 0), a.slab_w - 1);
+              if (lane == 0 && half == 0) {
+                a.slab_r[off] = w;
+                a.slab_t[off] = w;
+              }
+            }
+            const int slot = w0 + lane, col = (int)(w & 255u);
+            if (slot >= 1 && slot <= cnt && (col >> 7) == half) {
+              const uint32_t rb = *reinterpret_cast<const uint16_t*>(at(buf, tk, (col & 127) * 2));
+              a.slab_r[off] = (w & 0xFFFFu) | (rb << 16);
+              a.slab_t[off] = (w & 0xFFFFu) | (mul2(rb, w >> 16) << 16);
+            }
+            if (cnt < w0 + 32) break;
+          }
+        }
+        __syncwarp();
+      }
+    }
+  }
+
+  __syncwarp();
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  cluster.sync();
+  if (warp == 1) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512)
+                 : "memory");
+  }
+}
+
+// ---- host side -------------------------------------------------------------
+struct Operand {
+  const void* base;
+  int64_t rows, k;   // logical: rows x k; stored [rows][k] (K-major) or [k][rows] (mn)
+};
+
+inline int operand_map(CUtensorMap* map, const Operand& o, bool mn) {
+  // box of 64 contiguous elements (128 bytes); a pair CTA holds 128 rows: one K-major box of
+  // 128 rows, or two MN-major boxes of 64 rows x 64 k
+  return mn ? make_map(map, o.base, o.k, o.rows, 64) : make_map(map, o.base, o.rows, o.k, 128);
+}
+
+// out = bf16 of the sum over the ranges of k, in their order.
+__global__ void __launch_bounds__(256)
+sum_ranges_kernel(const float4* __restrict__ sums, uint2* __restrict__ out, int splits, size_t n4,
+                  const RunIf run_if) {
+  pdl_wait();
+  if (run_if.entries != nullptr && *run_if.entries <= run_if.limit) return;
+  const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
+  if (i >= n4) return;
+  float4 v[8];
+#pragma unroll
+  for (int s = 0; s < 8; ++s)
+    if (s < splits) v[s] = __ldcg(sums + (size_t)s * n4 + i);
+  float4 t = v[0];
+#pragma unroll
+  for (int s = 1; s < 8; ++s)
+    if (s < splits) {
+      t.x += v[s].x;
+      t.y += v[s].y;
+      t.z += v[s].z;
+      t.w += v[s].w;
+    }
+  out[i] = make_uint2(pack2(t.x, t.y), pack2(t.z, t.w));
+}
+
+// How the tiles of the last wave are cut along k: as many equal ranges as still fit the wave, at
+// least 4 k-steps each.  A product of less than one wave whose sums go to memory (`all`) takes up
+// to 8 ranges, added by a kernel of their own on all SMs; the last wave of a larger one up to 4,
+// added by the warps that arrive last.
+struct Split {
+  int64_t full_tiles;
+  int splits;
+};
+inline Split choose_split(int64_t tiles, int ksteps, int64_t slots, bool all) {
+  const int64_t tail = tiles % slots;
+  if (tail == 0) return {tiles, 1};
+  int64_t s = slots / tail;
+  if (s > ksteps / 4) s = ksteps / 4;
+  if (s > (all && tiles < slots ? 8 : 4)) s = all && tiles < slots ? 8 : 4;
+  if (s < 2) return {tiles, 1};
+  return {tiles - tail, (int)s};
+}
+inline size_t part_bytes(int64_t tiles, int ksteps, int64_t slots, bool all) {
+  const Split s = choose_split(tiles, ksteps, slots, all);
+  return s.splits < 2 ? 0 : (size_t)(tiles - s.full_tiles) * s.splits * kTile * kTile * sizeof(float);
+}
+
+template <int EPI, bool A_MN, bool B_MN>
+int launch(const char* fn, const Operand& a0, const Operand& a1, const Operand& b0,
+           const Operand& b1, Args args, int64_t row_capacity, int sm_count, cudaStream_t stream) {
+  constexpr bool kBuf = EPI != kStore;
+  constexpr int STAGES = kBuf ? 5 : 6;
+  constexpr size_t smem = (size_t)STAGES * kStageBytes + (kBuf ? kBufBytes : 0) + 1024;
+  CUtensorMap ma0, ma1, mb0, mb1;
+  if (int rc = operand_map(&ma0, a0, A_MN)) return rc;
+  if (int rc = operand_map(&ma1, a1, A_MN)) return rc;
+  if (int rc = operand_map(&mb0, b0, B_MN)) return rc;
+  if (int rc = operand_map(&mb1, b1, B_MN)) return rc;
+  auto kern = pair_gemm_kernel<EPI, A_MN, B_MN, STAGES>;
+  static size_t granted[64] = {0};
+  if (int rc = ensure_dynamic_smem(kern, smem, granted, fn)) return rc;
+  const int64_t tiles = (row_capacity + kTile - 1) / kTile * args.n_tiles;
+  const int64_t slots = sm_count / 2;
+  const Split sp = EPI != kGateUp && EPI != kGateUpHp && args.part != nullptr && args.counters != nullptr && args.rows_ptr == nullptr
+                       ? choose_split(tiles, args.ksteps, slots, EPI == kStore)
+                       : Split{tiles, 1};
+  args.full_tiles = (int)sp.full_tiles;
+  args.splits = sp.splits;
+  const bool sum_after = EPI == kStore && sp.splits > 1 && sp.full_tiles == 0 &&
+                         args.ld == (long long)args.n_tiles * kTile;
+  args.sums = sum_after ? args.part : nullptr;
+  const int64_t items = sp.full_tiles + (tiles - sp.full_tiles) * sp.splits;
+  const int64_t pairs = items < slots ? items : slots;
+  args.group = args.n_tiles >= 10 ? 8 : (int)((slots + args.n_tiles - 1) / args.n_tiles);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(2 * pairs), 1, 1);
+  cfg.blockDim = dim3(kThreads, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = add_pdl_attribute(attr, 1);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, ma0, ma1, mb0, mb1, args);
+  if (e != cudaSuccess) return fail(B200_ECUDA, "%s: launch: %s", fn, cudaGetErrorString(e));
+  if (sum_after) {
+    const size_t n4 = (size_t)args.rows * args.n_tiles * kTile / 4;
+    cudaLaunchConfig_t sum = {};
+    sum.gridDim = dim3((unsigned)((n4 + 255) / 256), 1, 1);
+    sum.blockDim = dim3(256, 1, 1);
+    sum.stream = stream;
+    cudaLaunchAttribute sattr[1];
+    sum.attrs = sattr;
+    sum.numAttrs = add_pdl_attribute(sattr, 0);
+    e = cudaLaunchKernelEx(&sum, sum_ranges_kernel, reinterpret_cast<const float4*>(args.sums),
+                           reinterpret_cast<uint2*>(args.out), args.splits, n4, args.run_if);
+    if (e != cudaSuccess) return fail(B200_ECUDA, "%s: launch: %s", fn, cudaGetErrorString(e));
+  }
+  return B200_OK;
+}
+
+}  // namespace pg
+}  // namespace
+}  // namespace b200

@@ -1,12 +1,10 @@
 // Gate projection + ReLU + TwELL pack on the 5th-generation tensor cores.
 //
-// Kernels of this file, by token count: twell_pack_tc_splitk_(wide_)kernel (17..32 tokens, D
-// split over a cluster), twell_pack_tc_splitk_mid_kernel (33..256, 128-token tiles, D split),
-// twell_pack_tc_wide_kernel (256-token tiles, one CTA per SM, sixteen epilogue warps: the
-// default above that) and twell_pack_tc_kernel, described first (64- / 128-token tiles, four
-// epilogue warps).
+// Kernels of this file, by token count: twell_pack_tc_splitk_(wide_)kernel (17..32 tokens) and
+// twell_pack_tc_splitk_mid_kernel (33..128, 128-token tiles), both with D split over a cluster.
+// Larger calls run on pairs of SMs (pair_gemm.cuh).
 //
-// CTA tile: one 256-neuron TwELL tile x NTOK tokens (64 or 128) x all of D.
+// CTA tile: one 256-neuron TwELL tile x NTOK tokens x a slice of D.
 // Neurons ride the MMA M axis as two 128-row accumulators, tokens the N axis:
 //   D0[128, NTOK] = W[tile*256      .. +128, :] . X[tok0 .. +NTOK, :]^T
 //   D1[128, NTOK] = W[tile*256 + 128 .. +128, :] . X[tok0 .. +NTOK, :]^T
@@ -14,7 +12,7 @@
 // TMA (cp.async.bulk.tensor, 128-byte swizzle, no multicast) into a ring of shared
 // memory stages; one elected thread issues tcgen05.mma (kind::f16, fp32 accumulate
 // in TMEM); tcgen05.commit releases a stage back to the producer and, after the
-// last k step, hands the accumulators to four epilogue warps.
+// last k step, hands the accumulators to the epilogue warps.
 //
 // In TMEM a lane is a neuron and a column is a token, so after tcgen05.ld the 32
 // lanes of an epilogue warp hold 32 consecutive neurons of one token per register:
@@ -38,175 +36,15 @@
 namespace cg = cooperative_groups;
 
 namespace b200 {
+
+int pair_gemm_status();
+
 namespace {
 
 __device__ int g_tc_error = 0;
 
-// grid = (H / 256, ceil(M / NTOK)).  Dynamic shared memory: STAGES x (A0 | A1 | B), 1024-aligned.
-template <int NTOK, int STAGES, int MINB>
-__global__ void __launch_bounds__(kThreadsTc, MINB)
-twell_pack_tc_kernel(const __grid_constant__ CUtensorMap tmap_w,
-                     const __grid_constant__ CUtensorMap tmap_x, const float* __restrict__ bias,
-                     uint32_t* __restrict__ packed, int M, int D, int slab_w, int row_words,
-                     int group) {
-  constexpr int kBTileBytes = NTOK * 128;
-  constexpr int kStageBytes = 2 * kATileBytes + kBTileBytes;
-  constexpr uint32_t kTmemCols = 2 * NTOK;  // 128 or 256: a power of two >= 32
-  constexpr uint32_t kIdesc = umma_idesc(128, NTOK);
-
-  extern __shared__ __align__(1024) unsigned char smem_raw[];
-  unsigned char* smem = reinterpret_cast<unsigned char*>(
-      (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  __shared__ __align__(8) uint64_t full_bar[STAGES], empty_bar[STAGES], acc_bar;
-  __shared__ uint32_t tmem_slot;
-  __shared__ volatile int abort_s;
-  __shared__ uint32_t masks_s[32][8];
-  __shared__ int prefix_s[32][8];
-
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  int tile, mblk;
-  raster_remap(group, tile, mblk);
-  const int m0 = mblk * NTOK;
-  const int ksteps = D / kStageK;
-
-  if (threadIdx.x == 0) {
-#pragma unroll
-    for (int s = 0; s < STAGES; ++s) {
-      mbar_init(&full_bar[s], 1);
-      mbar_init(&empty_bar[s], 1);
-    }
-    mbar_init(&acc_bar, 1);
-    abort_s = 0;
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-                 ::"r"(smem_u32(&tmem_slot)), "r"(kTmemCols)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem_base = tmem_slot;
-
-  if (warp == 0) {
-    // ---- TMA producer ----
-    if (lane == 0) {
-      for (int k = 0; k < ksteps && !abort_s; ++k) {
-        const int s = k % STAGES;
-        const uint32_t phase = (uint32_t)(k / STAGES) & 1u;
-        if (!mbar_wait(&empty_bar[s], phase ^ 1u)) {
-          abort_s = 1;
-          atomicExch(&g_tc_error, 1);
-          break;
-        }
-        unsigned char* st = smem + (size_t)s * kStageBytes;
-        mbar_expect_tx(&full_bar[s], (uint32_t)kStageBytes);
-        tma_load_2d(st, &tmap_w, k * kStageK, tile * kTileN, &full_bar[s]);
-        tma_load_2d(st + kATileBytes, &tmap_w, k * kStageK, tile * kTileN + 128, &full_bar[s]);
-        tma_load_2d(st + 2 * kATileBytes, &tmap_x, k * kStageK, m0, &full_bar[s]);
-      }
-    }
-  } else if (warp == 1) {
-    // ---- MMA issuer ----
-    if (lane == 0) {
-      for (int k = 0; k < ksteps && !abort_s; ++k) {
-        const int s = k % STAGES;
-        const uint32_t phase = (uint32_t)(k / STAGES) & 1u;
-        if (!mbar_wait(&full_bar[s], phase)) {
-          abort_s = 1;
-          atomicExch(&g_tc_error, 2);
-          break;
-        }
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t a0 = smem_u32(smem + (size_t)s * kStageBytes);
-        const uint64_t da0 = umma_desc(a0), da1 = umma_desc(a0 + kATileBytes),
-                       db = umma_desc(a0 + 2 * kATileBytes);
-#pragma unroll
-        for (int kk = 0; kk < kStageK / 16; ++kk) {
-          const uint32_t acc = (k > 0 || kk > 0) ? 1u : 0u;
-          // +32 bytes per 16 k-values inside the 128-byte swizzled row (encoded >> 4)
-          umma_bf16(tmem_base, da0 + 2 * kk, db + 2 * kk, kIdesc, acc);
-          umma_bf16(tmem_base + NTOK, da1 + 2 * kk, db + 2 * kk, kIdesc, acc);
-        }
-        umma_commit(&empty_bar[s]);  // stage reusable once these MMAs have read it
-      }
-      if (!abort_s) umma_commit(&acc_bar);  // accumulators complete
-    }
-  } else {
-    // ---- epilogue: warps 2..5 own TMEM lane quarters 2, 3, 0, 1 ----
-    const int q = warp & 3;
-    const int et = threadIdx.x - 64;  // 0..127
-    bool ok = mbar_wait(&acc_bar, 0u);
-    if (!ok) {
-      abort_s = 1;
-      atomicExch(&g_tc_error, 3);
-    }
-    ok = epi_barrier_and(ok);  // the same decision in all 128 epilogue threads
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const int n_lo = tile * kTileN + q * 32 + lane;  // neuron of accumulator 0; +128 for 1
-    const float b_lo = bias != nullptr ? bias[n_lo] : 0.f;
-    const float b_hi = bias != nullptr ? bias[n_lo + 128] : 0.f;
-    const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16);
-    for (int tb = 0; tb < NTOK / 32 && ok; ++tb) {
-      float v0[32], v1[32];
-      tmem_ld32(lane_addr + (uint32_t)(tb * 32), v0);
-      tmem_ld32(lane_addr + (uint32_t)(NTOK + tb * 32), v1);
-#pragma unroll
-      for (int c = 0; c < 32; ++c) {
-        const bool valid = m0 + tb * 32 + c < M;
-        v0[c] += b_lo;
-        v1[c] += b_hi;
-        const uint32_t k0 = __ballot_sync(0xffffffffu, valid && v0[c] > 0.f);
-        const uint32_t k1 = __ballot_sync(0xffffffffu, valid && v1[c] > 0.f);
-        if (lane == 0) {
-          masks_s[c][q] = k0;
-          masks_s[c][4 + q] = k1;
-        }
-      }
-      epi_barrier();
-      if (et < 32) {
-        const int tok = m0 + tb * 32 + et;
-        int run = 0;
-#pragma unroll
-        for (int ch = 0; ch < 8; ++ch) {
-          prefix_s[et][ch] = run;
-          run += __popc(masks_s[et][ch]);
-        }
-        if (tok < M) packed[(size_t)tok * row_words + (size_t)tile * slab_w] = (uint32_t)run;
-      }
-      epi_barrier();
-#pragma unroll
-      for (int c = 0; c < 32; ++c) {
-        const int tok = m0 + tb * 32 + c;
-        uint32_t* slab = packed + (size_t)tok * row_words + (size_t)tile * slab_w;
-        const uint32_t k0 = masks_s[c][q], k1 = masks_s[c][4 + q];
-        if ((k0 >> lane) & 1u) {
-          const int slot = prefix_s[c][q] + __popc(k0 & lanemask_lt());
-          if (slot < slab_w - 1) slab[1 + slot] = (uint32_t)n_lo | (bf16_bits(v0[c]) << 16);
-        }
-        if ((k1 >> lane) & 1u) {
-          const int slot = prefix_s[c][4 + q] + __popc(k1 & lanemask_lt());
-          if (slot < slab_w - 1) slab[1 + slot] = (uint32_t)(n_lo + 128) | (bf16_bits(v1[c]) << 16);
-        }
-      }
-      epi_barrier();  // masks_s / prefix_s are rewritten by the next token block
-    }
-  }
-
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  if (warp == 1) {
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base),
-                 "r"(kTmemCols)
-                 : "memory");
-  }
-}
-
 // ---------------------------------------------------------------------------
-// Decode variant (M <= 32): the same TMA -> tcgen05 pipeline, with the reduction
+// Decode variant (M <= 32): the TMA -> tcgen05 pipeline with the reduction
 // dimension split over a cluster of CL CTAs so that (H/256)*CL CTAs stream W_gate
 // concurrently.  CTA `crank` multiplies all 256 neurons of the tile by its slice of D for
 // up to 32 tokens; the partial accumulators leave TMEM through registers and are pushed
@@ -399,189 +237,6 @@ twell_pack_tc_splitk_kernel(const __grid_constant__ CUtensorMap tmap_w,
     const int slot = cnt_chunk[tl][nl / 32] + __popc(mask[i] & lanemask_lt());
     if (((mask[i] >> lane) & 1u) && slot < slab_w - 1)
       slab[1 + slot] = (uint32_t)(neuron0 + nl) | (bf16_bits(z[i]) << 16);
-  }
-}
-
-// ---------------------------------------------------------------------------
-// Large-M kernel with sixteen epilogue warps: ONE CTA per SM computes 256 neurons x 256 tokens
-// (two 128-lane accumulators of 256 columns = all of TMEM; a stage of 64 k-values is 32 KB of
-// weights + 32 KB of tokens, i.e. 131 flop per staged byte against 87 for the 128-token tile),
-// and the pack epilogue - which four warps need about 2 us per 32-token block for - is spread
-// over four groups of four warps that each take every fourth token block.  The epilogue
-// reads the accumulators twice (signs first, values again when the slots are known) so that a
-// thread holds 32 instead of 64 of them.
-// Threads: warp 0 producer, warp 1 mma, warps 2..17 epilogue (group = (warp - 2) / 4, TMEM
-// lane quarter = warp % 4).  grid = (H / 256, ceil(M / 256)).
-// ---------------------------------------------------------------------------
-constexpr int kThreadsTcWideM = 64 + 512;
-
-template <int STAGES>
-__global__ void __launch_bounds__(kThreadsTcWideM, 1)
-twell_pack_tc_wide_kernel(const __grid_constant__ CUtensorMap tmap_w,
-                          const __grid_constant__ CUtensorMap tmap_x,
-                          const float* __restrict__ bias, uint32_t* __restrict__ packed, int M,
-                          int D, int slab_w, int row_words, int group) {
-  constexpr int NTOK = 256;
-  constexpr int kBTileBytes = NTOK * 128;
-  constexpr int kStageBytes = 2 * kATileBytes + kBTileBytes;
-  constexpr uint32_t kTmemCols = 2 * NTOK;
-  constexpr uint32_t kIdesc = umma_idesc(128, NTOK);
-
-  extern __shared__ __align__(1024) unsigned char smem_raw[];
-  unsigned char* smem = reinterpret_cast<unsigned char*>(
-      (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  __shared__ __align__(8) uint64_t full_bar[STAGES], empty_bar[STAGES], acc_bar;
-  __shared__ uint32_t tmem_slot;
-  __shared__ volatile int abort_s;
-  __shared__ uint32_t masks_s[4][32][8];
-  __shared__ int prefix_s[4][32][8];
-
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  int tile, mblk;
-  raster_remap(group, tile, mblk);
-  const int m0 = mblk * NTOK;
-  const int ksteps = D / kStageK;
-
-  if (threadIdx.x == 0) {
-#pragma unroll
-    for (int s = 0; s < STAGES; ++s) {
-      mbar_init(&full_bar[s], 1);
-      mbar_init(&empty_bar[s], 1);
-    }
-    mbar_init(&acc_bar, 1);
-    abort_s = 0;
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-                 ::"r"(smem_u32(&tmem_slot)), "r"(kTmemCols)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem_base = tmem_slot;
-
-  if (warp == 0) {
-    if (lane == 0) {
-      for (int k = 0; k < ksteps && !abort_s; ++k) {
-        const int s = k % STAGES;
-        const uint32_t phase = (uint32_t)(k / STAGES) & 1u;
-        if (!mbar_wait(&empty_bar[s], phase ^ 1u)) {
-          abort_s = 1;
-          atomicExch(&g_tc_error, 1);
-          break;
-        }
-        unsigned char* st = smem + (size_t)s * kStageBytes;
-        mbar_expect_tx(&full_bar[s], (uint32_t)kStageBytes);
-        tma_load_2d(st, &tmap_w, k * kStageK, tile * kTileN, &full_bar[s]);  // 256 rows: A0 | A1
-        tma_load_2d(st + 2 * kATileBytes, &tmap_x, k * kStageK, m0, &full_bar[s]);
-      }
-    }
-  } else if (warp == 1) {
-    if (lane == 0) {
-      for (int k = 0; k < ksteps && !abort_s; ++k) {
-        const int s = k % STAGES;
-        const uint32_t phase = (uint32_t)(k / STAGES) & 1u;
-        if (!mbar_wait(&full_bar[s], phase)) {
-          abort_s = 1;
-          atomicExch(&g_tc_error, 2);
-          break;
-        }
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t a0 = smem_u32(smem + (size_t)s * kStageBytes);
-        const uint64_t da0 = umma_desc(a0), da1 = umma_desc(a0 + kATileBytes),
-                       db = umma_desc(a0 + 2 * kATileBytes);
-#pragma unroll
-        for (int kk = 0; kk < kStageK / 16; ++kk) {
-          const uint32_t acc = (k > 0 || kk > 0) ? 1u : 0u;
-          umma_bf16(tmem_base, da0 + 2 * kk, db + 2 * kk, kIdesc, acc);
-          umma_bf16(tmem_base + NTOK, da1 + 2 * kk, db + 2 * kk, kIdesc, acc);
-        }
-        umma_commit(&empty_bar[s]);
-      }
-      if (!abort_s) umma_commit(&acc_bar);
-    }
-  } else {
-    const int q = warp & 3;
-    const int grp = (warp - 2) >> 2;              // 0..3
-    const int gt = (int)threadIdx.x - 64 - grp * 128;  // 0..127 inside the group
-    const int bar_id = 2 + grp;
-    bool ok = mbar_wait(&acc_bar, 0u);
-    if (!ok) {
-      abort_s = 1;
-      atomicExch(&g_tc_error, 3);
-    }
-    ok = named_barrier_and(1, 512, ok);  // the same decision in all 512 epilogue threads
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const int n_lo = tile * kTileN + q * 32 + lane;  // neuron of accumulator 0; +128 for 1
-    const float b_lo = bias != nullptr ? bias[n_lo] : 0.f;
-    const float b_hi = bias != nullptr ? bias[n_lo + 128] : 0.f;
-    const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16);
-    uint32_t (*masks)[8] = masks_s[grp];
-    int (*prefix)[8] = prefix_s[grp];
-    for (int tb = grp; tb < NTOK / 32 && ok; tb += 4) {
-      if (m0 + tb * 32 >= M) break;  // the same in every thread of the group
-      float v[32];
-      // signs
-      tmem_ld32(lane_addr + (uint32_t)(tb * 32), v);
-#pragma unroll
-      for (int c = 0; c < 32; ++c) {
-        const uint32_t k = __ballot_sync(0xffffffffu, m0 + tb * 32 + c < M && v[c] + b_lo > 0.f);
-        if (lane == 0) masks[c][q] = k;
-      }
-      tmem_ld32(lane_addr + (uint32_t)(NTOK + tb * 32), v);
-#pragma unroll
-      for (int c = 0; c < 32; ++c) {
-        const uint32_t k = __ballot_sync(0xffffffffu, m0 + tb * 32 + c < M && v[c] + b_hi > 0.f);
-        if (lane == 0) masks[c][4 + q] = k;
-      }
-      named_barrier(bar_id, 128);
-      if (gt < 32) {
-        const int tok = m0 + tb * 32 + gt;
-        int run = 0;
-#pragma unroll
-        for (int ch = 0; ch < 8; ++ch) {
-          prefix[gt][ch] = run;
-          run += __popc(masks[gt][ch]);
-        }
-        if (tok < M) packed[(size_t)tok * row_words + (size_t)tile * slab_w] = (uint32_t)run;
-      }
-      named_barrier(bar_id, 128);
-      // values (accumulator 1 is still in v; accumulator 0 is read again)
-#pragma unroll
-      for (int c = 0; c < 32; ++c) {
-        const uint32_t k = masks[c][4 + q];
-        if ((k >> lane) & 1u) {
-          const int slot = prefix[c][4 + q] + __popc(k & lanemask_lt());
-          if (slot < slab_w - 1)
-            packed[(size_t)(m0 + tb * 32 + c) * row_words + (size_t)tile * slab_w + 1 + slot] =
-                (uint32_t)(n_lo + 128) | (bf16_bits(v[c] + b_hi) << 16);
-        }
-      }
-      tmem_ld32(lane_addr + (uint32_t)(tb * 32), v);
-#pragma unroll
-      for (int c = 0; c < 32; ++c) {
-        const uint32_t k = masks[c][q];
-        if ((k >> lane) & 1u) {
-          const int slot = prefix[c][q] + __popc(k & lanemask_lt());
-          if (slot < slab_w - 1)
-            packed[(size_t)(m0 + tb * 32 + c) * row_words + (size_t)tile * slab_w + 1 + slot] =
-                (uint32_t)n_lo | (bf16_bits(v[c] + b_lo) << 16);
-        }
-      }
-      named_barrier(bar_id, 128);  // masks / prefix are rewritten by the group's next block
-    }
-  }
-
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  if (warp == 1) {
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base),
-                 "r"(kTmemCols)
-                 : "memory");
   }
 }
 
@@ -783,7 +438,7 @@ twell_pack_tc_splitk_wide_kernel(const __grid_constant__ CUtensorMap tmap_w,
 }
 
 // ---------------------------------------------------------------------------
-// Split-k kernel for 33..256 tokens: the decode kernel above with 128-token tiles.  A tile of
+// Split-k kernel for 33..128 tokens (up to 256 on request): the decode kernel above with 128-token tiles.  A tile of
 // 256 neurons x 128 tokens has only H / 256 CTAs to itself when d_model is not split (32 at
 // d_ff 8192: 32 SMs walking 32 latency-bound k-steps, 31-36 us per call whatever the token
 // count); split four ways over a cluster every SM streams a quarter of the weight rows.
@@ -981,45 +636,6 @@ twell_pack_tc_splitk_mid_kernel(const __grid_constant__ CUtensorMap tmap_w,
 }
 
 // ---- host side -------------------------------------------------------------
-template <int NTOK, int STAGES, int MINB = 1>
-int launch_tc(const void* x, const void* w, const float* bias, void* packed, int64_t M, int64_t D,
-              int64_t H, int cf, cudaStream_t stream) {
-  CUtensorMap map_w, map_x;
-  if (int rc = make_map(&map_w, w, H, D, 128)) return rc;
-  if (int rc = make_map(&map_x, x, M, D, NTOK)) return rc;
-  const size_t smem = (size_t)STAGES * (2 * kATileBytes + NTOK * 128) + 1024;
-  auto kern = twell_pack_tc_kernel<NTOK, STAGES, MINB>;
-  static size_t granted[64] = {0};
-  if (int rc = ensure_dynamic_smem(kern, smem, granted, "b200_twell_pack")) return rc;
-  const int slab_w = kTileN / cf;
-  const int tiles = (int)(H / kTileN);
-  dim3 grid((unsigned)tiles, (unsigned)((M + NTOK - 1) / NTOK), 1);
-  kern<<<grid, kThreadsTc, smem, stream>>>(map_w, map_x, bias, static_cast<uint32_t*>(packed),
-                                           (int)M, (int)D, slab_w, tiles * slab_w,
-                                           raster_group(H * D * 2, (int64_t)NTOK * D * 2));
-  return check_launch("b200_twell_pack (tcgen05)");
-}
-
-template <int STAGES>
-int launch_tc_wide(const void* x, const void* w, const float* bias, void* packed, int64_t M,
-                   int64_t D, int64_t H, int cf, cudaStream_t stream) {
-  CUtensorMap map_w, map_x;
-  if (int rc = make_map(&map_w, w, H, D, 256)) return rc;
-  if (int rc = make_map(&map_x, x, M, D, 256)) return rc;
-  const size_t smem = (size_t)STAGES * (2 * kATileBytes + 256 * 128) + 1024;
-  auto kern = twell_pack_tc_wide_kernel<STAGES>;
-  static size_t granted[64] = {0};
-  if (int rc = ensure_dynamic_smem(kern, smem, granted, "b200_twell_pack")) return rc;
-  const int slab_w = kTileN / cf;
-  const int tiles = (int)(H / kTileN);
-  dim3 grid((unsigned)tiles, (unsigned)((M + 255) / 256), 1);
-  kern<<<grid, kThreadsTcWideM, smem, stream>>>(map_w, map_x, bias,
-                                                static_cast<uint32_t*>(packed), (int)M, (int)D,
-                                                slab_w, tiles * slab_w,
-                                                raster_group(H * D * 2, (int64_t)256 * D * 2));
-  return check_launch("b200_twell_pack (tcgen05, 256-token tiles)");
-}
-
 template <int CL, int STAGES>
 int launch_tc_splitk_mid(const void* x, const void* w, const float* bias, void* packed, int64_t M,
                          int64_t D, int64_t H, int cf, cudaStream_t stream) {
@@ -1122,36 +738,9 @@ int twell_pack_tc_splitk8(const void* x, const void* w, const float* bias, void*
   return launch_tc_splitk<8, 4>(x, w, bias, packed, M, D, H, cf, stream);
 }
 
-// Large-M path.  Needs D % 64 == 0 (guaranteed by D % 256 == 0).
-int twell_pack_tc(const void* x, const void* w, const float* bias, void* packed, int64_t M,
-                  int64_t D, int64_t H, int cf, cudaStream_t stream) {
-  // Above 64 tokens: one CTA per SM on 256-token tiles with sixteen epilogue warps.  Measured
-  // on B200 against two co-resident 128-token CTAs per SM (four epilogue warps each) and
-  // cuBLAS matmul + relu, TFLOP/s at (M, D, H): (2048, 2048, 8192) 996 / 826 / 1063;
-  // (16384, 2048, 8192) 1222 / 995 / 1273; (16384, 2048, 11008) 1221 / 1002 / 1260;
-  // (2048, 4096, 16384) 1299 / 1102 / 1363; (16384, 4096, 16384) 1288 / 1222 / 1391;
-  // (16384, 1024, 4096) 855 / 681 / 994; at 100 tokens (D 2048, H 8192) 30.4 against 34.6 us
-  // for one 128-token tile per CTA.  B200_PACK_TILE=128 keeps the 128-token forms.
-  static const int tile_tokens = [] {
-    const char* e = getenv("B200_PACK_TILE");
-    return e != nullptr ? atoi(e) : 256;
-  }();
-  if (M > 64 && tile_tokens != 128) return launch_tc_wide<3>(x, w, bias, packed, M, D, H, cf, stream);
-  if (M >= 1024) return launch_tc<128, 2, 2>(x, w, bias, packed, M, D, H, cf, stream);
-  if (M > 64) return launch_tc<128, 4>(x, w, bias, packed, M, D, H, cf, stream);
-  return launch_tc<64, 4>(x, w, bias, packed, M, D, H, cf, stream);
-}
-
 // (A 2-way split - 64 CTAs streaming 512 KB each at H = 8192 - was measured at 16.8 us against
 // 12.8 us for the 4-way split: one SM pulls about 64 GB/s through TMA, so the weight stream
 // needs well over 100 CTAs to reach the HBM rate.)
-
-// Two co-resident CTAs of 128 tokens per SM (2 x 256 TMEM columns, 2 x 2 stages): one CTA's
-// pack epilogue runs under the other's MMAs.
-int twell_pack_tc_pair(const void* x, const void* w, const float* bias, void* packed, int64_t M,
-                       int64_t D, int64_t H, int cf, cudaStream_t stream) {
-  return launch_tc<128, 2, 2>(x, w, bias, packed, M, D, H, cf, stream);
-}
 
 // 33..256 tokens: split-k over a cluster of `split` (4 or 2) CTAs with 128-token tiles.
 int twell_pack_tc_splitk_mid(const void* x, const void* w, const float* bias, void* packed,
@@ -1172,19 +761,14 @@ int twell_pack_mid_split(int64_t M, int64_t H, int sm_count) {
   return 0;
 }
 
-// One CTA per SM, 256 neurons x 256 tokens per tile, sixteen epilogue warps.
-int twell_pack_tc_wide(const void* x, const void* w, const float* bias, void* packed, int64_t M,
-                       int64_t D, int64_t H, int cf, cudaStream_t stream) {
-  return launch_tc_wide<3>(x, w, bias, packed, M, D, H, cf, stream);
-}
-
 // Error word raised by a bounded wait that gave up (0 = none).  Reads and clears it;
 // synchronises the device.
 int twell_pack_tc_status() {
   int v = 0, zero = 0;
   if (cudaMemcpyFromSymbol(&v, g_tc_error, sizeof(int)) != cudaSuccess) return -1;
   if (v != 0) cudaMemcpyToSymbol(g_tc_error, &zero, sizeof(int));
-  return v;
+  const int pair = pair_gemm_status();
+  return v != 0 ? v : pair;
 }
 
 }  // namespace b200

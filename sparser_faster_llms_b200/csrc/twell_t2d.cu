@@ -122,7 +122,7 @@ twell_t2d_kernel(const __nv_bfloat16* x, const uint32_t* __restrict__ packed,
                  __nv_bfloat16* out, int M, int tiles, int slab_w, int cs, int nc,
                  float* ws_partial, unsigned int* ws_counter,
                  const unsigned char* __restrict__ skip_rows,
-                 const __grid_constant__ FusedAr ar) {
+                 const __grid_constant__ FusedAr ar, const RunIf run_if) {
   constexpr int D = NI * 256;
   constexpr int NTHREADS = NI * 32;
   __shared__ int tile_off[kMaxTiles + 1];
@@ -143,6 +143,7 @@ twell_t2d_kernel(const __nv_bfloat16* x, const uint32_t* __restrict__ packed,
   // Rows routed to the dense tensor-core path: every CTA of every cluster of the row leaves
   // (the row is uniform per cluster, so no cluster barrier is left half-attended).
   if (skip_rows != nullptr && skip_rows[row]) return;
+  if (run_if.entries != nullptr && *run_if.entries > run_if.limit) return;
   // Fused all-reduce: every CTA reads the call epoch now (the round trip hides under the slab
   // load).  It is advanced by the last (token, slice) group to finish, which cannot happen
   // before every CTA of the grid has contributed its partial sums, i.e. has started.
@@ -440,7 +441,7 @@ template <int NI, bool GATED, bool HP>
 int launch_t2d(const void* x, const void* packed, const void* up, const void* down, void* out,
                int64_t M, int64_t H, int cf, int cs, int nc, float* ws_partial,
                unsigned int* ws_counter, const unsigned char* skip_rows, const FusedAr& ar,
-               cudaStream_t stream) {
+               const RunIf& run_if, cudaStream_t stream) {
   const int slab_w = kTileN / cf;
   const int tiles = (int)(H / kTileN);
   auto kern = twell_t2d_kernel<NI, GATED, HP>;
@@ -487,7 +488,8 @@ int launch_t2d(const void* x, const void* packed, const void* up, const void* do
       &cfg, kern, reinterpret_cast<const __nv_bfloat16*>(x),
       reinterpret_cast<const uint32_t*>(packed), reinterpret_cast<const __nv_bfloat16*>(up),
       reinterpret_cast<const __nv_bfloat16*>(down), reinterpret_cast<__nv_bfloat16*>(out), (int)M,
-      tiles, slab_w, cs, nc, ws_partial, ws_counter, skip_rows, ar);
+      tiles, slab_w, cs, nc, ws_partial, ws_counter, skip_rows, ar,
+      run_if);
   if (e != cudaSuccess) return fail(B200_ECUDA, "twell_t2d: launch: %s", cudaGetErrorString(e));
   return B200_OK;
 }
@@ -496,12 +498,12 @@ template <bool GATED, bool HP>
 int dispatch_ni(int ni, const void* x, const void* packed, const void* up, const void* down,
                 void* out, int64_t M, int64_t H, int cf, int cs, int nc, float* ws_partial,
                 unsigned int* ws_counter, const unsigned char* skip_rows, const FusedAr& ar,
-                cudaStream_t stream) {
+                const RunIf& run_if, cudaStream_t stream) {
   switch (ni) {
 #define B200_CASE(N)                                                                           \
   case N:                                                                                      \
     return launch_t2d<N, GATED, HP>(x, packed, up, down, out, M, H, cf, cs, nc, ws_partial,   \
-                                    ws_counter, skip_rows, ar, stream);
+                                    ws_counter, skip_rows, ar, run_if, stream);
     B200_CASE(1) B200_CASE(2) B200_CASE(3) B200_CASE(4) B200_CASE(5) B200_CASE(6) B200_CASE(7)
     B200_CASE(8) B200_CASE(9) B200_CASE(10) B200_CASE(11) B200_CASE(12) B200_CASE(13)
     B200_CASE(14) B200_CASE(15) B200_CASE(16)
@@ -551,7 +553,7 @@ int twell_t2d_launch(bool gated, bool hp, const void* x, const void* packed, con
                      const void* down, void* out, int64_t M, int64_t D, int64_t H, int cf,
                      void* workspace, size_t workspace_bytes, int sm_count, cudaStream_t stream,
                      const unsigned char* skip_rows = nullptr,
-                     const FusedAr* fused_ar = nullptr) {
+                     const FusedAr* fused_ar = nullptr, const RunIf& run_if = {nullptr, 0u}) {
   int cs = 1, nc = 1;
   t2d_shape(M, D, sm_count, workspace != nullptr ? workspace_bytes : 0, &cs, &nc);
   FusedAr far = {};
@@ -573,14 +575,18 @@ int twell_t2d_launch(bool gated, bool hp, const void* x, const void* packed, con
   auto run = [&](int cs_, int nc_) {
     if (gated) {
       return hp ? dispatch_ni<true, true>(ni, x, packed, up, down, out, M, H, cf, cs_, nc_, partial,
-                                          counters, skip_rows, far, stream)
+                                          counters, skip_rows, far, run_if,
+                                         stream)
                 : dispatch_ni<true, false>(ni, x, packed, up, down, out, M, H, cf, cs_, nc_,
-                                           partial, counters, skip_rows, far, stream);
+                                           partial, counters, skip_rows, far, run_if,
+                                         stream);
     }
     return hp ? dispatch_ni<false, true>(ni, x, packed, up, down, out, M, H, cf, cs_, nc_, partial,
-                                         counters, skip_rows, far, stream)
+                                         counters, skip_rows, far, run_if,
+                                         stream)
               : dispatch_ni<false, false>(ni, x, packed, up, down, out, M, H, cf, cs_, nc_,
-                                          partial, counters, skip_rows, far, stream);
+                                          partial, counters, skip_rows, far, run_if,
+                                         stream);
   };
   int rc = run(cs, nc);
   // A fused call whose clusters are not all resident at once is retried with smaller clusters

@@ -466,10 +466,26 @@ def _gated_mlp(layer_number, A, UP, DOWN, C_packed, OUT, highest_precision, cf) 
                   flags, thr, cap, ws_ptr, ws_bytes, *_lib.workspace(dev))
         route["last"] = (m, d, h, cap)
     else:
-        _lib.call("b200_twell_gated_mlp", dev, A.data_ptr(), GATE.data_ptr(),
+        scratch, scratch_bytes = _mlp_scratch(dev, m, d, h, True, flags)
+        _lib.call("b200_twell_gated_mlp_scratch", dev, A.data_ptr(), GATE.data_ptr(),
                   _lib.ptr(entry["bias"]), UP.data_ptr(), DOWN.data_ptr(), C_packed.data_ptr(),
-                  OUT.data_ptr(), m, d, h, cf, flags, *_lib.workspace(dev))
+                  OUT.data_ptr(), m, d, h, cf, flags, *_lib.workspace(dev), _lib.ptr(scratch),
+                  scratch_bytes)
     entry["m"] = m
+
+
+_DENSE_FROM_TOKENS = 64  # no shape has a use for scratch below this many tokens
+
+
+def _mlp_scratch(dev, m, d, h, gated, flags) -> tuple[torch.Tensor | None, int]:
+    """Hidden matrix and partial sums of a call that runs on the tensor cores (None: it does
+    not).  From torch's allocator on every call, so calls on several streams never share it."""
+    if m < _DENSE_FROM_TOKENS:
+        return None, 0
+    need = int(_lib.load_library().b200_twell_mlp_scratch_bytes(m, d, h, int(gated), flags))
+    if need == 0:
+        return None, 0
+    return torch.empty(need, dtype=torch.uint8, device=dev), need
 
 
 # One growing scratch buffer per device for the dense-row route (calls on a stream are
@@ -559,9 +575,10 @@ def _plain_mlp(layer_number, A, DOWN, C_packed, OUT, num_splits) -> None:
         raise ValueError(f"UP/DOWN must both be [{h}, {d}]")
     _check_packed(C_packed, m, h, entry["cf"], "C_packed")
     dev = _same_device(A, UP, DOWN, C_packed, OUT)
-    _lib.call("b200_twell_mlp", dev, A.data_ptr(), UP.data_ptr(), DOWN.data_ptr(),
+    scratch, scratch_bytes = _mlp_scratch(dev, m, d, h, False, 0)
+    _lib.call("b200_twell_mlp_scratch", dev, A.data_ptr(), UP.data_ptr(), DOWN.data_ptr(),
               C_packed.data_ptr(), OUT.data_ptr(), m, d, h, entry["cf"], int(num_splits),
-              *_lib.workspace(dev))
+              *_lib.workspace(dev), _lib.ptr(scratch), scratch_bytes)
     entry["m"] = m
 
 
