@@ -217,6 +217,39 @@ int b200_twell_mlp(const void* x, const void* up, const void* down, void* packed
  * ------------------------------------------------------------------------ */
 
 /*
+ * The whole forward of ff_forward_cuda_gated (custom_models/hybrid_modules/custom_op.cpp:40-137) on
+ * the tensor cores: P = slabs of relu(x g^T), R = (x k^T) on P's pattern, T = R * P, out = T v,
+ * l0 / l1 = mean positives / mean sum |T| per row.  x, out [M, D]; g, k, v [H, D] bf16; p / r / t
+ * slab arrays.  Up to tail_rows overflowed rows (ascending) leave the slabs - the sign bit of
+ * their count words in p, r, t is set - and are computed from their dense gate values; entries of
+ * later ones past a slab's capacity are lost and counted in *dropped.  *n_over = overflowed rows.
+ * l0, l1, dropped, n_over are device scalars.
+ *   scratch: b200_hybrid_train_scratch_bytes(M, D, H, tail_rows, 0) bytes, 256-byte aligned,
+ *     uninitialised; workspace as for the contraction (may be NULL).
+ */
+size_t b200_hybrid_train_scratch_bytes(int64_t M, int64_t D, int64_t H, int64_t tail_rows,
+                                       int backward);
+
+int b200_hybrid_train_forward(const void* x, const void* g, const void* k, const void* v,
+                              void* out, void* p_slab, void* r_slab, void* t_slab, float* l0,
+                              float* l1, int* dropped, int* n_over, int64_t M, int64_t D,
+                              int64_t H, int cf, int64_t tail_rows, void* workspace,
+                              size_t workspace_bytes, void* scratch, size_t scratch_bytes,
+                              void* stream);
+
+/*
+ * The backward (custom_op.cpp:139-282) from the slabs of the forward and the gradients of out
+ * ([M, D] bf16) and l1 (device scalar, may be NULL): dx [M, D], dg, dk, dv [H, D] bf16.
+ * tail_rows: at least the number of flagged rows to restore; scratch as above with backward = 1.
+ */
+int b200_hybrid_train_backward(const void* x, const void* g, const void* k, const void* v,
+                               const void* p_slab, const void* r_slab, const void* g_out,
+                               const float* l1_grad, void* dx, void* dg, void* dk, void* dv,
+                               int64_t M, int64_t D, int64_t H, int cf, int64_t tail_rows,
+                               void* workspace, size_t workspace_bytes, void* scratch,
+                               size_t scratch_bytes, void* stream);
+
+/*
  * Forward: R = (x k_w^T) sampled at P's pattern (bf16), T = R * P (bf16 multiply),
  * row_l1[r] = sum |T[r,:]| (fp32), row_nnz[r] = true positive count of the row,
  * row_drop[r] = entries of the row lost to slab overflow.  Replaces

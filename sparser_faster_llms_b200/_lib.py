@@ -44,6 +44,16 @@ _PROTOTYPES = {
                                      c_void_p]),
     "b200_twell_t2d": (c_int, [c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int,
                                c_int, c_void_p, c_size_t, c_void_p]),
+    "b200_hybrid_train_scratch_bytes": (c_size_t, [c_int64] * 4 + [c_int]),
+    # x, g, k, v, out, p, r, t, l0, l1, dropped, n_over, M, D, H, cf, tail_rows, ws, ws_bytes,
+    # scratch, scratch_bytes, stream
+    "b200_hybrid_train_forward": (c_int, [c_void_p] * 12 + [c_int64, c_int64, c_int64, c_int,
+                                          c_int64, c_void_p, c_size_t, c_void_p, c_size_t,
+                                          c_void_p]),
+    # x, g, k, v, p, r, g_out, l1_grad, dx, dg, dk, dv, then as above
+    "b200_hybrid_train_backward": (c_int, [c_void_p] * 12 + [c_int64, c_int64, c_int64, c_int,
+                                           c_int64, c_void_p, c_size_t, c_void_p, c_size_t,
+                                           c_void_p]),
     "b200_hybrid_sddmm_fwd": (c_int, [c_void_p] * 8 + [c_int64, c_int64, c_int64, c_int, c_void_p]),
     "b200_hybrid_sddmm_bwd": (c_int, [c_void_p] * 7 + [c_int64, c_int64, c_int64, c_int,
                                                        c_void_p]),

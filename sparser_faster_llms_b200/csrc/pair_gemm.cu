@@ -1,6 +1,8 @@
 // The fused MLPs on the paired tensor-core GEMM (pair_gemm.cuh) for calls of more than a few
 // dozen tokens: gate GEMM with the pack epilogue, up GEMM whose epilogue multiplies by the slab
 // pattern, down GEMM over the resulting hidden matrix.
+#include <initializer_list>
+
 #include "pair_gemm.cuh"
 
 namespace b200 {
@@ -234,6 +236,385 @@ int pair_mlp(bool gated, bool hp, const void* x, const void* gate, const float* 
   }
   return B200_OK;
 }
+
+// ---- hybrid training operator --------------------------------------------------------------------
+namespace {
+
+// Overflow bookkeeping of one call, zero-filled before it.
+struct RowState {
+  int n_tail;       // rows taken out of the slabs
+  int n_over;       // rows with an overflowed tile
+  int dropped;      // entries lost to the slabs' capacity
+  unsigned int done;
+  unsigned long long nnz;
+};
+
+// Forward (BWD = false): a warp per row adds up the count words; the block that finishes last
+// writes l0 and the lost entries, and lists the first `cap` overflowed rows in ascending order.
+// Backward: the listed rows are those whose count words carry the sign bit.
+// row_slot[r]: place of row r in the list, else -1.
+template <bool BWD>
+__global__ void __launch_bounds__(256)
+tail_rows_kernel(const uint32_t* __restrict__ P, int M, int tiles, int W, int cap,
+                 unsigned char* __restrict__ flags, int* __restrict__ row_slot,
+                 int* __restrict__ row_drop, int* __restrict__ rows, RowState* __restrict__ state,
+                 float* __restrict__ l0, int* __restrict__ dropped, int* __restrict__ n_over,
+                 float inv_m) {
+  __shared__ unsigned long long nnz_s;
+  __shared__ int over_s, drop_s, warp_sum[8];
+  __shared__ bool last_s;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (tid == 0) {
+    nnz_s = 0;
+    over_s = drop_s = 0;
+  }
+  __syncthreads();
+  const size_t rw = (size_t)tiles * W;
+  if (BWD) {
+    const int r = blockIdx.x * 256 + tid;
+    const bool f = r < M && (int)P[(size_t)r * rw] < 0;
+    if (r < M) {
+      flags[r] = f;
+      row_slot[r] = -1;
+    }
+    const int n = __syncthreads_count(f);
+    if (tid == 0) over_s = n;
+  } else {
+    for (int i = 0; i < 4; ++i) {
+      const int r = blockIdx.x * 32 + warp * 4 + i;
+      if (r >= M) break;
+      int nnz = 0, drop = 0;
+      for (int t = lane; t < tiles; t += 32) {
+        const int c = (int)P[(size_t)r * rw + (size_t)t * W];
+        nnz += c;
+        drop += max(c - (W - 1), 0);
+      }
+      nnz = __reduce_add_sync(0xffffffffu, nnz);
+      drop = __reduce_add_sync(0xffffffffu, drop);
+      if (lane == 0) {
+        flags[r] = drop > 0;
+        row_slot[r] = -1;
+        row_drop[r] = drop;
+        atomicAdd(&nnz_s, (unsigned long long)nnz);
+        if (drop > 0) {
+          atomicAdd(&over_s, 1);
+          atomicAdd(&drop_s, drop);
+        }
+      }
+    }
+  }
+  __threadfence();
+  __syncthreads();
+  if (tid == 0) {
+    if (!BWD) atomicAdd(&state->nnz, nnz_s);
+    if (over_s != 0) atomicAdd(&state->n_over, over_s);
+    if (!BWD && drop_s != 0) atomicAdd(&state->dropped, drop_s);
+    __threadfence();
+    last_s = atomicAdd(&state->done, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last_s) return;
+  __threadfence();
+  const int over = *(volatile int*)&state->n_over;
+  int lost = *(volatile int*)&state->dropped;
+  if (over > 0 && cap > 0) {
+    const int per = (M + 255) / 256, r0 = tid * per, r1 = min(M, r0 + per);
+    int mine = 0;
+    for (int r = r0; r < r1; ++r) mine += __ldcg(flags + r);
+    int inc = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += v;
+    }
+    if (lane == 31) warp_sum[warp] = inc;
+    if (tid == 0) drop_s = 0;
+    __syncthreads();
+    int pos = inc - mine;
+    for (int w = 0; w < warp; ++w) pos += warp_sum[w];
+    int kept = 0;
+    for (int r = r0; r < r1 && pos < cap; ++r) {
+      if (!__ldcg(flags + r)) continue;
+      rows[pos] = r;
+      row_slot[r] = pos++;
+      if (!BWD) kept += __ldcg(row_drop + r);
+    }
+    if (kept) atomicAdd(&drop_s, kept);
+    __syncthreads();
+    lost -= drop_s;
+  }
+  if (tid == 0) {
+    state->n_tail = min(over, cap);
+    if (!BWD) {
+      *l0 = (float)(*(volatile unsigned long long*)&state->nnz) * inv_m;
+      *dropped = lost;
+      *n_over = over;
+    }
+  }
+}
+
+// One block per listed row: copies the row of x and (FLAG) sets the sign bit of its count words.
+template <bool FLAG>
+__global__ void __launch_bounds__(128)
+tail_gather_kernel(uint32_t* __restrict__ P, const uint4* __restrict__ x,
+                   const int* __restrict__ rows, const RowState* __restrict__ state,
+                   uint4* __restrict__ xt, int tiles, int W, int vec_per_row) {
+  if ((int)blockIdx.x >= state->n_tail) return;
+  const int r = rows[blockIdx.x];
+  if (FLAG)
+    for (int t = threadIdx.x; t < tiles; t += 128)
+      P[((size_t)r * tiles + t) * W] |= 0x80000000u;
+  for (int v = threadIdx.x; v < vec_per_row; v += 128)
+    xt[(size_t)blockIdx.x * vec_per_row + v] = __ldg(x + (size_t)r * vec_per_row + v);
+}
+
+// l1 = inv_m * sum of n partial sums, in a fixed order.
+__global__ void __launch_bounds__(1024)
+l1_sum_kernel(const float* __restrict__ part, int n, float inv_m, float* __restrict__ l1) {
+  __shared__ float warp_s[32];
+  float s = 0.f;
+  for (int i = threadIdx.x; i < n; i += 1024) s += part[i];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if ((threadIdx.x & 31) == 0) warp_s[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    s = warp_s[threadIdx.x];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (threadIdx.x == 0) *l1 = s * inv_m;
+  }
+}
+
+// Scratch of a training call; `tail` rows at most leave the slabs.
+struct TrainWs {
+  RowState* state;
+  unsigned char* flags;
+  int *row_slot, *row_drop, *rows;
+  __nv_bfloat16 *xt, *pt, *rt;   // tail rows: x, gate values, up products
+  __nv_bfloat16 *t, *dru;        // [M, H] and (backward) [M, 2 H]
+  float *l1_part, *part;
+  size_t total;
+};
+
+TrainWs train_ws(void* base, int64_t M, int64_t D, int64_t H, int64_t tail, bool bwd) {
+  unsigned char* p = static_cast<unsigned char*>(base);
+  size_t off = 0;
+  auto take = [&](size_t bytes) {
+    unsigned char* q = p + off;
+    off += align256(bytes);
+    return q;
+  };
+  TrainWs w = {};
+  w.state = reinterpret_cast<RowState*>(take(sizeof(RowState)));
+  w.flags = take((size_t)M);
+  w.row_slot = reinterpret_cast<int*>(take((size_t)M * 4));
+  w.row_drop = reinterpret_cast<int*>(take((size_t)M * 4));
+  w.rows = reinterpret_cast<int*>(take((size_t)tail * 4));
+  w.xt = reinterpret_cast<__nv_bfloat16*>(take((size_t)tail * D * 2));
+  w.pt = reinterpret_cast<__nv_bfloat16*>(take((size_t)tail * H * 2));
+  if (bwd) w.rt = reinterpret_cast<__nv_bfloat16*>(take((size_t)tail * H * 2));
+  w.t = reinterpret_cast<__nv_bfloat16*>(take((size_t)M * H * 2));
+  if (bwd) w.dru = reinterpret_cast<__nv_bfloat16*>(take((size_t)M * H * 4));
+  const int64_t mt = (M + pg::kTile - 1) / pg::kTile, nt = H / pg::kTile, slots = sm_count() / 2;
+  if (!bwd) w.l1_part = reinterpret_cast<float*>(take((size_t)mt * nt * 16 * 4));
+  size_t part = pg::part_bytes(mt * nt, (int)(D / kStageK), slots, false);
+  auto more = [&](size_t b) { part = b > part ? b : part; };
+  more(pg::part_bytes(mt * (D / pg::kTile), (int)((bwd ? 2 : 1) * H / kStageK), slots, true));
+  if (bwd)
+    more(pg::part_bytes(3 * nt * (D / pg::kTile), (int)((M + kStageK - 1) / kStageK), slots, false));
+  w.part = reinterpret_cast<float*>(take(part));
+  w.total = off;
+  return w;
+}
+
+// Dense products of the listed tail rows: out[i, :] = xt[i, :] w^T (relu), device-side row count.
+int tail_product(const TrainWs& w, const void* weight, __nv_bfloat16* out, bool relu, int64_t tail,
+                 int64_t D, int64_t H, cudaStream_t stream) {
+  pg::Args a = base_args(tail, H, D);
+  a.rows_ptr = &w.state->n_tail;
+  a.out = out;
+  a.ld = H;
+  a.wide = 1;
+  a.relu = relu;
+  const pg::Operand ox = {w.xt, tail, D}, ow = {weight, H, D};
+  return pg::launch<pg::kStore, false, false>("tail rows", ox, ox, ow, ow, a, tail, sm_count(),
+                                              stream);
+}
+
+int train_check(const char* fn, int64_t M, int64_t D, int64_t H, int cf, int64_t tail,
+                std::initializer_list<const void*> ptrs, const void* scratch, size_t scratch_bytes,
+                size_t need) {
+  if (int rc = check_dims(fn, M, D, H, cf)) return rc;
+  if (M == 0) return fail(B200_EINVAL, "%s: M must be > 0", fn);
+  if (M > (int64_t)1 << 22) return fail(B200_EUNSUPPORTED, "%s: M > 2^22 rows", fn);
+  if (tail < 0 || tail > M) return fail(B200_EINVAL, "%s: need 0 <= tail_rows <= M", fn);
+  for (const void* p : ptrs) {
+    if (p == nullptr) return fail(B200_ENULL, "%s: NULL pointer", fn);
+    if (!aligned16(p)) return fail(B200_EALIGN, "%s: a pointer is not 16-byte aligned", fn);
+  }
+  if (scratch == nullptr) return fail(B200_ENULL, "%s: scratch is NULL", fn);
+  if (reinterpret_cast<uintptr_t>(scratch) & 255u)
+    return fail(B200_EALIGN, "%s: scratch is not 256-byte aligned", fn);
+  if (scratch_bytes < need)
+    return fail(B200_EWORKSPACE, "%s: scratch holds %zu bytes, %zu needed", fn, scratch_bytes, need);
+  return B200_OK;
+}
+
+unsigned int* split_counters(void* workspace, size_t workspace_bytes) {
+  return workspace != nullptr && workspace_bytes >= 16384 ? static_cast<unsigned int*>(workspace)
+                                                          : nullptr;
+}
+
+}  // namespace
+
+}  // namespace b200
+
+using namespace b200;
+
+extern "C" size_t b200_hybrid_train_scratch_bytes(int64_t M, int64_t D, int64_t H, int64_t tail_rows,
+                                                  int backward) {
+  if (M <= 0 || D < 256 || H < 256 || D % 256 || H % 256 || tail_rows < 0) return 0;
+  return train_ws(nullptr, M, D, H, tail_rows, backward != 0).total;
+}
+
+extern "C" int b200_hybrid_train_forward(const void* x, const void* g, const void* k, const void* v,
+                                         void* out, void* p_slab, void* r_slab, void* t_slab,
+                                         float* l0, float* l1, int* dropped, int* n_over, int64_t M,
+                                         int64_t D, int64_t H, int cf, int64_t tail_rows,
+                                         void* workspace, size_t workspace_bytes, void* scratch,
+                                         size_t scratch_bytes, void* stream) {
+  const char* fn = "b200_hybrid_train_forward";
+  const TrainWs w = train_ws(scratch, M, D, H, tail_rows, false);
+  if (int rc = train_check(fn, M, D, H, cf, tail_rows,
+                           {x, g, k, v, out, p_slab, r_slab, t_slab}, scratch, scratch_bytes,
+                           w.total))
+    return rc;
+  if (l0 == nullptr || l1 == nullptr || dropped == nullptr || n_over == nullptr)
+    return fail(B200_ENULL, "%s: NULL result pointer", fn);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  unsigned int* counters = split_counters(workspace, workspace_bytes);
+  const int tiles = (int)(H / kTileN), W = kTileN / cf;
+  const float inv_m = 1.f / (float)M;
+  if (cudaMemsetAsync(w.state, 0, sizeof(RowState), st) != cudaSuccess)
+    return fail(B200_ECUDA, "%s: cudaMemsetAsync failed", fn);
+  // the gate pattern
+  pdl_suppressed() = true;  // its predecessor is the memset
+  int rc = M > 128 ? pair_pack(x, g, nullptr, p_slab, nullptr, M, D, H, cf, nullptr, w.part,
+                               counters, st)
+                   : b200_twell_pack(x, g, nullptr, p_slab, M, D, H, cf, stream);
+  pdl_suppressed() = false;
+  if (rc) return rc;
+  tail_rows_kernel<false><<<(unsigned)((M + 31) / 32), 256, 0, st>>>(
+      static_cast<const uint32_t*>(p_slab), (int)M, tiles, W, (int)tail_rows, w.flags, w.row_slot,
+      w.row_drop, w.rows, w.state, l0, dropped, n_over, inv_m);
+  if (int e = check_launch(fn)) return e;
+  if (tail_rows > 0) {
+    tail_gather_kernel<true><<<(unsigned)tail_rows, 128, 0, st>>>(
+        static_cast<uint32_t*>(p_slab), static_cast<const uint4*>(x), w.rows, w.state,
+        reinterpret_cast<uint4*>(w.xt), tiles, W, (int)(D / 8));
+    if (int e = check_launch(fn)) return e;
+    if (int e = tail_product(w, g, w.pt, true, tail_rows, D, H, st)) return e;
+  }
+  // R, T
+  pg::Args a = base_args(M, H, D);
+  a.slab_p = static_cast<uint32_t*>(p_slab);
+  a.slab_r = static_cast<uint32_t*>(r_slab);
+  a.slab_t = static_cast<uint32_t*>(t_slab);
+  a.slab_w = W;
+  a.row_words = tiles * W;
+  a.row_slot = tail_rows > 0 ? w.row_slot : nullptr;
+  a.tail_p = w.pt;
+  a.out = w.t;
+  a.ld = H;
+  a.wide = 1;
+  a.l1_part = w.l1_part;
+  a.part = w.part;
+  a.counters = counters;
+  const pg::Operand ox = {x, M, D}, ok = {k, H, D};
+  if (int e = pg::launch<pg::kFwd, false, false>(fn, ox, ox, ok, ok, a, M, sm_count(), st)) return e;
+  if (int e = pair_down(w.t, 1, v, out, M, D, H, {nullptr, 0u}, w.part, counters, st)) return e;
+  l1_sum_kernel<<<1, 1024, 0, st>>>(w.l1_part, (int)((M + pg::kTile - 1) / pg::kTile) * tiles * 16,
+                                    inv_m, l1);
+  return check_launch(fn);
+}
+
+extern "C" int b200_hybrid_train_backward(const void* x, const void* g, const void* k, const void* v,
+                                          const void* p_slab, const void* r_slab,
+                                          const void* g_out, const float* l1_grad, void* dx,
+                                          void* dg, void* dk, void* dv, int64_t M, int64_t D,
+                                          int64_t H, int cf, int64_t tail_rows, void* workspace,
+                                          size_t workspace_bytes, void* scratch,
+                                          size_t scratch_bytes, void* stream) {
+  const char* fn = "b200_hybrid_train_backward";
+  const TrainWs w = train_ws(scratch, M, D, H, tail_rows, true);
+  if (int rc = train_check(fn, M, D, H, cf, tail_rows,
+                           {x, g, k, v, p_slab, r_slab, g_out, dx, dg, dk, dv}, scratch,
+                           scratch_bytes, w.total))
+    return rc;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  unsigned int* counters = split_counters(workspace, workspace_bytes);
+  const int tiles = (int)(H / kTileN), W = kTileN / cf;
+  if (tail_rows > 0) {
+    if (cudaMemsetAsync(w.state, 0, sizeof(RowState), st) != cudaSuccess)
+      return fail(B200_ECUDA, "%s: cudaMemsetAsync failed", fn);
+    tail_rows_kernel<true><<<(unsigned)((M + 255) / 256), 256, 0, st>>>(
+        static_cast<const uint32_t*>(p_slab), (int)M, tiles, W, (int)tail_rows, w.flags, w.row_slot,
+        w.row_drop, w.rows, w.state, nullptr, nullptr, nullptr, 0.f);
+    tail_gather_kernel<false><<<(unsigned)tail_rows, 128, 0, st>>>(
+        nullptr, static_cast<const uint4*>(x), w.rows, w.state, reinterpret_cast<uint4*>(w.xt),
+        tiles, W, (int)(D / 8));
+    if (int e = check_launch(fn)) return e;
+    if (int e = tail_product(w, g, w.pt, true, tail_rows, D, H, st)) return e;
+    if (int e = tail_product(w, k, w.rt, false, tail_rows, D, H, st)) return e;
+  }
+  // dT = g_out V^T on the pattern; dR = dT P, dU = dT R, T = R P
+  pg::Args a = base_args(M, H, D);
+  a.slab_p = const_cast<uint32_t*>(static_cast<const uint32_t*>(p_slab));
+  a.slab_r = const_cast<uint32_t*>(static_cast<const uint32_t*>(r_slab));
+  a.slab_w = W;
+  a.row_words = tiles * W;
+  a.row_slot = tail_rows > 0 ? w.row_slot : nullptr;
+  a.tail_p = w.pt;
+  a.tail_r = w.rt;
+  a.out = w.dru;
+  a.ld = 2 * H;
+  a.dense_t = w.t;
+  a.ld_t = H;
+  a.wide = 1;
+  a.l1_grad = l1_grad;
+  a.inv_m = 1.f / (float)M;
+  a.part = w.part;
+  a.counters = counters;
+  const pg::Operand og = {g_out, M, D}, ov = {v, H, D};
+  if (int e = pg::launch<pg::kBwd, false, false>(fn, og, og, ov, ov, a, M, sm_count(), st)) return e;
+  // dX = [dR | dU] [K; G]
+  pg::Args b = base_args(M, D, 2 * H);
+  b.seg_ksteps = (int)(H / kStageK);
+  b.out = static_cast<__nv_bfloat16*>(dx);
+  b.ld = D;
+  b.wide = aligned32(dx);
+  b.part = w.part;
+  b.counters = counters;
+  const pg::Operand odru = {w.dru, M, 2 * H}, okd = {k, D, H}, ogd = {g, D, H};
+  if (int e = pg::launch<pg::kStore, false, true>(fn, odru, odru, okd, ogd, b, M, sm_count(), st))
+    return e;
+  // [dK; dG] = [dR | dU]^T X and dV = T^T g_out in one launch
+  pg::Args c = base_args(3 * H, D, M);
+  c.second_mt = (int)(2 * H / pg::kTile);
+  c.out = static_cast<__nv_bfloat16*>(dk);
+  c.out_more[0] = static_cast<__nv_bfloat16*>(dg);
+  c.out_more[1] = static_cast<__nv_bfloat16*>(dv);
+  c.out_mt = (int)(H / pg::kTile);
+  c.ld = D;
+  c.wide = aligned32(dk) && aligned32(dg) && aligned32(dv);
+  c.part = w.part;
+  c.counters = counters;
+  const pg::Operand a0 = {w.dru, 2 * H, M}, a1 = {w.t, H, M}, b0 = {x, D, M}, b1 = {g_out, D, M};
+  return pg::launch<pg::kStore, true, true>(fn, a0, a1, b0, b1, c, 3 * H, sm_count(), st);
+}
+
+namespace b200 {
 
 // Error word raised by a bounded wait that gave up (0 = none).  Reads and clears it; synchronises.
 int pair_gemm_status() {

@@ -41,6 +41,7 @@ constexpr int kThreads = 320;
 constexpr int kTile = 256;                   // rows and columns per pair
 constexpr int kOperandBytes = 128 * 128;     // one CTA's half of A or B per 64-k stage
 constexpr int kStageBytes = 2 * kOperandBytes;
+constexpr int kBatch = 16;                   // slab rows whose words are in flight at a time
 constexpr int kBufBytes = 8 * 32 * 256;       // pattern buffers: 32 rows x 256 bytes per epilogue warp
 
 enum Epilogue {
@@ -66,6 +67,9 @@ struct Args {
   __nv_bfloat16* out;        // dense result, row stride ld
   long long ld;
   int wide;                  // out rows are 32-byte aligned
+  int relu;                  // kStore
+  __nv_bfloat16* out_more[2];  // kStore: results of the row tiles from out_mt and 2 out_mt on
+  int out_mt;                // 0: all rows in out
   const float* bias;         // packs; bias16: 16-byte aligned
   int bias16;
   // slab operands [rows][row_words], slab_w words per 256 columns
@@ -79,7 +83,7 @@ struct Args {
   const __nv_bfloat16* tail_r;
   __nv_bfloat16* dense_t;    // kBwd: T, row stride ld_t
   long long ld_t;
-  float* l1_part;            // kFwd: [2 n_tiles][rows] sums of |T|
+  float* l1_part;            // kFwd: [tiles][16] sums of |T|
   const float* l1_grad;      // kBwd: device scalar or null
   float inv_m;
   int keep_all;              // kGateUp: values past a slab's capacity still count in the product
@@ -211,18 +215,18 @@ __device__ __forceinline__ void load_values(const Args& a, unsigned char* buf, i
     *reinterpret_cast<uint4*>(buf + lane * 256 + i * 16) = make_uint4(0u, 0u, 0u, 0u);
   __syncwarp();
   const uint32_t* base = a.slab_p + (size_t)nt * a.slab_w;
-  for (int t0 = 0; t0 < 32; t0 += 8) {
+  for (int t0 = 0; t0 < 32; t0 += kBatch) {
     if (row0 + t0 >= rows) break;
-    int cnt[8], most = 0;
+    int cnt[kBatch], most = 0;
     for (int w0 = 0; w0 < a.slab_w; w0 += 32) {
-      uint32_t w[8];
+      uint32_t w[kBatch];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
+      for (int j = 0; j < kBatch; ++j) {
         const int row = row0 + t0 + j;
         w[j] = row < rows ? base[(size_t)row * a.row_words + w0 + lane] : 0u;
       }
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
+      for (int j = 0; j < kBatch; ++j) {
         if (w0 == 0) {
           cnt[j] = min(max((int)__shfl_sync(0xffffffffu, w[j], 0), 0), a.slab_w - 1);
           most = max(most, cnt[j]);
@@ -261,20 +265,20 @@ __device__ __forceinline__ void load_pairs(const Args& a, unsigned char* buf, in
     *reinterpret_cast<uint4*>(buf + lane * 256 + i * 16) = make_uint4(0u, 0u, 0u, 0u);
   __syncwarp();
   const size_t tile_off = (size_t)nt * a.slab_w;
-  for (int t0 = 0; t0 < 32; t0 += 8) {
+  for (int t0 = 0; t0 < 32; t0 += kBatch) {
     if (row0 + t0 >= rows) break;
-    int cnt[8], most = 0;
+    int cnt[kBatch], most = 0;
     for (int w0 = 0; w0 < a.slab_w; w0 += 32) {
-      uint32_t w[8], r[8];
+      uint32_t w[kBatch], r[kBatch];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
+      for (int j = 0; j < kBatch; ++j) {
         const int row = row0 + t0 + j;
         const size_t off = (size_t)row * a.row_words + tile_off + w0 + lane;
         w[j] = row < rows ? a.slab_p[off] : 0u;
         r[j] = row < rows ? a.slab_r[off] : 0u;
       }
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
+      for (int j = 0; j < kBatch; ++j) {
         if (w0 == 0) {
           cnt[j] = min(max((int)__shfl_sync(0xffffffffu, w[j], 0), 0), a.slab_w - 1);
           most = max(most, cnt[j]);
@@ -552,6 +556,10 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap map_a0,
       const int row = row0 + lane;
       const bool live = row < rows;
       __nv_bfloat16* out = a.out + (size_t)row * a.ld + nt * kTile + half * 128;
+      if (EPI == kStore && a.out_mt > 0 && mt >= a.out_mt) {
+        const int o = mt / a.out_mt;
+        out = a.out_more[o - 1] + (size_t)(row - o * a.out_mt * kTile) * a.ld + nt * kTile + half * 128;
+      }
       auto load_pattern = [&]() {
         if (EPI == kMul || EPI == kMulHp || EPI == kFwd)
           load_values(a, buf, row0, rows, nt, half, lane);
@@ -717,7 +725,9 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap map_a0,
           if (EPI == kStore) {
             uint32_t w[16];
 #pragma unroll
-            for (int p = 0; p < 16; ++p) w[p] = pack2(v[2 * p], v[2 * p + 1]);
+            for (int p = 0; p < 16; ++p)
+              w[p] = a.relu ? pack2(fmaxf(v[2 * p], 0.f), fmaxf(v[2 * p + 1], 0.f))
+                            : pack2(v[2 * p], v[2 * p + 1]);
             if (live) store64(out + cb * 32, w, a.wide);
           } else if (EPI == kMul || EPI == kGateUp || EPI == kFwd) {
             uint32_t w[16];
@@ -733,7 +743,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap map_a0,
                 const uint32_t m = nonzero2(g[p]);
                 r[p] = pack2(v[c], v[c + 1]) & m;      // never touch u where nothing is stored
                 w[4 * j + p] = mul2(g[p], r[p]) & m;
-                if (EPI == kFwd) {
+                if (EPI == kFwd && live) {
                   l1 += fabsf(lo_f(w[4 * j + p]));
                   l1 += fabsf(hi_f(w[4 * j + p]));
                 }
@@ -786,34 +796,48 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap map_a0,
             }
           }
         }
-        if (EPI == kFwd && live) a.l1_part[(size_t)(nt * 2 + half) * rows + row] = l1;
+        if (EPI == kFwd) {  // one sum of |T| per warp and tile
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) l1 += __shfl_xor_sync(0xffffffffu, l1, o);
+          if (lane == 0) a.l1_part[((size_t)im.tile * 2 + crank) * 8 + q * 2 + half] = l1;
+        }
         if (src.part == nullptr) release();
         __syncwarp();
       }
       if (EPI == kFwd) {
         // R and T in the slots of P, from the R values left in the pattern buffer
         const size_t tile_off = (size_t)nt * a.slab_w;
-        for (int tk = 0; tk < 32; ++tk) {
-          const int r = row0 + tk;
-          if (r >= rows) break;
-          int cnt = 0;
+        for (int t0 = 0; t0 < 32; t0 += kBatch) {
+          if (row0 + t0 >= rows) break;
+          int cnt[kBatch], most = 0;
           for (int w0 = 0; w0 < a.slab_w; w0 += 32) {
-            const size_t off = (size_t)r * a.row_words + tile_off + w0 + lane;
-            const uint32_t w = a.slab_p[off];
-            if (w0 == 0) {
-              cnt = min(max((int)__shfl_sync(0xffffffffu, w, 0), 0), a.slab_w - 1);
-              if (lane == 0 && half == 0) {
-                a.slab_r[off] = w;
-                a.slab_t[off] = w;
+            uint32_t w[kBatch];
+#pragma unroll
+            for (int j = 0; j < kBatch; ++j) {
+              const int r = row0 + t0 + j;
+              w[j] = r < rows ? a.slab_p[(size_t)r * a.row_words + tile_off + w0 + lane] : 0u;
+            }
+#pragma unroll
+            for (int j = 0; j < kBatch; ++j) {
+              const int r = row0 + t0 + j;
+              const size_t off = (size_t)r * a.row_words + tile_off + w0 + lane;
+              if (w0 == 0) {
+                cnt[j] = min(max((int)__shfl_sync(0xffffffffu, w[j], 0), 0), a.slab_w - 1);
+                most = max(most, cnt[j]);
+                if (lane == 0 && half == 0 && r < rows) {
+                  a.slab_r[off] = w[j];
+                  a.slab_t[off] = w[j];
+                }
+              }
+              const int slot = w0 + lane, col = (int)(w[j] & 255u);
+              if (slot >= 1 && slot <= cnt[j] && (col >> 7) == half) {
+                const uint32_t rb =
+                    *reinterpret_cast<const uint16_t*>(at(buf, t0 + j, (col & 127) * 2));
+                a.slab_r[off] = (w[j] & 0xFFFFu) | (rb << 16);
+                a.slab_t[off] = (w[j] & 0xFFFFu) | (mul2(rb, w[j] >> 16) << 16);
               }
             }
-            const int slot = w0 + lane, col = (int)(w & 255u);
-            if (slot >= 1 && slot <= cnt && (col >> 7) == half) {
-              const uint32_t rb = *reinterpret_cast<const uint16_t*>(at(buf, tk, (col & 127) * 2));
-              a.slab_r[off] = (w & 0xFFFFu) | (rb << 16);
-              a.slab_t[off] = (w & 0xFFFFu) | (mul2(rb, w >> 16) << 16);
-            }
-            if (cnt < w0 + 32) break;
+            if (most < w0 + 32) break;
           }
         }
         __syncwarp();
@@ -905,13 +929,14 @@ int launch(const char* fn, const Operand& a0, const Operand& a1, const Operand& 
   if (int rc = ensure_dynamic_smem(kern, smem, granted, fn)) return rc;
   const int64_t tiles = (row_capacity + kTile - 1) / kTile * args.n_tiles;
   const int64_t slots = sm_count / 2;
+  const bool can_sum = EPI == kStore && args.out_mt == 0 && !args.relu &&
+                       args.ld == (long long)args.n_tiles * kTile;
   const Split sp = EPI != kGateUp && EPI != kGateUpHp && args.part != nullptr && args.counters != nullptr && args.rows_ptr == nullptr
-                       ? choose_split(tiles, args.ksteps, slots, EPI == kStore)
+                       ? choose_split(tiles, args.ksteps, slots, can_sum)
                        : Split{tiles, 1};
   args.full_tiles = (int)sp.full_tiles;
   args.splits = sp.splits;
-  const bool sum_after = EPI == kStore && sp.splits > 1 && sp.full_tiles == 0 &&
-                         args.ld == (long long)args.n_tiles * kTile;
+  const bool sum_after = can_sum && sp.splits > 1 && sp.full_tiles == 0;
   args.sums = sum_after ? args.part : nullptr;
   const int64_t items = sp.full_tiles + (tiles - sp.full_tiles) * sp.splits;
   const int64_t pairs = items < slots ? items : slots;

@@ -63,49 +63,28 @@ _CONFIG = {
     "discard_overflow": 0,
     # average stored entries per row the column lists are sized for
     "csc_entries_per_row": 512,
-    # weight gradients dK / dG / dV: "sparse" = column lists + transposed SpMM, "dense" =
-    # scatter to a K-major matrix + tcgen05 GEMM, "auto" = dense from 2048 tokens on
+    # backward: "dense" / "auto" = tensor-core products with the slab pattern in their epilogues,
+    # "sparse" = gathers along slabs and column lists
     "weight_gradient_mode": "auto",
     # size the tail from the overflow count observed on earlier calls instead of always
     # computing tail_rows_regular rows (see set_tail_rows_adaptive)
     "tail_rows_adaptive": 0,
 }
-_LAST_TRANSPOSE_OVERFLOW: torch.Tensor | None = None
+_LAST_TRANSPOSE_OVERFLOW: torch.Tensor | torch.device | None = None
 _PERF: dict[str, list[float]] = {}
 _PERF_ENABLED = os.environ.get("SPARSE_ENABLE_PERF_PROFILING", "0") not in ("0", "", "false", "False")
 
 
 def set_weight_gradient_mode(mode: str) -> None:
-    """``"sparse"``, ``"dense"`` or ``"auto"`` (default: dense from 2048 tokens on).  The three
-    weight gradients reduce over all tokens and are dense ``[H, D]`` matrices, so they can run
-    as tensor-core GEMMs over a scattered K-major copy of the slab instead of gathers along
-    column lists.  Measured on B200 (16384 tokens, D = 1024, H = 4096, 41 positives per token)
-    the two forms take the same time (0.79 ms for the three products against 0.78 ms including
-    the lists: the GEMM has only 128 tiles and is bound by the operand stream into each SM);
-    the dense form is deterministic, whereas the order inside a column list follows atomic
-    arrival.  No reference counterpart: the reference always transposes the hybrid container
-    and runs its SpMM (custom_op.cpp:247-269)."""
+    """``"dense"`` and ``"auto"`` (the default): the backward runs as dense tensor-core products
+    whose epilogues apply the slab pattern (``csrc/pair_gemm.cu``); deterministic.  ``"sparse"``:
+    gathers along the slabs and along column lists, whose order follows atomic arrival.  Measured
+    on B200 (16384 tokens, D = 1024, H = 4096, 41 positives per token), forward + backward: see
+    ``csrc/pair_gemm.cu``.  No reference counterpart: the reference always transposes the hybrid
+    container and runs its SpMM (custom_op.cpp:247-269)."""
     if mode not in ("sparse", "dense", "auto"):
         raise ValueError("mode must be 'sparse', 'dense' or 'auto'")
     _CONFIG["weight_gradient_mode"] = mode
-
-
-def _dense_weight_gradients(m: int) -> bool:
-    mode = _CONFIG["weight_gradient_mode"]
-    return mode == "dense" or (mode == "auto" and m >= 2048)
-
-
-_WGRAD_WS: dict[int, torch.Tensor] = {}
-
-
-def _wgrad_workspace(dev: torch.device, m: int, d: int, h: int) -> torch.Tensor:
-    need = int(_lib.load_library().b200_hybrid_wgrad_workspace_bytes(m, d, h))
-    key = dev.index if dev.index is not None else torch.cuda.current_device()
-    buf = _WGRAD_WS.get(key)
-    if buf is None or buf.numel() < need:
-        buf = torch.empty(need, dtype=torch.uint8, device=dev)
-        _WGRAD_WS[key] = buf
-    return buf
 
 
 def set_tail_rows_adaptive(on: bool) -> None:
@@ -263,54 +242,32 @@ def ff_forward_impl(X: torch.Tensor, G: torch.Tensor, K: torch.Tensor, V: torch.
     Xf = X.reshape(m, d).contiguous()
     G, K, V = G.contiguous(), K.contiguous(), V.contiguous()
     shape = _slab_shape(m, h, cf)
+    i32, f32 = dict(dtype=torch.int32, device=dev), dict(dtype=torch.float32, device=dev)
+    P, R, T = (torch.empty(shape, **i32) for _ in range(3))
+    out = torch.empty_like(Xf)
+    if m == 0:
+        zero = torch.zeros((), **f32)
+        return out.reshape(X.shape), zero, zero.clone(), P, R, T, torch.zeros((), **i32)
     tail_key = (dev.index, G.data_ptr(), m, h)
-    cap = _tail_capacity(tail_key, m) if m > 0 else 0
+    cap = _tail_capacity(tail_key, m)
+    l0, l1 = torch.empty((), **f32), torch.empty((), **f32)
+    dropped, n_over = torch.empty((), **i32), torch.empty((), **i32)
     with _Timer("ff_forward_gated_total"):
-        P = torch.empty(shape, dtype=torch.int32, device=dev)
-        with _Timer("gate_gemm_pack"):
-            _lib.call("b200_twell_pack", dev, Xf.data_ptr(), G.data_ptr(), None, P.data_ptr(),
-                      m, d, h, cf)
-        inv_m = 1.0 / max(m, 1)
-        tail = None
-        adaptive = bool(_CONFIG["tail_rows_adaptive"]) and m > 0 and \
-            not _CONFIG["discard_overflow"] and _CONFIG["tail_rows_regular"] > 0
-        if cap > 0 or adaptive:
-            cnt = _count_view(P, m, h, cf)
-            over = (cnt > TILE // cf - 1).any(dim=1)
-            if adaptive:
-                _tail_observe(tail_key, over.sum())
-        if cap > 0:
-            # rows with an overflowed tile leave the slabs: flag their count words
-            in_tail = over & (over.cumsum(0) <= cap) if cap < m else over
-            l0 = cnt.sum(dtype=torch.float32) * inv_m
-            cnt.bitwise_or_(in_tail.to(torch.int32).mul_(_INT_MIN).unsqueeze(1))
-            tail = _tail_index(in_tail, cap, m)
-        R = torch.empty_like(P)
-        T = torch.empty_like(P)
-        row_l1 = torch.empty(m, dtype=torch.float32, device=dev)
-        row_nnz = torch.empty(m, dtype=torch.int32, device=dev)
-        row_drop = torch.empty(m, dtype=torch.int32, device=dev)
-        with _Timer("sddmm_R_T"):
-            _lib.call("b200_hybrid_sddmm_fwd", dev, Xf.data_ptr(), K.data_ptr(), P.data_ptr(),
-                      R.data_ptr(), T.data_ptr(), row_l1.data_ptr(), row_nnz.data_ptr(),
-                      row_drop.data_ptr(), m, d, h, cf)
-        with _Timer("spmm_out"):
-            out = _spmm(T, V, m, d, h, cf, pad_rows=1 if tail is not None else 0)
-        l1 = row_l1.sum()
-        if tail is None:
-            l0 = row_nnz.sum(dtype=torch.float32) * inv_m
-        else:
-            with _Timer("dense_tail_forward"):
-                idx, valid, scatter = tail
-                Xt = Xf[idx] * valid.unsqueeze(1)
-                Pt = torch.relu(Xt @ G.t())
-                Tt = (Xt @ K.t()) * Pt
-                out.index_copy_(0, scatter, Tt @ V)
-                l1 = l1 + Tt.abs().sum(dtype=torch.float32)
-            out = out[:m]
-        l1 = l1 * inv_m
-        dropped = row_drop.sum(dtype=torch.int32)
+        scratch = _train_scratch(dev, m, d, h, cap, 0)
+        _lib.call("b200_hybrid_train_forward", dev, Xf.data_ptr(), G.data_ptr(), K.data_ptr(),
+                  V.data_ptr(), out.data_ptr(), P.data_ptr(), R.data_ptr(), T.data_ptr(),
+                  l0.data_ptr(), l1.data_ptr(), dropped.data_ptr(), n_over.data_ptr(), m, d, h, cf,
+                  cap, *_lib.workspace(dev), scratch.data_ptr(), scratch.numel())
+    if _CONFIG["tail_rows_adaptive"] and not _CONFIG["discard_overflow"] \
+            and _CONFIG["tail_rows_regular"] > 0:
+        _tail_observe(tail_key, n_over)
     return out.reshape(X.shape), l0, l1, P, R, T, dropped
+
+
+def _train_scratch(dev: torch.device, m: int, d: int, h: int, tail: int, bwd: int) -> torch.Tensor:
+    """Intermediate matrices of one call, from torch's allocator (never shared between calls)."""
+    need = int(_lib.load_library().b200_hybrid_train_scratch_bytes(m, d, h, tail, bwd))
+    return torch.empty(need, dtype=torch.uint8, device=dev)
 
 
 _CSC_SCRATCH: dict[tuple, dict[str, torch.Tensor]] = {}
@@ -350,17 +307,30 @@ def ff_backward_impl(X, G, K, V, P, R, T, gR, gl0, gl1):
     if gl1 is not None:
         gl1_dev = gl1.detach().to(device=dev, dtype=torch.float32).reshape(1).contiguous()
     # tail rows: flagged count words (sign bit) in P, set by the forward
-    tail = None
+    tail, cap = None, 0
     if m > 0 and not _CONFIG["discard_overflow"] and _CONFIG["tail_rows_regular"] > 0:
         cap = min(int(_CONFIG["tail_rows_regular"]), m)
-        if _CONFIG["tail_rows_adaptive"]:
-            st = _TAIL_SEEN.get((dev.index, G.data_ptr(), m, h))
-            if st is not None and st["cap_fwd"] is not None:
-                cap = min(cap, st["cap_fwd"])  # what the forward(s) since the last backward used
-                st["cap_fwd"] = None
-        if cap > 0:
-            flagged = (_count_view(P, m, h, cf) < 0).any(dim=1)
-            tail = _tail_index(flagged, cap, m)
+    if m > 0 and _CONFIG["weight_gradient_mode"] != "sparse":
+        dX = torch.empty_like(Xf)
+        dG, dK, dV = torch.empty_like(G), torch.empty_like(K), torch.empty_like(V)
+        with _Timer("ff_backward_gated_total"):
+            scratch = _train_scratch(dev, m, d, h, cap, 1)
+            _lib.call("b200_hybrid_train_backward", dev, Xf.data_ptr(), G.data_ptr(),
+                      K.data_ptr(), V.data_ptr(), P.data_ptr(), R.data_ptr(), gRf.data_ptr(),
+                      _lib.ptr(gl1_dev), dX.data_ptr(), dG.data_ptr(), dK.data_ptr(),
+                      dV.data_ptr(), m, d, h, cf, cap, *_lib.workspace(dev), scratch.data_ptr(),
+                      scratch.numel())
+        _LAST_TRANSPOSE_OVERFLOW = dev  # no column lists: nothing can overflow
+        return dX.reshape(X.shape), dG, dK, dV
+    # "sparse": gathers along the slabs and along column lists
+    if cap > 0 and _CONFIG["tail_rows_adaptive"]:
+        st = _TAIL_SEEN.get((dev.index, G.data_ptr(), m, h))
+        if st is not None and st["cap_fwd"] is not None:
+            cap = min(cap, st["cap_fwd"])  # what the forward(s) since the last backward used
+            st["cap_fwd"] = None
+    if cap > 0:
+        flagged = (_count_view(P, m, h, cf) < 0).any(dim=1)
+        tail = _tail_index(flagged, cap, m)
     pad = 1 if tail is not None else 0
     with _Timer("ff_backward_gated_total"):
         dR = torch.empty_like(P)
@@ -373,18 +343,7 @@ def ff_backward_impl(X, G, K, V, P, R, T, gR, gl0, gl1):
         dK = torch.empty((h, d), dtype=torch.bfloat16, device=dev)
         dG = torch.empty_like(dK)
         dV = torch.empty_like(dK)
-        if _dense_weight_gradients(m):
-            ws = _wgrad_workspace(dev, m, d, h)
-            with _Timer("wgrad_dense_dK_dG"):
-                _lib.call("b200_hybrid_wgrad_dense", dev, dR.data_ptr(), Xf.data_ptr(),
-                          dK.data_ptr(), m, d, h, cf, 0, ws.data_ptr(), ws.numel())
-                _lib.call("b200_hybrid_wgrad_dense", dev, dU.data_ptr(), Xf.data_ptr(),
-                          dG.data_ptr(), m, d, h, cf, 1, ws.data_ptr(), ws.numel())
-            with _Timer("wgrad_dense_dV"):
-                _lib.call("b200_hybrid_wgrad_dense", dev, T.data_ptr(), gRf.data_ptr(),
-                          dV.data_ptr(), m, d, h, cf, 0, ws.data_ptr(), ws.numel())
-            _LAST_TRANSPOSE_OVERFLOW = torch.zeros((), dtype=torch.int32, device=dev)
-        else:
+        if m > 0:
             sc = _csc_scratch(dev, m, h)
             overflow = torch.empty(1, dtype=torch.int32, device=dev)
             with _Timer("column_lists"):
@@ -400,6 +359,9 @@ def ff_backward_impl(X, G, K, V, P, R, T, gR, gl0, gl1):
                           sc["row"].data_ptr(), sc["pos"].data_ptr(), sc["cap"], gRf.data_ptr(),
                           dV.data_ptr(), None, h, d)
             _LAST_TRANSPOSE_OVERFLOW = overflow.reshape(())
+        else:
+            for t in (dK, dG, dV):
+                t.zero_()
         if tail is not None:
             # the flagged rows, dense (gate, up and the pattern recomputed from X)
             with _Timer("dense_tail_backward"):
@@ -476,10 +438,11 @@ def _autograd_backward(ctx, g_out, g_l0, g_l1, g_p, g_r, g_t):
     X, G, K, V, P, R, T = ctx.saved_tensors
     if g_out is None:
         g_out = torch.zeros_like(X)
-    zero = torch.zeros((), dtype=torch.float32, device=X.device)
+    if g_l1 is None:
+        g_l1 = torch.zeros((), dtype=torch.float32, device=X.device)
     dX, dG, dK, dV = torch.ops.sparse_ops.ff_backward_gated(
-        X, G, K, V, P, R, T, g_out.to(torch.bfloat16), zero if g_l0 is None else g_l0,
-        zero if g_l1 is None else g_l1)
+        X, G, K, V, P, R, T, g_out.to(torch.bfloat16), g_l1 if g_l0 is None else g_l0,  # ignored
+        g_l1)
     return dX, dG, dK, dV
 
 
@@ -535,6 +498,8 @@ def _set_knob(key: str, v: int) -> None:
 def _get_last_transpose_overflow() -> torch.Tensor:
     if _LAST_TRANSPOSE_OVERFLOW is None:
         raise RuntimeError("No backward pass has been run yet")
+    if isinstance(_LAST_TRANSPOSE_OVERFLOW, torch.device):
+        return torch.zeros((), dtype=torch.int32, device=_LAST_TRANSPOSE_OVERFLOW)
     return _LAST_TRANSPOSE_OVERFLOW
 
 
