@@ -525,14 +525,11 @@ extern "C" int b200_hybrid_train_forward(const void* x, const void* g, const voi
   a.row_words = tiles * W;
   a.row_slot = tail_rows > 0 ? w.row_slot : nullptr;
   a.tail_p = w.pt;
-  a.out = w.t;
-  a.ld = H;
-  a.wide = 1;
   a.l1_part = w.l1_part;
   a.part = w.part;
   a.counters = counters;
-  const pg::Operand ox = {x, M, D}, ok = {k, H, D};
-  if (int e = pg::launch<pg::kFwd, false, false>(fn, ox, ox, ok, ok, a, M, sm_count(), st)) return e;
+  const pg::Operand ox = {x, M, D}, ok = {k, H, D}, ot = {w.t, M, H};
+  if (int e = pg::launch<pg::kFwd, false, false>(fn, ox, ot, ok, ot, a, M, sm_count(), st)) return e;
   if (int e = pair_down(w.t, 1, v, out, M, D, H, {nullptr, 0u}, w.part, counters, st)) return e;
   l1_sum_kernel<<<1, 1024, 0, st>>>(w.l1_part, (int)((M + pg::kTile - 1) / pg::kTile) * tiles * 16,
                                     inv_m, l1);
@@ -577,17 +574,12 @@ extern "C" int b200_hybrid_train_backward(const void* x, const void* g, const vo
   a.row_slot = tail_rows > 0 ? w.row_slot : nullptr;
   a.tail_p = w.pt;
   a.tail_r = w.rt;
-  a.out = w.dru;
-  a.ld = 2 * H;
-  a.dense_t = w.t;
-  a.ld_t = H;
-  a.wide = 1;
   a.l1_grad = l1_grad;
   a.inv_m = 1.f / (float)M;
   a.part = w.part;
   a.counters = counters;
-  const pg::Operand og = {g_out, M, D}, ov = {v, H, D};
-  if (int e = pg::launch<pg::kBwd, false, false>(fn, og, og, ov, ov, a, M, sm_count(), st)) return e;
+  const pg::Operand og = {g_out, M, D}, ov = {v, H, D}, odu = {w.dru, M, 2 * H}, ot = {w.t, M, H};
+  if (int e = pg::launch<pg::kBwd, false, false>(fn, og, odu, ov, ot, a, M, sm_count(), st)) return e;
   // dX = [dR | dU] [K; G]
   pg::Args b = base_args(M, D, 2 * H);
   b.seg_ksteps = (int)(H / kStageK);

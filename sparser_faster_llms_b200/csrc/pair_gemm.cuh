@@ -42,7 +42,6 @@ constexpr int kTile = 256;                   // rows and columns per pair
 constexpr int kOperandBytes = 128 * 128;     // one CTA's half of A or B per 64-k stage
 constexpr int kStageBytes = 2 * kOperandBytes;
 constexpr int kBatch = 16;                   // slab rows whose words are in flight at a time
-constexpr int kBufBytes = 8 * 32 * 256;       // pattern buffers: 32 rows x 256 bytes per epilogue warp
 
 enum Epilogue {
   kStore = 0,    // out[row, col] = bf16(acc)
@@ -55,6 +54,12 @@ enum Epilogue {
   kFwd = 4,      // training forward: R = bf16(acc) and T = R * P as slabs, T dense, l1 partial sums
   kBwd = 5       // training backward: dense [dR | dU] and T from acc = dT
 };
+
+// Shared memory of the eight epilogue warps: 32 rows x 256 bytes of pattern each, or the blocks of
+// the training epilogues.
+__host__ __device__ constexpr int buf_bytes(int epi) {
+  return epi == kStore ? 0 : epi == kBwd ? 8 * 3 * 4096 : 8 * 32 * 256;
+}
 
 struct Args {
   int rows;                  // rows of the product (device count in rows_ptr when not null)
@@ -81,8 +86,6 @@ struct Args {
   const int* row_slot;
   const __nv_bfloat16* tail_p;
   const __nv_bfloat16* tail_r;
-  __nv_bfloat16* dense_t;    // kBwd: T, row stride ld_t
-  long long ld_t;
   float* l1_part;            // kFwd: [tiles][16] sums of |T|
   const float* l1_grad;      // kBwd: device scalar or null
   float inv_m;
@@ -256,59 +259,6 @@ __device__ __forceinline__ void load_values(const Args& a, unsigned char* buf, i
   __syncwarp();
 }
 
-// The same with P and R interleaved (u32 = P | R << 16) for columns [64 quarter, +64) of the tile.
-__device__ __forceinline__ void load_pairs(const Args& a, unsigned char* buf, int row0, int rows,
-                                           int nt, int quarter, int lane) {
-  __syncwarp();
-#pragma unroll
-  for (int i = 0; i < 16; ++i)
-    *reinterpret_cast<uint4*>(buf + lane * 256 + i * 16) = make_uint4(0u, 0u, 0u, 0u);
-  __syncwarp();
-  const size_t tile_off = (size_t)nt * a.slab_w;
-  for (int t0 = 0; t0 < 32; t0 += kBatch) {
-    if (row0 + t0 >= rows) break;
-    int cnt[kBatch], most = 0;
-    for (int w0 = 0; w0 < a.slab_w; w0 += 32) {
-      uint32_t w[kBatch], r[kBatch];
-#pragma unroll
-      for (int j = 0; j < kBatch; ++j) {
-        const int row = row0 + t0 + j;
-        const size_t off = (size_t)row * a.row_words + tile_off + w0 + lane;
-        w[j] = row < rows ? a.slab_p[off] : 0u;
-        r[j] = row < rows ? a.slab_r[off] : 0u;
-      }
-#pragma unroll
-      for (int j = 0; j < kBatch; ++j) {
-        if (w0 == 0) {
-          cnt[j] = min(max((int)__shfl_sync(0xffffffffu, w[j], 0), 0), a.slab_w - 1);
-          most = max(most, cnt[j]);
-        }
-        const int slot = w0 + lane, col = (int)(w[j] & 255u);
-        if (slot >= 1 && slot <= cnt[j] && (col >> 6) == quarter)
-          *reinterpret_cast<uint32_t*>(at(buf, t0 + j, (col & 63) * 4)) =
-              __byte_perm(w[j], r[j], 0x7632);
-      }
-      if (most < w0 + 32) break;
-    }
-  }
-  if (a.row_slot != nullptr) {
-    const int mine = row0 + lane < rows ? a.row_slot[row0 + lane] : -1;
-    uint32_t todo = __ballot_sync(0xffffffffu, mine >= 0);
-    __syncwarp();
-    while (todo != 0u) {
-      const int t = __ffs(todo) - 1;
-      todo &= todo - 1;
-      const int slot = __shfl_sync(0xffffffffu, mine, t);
-      const size_t off = (size_t)slot * a.n_tiles * kTile + nt * kTile + quarter * 64 + lane * 2;
-      const uint32_t p2 = *reinterpret_cast<const uint32_t*>(a.tail_p + off);
-      const uint32_t r2 = *reinterpret_cast<const uint32_t*>(a.tail_r + off);
-      *reinterpret_cast<uint2*>(at(buf, t, lane * 8)) =
-          make_uint2(__byte_perm(p2, r2, 0x5410), __byte_perm(p2, r2, 0x7632));
-    }
-  }
-  __syncwarp();
-}
-
 // The 32 sums of a lane's row in the 32 columns at `col` of the warp's block: from TMEM, or, for a
 // split tile, the ranges' sums added in order.
 struct Source {
@@ -336,6 +286,264 @@ __device__ __forceinline__ void fetch32(const Source& src, int cb, float (&v)[32
     }
 #pragma unroll
     for (int c = 0; c < 32; ++c) v[c] = (v[c] + u[c]) + w[c];
+  }
+}
+
+// ---- training epilogues: sums -> slab entries and zero-filled dense tiles -----------------------
+// Only 1 - 3 % of the sums are on the pattern, so the arithmetic runs per stored entry instead of
+// per column: a 64-column block of sums goes to shared memory as bf16, the lanes pick their
+// entries out of it, and the dense operands of the following products are zero-filled blocks with
+// the entries scattered in, written by TMA (128-byte rows, clipped at the last row).  What bounds
+// them is the dense writes and the MMAs of the next tile.  Against expanding the pattern to a dense
+// tile and computing every column (two warps per scheduler, some 5000 instructions per warp and
+// tile), 16384 tokens, D 1024, H 4096, 1 %: forward 229 -> 114 us, backward 317 -> 161 us (134 and
+// 403 MB written: 22 and 67 us at copy speed; the product alone 96 us).  The backward gives up one
+// of five operand stages for its third block per warp.
+
+constexpr int kBlockBytes = 32 * 128;        // 32 rows x 64 columns of bf16, 128-byte swizzle
+constexpr int kAhead = 16;                   // slab words per row that are fetched ahead
+
+// Byte of column `col` in row `row` of a block: the layout of SWIZZLE_128B.
+__device__ __forceinline__ unsigned char* blk(unsigned char* buf, int row, int col) {
+  return buf + row * 128 + ((((col >> 3) ^ row) & 7) << 4) + (col & 7) * 2;
+}
+__device__ __forceinline__ void zero_row(unsigned char* buf, int row) {
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+    *reinterpret_cast<uint4*>(buf + row * 128 + ((i ^ (row & 7)) << 4)) = make_uint4(0u, 0u, 0u, 0u);
+}
+__device__ __forceinline__ uint32_t lds16(const unsigned char* p) {
+  return *reinterpret_cast<const uint16_t*>(p);
+}
+__device__ __forceinline__ void sts16(unsigned char* p, uint32_t v) {
+  *reinterpret_cast<uint16_t*>(p) = (uint16_t)v;
+}
+__device__ __forceinline__ void tma_store(const CUtensorMap* map, const void* src, int c0, int c1) {
+  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];"
+               ::"l"(map), "r"(c0), "r"(c1), "r"(smem_u32(src))
+               : "memory");
+}
+__device__ __forceinline__ void tma_store_commit() {
+  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+__device__ __forceinline__ void tma_store_wait_read() {
+  asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+}
+__device__ __forceinline__ void tma_store_wait() {
+  asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+}
+
+// Slab words [w0, w0 + 16) of the warp's 32 rows: register pair g of a lane holds words
+// w0 + 2 (lane & 7) and the next of row 4 g + lane / 8, i.e. 64 contiguous bytes per row.
+__device__ __forceinline__ void load_words(const uint32_t* slab, const Args& a, int row0, int rows,
+                                           int nt, int w0, int lane, uint2 (&w)[8]) {
+  const size_t off = (size_t)nt * a.slab_w + w0 + (lane & 7) * 2;
+#pragma unroll
+  for (int g = 0; g < 8; ++g) {
+    const int row = row0 + g * 4 + (lane >> 3);
+    w[g] = row < rows ? *reinterpret_cast<const uint2*>(slab + (size_t)row * a.row_words + off)
+                      : make_uint2(0u, 0u);
+  }
+}
+
+// Stored entries per row (as load_words lays rows out) and the largest count of the 32 rows.
+// Counts with the sign bit set belong to rows taken out of the slabs: no entries.
+__device__ __forceinline__ int row_counts(const Args& a, const uint2 (&w)[8], int lane, int (&cnt)[8]) {
+  int most = 0;
+#pragma unroll
+  for (int g = 0; g < 8; ++g) {
+    cnt[g] = min(max((int)__shfl_sync(0xffffffffu, w[g].x, lane & 24), 0), a.slab_w - 1);
+    most = max(most, cnt[g]);
+  }
+  return __reduce_max_sync(0xffffffffu, most);
+}
+
+// dT of one column pair (or one column in the low half): the bf16 sum, shifted by the l1 gradient
+// times the sign of R.
+__device__ __forceinline__ uint32_t shifted2(uint32_t dt, uint32_t r2, float shift) {
+  if (shift == 0.f) return dt;
+  const float r0 = lo_f(r2), r1 = hi_f(r2);
+  const float s0 = r0 > 0.f ? shift : (r0 < 0.f ? -shift : 0.f);
+  const float s1 = r1 > 0.f ? shift : (r1 < 0.f ? -shift : 0.f);
+  return pack2(lo_f(dt) + s0, hi_f(dt) + s1);
+}
+
+// Sums of columns [64 hc, +64) of the warp's block as bf16 rows (lane = row).
+__device__ __forceinline__ void sums_to_block(const Source& src, int hc, unsigned char* buf, int lane) {
+#pragma unroll
+  for (int cb = 0; cb < 2; ++cb) {
+    float v[32];
+    fetch32(src, hc * 2 + cb, v);
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      *reinterpret_cast<uint4*>(buf + lane * 128 + (((cb * 4 + j) ^ (lane & 7)) << 4)) =
+          make_uint4(pack2(v[8 * j], v[8 * j + 1]), pack2(v[8 * j + 2], v[8 * j + 3]),
+                     pack2(v[8 * j + 4], v[8 * j + 5]), pack2(v[8 * j + 6], v[8 * j + 7]));
+  }
+}
+
+// Calls f(row, column in the 64-column block, slab offset, P word, R word) for this lane's stored
+// entries of block `quarter` of tile nt; pw / rw hold the first kAhead words of every row.
+template <bool WITH_R, typename F>
+__device__ __forceinline__ void for_entries(const Args& a, int row0, int rows, int nt, int quarter,
+                                            int lane, const uint2 (&pw)[8], const uint2 (&rw)[8],
+                                            const int (&cnt)[8], int most, F f) {
+  auto batch = [&](int w0, const uint2 (&p)[8], const uint2 (&r)[8]) {
+#pragma unroll
+    for (int g = 0; g < 8; ++g) {
+      const int row = g * 4 + (lane >> 3), slot = w0 + (lane & 7) * 2;
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const uint32_t w = e == 0 ? p[g].x : p[g].y;
+        if (slot + e >= 1 && slot + e <= cnt[g] && ((int)(w & 255u) >> 6) == quarter)
+          f(row, (int)(w & 63u),
+            (size_t)(row0 + row) * a.row_words + (size_t)nt * a.slab_w + slot + e, w,
+            WITH_R ? (e == 0 ? r[g].x : r[g].y) : 0u);
+      }
+    }
+  };
+  batch(0, pw, rw);
+#pragma unroll 1
+  for (int w0 = kAhead; w0 <= most; w0 += kAhead) {
+    uint2 p[8], r[8];
+    load_words(a.slab_p, a, row0, rows, nt, w0, lane, p);
+    if (WITH_R) load_words(a.slab_r, a, row0, rows, nt, w0, lane, r);
+    batch(w0, p, r);
+  }
+}
+
+// Calls f(row, offset of this lane's two columns in the rows of tail_p / tail_r, their place in the
+// block) for every row of the warp that is out of the slabs; all lanes take part.
+template <typename F>
+__device__ __forceinline__ void for_tail_rows(const Args& a, int slot, int nt, int quarter, int lane,
+                                              F f) {
+  uint32_t todo = __ballot_sync(0xffffffffu, slot >= 0);
+  while (todo != 0u) {
+    const int t = __ffs(todo) - 1;
+    todo &= todo - 1;
+    const int s = __shfl_sync(0xffffffffu, slot, t);
+    f(t, (size_t)s * a.n_tiles * kTile + nt * kTile + quarter * 64 + lane * 2, lane * 2);
+  }
+}
+
+// Training forward: R and T in the slots of P, T as a dense matrix, this lane's part of sum |T|.
+// buf: two blocks.  release() is called once the accumulator has been read.
+template <typename Release>
+__device__ __forceinline__ float forward_tile(const Args& a, const CUtensorMap* map_t, const Source& src,
+                                              unsigned char* buf, int row0, int rows, int nt, int half,
+                                              int lane, const uint2 (&pw)[8], int tail_slot,
+                                              Release release) {
+  int cnt[8];
+  const int most = row_counts(a, pw, lane, cnt);
+  unsigned char *bx = buf, *bt = buf + kBlockBytes;
+  float l1 = 0.f;
+  if (half == 0 && (lane & 7) == 0) {
+#pragma unroll
+    for (int g = 0; g < 8; ++g) {
+      const int row = row0 + g * 4 + (lane >> 3);
+      if (row >= rows) continue;
+      const size_t off = (size_t)row * a.row_words + (size_t)nt * a.slab_w;
+      a.slab_r[off] = pw[g].x;
+      a.slab_t[off] = pw[g].x;
+    }
+  }
+#pragma unroll 1
+  for (int hc = 0; hc < 2; ++hc) {
+    const int quarter = 2 * half + hc;
+    if (lane == 0) tma_store_wait_read();
+    __syncwarp();
+    sums_to_block(src, hc, bx, lane);
+    zero_row(bt, lane);
+    if (hc == 1) release();
+    __syncwarp();
+    for_entries<false>(a, row0, rows, nt, quarter, lane, pw, pw, cnt, most,
+                       [&](int row, int col, size_t off, uint32_t p, uint32_t) {
+                         const uint32_t m = nonzero2(p >> 16);
+                         const uint32_t r = lds16(blk(bx, row, col)) & m;
+                         const uint32_t t = mul2(p >> 16, r) & m;
+                         l1 += fabsf(lo_f(t));
+                         sts16(blk(bt, row, col), t);
+                         a.slab_r[off] = (p & 0xFFFFu) | (r << 16);
+                         a.slab_t[off] = (p & 0xFFFFu) | (t << 16);
+                       });
+    for_tail_rows(a, tail_slot, nt, quarter, lane, [&](int row, size_t off, int col) {
+      const uint32_t p2 = *reinterpret_cast<const uint32_t*>(a.tail_p + off), m = nonzero2(p2);
+      const uint32_t r2 = *reinterpret_cast<const uint32_t*>(blk(bx, row, col)) & m;
+      const uint32_t t2 = mul2(p2, r2) & m;
+      l1 += fabsf(lo_f(t2));
+      l1 += fabsf(hi_f(t2));
+      *reinterpret_cast<uint32_t*>(blk(bt, row, col)) = t2;
+    });
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncwarp();
+    if (lane == 0 && row0 < rows) {
+      tma_store(map_t, bt, nt * kTile + quarter * 64, row0);
+      tma_store_commit();
+    }
+  }
+  return l1;
+}
+
+// Training backward: dense [dR | dU] and T from dT.  buf: three blocks; the one that held dT is
+// used again for T.
+template <typename Release>
+__device__ __forceinline__ void backward_tile(const Args& a, const CUtensorMap* map_dru,
+                                              const CUtensorMap* map_t, const Source& src,
+                                              unsigned char* buf, int row0, int rows, int nt, int half,
+                                              int lane, const uint2 (&pw)[8], const uint2 (&rw)[8],
+                                              int tail_slot, float shift, Release release) {
+  int cnt[8];
+  const int most = row_counts(a, pw, lane, cnt);
+  unsigned char *bx = buf, *br = buf + kBlockBytes, *bu = buf + 2 * kBlockBytes;
+#pragma unroll 1
+  for (int hc = 0; hc < 2; ++hc) {
+    const int quarter = 2 * half + hc;
+    if (lane == 0) tma_store_wait_read();
+    __syncwarp();
+    sums_to_block(src, hc, bx, lane);
+    zero_row(br, lane);
+    zero_row(bu, lane);
+    if (hc == 1) release();
+    __syncwarp();
+    for_entries<true>(a, row0, rows, nt, quarter, lane, pw, rw, cnt, most,
+                      [&](int row, int col, size_t, uint32_t p, uint32_t r) {
+                        p >>= 16;
+                        r >>= 16;
+                        const uint32_t m = nonzero2(p);
+                        const uint32_t dt = shifted2(lds16(blk(bx, row, col)), r, shift) & m;
+                        sts16(blk(br, row, col), mul2(dt, p) & m);
+                        sts16(blk(bu, row, col), mul2(dt, r) & m);
+                      });
+    for_tail_rows(a, tail_slot, nt, quarter, lane, [&](int row, size_t off, int col) {
+      const uint32_t p2 = *reinterpret_cast<const uint32_t*>(a.tail_p + off), m = nonzero2(p2);
+      const uint32_t r2 = *reinterpret_cast<const uint32_t*>(a.tail_r + off);
+      const uint32_t dt =
+          shifted2(*reinterpret_cast<const uint32_t*>(blk(bx, row, col)), r2, shift) & m;
+      *reinterpret_cast<uint32_t*>(blk(br, row, col)) = mul2(dt, p2) & m;
+      *reinterpret_cast<uint32_t*>(blk(bu, row, col)) = mul2(dt, r2) & m;
+    });
+    __syncwarp();
+    zero_row(bx, lane);
+    __syncwarp();
+    for_entries<true>(a, row0, rows, nt, quarter, lane, pw, rw, cnt, most,
+                      [&](int row, int col, size_t, uint32_t p, uint32_t r) {
+                        p >>= 16;
+                        sts16(blk(bx, row, col), mul2(r >> 16, p) & nonzero2(p));
+                      });
+    for_tail_rows(a, tail_slot, nt, quarter, lane, [&](int row, size_t off, int col) {
+      const uint32_t p2 = *reinterpret_cast<const uint32_t*>(a.tail_p + off);
+      const uint32_t r2 = *reinterpret_cast<const uint32_t*>(a.tail_r + off);
+      *reinterpret_cast<uint32_t*>(blk(bx, row, col)) = mul2(r2, p2) & nonzero2(p2);
+    });
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncwarp();
+    if (lane == 0 && row0 < rows) {
+      const int c = nt * kTile + quarter * 64;
+      tma_store(map_dru, br, c, row0);
+      tma_store(map_dru, bu, a.n_tiles * kTile + c, row0);
+      tma_store(map_t, bx, c, row0);
+      tma_store_commit();
+    }
   }
 }
 
@@ -370,6 +578,8 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap map_a0,
   constexpr uint32_t kIdesc = umma_idesc(256, 256) | (A_MN ? 1u << 15 : 0u) | (B_MN ? 1u << 16 : 0u);
   constexpr bool kGate2 = EPI == kGateUp || EPI == kGateUpHp;
   constexpr bool kIsPack = EPI == kPack || EPI == kPackDense || kGate2;
+  constexpr bool kTrain = EPI == kFwd || EPI == kBwd;
+  constexpr int kBufBytes = buf_bytes(EPI) / 8;  // of one epilogue warp
   constexpr int kPhases = kGate2 ? 2 : 1;  // accumulators per item
 
   // Without a device-side choice or row count the set-up below runs while the predecessor drains.
@@ -523,7 +733,8 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap map_a0,
   } else {
     // ---- epilogue: warp = (lane quarter, column half) ----
     const int q = warp & 3, half = (warp - 2) >> 2;
-    unsigned char* buf = smem + (size_t)STAGES * kStageBytes + (size_t)(warp - 2) * 32 * 256;
+    unsigned char* buf =
+        smem + (size_t)STAGES * kStageBytes + (size_t)(warp - 2) * kBufBytes;
     const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(half * 128);
     float shift = 0.f;
     if (EPI == kBwd && a.l1_grad != nullptr) shift = __ldg(a.l1_grad) * a.inv_m;
@@ -560,10 +771,15 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap map_a0,
         const int o = mt / a.out_mt;
         out = a.out_more[o - 1] + (size_t)(row - o * a.out_mt * kTile) * a.ld + nt * kTile + half * 128;
       }
+      uint2 pw[kTrain ? 8 : 1], rw[EPI == kBwd ? 8 : 1];  // the rows' first slab words
+      int tail_slot = -1;
       auto load_pattern = [&]() {
-        if (EPI == kMul || EPI == kMulHp || EPI == kFwd)
-          load_values(a, buf, row0, rows, nt, half, lane);
-        if (EPI == kBwd) load_pairs(a, buf, row0, rows, nt, 2 * half, lane);
+        if constexpr (EPI == kMul || EPI == kMulHp) load_values(a, buf, row0, rows, nt, half, lane);
+        if constexpr (kTrain) {
+          load_words(a.slab_p, a, row0, rows, nt, 0, lane, pw);
+          if (a.row_slot != nullptr && live) tail_slot = a.row_slot[row];
+        }
+        if constexpr (EPI == kBwd) load_words(a.slab_r, a, row0, rows, nt, 0, lane, rw);
       };
       // the pattern is fetched under the MMAs of this tile (a split tile's only by the warp that
       // finishes it)
@@ -715,11 +931,23 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap map_a0,
         src = Source{lane_addr + (uint32_t)((i & 1) * 256), nullptr, 1};
       }
 
-      if (!kIsPack || kGate2) {
-        float l1 = 0.f;
+      if constexpr (kTrain) {
+        auto done = [&]() {
+          if (src.part == nullptr) release();
+        };
+        if constexpr (EPI == kFwd) {
+          float l1 = forward_tile(a, &map_a1, src, buf, row0, rows, nt, half, lane, pw, tail_slot, done);
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) l1 += __shfl_xor_sync(0xffffffffu, l1, o);
+          if (lane == 0)  // one sum of |T| per warp and tile
+            a.l1_part[((size_t)im.tile * 2 + crank) * 8 + q * 2 + half] = l1;
+        } else {
+          backward_tile(a, &map_a1, &map_b1, src, buf, row0, rows, nt, half, lane, pw, rw, tail_slot,
+                        shift, done);
+        }
+      } else if (!kIsPack || kGate2) {
 #pragma unroll 1
         for (int cb = 0; cb < 4; ++cb) {
-          if (EPI == kBwd && cb == 2) load_pairs(a, buf, row0, rows, nt, 2 * half + 1, lane);
           float v[32];
           fetch32(src, cb, v);
           if (EPI == kStore) {
@@ -729,26 +957,18 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap map_a0,
               w[p] = a.relu ? pack2(fmaxf(v[2 * p], 0.f), fmaxf(v[2 * p + 1], 0.f))
                             : pack2(v[2 * p], v[2 * p + 1]);
             if (live) store64(out + cb * 32, w, a.wide);
-          } else if (EPI == kMul || EPI == kGateUp || EPI == kFwd) {
+          } else if (EPI == kMul || EPI == kGateUp) {
             uint32_t w[16];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-              uint4* gp = reinterpret_cast<uint4*>(at(buf, lane, cb * 64 + j * 16));
-              const uint4 g4 = *gp;
+              const uint4 g4 = *reinterpret_cast<const uint4*>(at(buf, lane, cb * 64 + j * 16));
               const uint32_t g[4] = {g4.x, g4.y, g4.z, g4.w};
-              uint32_t r[4];
 #pragma unroll
               for (int p = 0; p < 4; ++p) {
                 const int c = 8 * j + 2 * p;
-                const uint32_t m = nonzero2(g[p]);
-                r[p] = pack2(v[c], v[c + 1]) & m;      // never touch u where nothing is stored
-                w[4 * j + p] = mul2(g[p], r[p]) & m;
-                if (EPI == kFwd && live) {
-                  l1 += fabsf(lo_f(w[4 * j + p]));
-                  l1 += fabsf(hi_f(w[4 * j + p]));
-                }
+                const uint32_t m = nonzero2(g[p]);     // never touch u where nothing is stored
+                w[4 * j + p] = mul2(g[p], pack2(v[c], v[c + 1]) & m) & m;
               }
-              if (EPI == kFwd) *gp = make_uint4(r[0], r[1], r[2], r[3]);
             }
             if (live) store64(out + cb * 32, w, a.wide);
           } else if (EPI == kMulHp || EPI == kGateUpHp) {
@@ -764,85 +984,13 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap map_a0,
               store64(out + h + cb * 32, w1, a.wide);
               store64(out + 2 * h + cb * 32, w2, a.wide);
             }
-          } else if (EPI == kBwd) {
-            uint32_t dr[16], du[16], tt[16];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              const uint4 g4 =
-                  *reinterpret_cast<const uint4*>(at(buf, lane, (cb & 1) * 128 + j * 16));
-#pragma unroll
-              for (int p = 0; p < 2; ++p) {
-                const uint32_t x0 = p == 0 ? g4.x : g4.z, x1 = p == 0 ? g4.y : g4.w;
-                const int c = 4 * j + 2 * p, o = 2 * j + p;
-                const uint32_t p2 = __byte_perm(x0, x1, 0x5410), r2 = __byte_perm(x0, x1, 0x7632);
-                const uint32_t m = nonzero2(p2);
-                uint32_t dt = pack2(v[c], v[c + 1]);
-                if (shift != 0.f) {
-                  const float r0 = lo_f(r2), r1 = hi_f(r2);
-                  const float s0 = r0 > 0.f ? shift : (r0 < 0.f ? -shift : 0.f);
-                  const float s1 = r1 > 0.f ? shift : (r1 < 0.f ? -shift : 0.f);
-                  dt = pack2(lo_f(dt) + s0, hi_f(dt) + s1);
-                }
-                dt &= m;
-                dr[o] = mul2(dt, p2) & m;
-                du[o] = mul2(dt, r2) & m;
-                tt[o] = mul2(r2, p2) & m;
-              }
-            }
-            if (live) {
-              store64(out + cb * 32, dr, a.wide);
-              store64(out + (size_t)a.n_tiles * kTile + cb * 32, du, a.wide);
-              store64(a.dense_t + (size_t)row * a.ld_t + nt * kTile + half * 128 + cb * 32, tt, a.wide);
-            }
           }
-        }
-        if (EPI == kFwd) {  // one sum of |T| per warp and tile
-#pragma unroll
-          for (int o = 16; o > 0; o >>= 1) l1 += __shfl_xor_sync(0xffffffffu, l1, o);
-          if (lane == 0) a.l1_part[((size_t)im.tile * 2 + crank) * 8 + q * 2 + half] = l1;
         }
         if (src.part == nullptr) release();
         __syncwarp();
       }
-      if (EPI == kFwd) {
-        // R and T in the slots of P, from the R values left in the pattern buffer
-        const size_t tile_off = (size_t)nt * a.slab_w;
-        for (int t0 = 0; t0 < 32; t0 += kBatch) {
-          if (row0 + t0 >= rows) break;
-          int cnt[kBatch], most = 0;
-          for (int w0 = 0; w0 < a.slab_w; w0 += 32) {
-            uint32_t w[kBatch];
-#pragma unroll
-            for (int j = 0; j < kBatch; ++j) {
-              const int r = row0 + t0 + j;
-              w[j] = r < rows ? a.slab_p[(size_t)r * a.row_words + tile_off + w0 + lane] : 0u;
-            }
-#pragma unroll
-            for (int j = 0; j < kBatch; ++j) {
-              const int r = row0 + t0 + j;
-              const size_t off = (size_t)r * a.row_words + tile_off + w0 + lane;
-              if (w0 == 0) {
-                cnt[j] = min(max((int)__shfl_sync(0xffffffffu, w[j], 0), 0), a.slab_w - 1);
-                most = max(most, cnt[j]);
-                if (lane == 0 && half == 0 && r < rows) {
-                  a.slab_r[off] = w[j];
-                  a.slab_t[off] = w[j];
-                }
-              }
-              const int slot = w0 + lane, col = (int)(w[j] & 255u);
-              if (slot >= 1 && slot <= cnt[j] && (col >> 7) == half) {
-                const uint32_t rb =
-                    *reinterpret_cast<const uint16_t*>(at(buf, t0 + j, (col & 127) * 2));
-                a.slab_r[off] = (w[j] & 0xFFFFu) | (rb << 16);
-                a.slab_t[off] = (w[j] & 0xFFFFu) | (mul2(rb, w[j] >> 16) << 16);
-              }
-            }
-            if (most < w0 + 32) break;
-          }
-        }
-        __syncwarp();
-      }
     }
+    if (kTrain && lane == 0) tma_store_wait();
   }
 
   __syncwarp();
@@ -916,14 +1064,19 @@ inline size_t part_bytes(int64_t tiles, int ksteps, int64_t slots, bool all) {
 template <int EPI, bool A_MN, bool B_MN>
 int launch(const char* fn, const Operand& a0, const Operand& a1, const Operand& b0,
            const Operand& b1, Args args, int64_t row_capacity, int sm_count, cudaStream_t stream) {
-  constexpr bool kBuf = EPI != kStore;
-  constexpr int STAGES = kBuf ? 5 : 6;
-  constexpr size_t smem = (size_t)STAGES * kStageBytes + (kBuf ? kBufBytes : 0) + 1024;
+  constexpr bool kTrain = EPI == kFwd || EPI == kBwd;
+  constexpr int STAGES = EPI == kStore ? 6 : EPI == kBwd ? 4 : 5;
+  constexpr size_t smem = (size_t)STAGES * kStageBytes + buf_bytes(EPI) + 1024;
   CUtensorMap ma0, ma1, mb0, mb1;
   if (int rc = operand_map(&ma0, a0, A_MN)) return rc;
-  if (int rc = operand_map(&ma1, a1, A_MN)) return rc;
   if (int rc = operand_map(&mb0, b0, B_MN)) return rc;
-  if (int rc = operand_map(&mb1, b1, B_MN)) return rc;
+  if (kTrain) {  // a1, b1: the dense results, stored in blocks of 32 rows
+    if (int rc = make_map(&ma1, a1.base, a1.rows, a1.k, 32)) return rc;
+    if (int rc = make_map(&mb1, b1.base, b1.rows, b1.k, 32)) return rc;
+  } else {
+    if (int rc = operand_map(&ma1, a1, A_MN)) return rc;
+    if (int rc = operand_map(&mb1, b1, B_MN)) return rc;
+  }
   auto kern = pair_gemm_kernel<EPI, A_MN, B_MN, STAGES>;
   static size_t granted[64] = {0};
   if (int rc = ensure_dynamic_smem(kern, smem, granted, fn)) return rc;

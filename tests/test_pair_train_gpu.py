@@ -100,3 +100,10 @@ def test_overflowed_rows_within_and_beyond_the_tail(m):
     assert taken == 5 and left == (m + 8) // 9 - 5
     taken, left = run_case(m, 512, 2048, 0.03, hot=9, tail=0)
     assert taken == 0 and left == (m + 8) // 9
+
+
+@pytest.mark.parametrize("width,density", [(64, 0.1), (128, 0.2), (512, 0.05), (512, 0.35)])
+def test_entry_counts_around_the_words_fetched_ahead(width, density):
+    """Means of 26 / 51 / 13 / 90 entries per 256-neuron tile: more than the 16 slab words that
+    are fetched ahead, a few of them only, and (first two) full slabs with overflowed rows."""
+    run_case(97, 256, 768, density, width=width)
