@@ -15,6 +15,7 @@ from __future__ import annotations
 import torch
 
 from . import _lib
+from .twell import _BaseTwELLMLP
 
 
 class GraphedFFNStack:
@@ -47,37 +48,67 @@ class GraphedFFNStack:
         self.y_host = torch.zeros(out_shape, dtype=torch.bfloat16).pin_memory()
         self.stream = torch.cuda.Stream(dev)
         self.copy_stream = torch.cuda.Stream(dev)
+        self.result_stream = torch.cuda.Stream(dev)
         self.copy_chunk = max(1, int(copy_chunk))
         self.graph: torch.cuda.CUDAGraph | None = None
         self._capture()
+
+    def _chunks(self, single: int) -> list[tuple[int, int]]:
+        """Layer ranges of the transfers, ``copy_chunk`` layers each, counted from the layer
+        ``single`` (the first or the last), which is a range of its own."""
+        n, c = self.layers, self.copy_chunk
+        cuts = range(1, n, c) if single == 0 else range(n - 1, 0, -c)
+        bounds = sorted({0, n, *cuts})
+        return list(zip(bounds[:-1], bounds[1:]))
+
+    @staticmethod
+    def _writes_into(mlp) -> bool:
+        """Whether the module can be given the tensor it writes: this package's own forward, not
+        in place, with nothing hooked to it."""
+        return (isinstance(mlp, _BaseTwELLMLP) and type(mlp).forward is _BaseTwELLMLP.forward
+                and "forward" not in vars(mlp) and not mlp.inplace
+                and not (mlp._forward_hooks or mlp._forward_pre_hooks))
 
     def _body(self) -> None:
         # The host -> device copies run on a second stream in chunks of a few layers, each
         # chunk followed by an event the compute stream waits on: layer l starts as soon as
         # its own input has arrived, and the rest of the transfer hides under the kernels.
         # The first chunk is a single layer, so the compute stream starts after one small copy.
+        # The results leave the same way on a third stream, the last layer by itself: what is
+        # left after the last kernel is one layer's copy instead of all of them (28 layers of
+        # 32 x 2048: 69 us).  A layer writes its row of y_dev itself; a copy per layer between
+        # the kernels costs its launch and, worse, the overlap of the next kernel's start.
         main = torch.cuda.current_stream(self.device)
         self.copy_stream.wait_stream(main)
-        bounds = [0, 1] + list(range(1 + self.copy_chunk, self.layers, self.copy_chunk))
-        bounds = [b for b in bounds if b < self.layers] + [self.layers]
         ready = {}
         with torch.cuda.stream(self.copy_stream):
-            for l0, l1 in zip(bounds[:-1], bounds[1:]):
+            for l0, l1 in self._chunks(0):
                 self.x_dev[l0:l1].copy_(self.x_host[l0:l1], non_blocking=True)
                 ev = torch.cuda.Event()
                 ev.record(self.copy_stream)
                 ready[l0] = ev
+        done = {} if self.return_last_only else {l1: l0 for l0, l1 in self._chunks(-1)}
         for l, mlp in enumerate(self.mlps):
             if l in ready:
                 main.wait_event(ready[l])
-            y = mlp(self.x_dev[l])
-            # only what is returned is gathered: with return_last_only the last layer's
-            # output goes to the host straight from the module's own tensor
-            if not self.return_last_only and y.data_ptr() != self.y_dev[l].data_ptr():
-                self.y_dev[l].copy_(y)
+            if not self.return_last_only and self._writes_into(mlp):
+                mlp._forward_into(self.x_dev[l], self.y_dev[l])
+            else:
+                y = mlp(self.x_dev[l])
+                # only what is returned is gathered: with return_last_only the last layer's
+                # output goes to the host straight from the module's own tensor
+                if not self.return_last_only and y.data_ptr() != self.y_dev[l].data_ptr():
+                    self.y_dev[l].copy_(y)
+            if l + 1 in done:
+                self.result_stream.wait_stream(main)
+                with torch.cuda.stream(self.result_stream):
+                    self.y_host[done[l + 1]:l + 1].copy_(self.y_dev[done[l + 1]:l + 1],
+                                                         non_blocking=True)
         main.wait_stream(self.copy_stream)
-        src = y.view(self.batch, self.d_model) if self.return_last_only else self.y_dev
-        self.y_host.copy_(src, non_blocking=True)
+        if self.return_last_only:
+            self.y_host.copy_(y.view(self.batch, self.d_model), non_blocking=True)
+        else:
+            main.wait_stream(self.result_stream)
 
     def _capture(self) -> None:
         with torch.cuda.device(self.device):

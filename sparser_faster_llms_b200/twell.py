@@ -851,6 +851,9 @@ class _BaseTwELLMLP(nn.Module):
     def _call_args(self) -> tuple[tuple, dict]:
         raise NotImplementedError
 
+    def _native(self, rows: torch.Tensor, packed: torch.Tensor, out: torch.Tensor) -> None:
+        raise NotImplementedError
+
     def _apply_dense_route(self) -> None:  # gated modules override
         pass
 
@@ -885,6 +888,15 @@ class _BaseTwELLMLP(nn.Module):
         out = self._entry[(shared, self.inplace)](self.layer_number, rows, *args, ext=self.ext,
                                                   **kwargs)
         return A if self.inplace else out.view(shape)
+
+    def _forward_into(self, A: torch.Tensor, out: torch.Tensor) -> None:
+        """The forward with its result in ``out`` (contiguous, the shape of ``A``)."""
+        rows = A.view(-1, A.shape[-1])
+        self._ensure_layer()
+        packed = (self.layer.prepare_shared_hidden_state(rows)
+                  if self.preallocate_shared_hidden_state
+                  else _temp_packed(self.layer_number, rows))
+        self._native(rows, packed, out.view(rows.shape))
 
     def destroy(self) -> None:
         if self.layer is not None:
@@ -924,6 +936,9 @@ class TwELLMLP(_BaseTwELLMLP):
     def _call_args(self):
         return (self.DOWN,), {"num_splits": self.num_splits}
 
+    def _native(self, rows, packed, out):
+        _plain_mlp(self.layer_number, rows, self.DOWN, packed, out, self.num_splits)
+
 
 class TwELLGatedMLP(_BaseTwELLMLP):
     """Fused gated TwELL MLP wrapper."""
@@ -954,6 +969,10 @@ class TwELLGatedMLP(_BaseTwELLMLP):
         return (self.UP, self.DOWN), {"highest_precision": self.highest_precision,
                                       "compression_factor": self.compression_factor,
                                       "flex_kernels": self.flex_kernels}
+
+    def _native(self, rows, packed, out):
+        _gated_mlp(self.layer_number, rows, self.UP, self.DOWN, packed, out,
+                   self.highest_precision, self.compression_factor)
 
     def enable_dense_route(self, dense_cap: int | None = None, nnz_threshold: int | None = None,
                            min_tokens: int = 256, dense_all_tokens: int | None = None) -> None:

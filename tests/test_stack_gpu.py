@@ -31,3 +31,24 @@ def test_graphed_stack_matches_eager_modules_and_dense_reference():
         runner.run(torch.zeros(L, B + 1, d, dtype=torch.bfloat16))
     for m in mods:
         m.destroy()
+
+
+@pytest.mark.parametrize("layers,chunk", [(1, 4), (2, 1), (5, 4), (6, 4), (9, 3)])
+def test_results_leave_in_chunks(layers, chunk):
+    """Every layer's row of the result, whatever the cut of the transfers; in-place and hooked
+    modules, which do not write into the result tensor, between the others."""
+    B, d, h = 2, 256, 512
+    ffn = [synthetic.make_ffn(d, h, seed=160 + l, density=0.05, skew_sigma=0.0) for l in range(layers)]
+    mods = [twell.TwELLGatedMLP(520 + l, f.gate.to(DEV), f.up.to(DEV), f.down.to(DEV), inplace=l == 1)
+            for l, f in enumerate(ffn)]
+    if layers > 3:
+        mods[3].register_forward_hook(lambda mod, args, out: out * 2)
+    runner = stack.GraphedFFNStack(mods, B, copy_chunk=chunk)
+    assert [b for r in runner._chunks(-1) for b in range(*r)] == list(range(layers))
+    for seed in (1, 2):
+        x = torch.stack([synthetic.make_tokens(B, d, seed=seed * 10 + l) for l in range(layers)])
+        y = runner.run(x).clone()
+        for l in range(layers):
+            assert torch.equal(mods[l](x[l].to(DEV)).cpu(), y[l])
+    for m in mods:
+        m.destroy()
