@@ -54,12 +54,19 @@ class GraphedFFNStack:
         self._capture()
 
     def _chunks(self, single: int) -> list[tuple[int, int]]:
-        """Layer ranges of the transfers, ``copy_chunk`` layers each, counted from the layer
-        ``single`` (the first or the last), which is a range of its own."""
-        n, c = self.layers, self.copy_chunk
-        cuts = range(1, n, c) if single == 0 else range(n - 1, 0, -c)
-        bounds = sorted({0, n, *cuts})
-        return list(zip(bounds[:-1], bounds[1:]))
+        """Layer ranges of the transfers, counted from the layer ``single`` (the first or the
+        last), which is a range of its own.  A range that starts a kernel late costs it some
+        3 us (measured at one token: its launch is no longer prepared under its predecessor),
+        so small layers go in few ranges: about 1 MB (some 20 us of transfer, the time of one
+        or two layers), then the rest.  Layers of more than 256 KB go ``copy_chunk`` at a time."""
+        n, layer_bytes = self.layers, 2 * self.batch * self.d_model
+        if layer_bytes > 256 << 10:
+            cuts = range(1, n, self.copy_chunk)
+        else:
+            cuts = (1, 1 + max(self.copy_chunk, (1 << 20) // max(layer_bytes, 1)))
+        bounds = sorted({0, n, *(min(c, n) for c in cuts)})
+        ranges = list(zip(bounds[:-1], bounds[1:]))
+        return ranges if single == 0 else [(n - b, n - a) for a, b in reversed(ranges)]
 
     @staticmethod
     def _writes_into(mlp) -> bool:
