@@ -61,13 +61,27 @@ inline int ensure_dynamic_smem(Kernel kern, size_t bytes, size_t (&granted)[64],
 // driver while its predecessor in the stream still runs; it must execute pdl_wait() before
 // its first global read of data the predecessor may write and before its first global write
 // (the wait returns once the predecessor grid has completed and its memory is visible).
-// No kernel here issues griddepcontrol.launch_dependents: with an explicit early trigger the
-// successor's CTAs become resident under the predecessor's tail and take shared memory and L1
-// from it (measured on B200, decode stack at batch 32: 0.79-0.83 ms per step against 0.70
-// without the attribute), whereas the implicit trigger at grid exit only removes the launch
-// latency between the two kernels (0.677 ms).  pdl_wait() is a no-op in a kernel launched
-// without the attribute.
+// pdl_wait() is a no-op in a kernel launched without the attribute.
+//
+// The contraction and the one-token layer kernel also issue pdl_trigger(): their successor's CTAs
+// become resident as their own CTAs leave, and use the time until pdl_wait() returns to set up
+// and to ask L2 for the first part of their weights (a quarter: asking for all of it, or from
+// inside the predecessor, fetches rows that are gone from L2 again when they are read).  Neither
+// alone gains much; together, 28 layers of D 2048, H 8192: one token 370 -> 342 us, 32 tokens
+// 757 -> 700 us.  The pack kernels do not: a contraction that is resident early has nothing to
+// fetch and takes shared memory and L1 from them (832 us at 32 tokens).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Lets the next kernel of the stream (launched with the attribute) become resident as this one's CTAs
+// leave; its pdl_wait() still waits for all of them.
+__device__ __forceinline__ void pdl_trigger() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// Asks L2 for a range (a multiple of 16 bytes).  Changes no value, so it may stand before pdl_wait().
+__device__ __forceinline__ void l2_prefetch(const void* p, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
 
 // Whether the decode kernels are launched with programmatic stream serialisation
 // (environment variable B200_PDL: "0" switches it off, anything else or unset keeps the

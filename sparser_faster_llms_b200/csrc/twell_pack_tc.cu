@@ -307,6 +307,9 @@ twell_pack_tc_splitk_wide_kernel(const __grid_constant__ CUtensorMap tmap_w,
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = tmem_slot;
+  if (threadIdx.x == 0)  // two of the eight k-steps at D 2048: one is slower (724 us), three level
+    for (int k = 0; k < 2 && k < ksteps; ++k)
+      tma_prefetch_2d(&tmap_w, k_base + k * kStageK, tile * kTileN);
   pdl_wait();
 
   if (warp == 0) {

@@ -213,6 +213,7 @@ twell_t2d_kernel(const __nv_bfloat16* x, const uint32_t* __restrict__ packed,
   for (int e = 0; e < 8; ++e) acc[e] = 0.f;
   int buf = 0;
 
+  pdl_trigger();
   const __nv_bfloat16* up_lane = up + warp * 256 + lane * 8;
   const __nv_bfloat16* down_lane = down + warp * 256 + lane * 8;
   const __nv_bfloat162* x2 = reinterpret_cast<const __nv_bfloat162*>(&xv);
