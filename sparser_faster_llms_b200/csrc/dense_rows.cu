@@ -876,10 +876,19 @@ struct DenseWs {
   __nv_bfloat16* hd;     // [cap_pad, H]
   __nv_bfloat16* h_all;  // [M, H]: every row's hidden values (the form of b200_twell_gated_mlp_hybrid
   float* part;           //   on paired tensor-core tiles) and its split-tile sums, over xd / hd
+  size_t routed;         // bytes without h_all and part
   size_t total;
 };
 
 size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
+
+// Whether a routed call takes every row through the paired tensor-core tiles: that needs the whole
+// [M, H] hidden matrix, so not where it is above 1 GB and above what the dense rows take anyway.
+bool pair_rows(int64_t M, int64_t D, int64_t H, int64_t cap) {
+  const int64_t hidden = M * H * 2, rows = cap * (D + H) * 2;
+  return pair_mlp_serves(M, D, H, true, false) &&
+         hidden <= (rows > ((int64_t)1 << 30) ? rows : (int64_t)1 << 30);
+}
 
 DenseWs dense_ws_layout(void* base, int64_t M, int64_t D, int64_t H, int64_t cap) {
   const int64_t cap_pad = (cap + kDenseTok - 1) / kDenseTok * kDenseTok;
@@ -896,8 +905,8 @@ DenseWs dense_ws_layout(void* base, int64_t M, int64_t D, int64_t H, int64_t cap
   off += align256((size_t)cap_pad * D * 2);
   w.hd = reinterpret_cast<__nv_bfloat16*>(p + off);
   off += align256((size_t)cap_pad * H * 2);
-  w.total = off;
-  if (pair_mlp_serves(M, D, H, true, false)) {
+  w.total = w.routed = off;
+  if (pair_rows(M, D, H, cap)) {
     off = (size_t)(reinterpret_cast<unsigned char*>(w.xd) - p);
     w.h_all = w.xd;
     off += align256((size_t)M * H * 2);
@@ -1233,9 +1242,9 @@ int b200_twell_gated_t2d_hybrid(const void* x, const void* packed, const void* g
   if (reinterpret_cast<uintptr_t>(hybrid_ws) & 255u)
     return fail(B200_EALIGN, "%s: hybrid_ws is not 256-byte aligned", fn);
   DenseWs w = dense_ws_layout(hybrid_ws, M, D, H, dense_cap);
-  if (hybrid_ws_bytes < w.total)
+  if (hybrid_ws_bytes < w.routed)
     return fail(B200_EWORKSPACE, "%s: hybrid_ws holds %zu bytes, %zu needed", fn, hybrid_ws_bytes,
-                w.total);
+                w.routed);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int tiles = (int)(H / kTileN), slab_w = kTileN / cf;
   const int64_t cap_pad = (dense_cap + kDenseTok - 1) / kDenseTok * kDenseTok;
@@ -1267,7 +1276,9 @@ int b200_twell_gated_mlp_hybrid(const void* x, const void* gate, const float* ga
                                 void* hybrid_ws, size_t hybrid_ws_bytes, void* workspace,
                                 size_t workspace_bytes, void* stream) {
   const char* fn = "b200_twell_gated_mlp_hybrid";
-  if (M > 0 && flags == 0 && D <= 4096 && pair_mlp_serves(M, D, H, true, false) && dense_cap > 0 &&
+  if (M > 0 && flags == 0 && D <= 4096 && dense_cap > 0 &&
+      pair_rows(M, D, H, dense_cap < M ? dense_cap : M) &&
+      hybrid_ws_bytes >= dense_ws_layout(nullptr, M, D, H, dense_cap < M ? dense_cap : M).total &&
       nnz_threshold >= 0 && M <= (int64_t)1 << 20 && hybrid_ws != nullptr && x && gate && up &&
       down && down_t && packed && out) {
     // Large calls: every row on the paired tensor-core tiles.  The hidden values of a routed row
@@ -1282,9 +1293,6 @@ int b200_twell_gated_mlp_hybrid(const void* x, const void* gate, const float* ga
       return fail(B200_EALIGN, "%s: hybrid_ws is not 256-byte aligned", fn);
     if (dense_cap > M) dense_cap = M;
     DenseWs w = dense_ws_layout(hybrid_ws, M, D, H, dense_cap);
-    if (hybrid_ws_bytes < w.total)
-      return fail(B200_EWORKSPACE, "%s: hybrid_ws holds %zu bytes, %zu needed", fn, hybrid_ws_bytes,
-                  w.total);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int tiles = (int)(H / kTileN), slab_w = kTileN / cf;
     if (int rc = pair_gate_up(false, x, gate, gate_bias, up, packed, w.h_all, M, D, H, cf, true, st))

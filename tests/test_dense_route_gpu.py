@@ -185,3 +185,28 @@ def test_all_rows_dense_on_256_token_tiles_for_both_products():
     assert _lib.load_library().b200_twell_hybrid_status() == 0
     assert row_rel_l2(y, ref).max() < REL_L2_ROW
     mod.destroy()
+
+
+def test_routed_call_with_a_workspace_for_the_routed_rows_only():
+    """A workspace that holds the dense rows but not the whole hidden matrix: the same call, served
+    row by row (what the function took before it had a use for more)."""
+    from sparser_faster_llms_b200 import _lib
+    m, d, h, cap = 700, 512, 4096, 64
+    ffn = synthetic.make_ffn(d, h, seed=5, density=0.03, skew_sigma=0.5, device=str(DEV))
+    x = synthetic.make_tokens(m, d, seed=6, device=str(DEV))
+    lib = _lib.load_library()
+    full = lib.b200_twell_hybrid_workspace_bytes(m, d, h, cap)
+    packed = twell.allocate_packed_output(m, h, device=DEV)
+    down_t = ffn.down.t().contiguous()
+    outs = []
+    for nbytes in (full, full - m * h):  # half of the hidden matrix missing
+        ws = torch.empty(nbytes, dtype=torch.uint8, device=DEV)
+        out = torch.empty_like(x)
+        _lib.call("b200_twell_gated_mlp_hybrid", torch.device(DEV), x.data_ptr(),
+                  ffn.gate.data_ptr(), None, ffn.up.data_ptr(), ffn.down.data_ptr(),
+                  down_t.data_ptr(), packed.data_ptr(), out.data_ptr(), m, d, h, 8, 0, h // 16, cap,
+                  ws.data_ptr(), nbytes, *_lib.workspace(torch.device(DEV)))
+        torch.cuda.synchronize()
+        outs.append(out.double())
+    # both forms round to bf16 at u, h, out (and the gather form every product): 1.2e-2 as above
+    assert ((outs[0] - outs[1]).norm() / outs[0].norm()).item() < 1.2e-2
