@@ -181,8 +181,16 @@ def ptr(t: torch.Tensor | None) -> int | None:
     return None if t is None else t.data_ptr()
 
 
+# Handle of a device's current stream by ordinal.  torch.cuda.current_stream builds a Stream object
+# around the same value, at 1.5 us a time.
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def current_stream_handle(device: torch.device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    index = getattr(device, "index", None)  # a method where a device is given by name
+    if _raw_stream is None or type(index) is not int:
+        return torch.cuda.current_stream(device).cuda_stream
+    return _raw_stream(index)
 
 
 _WORKSPACES: dict[tuple[int, int], torch.Tensor] = {}
@@ -193,9 +201,9 @@ def workspace(device: torch.device) -> tuple[int | None, int]:
     """(pointer, bytes) of the zero-initialised contraction workspace of ``device``'s current
     stream, created on first use.  During CUDA-graph capture no new workspace is created:
     ``(None, 0)`` is returned and the kernels use their workspace-free shape."""
-    stream = torch.cuda.current_stream(device)
+    device = torch.device(device)
     key = (device.index if device.index is not None else torch.cuda.current_device(),
-           stream.cuda_stream)
+           current_stream_handle(device))
     ws = _WORKSPACES.get(key)
     if ws is None:
         if torch.cuda.is_current_stream_capturing():
@@ -216,8 +224,10 @@ def workspace(device: torch.device) -> tuple[int | None, int]:
 
 def call(fn_name: str, device: torch.device, *args) -> None:
     """Invoke ``fn_name(*args, stream)`` on ``device``'s current stream and raise on error."""
-    lib = load_library()
-    fn = getattr(lib, fn_name)
-    with torch.cuda.device(device):
+    fn = getattr(load_library(), fn_name)
+    if device.index == torch.cuda.current_device():
         status = fn(*args, current_stream_handle(device))
+    else:
+        with torch.cuda.device(device):
+            status = fn(*args, current_stream_handle(device))
     check(fn_name, status)

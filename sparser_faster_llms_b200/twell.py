@@ -199,6 +199,9 @@ def packed_to_dense(packed: torch.Tensor, output_n: int, tile_n: int = 256,
 # argument checks shared by the functional wrappers
 # --------------------------------------------------------------------------
 def _need(t: torch.Tensor, name: str, dtype: torch.dtype, ndim: int = 2) -> torch.Tensor:
+    if (isinstance(t, torch.Tensor) and t.dtype is dtype and t.dim() == ndim and t.is_cuda
+            and t.is_contiguous()):
+        return t
     if not isinstance(t, torch.Tensor):
         raise TypeError(f"{name} must be a torch.Tensor")
     if t.dtype != dtype:
@@ -857,8 +860,13 @@ class _BaseTwELLMLP(nn.Module):
     def _apply_dense_route(self) -> None:  # gated modules override
         pass
 
+    def _weight(self, name: str) -> torch.Tensor:
+        """A weight by name, past nn.Module's attribute lookup while it is a buffer."""
+        t = self._buffers.get(name)
+        return getattr(self, name) if t is None else t
+
     def _ensure_layer(self) -> None:
-        weight = getattr(self, self._first)
+        weight = self._weight(self._first)
         entry = _D2T_LAYERS.get(self.layer_number)
         if (self.layer is not None and entry is not None
                 and entry["B"].data_ptr() == weight.data_ptr()):
@@ -879,7 +887,8 @@ class _BaseTwELLMLP(nn.Module):
 
     def forward(self, A: torch.Tensor) -> torch.Tensor:
         shape = A.shape
-        rows = A.view(-1, shape[-1])
+        flat = len(shape) == 2
+        rows = A if flat else A.view(-1, shape[-1])
         self._ensure_layer()
         shared = self.preallocate_shared_hidden_state
         args, kwargs = self._call_args()
@@ -887,7 +896,7 @@ class _BaseTwELLMLP(nn.Module):
             args = args + (self.layer.prepare_shared_hidden_state(rows),)
         out = self._entry[(shared, self.inplace)](self.layer_number, rows, *args, ext=self.ext,
                                                   **kwargs)
-        return A if self.inplace else out.view(shape)
+        return A if self.inplace else out if flat else out.view(shape)
 
     def _forward_into(self, A: torch.Tensor, out: torch.Tensor) -> None:
         """The forward with its result in ``out`` (contiguous, the shape of ``A``)."""
@@ -934,7 +943,7 @@ class TwELLMLP(_BaseTwELLMLP):
         self.num_splits = int(num_splits)
 
     def _call_args(self):
-        return (self.DOWN,), {"num_splits": self.num_splits}
+        return (self._weight("DOWN"),), {"num_splits": self.num_splits}
 
     def _native(self, rows, packed, out):
         _plain_mlp(self.layer_number, rows, self.DOWN, packed, out, self.num_splits)
@@ -966,7 +975,7 @@ class TwELLGatedMLP(_BaseTwELLMLP):
         self._down_t: torch.Tensor | None = None
 
     def _call_args(self):
-        return (self.UP, self.DOWN), {"highest_precision": self.highest_precision,
+        return (self._weight("UP"), self._weight("DOWN")), {"highest_precision": self.highest_precision,
                                       "compression_factor": self.compression_factor,
                                       "flex_kernels": self.flex_kernels}
 
