@@ -83,6 +83,10 @@ __device__ __forceinline__ void l2_prefetch(const void* p, uint32_t bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
 }
 
+__device__ __forceinline__ void l2_prefetch_line(const void* p) {
+  asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+}
+
 // Whether the decode kernels are launched with programmatic stream serialisation
 // (environment variable B200_PDL: "0" switches it off, anything else or unset keeps the
 // built-in default).

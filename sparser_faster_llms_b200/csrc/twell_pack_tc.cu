@@ -509,6 +509,9 @@ twell_pack_tc_splitk_mid_kernel(const __grid_constant__ CUtensorMap tmap_w,
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = tmem_slot;
+  if (threadIdx.x == 0)  // 37 tokens, H 5632, eager layers: 26.8 -> 26.4 us; 128, H 8192: 48.0 -> 47.4
+    for (int k = 0; k < 2 && k < ksteps; ++k)
+      tma_prefetch_2d(&tmap_w, k_base + k * kStageK, tile * kTileN);
   pdl_wait();
 
   bool ok = true;
