@@ -271,9 +271,9 @@ def pack_kernel_name(B: int, d: int, hl: int) -> str:
         return "twell_pack_kernel"
     if B <= 32:
         return "twell_pack_tc_splitk_wide_kernel"
-    if B <= 256 and tiles * 2 * -(-B // 128) <= 148:
+    if B <= 128 and tiles * 4 <= 148:
         return "twell_pack_tc_splitk_mid_kernel"
-    return "twell_pack_tc_wide_kernel" if B > 64 else "twell_pack_tc_kernel"
+    return "pair_gemm_kernel"
 
 
 def run_ours(args):
