@@ -447,7 +447,8 @@ int train_check(const char* fn, int64_t M, int64_t D, int64_t H, int cf, int64_t
                 size_t need) {
   if (int rc = check_dims(fn, M, D, H, cf)) return rc;
   if (M == 0) return fail(B200_EINVAL, "%s: M must be > 0", fn);
-  if (M > (int64_t)1 << 22) return fail(B200_EUNSUPPORTED, "%s: M > 2^22 rows", fn);
+  // row numbers, tiles and the sums of |T| (16 per tile of 256 x 256, H <= 65536) are 32-bit
+  if (M > (int64_t)1 << 26) return fail(B200_EUNSUPPORTED, "%s: M > 2^26 rows", fn);
   if (tail < 0 || tail > M) return fail(B200_EINVAL, "%s: need 0 <= tail_rows <= M", fn);
   for (const void* p : ptrs) {
     if (p == nullptr) return fail(B200_ENULL, "%s: NULL pointer", fn);

@@ -81,19 +81,9 @@ twell_pack_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __re
   const int tile = blockIdx.x / CL;
   const int m0 = blockIdx.y * TM;
   cluster.barrier_arrive();  // matched by barrier_wait() before the first remote store
-  const int tid = threadIdx.x;
-  if (M > 4) {
-    // the first quarter of this CTA's piece of every weight row, asked into L2 (28 layers of
-    // D 2048, H 8192: 8 tokens 697 -> 682 us; 2 tokens 524 -> 528)
-    const int piece = D / CL * 2, quarter = (piece + 511) / 512 * 128;
-    const unsigned char* rows = reinterpret_cast<const unsigned char*>(w) +
-                                (size_t)tile * kTileN * D * 2 + (size_t)crank * piece;
-    for (int r = tid; r < kTileN; r += NTHREADS)
-      for (int off = 0; off < quarter && off < piece; off += 128)
-        l2_prefetch_line(rows + (size_t)r * D * 2 + off);
-  }
   pdl_wait();                // nothing is read or written before the predecessor has completed
 
+  const int tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3;
 
