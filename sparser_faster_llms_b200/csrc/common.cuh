@@ -63,7 +63,7 @@ inline int ensure_dynamic_smem(Kernel kern, size_t bytes, size_t (&granted)[64],
 // (the wait returns once the predecessor grid has completed and its memory is visible).
 // pdl_wait() is a no-op in a kernel launched without the attribute.
 //
-// The contraction and the one-token layer kernel also issue pdl_trigger(): their successor's CTAs
+// The contraction of more than 16 tokens and the one-token layer kernel also issue pdl_trigger(): their successor's CTAs
 // become resident as their own CTAs leave, and use the time until pdl_wait() returns to set up
 // and to ask L2 for the first part of their weights (a quarter: asking for all of it, or from
 // inside the predecessor, fetches rows that are gone from L2 again when they are read).  Neither
@@ -81,10 +81,6 @@ __device__ __forceinline__ void pdl_trigger() {
 // Asks L2 for a range (a multiple of 16 bytes).  Changes no value, so it may stand before pdl_wait().
 __device__ __forceinline__ void l2_prefetch(const void* p, uint32_t bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
-}
-
-__device__ __forceinline__ void l2_prefetch_line(const void* p) {
-  asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
 }
 
 // Whether the decode kernels are launched with programmatic stream serialisation

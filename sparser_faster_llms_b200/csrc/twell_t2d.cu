@@ -213,7 +213,10 @@ twell_t2d_kernel(const __nv_bfloat16* x, const uint32_t* __restrict__ packed,
   for (int e = 0; e < 8; ++e) acc[e] = 0.f;
   int buf = 0;
 
-  pdl_trigger();
+  // Up to 16 tokens the successor is usually the mma.sync pack kernel, whose small CTAs would become
+  // resident beside this kernel's and slow its row loads (D 4096, H 16384, eager layers: 2 tokens
+  // 45.2 -> 48.8 us, 4 tokens 51.3 -> 56.2, 16 tokens 69.7 -> 71.7).
+  if (M > 16) pdl_trigger();
   const __nv_bfloat16* up_lane = up + warp * 256 + lane * 8;
   const __nv_bfloat16* down_lane = down + warp * 256 + lane * 8;
   const __nv_bfloat162* x2 = reinterpret_cast<const __nv_bfloat162*>(&xv);
