@@ -154,6 +154,25 @@ int b200_twell_mlp_scratch(const void* x, const void* up, const void* down, void
                            size_t scratch_bytes, void* stream);
 
 /*
+ * The same three with the hidden matrix held for at most max_rows tokens at a time, rounded down
+ * to a multiple of 256 (at least 256); it never takes more than 1 GB, max_rows 0 sets no other
+ * limit.  The chunks run one after another on the stream, through the same scratch.
+ */
+size_t b200_twell_mlp_scratch_bytes_chunked(int64_t M, int64_t D, int64_t H, int gated,
+                                            uint32_t flags, int64_t max_rows);
+
+int b200_twell_gated_mlp_chunked(const void* x, const void* gate, const float* gate_bias,
+                                 const void* up, const void* down, void* packed, void* out,
+                                 int64_t M, int64_t D, int64_t H, int cf, uint32_t flags,
+                                 void* workspace, size_t workspace_bytes, void* scratch,
+                                 size_t scratch_bytes, int64_t max_rows, void* stream);
+
+int b200_twell_mlp_chunked(const void* x, const void* up, const void* down, void* packed, void* out,
+                           int64_t M, int64_t D, int64_t H, int cf, int num_splits,
+                           void* workspace, size_t workspace_bytes, void* scratch,
+                           size_t scratch_bytes, int64_t max_rows, void* stream);
+
+/*
  * The fused gated MLP as ONE kernel for decode-sized calls (1 <= M <= 32): a thread-block
  * cluster per 256-neuron tile computes its slice of the gate, writes the slab words (same
  * bytes as b200_twell_pack) and at once contracts its own active neurons, and the tiles'

@@ -113,6 +113,15 @@ _PROTOTYPES = {
                                              c_void_p]),
     "b200_twell_mlp_scratch": (c_int, [c_void_p] * 5 + [c_int64, c_int64, c_int64, c_int, c_int,
                                        c_void_p, c_size_t, c_void_p, c_size_t, c_void_p]),
+    # the same with max_rows (before the stream)
+    "b200_twell_mlp_scratch_bytes_chunked": (c_size_t, [c_int64, c_int64, c_int64, c_int, c_uint32,
+                                                        c_int64]),
+    "b200_twell_gated_mlp_chunked": (c_int, [c_void_p] * 7 + [c_int64, c_int64, c_int64, c_int,
+                                             c_uint32, c_void_p, c_size_t, c_void_p, c_size_t,
+                                             c_int64, c_void_p]),
+    "b200_twell_mlp_chunked": (c_int, [c_void_p] * 5 + [c_int64, c_int64, c_int64, c_int, c_int,
+                                       c_void_p, c_size_t, c_void_p, c_size_t, c_int64,
+                                       c_void_p]),
     "b200_twell_decode_workspace_bytes": (c_size_t, [c_int64, c_int64, c_int64]),
     # x, gate, gate_bias, up, down, packed, out, M, D, H, cf, flags, ws, ws_bytes, prefetch,
     # prefetch_bytes, stream

@@ -63,14 +63,15 @@ int twell_gemv_layer(bool gated, bool hp, const void* x, const void* w, const fl
                      int64_t H, int cf, void* workspace, size_t workspace_bytes,
                      cudaStream_t stream);
 int pair_pack(const void* x, const void* w, const float* bias, void* packed, void* dense, int64_t M,
-              int64_t D, int64_t H, int cf, unsigned int* entries, float* part,
-              unsigned int* counters, cudaStream_t stream);
+              int64_t D, int64_t H, int cf, unsigned int* entries, const SplitRoom& room,
+              cudaStream_t stream);
 bool pair_mlp_serves(int64_t M, int64_t D, int64_t H, bool gated, bool hp);
-size_t pair_mlp_scratch_bytes(int64_t M, int64_t D, int64_t H, bool gated, bool hp);
+size_t pair_mlp_scratch_bytes(int64_t M, int64_t D, int64_t H, bool gated, bool hp,
+                              int64_t max_rows);
 int pair_mlp(bool gated, bool hp, const void* x, const void* gate, const float* bias,
              const void* up, const void* down, void* packed, void* out, int64_t M, int64_t D,
              int64_t H, int cf, void* workspace, size_t workspace_bytes, void* scratch,
-             cudaStream_t stream);
+             int64_t max_rows, cudaStream_t stream);
 int twell_decode_status();
 #ifdef B200_TRACE
 void twell_decode_trace(unsigned long long* out16);
@@ -215,7 +216,7 @@ int b200_twell_pack_select(const void* x, const void* w, const float* bias, void
   if (kernel == 0 && M > 32 && M <= 128 && twell_pack_mid_split(M, H, sm_count()) == 4)
     return twell_pack_tc_splitk_mid(x, w, bias, packed, M, D, H, cf, 4, st);
   if (kernel == 2 || kernel == 4 || kernel == 7 || (kernel == 0 && M > 32))
-    return pair_pack(x, w, bias, packed, nullptr, M, D, H, cf, nullptr, nullptr, nullptr, st);
+    return pair_pack(x, w, bias, packed, nullptr, M, D, H, cf, nullptr, {nullptr, 0, nullptr}, st);
   return twell_pack_small(x, w, bias, packed, M, D, H, cf, st);
 }
 
@@ -395,16 +396,40 @@ int b200_twell_gated_mlp(const void* x, const void* gate, const float* gate_bias
 namespace {
 // Whether a fused-MLP call runs on the paired tensor-core GEMM with the given scratch.
 bool pair_wanted(int64_t M, int64_t D, int64_t H, bool gated, bool hp, const void* scratch,
-                 size_t scratch_bytes) {
+                 size_t scratch_bytes, int64_t max_rows) {
   if (scratch == nullptr || M < 1 || D % 256 || H % 256 || D < 256 || D > 4096) return false;
-  const size_t need = pair_mlp_scratch_bytes(M, D, H, gated, hp);
+  const size_t need = pair_mlp_scratch_bytes(M, D, H, gated, hp, max_rows);
   return need != 0 && scratch_bytes >= need;
 }
 }  // namespace
 
-size_t b200_twell_mlp_scratch_bytes(int64_t M, int64_t D, int64_t H, int gated, uint32_t flags) {
+size_t b200_twell_mlp_scratch_bytes_chunked(int64_t M, int64_t D, int64_t H, int gated,
+                                            uint32_t flags, int64_t max_rows) {
   if (M <= 0 || D < 256 || D > 4096 || D % 256 || H < 256 || H > 65536 || H % 256) return 0;
-  return pair_mlp_scratch_bytes(M, D, H, gated != 0, (flags & B200_FLAG_HIGH_PRECISION) != 0);
+  return pair_mlp_scratch_bytes(M, D, H, gated != 0, (flags & B200_FLAG_HIGH_PRECISION) != 0,
+                                max_rows);
+}
+
+size_t b200_twell_mlp_scratch_bytes(int64_t M, int64_t D, int64_t H, int gated, uint32_t flags) {
+  return b200_twell_mlp_scratch_bytes_chunked(M, D, H, gated, flags, 0);
+}
+
+int b200_twell_gated_mlp_chunked(const void* x, const void* gate, const float* gate_bias,
+                                 const void* up, const void* down, void* packed, void* out,
+                                 int64_t M, int64_t D, int64_t H, int cf, uint32_t flags,
+                                 void* workspace, size_t workspace_bytes, void* scratch,
+                                 size_t scratch_bytes, int64_t max_rows, void* stream) {
+  const bool hp = (flags & B200_FLAG_HIGH_PRECISION) != 0;
+  if (pair_wanted(M, D, H, true, hp, scratch, scratch_bytes, max_rows)) {
+    B200_TRY(check_decode_args("b200_twell_gated_mlp", x, gate, gate_bias, up, down, packed, out,
+                               M, D, H, cf, flags, workspace, true));
+    B200_TRY(check_ptr("b200_twell_gated_mlp", "scratch", scratch));
+    return pair_mlp(true, hp, x, gate, gate_bias, up, down, packed, out, M, D, H, cf,
+                    workspace, workspace_bytes, scratch, max_rows,
+                    static_cast<cudaStream_t>(stream));
+  }
+  return b200_twell_gated_mlp(x, gate, gate_bias, up, down, packed, out, M, D, H, cf, flags,
+                              workspace, workspace_bytes, stream);
 }
 
 int b200_twell_gated_mlp_scratch(const void* x, const void* gate, const float* gate_bias,
@@ -412,16 +437,8 @@ int b200_twell_gated_mlp_scratch(const void* x, const void* gate, const float* g
                                  int64_t M, int64_t D, int64_t H, int cf, uint32_t flags,
                                  void* workspace, size_t workspace_bytes, void* scratch,
                                  size_t scratch_bytes, void* stream) {
-  const bool hp = (flags & B200_FLAG_HIGH_PRECISION) != 0;
-  if (pair_wanted(M, D, H, true, hp, scratch, scratch_bytes)) {
-    B200_TRY(check_decode_args("b200_twell_gated_mlp", x, gate, gate_bias, up, down, packed, out,
-                               M, D, H, cf, flags, workspace, true));
-    B200_TRY(check_ptr("b200_twell_gated_mlp", "scratch", scratch));
-    return pair_mlp(true, hp, x, gate, gate_bias, up, down, packed, out, M, D, H, cf,
-                    workspace, workspace_bytes, scratch, static_cast<cudaStream_t>(stream));
-  }
-  return b200_twell_gated_mlp(x, gate, gate_bias, up, down, packed, out, M, D, H, cf, flags,
-                              workspace, workspace_bytes, stream);
+  return b200_twell_gated_mlp_chunked(x, gate, gate_bias, up, down, packed, out, M, D, H, cf, flags,
+                                      workspace, workspace_bytes, scratch, scratch_bytes, 0, stream);
 }
 
 size_t b200_fused_allreduce_block_bytes(int64_t max_tokens, int64_t D) {
@@ -514,20 +531,29 @@ int b200_twell_mlp(const void* x, const void* up, const void* down, void* packed
                         stream);
 }
 
-int b200_twell_mlp_scratch(const void* x, const void* up, const void* down, void* packed, void* out,
+int b200_twell_mlp_chunked(const void* x, const void* up, const void* down, void* packed, void* out,
                            int64_t M, int64_t D, int64_t H, int cf, int num_splits,
                            void* workspace, size_t workspace_bytes, void* scratch,
-                           size_t scratch_bytes, void* stream) {
+                           size_t scratch_bytes, int64_t max_rows, void* stream) {
   if ((num_splits == 1 || num_splits == 2 || num_splits == 4 || num_splits == 8) &&
-      pair_wanted(M, D, H, false, false, scratch, scratch_bytes)) {
+      pair_wanted(M, D, H, false, false, scratch, scratch_bytes, max_rows)) {
     B200_TRY(check_decode_args("b200_twell_mlp", x, up, nullptr, nullptr, down, packed, out, M, D,
                                H, cf, 0, workspace, false));
     B200_TRY(check_ptr("b200_twell_mlp", "scratch", scratch));
     return pair_mlp(false, false, x, up, nullptr, nullptr, down, packed, out, M, D, H, cf,
-                    workspace, workspace_bytes, scratch, static_cast<cudaStream_t>(stream));
+                    workspace, workspace_bytes, scratch, max_rows,
+                    static_cast<cudaStream_t>(stream));
   }
   return b200_twell_mlp(x, up, down, packed, out, M, D, H, cf, num_splits, workspace,
                         workspace_bytes, stream);
+}
+
+int b200_twell_mlp_scratch(const void* x, const void* up, const void* down, void* packed, void* out,
+                           int64_t M, int64_t D, int64_t H, int cf, int num_splits,
+                           void* workspace, size_t workspace_bytes, void* scratch,
+                           size_t scratch_bytes, void* stream) {
+  return b200_twell_mlp_chunked(x, up, down, packed, out, M, D, H, cf, num_splits, workspace,
+                                workspace_bytes, scratch, scratch_bytes, 0, stream);
 }
 
 }  // extern "C"

@@ -129,6 +129,14 @@ struct RunIf {
   unsigned int limit;
 };
 
+// Room for a last wave of tiles that is cut along k: fp32 sums of the ranges, and counters that are
+// zero at rest.  A launch whose cut does not fit `bytes`, or that gets no room, runs uncut.
+struct SplitRoom {
+  float* part;
+  size_t bytes;
+  unsigned int* counters;
+};
+
 __device__ __forceinline__ uint32_t bf16_bits(float v) {
   return (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(v));
 }

@@ -42,8 +42,7 @@ int pair_gate_up(bool hp, const void* x, const void* gate, const float* bias, co
                  void* packed, void* hidden, int64_t M, int64_t D, int64_t H, int cf,
                  bool keep_all, cudaStream_t stream);
 int pair_down(const void* hidden, int terms, const void* down, void* out, int64_t M, int64_t D,
-              int64_t H, const RunIf& run_if, float* part, unsigned int* counters,
-              cudaStream_t stream);
+              int64_t H, const RunIf& run_if, const SplitRoom& room, cudaStream_t stream);
 
 namespace {
 
@@ -1306,9 +1305,10 @@ int b200_twell_gated_mlp_hybrid(const void* x, const void* gate, const float* ga
       truncate_rows_kernel<<<row_blocks, 256, 0, st>>>(static_cast<const uint32_t*>(packed), w.flags,
                                                       w.counters, (int)M, tiles, slab_w, w.h_all);
     if (int rc = check_launch(fn)) return rc;
-    return pair_down(w.h_all, 1, down, out, M, D, H, {nullptr, 0u}, w.part,
-                     workspace != nullptr && workspace_bytes >= 16384
-                         ? static_cast<unsigned int*>(workspace) : nullptr, st);
+    const SplitRoom room = {w.part, pair_part_bytes(M, D, H),
+                            workspace != nullptr && workspace_bytes >= 16384
+                                ? static_cast<unsigned int*>(workspace) : nullptr};
+    return pair_down(w.h_all, 1, down, out, M, D, H, {nullptr, 0u}, room, st);
   }
   if (int rc = b200_twell_pack(x, gate, gate_bias, packed, M, D, H, cf, stream)) return rc;
   return b200_twell_gated_t2d_hybrid(x, packed, gate, gate_bias, up, down, down_t, out, M, D, H,

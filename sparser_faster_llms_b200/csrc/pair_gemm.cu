@@ -17,14 +17,18 @@ namespace {
 
 constexpr int64_t kHiddenBytes = (int64_t)1 << 30;  // hidden matrix of one row chunk
 
-int64_t chunk_rows(int64_t M, int64_t H, int terms) {
-  const int64_t most = kHiddenBytes / (H * 2 * terms) / pg::kTile * pg::kTile;
+// Rows of all chunks but the last: whole tiles within kHiddenBytes and, where the caller sets it,
+// max_rows.
+int64_t chunk_rows(int64_t M, int64_t H, int terms, int64_t max_rows) {
+  int64_t most = kHiddenBytes / (H * 2 * terms) / pg::kTile * pg::kTile;
+  if (max_rows > 0 && max_rows < most)
+    most = max_rows < pg::kTile ? pg::kTile : max_rows / pg::kTile * pg::kTile;
   return M < most ? M : most;
 }
 
 size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
 
-// Largest split-tile buffer of the three products of a chunk of `rows` rows.
+// Largest split-tile buffer of the three products of a call of `rows` rows.
 size_t mlp_part_bytes(int64_t rows, int64_t D, int64_t H, int terms) {
   const int64_t mt = (rows + pg::kTile - 1) / pg::kTile, slots = sm_count() / 2;
   const size_t a = pg::part_bytes(mt * (H / pg::kTile), (int)(D / kStageK), slots, false);
@@ -43,13 +47,18 @@ pg::Args base_args(int64_t rows, int64_t n, int64_t k) {
 
 int aligned32(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 31u) == 0; }
 
+// The contraction workspace's zero-filled counters, or null.
+unsigned int* split_counters(void* workspace, size_t workspace_bytes) {
+  return workspace != nullptr && workspace_bytes >= 16384 ? static_cast<unsigned int*>(workspace)
+                                                          : nullptr;
+}
+
 }  // namespace
 
-// Slabs of relu(x W^T + bias); `dense`: also the stored values as an [M, H] matrix.  part /
-// counters may be null (no split of the last wave); entries: counter of stored entries or null.
+// Slabs of relu(x W^T + bias); `dense`: also the stored values as an [M, H] matrix.  entries: counter of stored entries or null.
 int pair_pack(const void* x, const void* w, const float* bias, void* packed, void* dense, int64_t M,
-              int64_t D, int64_t H, int cf, unsigned int* entries, float* part,
-              unsigned int* counters, cudaStream_t stream) {
+              int64_t D, int64_t H, int cf, unsigned int* entries, const SplitRoom& room,
+              cudaStream_t stream) {
   pg::Args a = base_args(M, H, D);
   a.bias = bias;
   a.bias16 = aligned16(bias);
@@ -57,8 +66,7 @@ int pair_pack(const void* x, const void* w, const float* bias, void* packed, voi
   a.slab_p = static_cast<uint32_t*>(packed);
   a.slab_w = kTileN / cf;
   a.row_words = (int)(H / kTileN) * a.slab_w;
-  a.part = part;
-  a.counters = counters;
+  pg::give_room(a, room);
   const pg::Operand ox = {x, M, D}, ow = {w, H, D};
   if (dense == nullptr)
     return pg::launch<pg::kPack, false, false>("b200_twell_pack", ox, ox, ow, ow, a, M, sm_count(),
@@ -74,7 +82,7 @@ int pair_pack(const void* x, const void* w, const float* bias, void* packed, voi
 // row_slot / tail_p: rows whose gate values come from a dense matrix instead (may be null).
 int pair_up(bool hp, const void* x, const void* packed, const void* up, void* hidden, int64_t M,
             int64_t D, int64_t H, int cf, const int* row_slot, const void* tail_p,
-            const RunIf& run_if, float* part, unsigned int* counters, cudaStream_t stream) {
+            const RunIf& run_if, const SplitRoom& room, cudaStream_t stream) {
   pg::Args a = base_args(M, H, D);
   a.run_if = run_if;
   a.slab_p = const_cast<uint32_t*>(static_cast<const uint32_t*>(packed));
@@ -85,8 +93,7 @@ int pair_up(bool hp, const void* x, const void* packed, const void* up, void* hi
   a.out = static_cast<__nv_bfloat16*>(hidden);
   a.ld = hp ? 3 * H : H;
   a.wide = aligned32(hidden);
-  a.part = part;
-  a.counters = counters;
+  pg::give_room(a, room);
   const pg::Operand ox = {x, M, D}, ou = {up, H, D};
   return hp ? pg::launch<pg::kMulHp, false, false>("up product", ox, ox, ou, ou, a, M, sm_count(),
                                                    stream)
@@ -96,16 +103,14 @@ int pair_up(bool hp, const void* x, const void* packed, const void* up, void* hi
 
 // out[M, D] = hidden[M, terms * H] [down; down; ...] with down [H, D] as it is stored.
 int pair_down(const void* hidden, int terms, const void* down, void* out, int64_t M, int64_t D,
-              int64_t H, const RunIf& run_if, float* part, unsigned int* counters,
-              cudaStream_t stream) {
+              int64_t H, const RunIf& run_if, const SplitRoom& room, cudaStream_t stream) {
   pg::Args a = base_args(M, D, terms * H);
   a.run_if = run_if;
   a.seg_ksteps = (int)(H / kStageK);
   a.out = static_cast<__nv_bfloat16*>(out);
   a.ld = D;
   a.wide = aligned32(out);
-  a.part = part;
-  a.counters = counters;
+  pg::give_room(a, room);
   const pg::Operand oh = {hidden, M, terms * H}, od = {down, D, H};
   return pg::launch<pg::kStore, false, true>("down product", oh, oh, od, od, a, M, sm_count(),
                                              stream);
@@ -179,27 +184,34 @@ static int64_t gather_entries(int64_t D, int64_t H, bool hp) {
 
 size_t pair_part_bytes(int64_t M, int64_t D, int64_t H) { return mlp_part_bytes(M, D, H, 1); }
 
-size_t pair_mlp_scratch_bytes(int64_t M, int64_t D, int64_t H, bool gated, bool hp) {
+// The split-tile buffer of a chunked call: which tiles are cut depends on their number, so the
+// shorter last chunk often needs more room than a full one.
+static size_t chunks_part_bytes(int64_t M, int64_t rows, int64_t D, int64_t H, int terms) {
+  const size_t full = mlp_part_bytes(rows, D, H, terms);
+  const size_t last = M % rows != 0 ? mlp_part_bytes(M % rows, D, H, terms) : 0;
+  return full > last ? full : last;
+}
+
+size_t pair_mlp_scratch_bytes(int64_t M, int64_t D, int64_t H, bool gated, bool hp,
+                              int64_t max_rows) {
   if (!pair_mlp_serves(M, D, H, gated, hp)) return 0;
   const int terms = hp ? 3 : 1;
-  const int64_t rows = chunk_rows(M, H, terms);
-  return align256((size_t)rows * H * 2 * terms) + 256 + mlp_part_bytes(rows, D, H, terms);
+  const int64_t rows = chunk_rows(M, H, terms, max_rows);
+  return align256((size_t)rows * H * 2 * terms) + 256 + chunks_part_bytes(M, rows, D, H, terms);
 }
 
 // workspace: the contraction workspace (its zero-filled counters; may be null).
 int pair_mlp(bool gated, bool hp, const void* x, const void* gate, const float* bias,
              const void* up, const void* down, void* packed, void* out, int64_t M, int64_t D,
              int64_t H, int cf, void* workspace, size_t workspace_bytes, void* scratch,
-             cudaStream_t stream) {
+             int64_t max_rows, cudaStream_t stream) {
   const int terms = hp ? 3 : 1;
-  const int64_t rows = chunk_rows(M, H, terms);
+  const int64_t rows = chunk_rows(M, H, terms, max_rows);
   const int64_t row_words = H / cf;
   unsigned char* p = static_cast<unsigned char*>(scratch) + align256((size_t)rows * H * 2 * terms);
   unsigned int* entries = reinterpret_cast<unsigned int*>(p);
-  float* part = reinterpret_cast<float*>(p + 256);
-  unsigned int* counters = workspace != nullptr && workspace_bytes >= 16384
-                               ? static_cast<unsigned int*>(workspace)
-                               : nullptr;
+  const SplitRoom room = {reinterpret_cast<float*>(p + 256), chunks_part_bytes(M, rows, D, H, terms),
+                          split_counters(workspace, workspace_bytes)};
   for (int64_t r0 = 0; r0 < M; r0 += rows) {
     const int64_t m = M - r0 < rows ? M - r0 : rows;
     const void* xc = static_cast<const __nv_bfloat16*>(x) + r0 * D;
@@ -219,15 +231,15 @@ int pair_mlp(bool gated, bool hp, const void* x, const void* gate, const float* 
     } else {
       pdl_suppressed() = choose;  // its predecessor is the memset
       const int rc = pair_pack(xc, gate, bias, pc, gated ? nullptr : scratch, m, D, H, cf,
-                               choose ? entries : nullptr, part, counters, stream);
+                               choose ? entries : nullptr, room, stream);
       pdl_suppressed() = false;
       if (rc) return rc;
       if (gated)
-        if (int rc = pair_up(hp, xc, pc, up, scratch, m, D, H, cf, nullptr, nullptr, run_if, part,
-                             counters, stream))
+        if (int rc = pair_up(hp, xc, pc, up, scratch, m, D, H, cf, nullptr, nullptr, run_if, room,
+                             stream))
           return rc;
     }
-    if (int rc = pair_down(scratch, terms, down, oc, m, D, H, run_if, part, counters, stream))
+    if (int rc = pair_down(scratch, terms, down, oc, m, D, H, run_if, room, stream))
       return rc;
     if (run_if.entries != nullptr)
       if (int rc = twell_t2d_launch(gated, hp, xc, pc, up, down, oc, m, D, H, cf, workspace,
@@ -394,7 +406,7 @@ struct TrainWs {
   __nv_bfloat16 *xt, *pt, *rt;   // tail rows: x, gate values, up products
   __nv_bfloat16 *t, *dru;        // [M, H] and (backward) [M, 2 H]
   float *l1_part, *part;
-  size_t total;
+  size_t part_bytes, total;
 };
 
 TrainWs train_ws(void* base, int64_t M, int64_t D, int64_t H, int64_t tail, bool bwd) {
@@ -424,6 +436,7 @@ TrainWs train_ws(void* base, int64_t M, int64_t D, int64_t H, int64_t tail, bool
   if (bwd)
     more(pg::part_bytes(3 * nt * (D / pg::kTile), (int)((M + kStageK - 1) / kStageK), slots, false));
   w.part = reinterpret_cast<float*>(take(part));
+  w.part_bytes = part;
   w.total = off;
   return w;
 }
@@ -462,11 +475,6 @@ int train_check(const char* fn, int64_t M, int64_t D, int64_t H, int cf, int64_t
   return B200_OK;
 }
 
-unsigned int* split_counters(void* workspace, size_t workspace_bytes) {
-  return workspace != nullptr && workspace_bytes >= 16384 ? static_cast<unsigned int*>(workspace)
-                                                          : nullptr;
-}
-
 }  // namespace
 
 }  // namespace b200
@@ -494,15 +502,15 @@ extern "C" int b200_hybrid_train_forward(const void* x, const void* g, const voi
   if (l0 == nullptr || l1 == nullptr || dropped == nullptr || n_over == nullptr)
     return fail(B200_ENULL, "%s: NULL result pointer", fn);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  unsigned int* counters = split_counters(workspace, workspace_bytes);
+  const SplitRoom room = {w.part, w.part_bytes, split_counters(workspace, workspace_bytes)};
   const int tiles = (int)(H / kTileN), W = kTileN / cf;
   const float inv_m = 1.f / (float)M;
   if (cudaMemsetAsync(w.state, 0, sizeof(RowState), st) != cudaSuccess)
     return fail(B200_ECUDA, "%s: cudaMemsetAsync failed", fn);
   // the gate pattern
   pdl_suppressed() = true;  // its predecessor is the memset
-  int rc = M > 128 ? pair_pack(x, g, nullptr, p_slab, nullptr, M, D, H, cf, nullptr, w.part,
-                               counters, st)
+  int rc = M > 128 ? pair_pack(x, g, nullptr, p_slab, nullptr, M, D, H, cf, nullptr, room,
+                               st)
                    : b200_twell_pack(x, g, nullptr, p_slab, M, D, H, cf, stream);
   pdl_suppressed() = false;
   if (rc) return rc;
@@ -527,11 +535,10 @@ extern "C" int b200_hybrid_train_forward(const void* x, const void* g, const voi
   a.row_slot = tail_rows > 0 ? w.row_slot : nullptr;
   a.tail_p = w.pt;
   a.l1_part = w.l1_part;
-  a.part = w.part;
-  a.counters = counters;
+  pg::give_room(a, room);
   const pg::Operand ox = {x, M, D}, ok = {k, H, D}, ot = {w.t, M, H};
   if (int e = pg::launch<pg::kFwd, false, false>(fn, ox, ot, ok, ot, a, M, sm_count(), st)) return e;
-  if (int e = pair_down(w.t, 1, v, out, M, D, H, {nullptr, 0u}, w.part, counters, st)) return e;
+  if (int e = pair_down(w.t, 1, v, out, M, D, H, {nullptr, 0u}, room, st)) return e;
   l1_sum_kernel<<<1, 1024, 0, st>>>(w.l1_part, (int)((M + pg::kTile - 1) / pg::kTile) * tiles * 16,
                                     inv_m, l1);
   return check_launch(fn);
@@ -551,7 +558,7 @@ extern "C" int b200_hybrid_train_backward(const void* x, const void* g, const vo
                            scratch_bytes, w.total))
     return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  unsigned int* counters = split_counters(workspace, workspace_bytes);
+  const SplitRoom room = {w.part, w.part_bytes, split_counters(workspace, workspace_bytes)};
   const int tiles = (int)(H / kTileN), W = kTileN / cf;
   if (tail_rows > 0) {
     if (cudaMemsetAsync(w.state, 0, sizeof(RowState), st) != cudaSuccess)
@@ -577,8 +584,7 @@ extern "C" int b200_hybrid_train_backward(const void* x, const void* g, const vo
   a.tail_r = w.rt;
   a.l1_grad = l1_grad;
   a.inv_m = 1.f / (float)M;
-  a.part = w.part;
-  a.counters = counters;
+  pg::give_room(a, room);
   const pg::Operand og = {g_out, M, D}, ov = {v, H, D}, odu = {w.dru, M, 2 * H}, ot = {w.t, M, H};
   if (int e = pg::launch<pg::kBwd, false, false>(fn, og, odu, ov, ot, a, M, sm_count(), st)) return e;
   // dX = [dR | dU] [K; G]
@@ -587,8 +593,7 @@ extern "C" int b200_hybrid_train_backward(const void* x, const void* g, const vo
   b.out = static_cast<__nv_bfloat16*>(dx);
   b.ld = D;
   b.wide = aligned32(dx);
-  b.part = w.part;
-  b.counters = counters;
+  pg::give_room(b, room);
   const pg::Operand odru = {w.dru, M, 2 * H}, okd = {k, D, H}, ogd = {g, D, H};
   if (int e = pg::launch<pg::kStore, false, true>(fn, odru, odru, okd, ogd, b, M, sm_count(), st))
     return e;
@@ -601,8 +606,7 @@ extern "C" int b200_hybrid_train_backward(const void* x, const void* g, const vo
   c.out_mt = (int)(H / pg::kTile);
   c.ld = D;
   c.wide = aligned32(dk) && aligned32(dg) && aligned32(dv);
-  c.part = w.part;
-  c.counters = counters;
+  pg::give_room(c, room);
   const pg::Operand a0 = {w.dru, 2 * H, M}, a1 = {w.t, H, M}, b0 = {x, D, M}, b1 = {g_out, D, M};
   return pg::launch<pg::kStore, true, true>(fn, a0, a1, b0, b1, c, 3 * H, sm_count(), st);
 }

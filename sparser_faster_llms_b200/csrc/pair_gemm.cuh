@@ -69,6 +69,7 @@ struct Args {
   float* sums;               // kStore, every tile split: fp32 sums [splits][rows][256 n_tiles]
   float* part;               // [items of split tiles][2][8 warps][128 columns][32 rows]
   unsigned int* counters;    // [split tiles][2][8], zero at rest
+  size_t part_bytes;         // host: size of part
   __nv_bfloat16* out;        // dense result, row stride ld
   long long ld;
   int wide;                  // out rows are 32-byte aligned
@@ -1056,9 +1057,16 @@ inline Split choose_split(int64_t tiles, int ksteps, int64_t slots, bool all) {
   if (s < 2) return {tiles, 1};
   return {tiles - tail, (int)s};
 }
-inline size_t part_bytes(int64_t tiles, int ksteps, int64_t slots, bool all) {
-  const Split s = choose_split(tiles, ksteps, slots, all);
+inline size_t split_bytes(const Split& s, int64_t tiles) {
   return s.splits < 2 ? 0 : (size_t)(tiles - s.full_tiles) * s.splits * kTile * kTile * sizeof(float);
+}
+inline size_t part_bytes(int64_t tiles, int ksteps, int64_t slots, bool all) {
+  return split_bytes(choose_split(tiles, ksteps, slots, all), tiles);
+}
+inline void give_room(Args& a, const SplitRoom& room) {
+  a.part = room.part;
+  a.part_bytes = room.bytes;
+  a.counters = room.counters;
 }
 
 template <int EPI, bool A_MN, bool B_MN>
@@ -1084,9 +1092,10 @@ int launch(const char* fn, const Operand& a0, const Operand& a1, const Operand& 
   const int64_t slots = sm_count / 2;
   const bool can_sum = EPI == kStore && args.out_mt == 0 && !args.relu &&
                        args.ld == (long long)args.n_tiles * kTile;
-  const Split sp = EPI != kGateUp && EPI != kGateUpHp && args.part != nullptr && args.counters != nullptr && args.rows_ptr == nullptr
-                       ? choose_split(tiles, args.ksteps, slots, can_sum)
-                       : Split{tiles, 1};
+  Split sp = EPI != kGateUp && EPI != kGateUpHp && args.part != nullptr && args.counters != nullptr && args.rows_ptr == nullptr
+                 ? choose_split(tiles, args.ksteps, slots, can_sum)
+                 : Split{tiles, 1};
+  if (split_bytes(sp, tiles) > args.part_bytes) sp = {tiles, 1};
   args.full_tiles = (int)sp.full_tiles;
   args.splits = sp.splits;
   const bool sum_after = can_sum && sp.splits > 1 && sp.full_tiles == 0;

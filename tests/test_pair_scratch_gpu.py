@@ -1,0 +1,48 @@
+"""Fused MLPs whose hidden matrix is held for a part of the tokens at a time: full chunks and a shorter
+last one whose tiles are cut along k, next to a guard region that no launch may touch.
+
+Same references and bounds as ``test_pair_gemm_gpu``: dyadic inputs, bit-exact slabs, outputs against
+the exact product of the oracle's hidden values.
+"""
+import pytest
+import torch
+
+from oracle import ffn_oracle as fo, twell_format as tf
+from sparser_faster_llms_b200 import _lib, synthetic, twell
+from test_pair_gemm_gpu import REL, hidden_of
+
+pytestmark = pytest.mark.gpu
+DEV = torch.device("cuda:0")
+GUARD = 32 << 20
+
+
+@pytest.mark.parametrize("m,d,h,max_rows,gated,hp", [
+    (640, 2048, 8192, 256, True, False), (1111, 1024, 4096, 512, True, False),
+    (700, 1024, 4096, 300, False, False), (4200, 2048, 8192, 1792, True, True)])
+def test_chunks_of_a_call(m, d, h, max_rows, gated, hp):
+    flags = _lib.FLAG_HIGH_PRECISION if hp else 0
+    lib = _lib.load_library()
+    need = lib.b200_twell_mlp_scratch_bytes_chunked(m, d, h, int(gated), flags, max_rows)
+    assert 0 < need < m * h * 2 * (3 if hp else 1) + GUARD
+    x, gate, up, down = synthetic.dyadic_case(m, d, h, seed=m + d)
+    want = tf.pack_preactivations(fo.gate_preactivation(x, gate).numpy(), 8)
+    xg, gg, ug, dg = (t.to(DEV) for t in (x, gate, up, down))
+    packed = twell.allocate_packed_output(m, h, device=DEV)
+    out = torch.empty_like(xg)
+    scratch = torch.full((need + GUARD,), 0x5A, dtype=torch.uint8, device=DEV)
+    ws = _lib.workspace(DEV)
+    if gated:
+        _lib.call("b200_twell_gated_mlp_chunked", DEV, xg.data_ptr(), gg.data_ptr(), None,
+                  ug.data_ptr(), dg.data_ptr(), packed.data_ptr(), out.data_ptr(), m, d, h, 8,
+                  flags, *ws, scratch.data_ptr(), need, max_rows)
+    else:
+        _lib.call("b200_twell_mlp_chunked", DEV, xg.data_ptr(), gg.data_ptr(), dg.data_ptr(),
+                  packed.data_ptr(), out.data_ptr(), m, d, h, 8, 2, *ws, scratch.data_ptr(), need,
+                  max_rows)
+    torch.cuda.synchronize()
+    assert lib.b200_twell_hybrid_status() == 0
+    assert (packed.cpu().view(torch.int32).numpy().view("uint32") == want).all()
+    assert bool((scratch[need:] == 0x5A).all())
+    rows = [0, max_rows // 256 * 256 - 1, max_rows // 256 * 256, m // 2, m - 129, m - 1]
+    ref = hidden_of(x[rows], up if gated else None, want[rows], h, 8, hp) @ down.double()
+    assert ((out[rows].double().cpu() - ref).norm() / ref.norm()).item() < REL

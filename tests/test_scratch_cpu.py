@@ -1,0 +1,73 @@
+"""Sizes of the scratch that calls on the paired tensor-core GEMM ask for, against what each of their
+launches writes.  A launch cuts its last wave of tiles along k, and how depends on the number of tiles,
+so every row chunk of a call is looked at by itself.  The library sizes for 148 SMs without a device."""
+import random
+
+import pytest
+
+from sparser_faster_llms_b200 import _lib, build
+
+PAIRS, TILE, STAGE_K = 74, 256, 64
+SHAPES = [(1024, 4096), (2048, 5632), (2048, 8192), (2048, 11008), (4096, 11008), (4096, 16384)]
+
+
+@pytest.fixture(scope="module")
+def lib():
+    build.build_library()
+    return _lib.load_library()
+
+
+def range_bytes(tiles, k, own_kernel):
+    """fp32 sums of the ranges that a product of `tiles` tiles is cut into."""
+    ksteps, tail = -(-k // STAGE_K), tiles % PAIRS
+    if tail == 0:
+        return 0
+    most = 8 if own_kernel and tiles < PAIRS else 4
+    splits = min(PAIRS // tail, ksteps // 4, most)
+    return 0 if splits < 2 else tail * splits * TILE * TILE * 4
+
+
+def chunks(m, h, terms, max_rows):
+    rows = (1 << 30) // (h * 2 * terms) // TILE * TILE
+    if max_rows:
+        rows = min(rows, max(TILE, max_rows // TILE * TILE))
+    rows = min(m, rows)
+    return [min(rows, m - r) for r in range(0, m, rows)]
+
+
+def mlp_need(m, d, h, terms, max_rows):
+    sizes = chunks(m, h, terms, max_rows)
+    cut = 0
+    for rows in set(sizes):
+        mt = -(-rows // TILE)
+        cut = max(cut, range_bytes(mt * (h // TILE), d, False),
+                  range_bytes(mt * (d // TILE), h * terms, True))
+    return sizes[0] * h * 2 * terms + 256 + cut
+
+
+def token_counts(h, terms):
+    rnd = random.Random(h + terms)
+    chunk = (1 << 30) // (h * 2 * terms) // TILE * TILE
+    edges = [k * chunk + e for k in (1, 2) for e in (-1, 0, 1, 100, 256, 777, 1024)]
+    return edges + [rnd.randint(64, 3 * chunk) for _ in range(60)]
+
+
+@pytest.mark.parametrize("d,h", SHAPES)
+@pytest.mark.parametrize("gated,flags", [(1, 0), (1, _lib.FLAG_HIGH_PRECISION), (0, 0)])
+def test_fused_mlp_scratch_holds_every_chunk(lib, d, h, gated, flags):
+    terms = 3 if flags else 1
+    seen = 0
+    for m in token_counts(h, terms):
+        got = lib.b200_twell_mlp_scratch_bytes(m, d, h, gated, flags)
+        assert got == 0 or got >= mlp_need(m, d, h, terms, 0), m
+        seen += got > 0
+    assert seen > 40
+
+
+@pytest.mark.parametrize("max_rows", [1, 256, 600, 4096])
+def test_chunked_scratch_holds_every_chunk(lib, max_rows):
+    for d, h in SHAPES:
+        for m in (320, 700, 1000, 5000, 70000):
+            got = lib.b200_twell_mlp_scratch_bytes_chunked(m, d, h, 1, 0, max_rows)
+            assert got == 0 or got >= mlp_need(m, d, h, 1, max_rows), (m, d, h)
+            assert got <= lib.b200_twell_mlp_scratch_bytes(m, d, h, 1, 0) + (1 << 26)
