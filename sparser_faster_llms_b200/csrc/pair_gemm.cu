@@ -192,12 +192,14 @@ static size_t chunks_part_bytes(int64_t M, int64_t rows, int64_t D, int64_t H, i
   return full > last ? full : last;
 }
 
+// 240 bytes of it take a 16-byte aligned scratch to the 256 bytes at which its parts begin (rows of
+// sums are written 32 bytes at a time).
 size_t pair_mlp_scratch_bytes(int64_t M, int64_t D, int64_t H, bool gated, bool hp,
                               int64_t max_rows) {
   if (!pair_mlp_serves(M, D, H, gated, hp)) return 0;
   const int terms = hp ? 3 : 1;
   const int64_t rows = chunk_rows(M, H, terms, max_rows);
-  return align256((size_t)rows * H * 2 * terms) + 256 + chunks_part_bytes(M, rows, D, H, terms);
+  return 240 + align256((size_t)rows * H * 2 * terms) + 256 + chunks_part_bytes(M, rows, D, H, terms);
 }
 
 // workspace: the contraction workspace (its zero-filled counters; may be null).
@@ -208,6 +210,7 @@ int pair_mlp(bool gated, bool hp, const void* x, const void* gate, const float* 
   const int terms = hp ? 3 : 1;
   const int64_t rows = chunk_rows(M, H, terms, max_rows);
   const int64_t row_words = H / cf;
+  scratch = reinterpret_cast<void*>(align256(reinterpret_cast<uintptr_t>(scratch)));
   unsigned char* p = static_cast<unsigned char*>(scratch) + align256((size_t)rows * H * 2 * terms);
   unsigned int* entries = reinterpret_cast<unsigned int*>(p);
   const SplitRoom room = {reinterpret_cast<float*>(p + 256), chunks_part_bytes(M, rows, D, H, terms),

@@ -46,3 +46,25 @@ def test_chunks_of_a_call(m, d, h, max_rows, gated, hp):
     rows = [0, max_rows // 256 * 256 - 1, max_rows // 256 * 256, m // 2, m - 129, m - 1]
     ref = hidden_of(x[rows], up if gated else None, want[rows], h, 8, hp) @ down.double()
     assert ((out[rows].double().cpu() - ref).norm() / ref.norm()).item() < REL
+
+
+@pytest.mark.parametrize("offset", [16, 48, 240])
+@pytest.mark.parametrize("m,hp", [(160, False), (4096, True)])
+def test_scratch_of_any_16_byte_alignment(m, hp, offset):
+    """Less than one wave of down tiles (sums written 32 bytes at a time), and several waves."""
+    d, h, flags = 2048, 8192, _lib.FLAG_HIGH_PRECISION if hp else 0
+    need = _lib.load_library().b200_twell_mlp_scratch_bytes(m, d, h, 1, flags)
+    x, *weights = synthetic.dyadic_case(m, d, h, seed=m)
+    xg, gg, ug, dg = (t.to(DEV) for t in (x, *weights))
+    packed = twell.allocate_packed_output(m, h, device=DEV)
+    scratch = torch.full((need + 512,), 0x5A, dtype=torch.uint8, device=DEV)
+    outs = []
+    for off in (0, offset):
+        outs.append(torch.empty_like(xg))
+        _lib.call("b200_twell_gated_mlp_scratch", DEV, xg.data_ptr(), gg.data_ptr(), None,
+                  ug.data_ptr(), dg.data_ptr(), packed.data_ptr(), outs[-1].data_ptr(), m, d, h, 8,
+                  flags, *_lib.workspace(DEV), scratch.data_ptr() + off, need)
+    torch.cuda.synchronize()
+    assert _lib.load_library().b200_twell_hybrid_status() == 0
+    assert torch.equal(outs[0], outs[1])
+    assert bool((scratch[need + offset:] == 0x5A).all())

@@ -42,7 +42,7 @@ def mlp_need(m, d, h, terms, max_rows):
         mt = -(-rows // TILE)
         cut = max(cut, range_bytes(mt * (h // TILE), d, False),
                   range_bytes(mt * (d // TILE), h * terms, True))
-    return sizes[0] * h * 2 * terms + 256 + cut
+    return 240 + sizes[0] * h * 2 * terms + 256 + cut  # 240: from 16-byte to 256-byte alignment
 
 
 def token_counts(h, terms):
