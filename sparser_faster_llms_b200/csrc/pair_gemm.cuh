@@ -548,6 +548,14 @@ __device__ __forceinline__ void backward_tile(const Args& a, const CUtensorMap* 
   }
 }
 
+// First term of h where rounding h to bf16 would leave bf16's range, and what it leaves: infinities
+// stand alone (inf - inf would put a NaN into the other terms), finite values keep the largest bf16.
+constexpr float kBf16Max = 0x1.FEp127f;
+__device__ __forceinline__ float first_term(float h) {
+  return fabsf(h) > kBf16Max && !isinf(h) ? copysignf(kBf16Max, h) : h;
+}
+__device__ __forceinline__ float rest_of(float h, float first) { return isinf(h) ? 0.f : h - first; }
+
 // h = g * u of 32 columns as three bf16 terms (24 bits of h), zero where g is.
 __device__ __forceinline__ void mul_hp(const uint4* g4, const float (&v)[32], uint32_t (&w0)[16],
                                        uint32_t (&w1)[16], uint32_t (&w2)[16]) {
@@ -560,8 +568,14 @@ __device__ __forceinline__ void mul_hp(const uint4* g4, const float (&v)[32], ui
       const float g0 = lo_f(g[p]), g1 = hi_f(g[p]);
       float h0 = g0 != 0.f ? g0 * v[c] : 0.f, h1 = g1 != 0.f ? g1 * v[c + 1] : 0.f;
       w0[o] = pack2(h0, h1);
-      h0 -= lo_f(w0[o]);
-      h1 -= hi_f(w0[o]);
+      if (fmaxf(fabsf(h0), fabsf(h1)) > kBf16Max) {
+        w0[o] = pack2(first_term(h0), first_term(h1));
+        h0 = rest_of(h0, lo_f(w0[o]));
+        h1 = rest_of(h1, hi_f(w0[o]));
+      } else {
+        h0 -= lo_f(w0[o]);
+        h1 -= hi_f(w0[o]);
+      }
       w1[o] = pack2(h0, h1);
       h0 -= lo_f(w1[o]);
       h1 -= hi_f(w1[o]);
