@@ -398,6 +398,16 @@ int b200_twell_gated_mlp_hybrid(const void* x, const void* gate, const float* ga
                                 void* hybrid_ws, size_t hybrid_ws_bytes, void* workspace,
                                 size_t workspace_bytes, void* stream);
 
+/* The same with the routing counts of b200_twell_hybrid_counters written to `counters` (3 device
+ * ints, may be NULL), so that hybrid_ws is free for other use once the stream is past the call. */
+int b200_twell_gated_mlp_hybrid_counted(const void* x, const void* gate, const float* gate_bias,
+                                        const void* up, const void* down, const void* down_t,
+                                        void* packed, void* out, int64_t M, int64_t D, int64_t H,
+                                        int cf, uint32_t flags, int64_t nnz_threshold,
+                                        int64_t dense_cap, void* hybrid_ws, size_t hybrid_ws_bytes,
+                                        void* workspace, size_t workspace_bytes, int* counters,
+                                        void* stream);
+
 /*
  * Every row on the dense route, with no slab, routing or gather: for token counts so
  * large that the weights are amortised and the per-entry gather cannot win.

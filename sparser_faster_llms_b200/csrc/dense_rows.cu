@@ -1218,12 +1218,16 @@ size_t b200_twell_hybrid_workspace_bytes(int64_t M, int64_t D, int64_t H, int64_
   return dense_ws_layout(nullptr, M, D, H, dense_cap).total;
 }
 
-int b200_twell_gated_t2d_hybrid(const void* x, const void* packed, const void* gate,
-                                const float* gate_bias, const void* up, const void* down,
-                                const void* down_t, void* out, int64_t M, int64_t D, int64_t H,
-                                int cf, uint32_t flags, int64_t nnz_threshold, int64_t dense_cap,
-                                void* hybrid_ws, size_t hybrid_ws_bytes, void* workspace,
-                                size_t workspace_bytes, void* stream) {
+}  // extern "C"
+
+namespace {
+
+// counters: where the routing counts go instead of the workspace (may be null).
+int t2d_hybrid(const void* x, const void* packed, const void* gate, const float* gate_bias,
+               const void* up, const void* down, const void* down_t, void* out, int64_t M, int64_t D,
+               int64_t H, int cf, uint32_t flags, int64_t nnz_threshold, int64_t dense_cap,
+               void* hybrid_ws, size_t hybrid_ws_bytes, void* workspace, size_t workspace_bytes,
+               int* counters, void* stream) {
   const char* fn = "b200_twell_gated_t2d_hybrid";
   if (int rc = check_dims(fn, M, D, H, cf)) return rc;
   if (flags & ~B200_FLAG_HIGH_PRECISION) return fail(B200_EINVAL, "%s: unknown flags 0x%x", fn, flags);
@@ -1244,6 +1248,7 @@ int b200_twell_gated_t2d_hybrid(const void* x, const void* packed, const void* g
   if (hybrid_ws_bytes < w.routed)
     return fail(B200_EWORKSPACE, "%s: hybrid_ws holds %zu bytes, %zu needed", fn, hybrid_ws_bytes,
                 w.routed);
+  if (counters != nullptr) w.counters = counters;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int tiles = (int)(H / kTileN), slab_w = kTileN / cf;
   const int64_t cap_pad = (dense_cap + kDenseTok - 1) / kDenseTok * kDenseTok;
@@ -1268,13 +1273,31 @@ int b200_twell_gated_t2d_hybrid(const void* x, const void* packed, const void* g
                                   w.counters, D, dense_cap, st);
 }
 
-int b200_twell_gated_mlp_hybrid(const void* x, const void* gate, const float* gate_bias,
-                                const void* up, const void* down, const void* down_t,
-                                void* packed, void* out, int64_t M, int64_t D, int64_t H, int cf,
-                                uint32_t flags, int64_t nnz_threshold, int64_t dense_cap,
+}  // namespace
+
+extern "C" {
+
+int b200_twell_gated_t2d_hybrid(const void* x, const void* packed, const void* gate,
+                                const float* gate_bias, const void* up, const void* down,
+                                const void* down_t, void* out, int64_t M, int64_t D, int64_t H,
+                                int cf, uint32_t flags, int64_t nnz_threshold, int64_t dense_cap,
                                 void* hybrid_ws, size_t hybrid_ws_bytes, void* workspace,
                                 size_t workspace_bytes, void* stream) {
+  return t2d_hybrid(x, packed, gate, gate_bias, up, down, down_t, out, M, D, H, cf, flags,
+                    nnz_threshold, dense_cap, hybrid_ws, hybrid_ws_bytes, workspace,
+                    workspace_bytes, nullptr, stream);
+}
+
+int b200_twell_gated_mlp_hybrid_counted(const void* x, const void* gate, const float* gate_bias,
+                                        const void* up, const void* down, const void* down_t,
+                                        void* packed, void* out, int64_t M, int64_t D, int64_t H,
+                                        int cf, uint32_t flags, int64_t nnz_threshold,
+                                        int64_t dense_cap, void* hybrid_ws, size_t hybrid_ws_bytes,
+                                        void* workspace, size_t workspace_bytes, int* counters,
+                                        void* stream) {
   const char* fn = "b200_twell_gated_mlp_hybrid";
+  if (reinterpret_cast<uintptr_t>(counters) & 3u)
+    return fail(B200_EALIGN, "%s: counters is not 4-byte aligned", fn);
   if (M > 0 && flags == 0 && D <= 4096 && dense_cap > 0 &&
       pair_rows(M, D, H, dense_cap < M ? dense_cap : M) &&
       hybrid_ws_bytes >= dense_ws_layout(nullptr, M, D, H, dense_cap < M ? dense_cap : M).total &&
@@ -1292,6 +1315,7 @@ int b200_twell_gated_mlp_hybrid(const void* x, const void* gate, const float* ga
       return fail(B200_EALIGN, "%s: hybrid_ws is not 256-byte aligned", fn);
     if (dense_cap > M) dense_cap = M;
     DenseWs w = dense_ws_layout(hybrid_ws, M, D, H, dense_cap);
+    if (counters != nullptr) w.counters = counters;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int tiles = (int)(H / kTileN), slab_w = kTileN / cf;
     if (int rc = pair_gate_up(false, x, gate, gate_bias, up, packed, w.h_all, M, D, H, cf, true, st))
@@ -1311,9 +1335,21 @@ int b200_twell_gated_mlp_hybrid(const void* x, const void* gate, const float* ga
     return pair_down(w.h_all, 1, down, out, M, D, H, {nullptr, 0u}, room, st);
   }
   if (int rc = b200_twell_pack(x, gate, gate_bias, packed, M, D, H, cf, stream)) return rc;
-  return b200_twell_gated_t2d_hybrid(x, packed, gate, gate_bias, up, down, down_t, out, M, D, H,
-                                     cf, flags, nnz_threshold, dense_cap, hybrid_ws,
-                                     hybrid_ws_bytes, workspace, workspace_bytes, stream);
+  return t2d_hybrid(x, packed, gate, gate_bias, up, down, down_t, out, M, D, H, cf, flags,
+                    nnz_threshold, dense_cap, hybrid_ws, hybrid_ws_bytes, workspace,
+                    workspace_bytes, counters, stream);
+}
+
+int b200_twell_gated_mlp_hybrid(const void* x, const void* gate, const float* gate_bias,
+                                const void* up, const void* down, const void* down_t,
+                                void* packed, void* out, int64_t M, int64_t D, int64_t H, int cf,
+                                uint32_t flags, int64_t nnz_threshold, int64_t dense_cap,
+                                void* hybrid_ws, size_t hybrid_ws_bytes, void* workspace,
+                                size_t workspace_bytes, void* stream) {
+  return b200_twell_gated_mlp_hybrid_counted(x, gate, gate_bias, up, down, down_t, packed, out, M, D,
+                                             H, cf, flags, nnz_threshold, dense_cap, hybrid_ws,
+                                             hybrid_ws_bytes, workspace, workspace_bytes, nullptr,
+                                             stream);
 }
 
 /* Every row on the dense route, without slab, routing or gather: Hd = relu(x Wg^T + b) *

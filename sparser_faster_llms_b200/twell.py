@@ -20,7 +20,6 @@ pybind extension.  Differences a caller can observe:
 """
 from __future__ import annotations
 
-import ctypes
 import os
 from pathlib import Path
 from types import SimpleNamespace
@@ -452,22 +451,24 @@ def _gated_mlp(layer_number, A, UP, DOWN, C_packed, OUT, highest_precision, cf) 
     elif (route is not None and route["dense_all_tokens"] is not None
             and m >= route["dense_all_tokens"]):
         # so many tokens that every row is cheaper as dense GEMMs: no slab is produced
-        ws_ptr, _ = _hybrid_workspace(dev, m, d, h, 0)
+        ws = _hybrid_workspace(dev, m, d, h, 0)
         _lib.call("b200_dense_gated_mlp", dev, A.data_ptr(), GATE.data_ptr(),
-                  _lib.ptr(entry["bias"]), UP.data_ptr(), route["DOWN_T"].data_ptr(), ws_ptr,
-                  OUT.data_ptr(), m, d, h)
+                  _lib.ptr(entry["bias"]), UP.data_ptr(), route["DOWN_T"].data_ptr(),
+                  ws.data_ptr(), OUT.data_ptr(), m, d, h)
         route["last"] = None
     elif route is not None and m >= route["min_tokens"]:
         cap = route["dense_cap"]
         cap = min(m, (max(128, m // 4) + 127) // 128 * 128) if cap is None else min(m, int(cap))
         thr = route["nnz_threshold"]
         thr = h // 16 if thr is None else int(thr)
-        ws_ptr, ws_bytes = _hybrid_workspace(dev, m, d, h, cap)
-        _lib.call("b200_twell_gated_mlp_hybrid", dev, A.data_ptr(), GATE.data_ptr(),
+        ws = _hybrid_workspace(dev, m, d, h, cap)
+        counters = torch.empty(3, dtype=torch.int32, device=dev)
+        _lib.call("b200_twell_gated_mlp_hybrid_counted", dev, A.data_ptr(), GATE.data_ptr(),
                   _lib.ptr(entry["bias"]), UP.data_ptr(), DOWN.data_ptr(),
                   route["DOWN_T"].data_ptr(), C_packed.data_ptr(), OUT.data_ptr(), m, d, h, cf,
-                  flags, thr, cap, ws_ptr, ws_bytes, *_lib.workspace(dev))
-        route["last"] = (m, d, h, cap)
+                  flags, thr, cap, ws.data_ptr(), ws.numel(), *_lib.workspace(dev),
+                  counters.data_ptr())
+        route["last"] = counters
     else:
         scratch, scratch_bytes = _mlp_scratch(dev, m, d, h, True, flags)
         _lib.call("b200_twell_gated_mlp_scratch", dev, A.data_ptr(), GATE.data_ptr(),
@@ -491,22 +492,14 @@ def _mlp_scratch(dev, m, d, h, gated, flags) -> tuple[torch.Tensor | None, int]:
     return torch.empty(need, dtype=torch.uint8, device=dev), need
 
 
-# One growing scratch buffer per device for the dense-row route (calls on a stream are
-# serialised, so all layers share it).
-_HYBRID_WS: dict[int, torch.Tensor] = {}
-
-
-def _hybrid_workspace(dev: torch.device, m: int, d: int, h: int, cap: int) -> tuple[int, int]:
+def _hybrid_workspace(dev: torch.device, m: int, d: int, h: int, cap: int) -> torch.Tensor:
+    """Scratch of one dense-row call: the hidden matrix and the routed rows.  Like
+    :func:`_mlp_scratch` from torch's allocator on every call."""
     if cap > 0:
         need = int(_lib.load_library().b200_twell_hybrid_workspace_bytes(m, d, h, cap))
     else:  # all rows dense: only the [M, H] bf16 hidden state
         need = m * h * 2
-    key = dev.index if dev.index is not None else torch.cuda.current_device()
-    buf = _HYBRID_WS.get(key)
-    if buf is None or buf.numel() < need:
-        buf = torch.empty(need, dtype=torch.uint8, device=dev)
-        _HYBRID_WS[key] = buf
-    return buf.data_ptr(), buf.numel()
+    return torch.empty(need, dtype=torch.uint8, device=dev)
 
 
 def set_d2t_layer_dense_route(layer_number: int, DOWN_T: torch.Tensor | None, *,
@@ -551,19 +544,12 @@ def set_d2t_layer_fused_allreduce(layer_number: int, fused) -> None:
 
 def d2t_layer_dense_route_counters(layer_number: int) -> dict | None:
     """``{"dense_rows", "lossy_rows_left_sparse", "qualified_rows"}`` of the last routed call
-    of this layer, or None if it has not run one.  Synchronises the device; valid only until
-    another layer's routed call reuses the shared scratch buffer."""
+    of this layer, or None if it has not run one.  Synchronises the device."""
     route = _layer(layer_number).get("dense_route")
     if route is None or route["last"] is None:
         return None
-    m, d, h, cap = route["last"]
-    dev = route["DOWN_T"].device
-    key = dev.index if dev.index is not None else torch.cuda.current_device()
-    out = (ctypes.c_int * 3)()
-    with torch.cuda.device(dev):
-        _lib.check("b200_twell_hybrid_counters",
-                   _lib.load_library().b200_twell_hybrid_counters(
-                       _HYBRID_WS[key].data_ptr(), m, d, h, cap, out))
+    torch.cuda.synchronize(route["last"].device)  # the call may have run on any stream
+    out = route["last"].tolist()
     return {"dense_rows": out[0], "lossy_rows_left_sparse": out[1], "qualified_rows": out[2]}
 
 

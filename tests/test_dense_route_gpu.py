@@ -210,3 +210,29 @@ def test_routed_call_with_a_workspace_for_the_routed_rows_only():
         outs.append(out.double())
     # both forms round to bf16 at u, h, out (and the gather form every product): 1.2e-2 as above
     assert ((outs[0] - outs[1]).norm() / outs[0].norm()).item() < 1.2e-2
+
+
+def test_routed_calls_on_two_streams_share_no_scratch():
+    """Two layers called in turn on streams of their own: the hidden matrix of one call must not
+    reach the other's product, and each layer keeps the counts of its own last call."""
+    m, d, h = 1024, 1024, 4096
+    xs, mods, want = [], [], []
+    for i in range(2):
+        ffn, x, _, _ = make_case(m, d, h, seed=640 + i)
+        mods.append(modules(7100 + 2 * i, ffn, nnz_threshold=h // 16, dense_cap=m,
+                            min_tokens=128)[1])
+        xs.append(x.to(DEV))
+        want.append((mods[i](xs[i]).clone(), mods[i].dense_route_counters()))
+    assert want[0][1] != want[1][1]
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    torch.cuda.synchronize()
+    got = [[], []]
+    for _ in range(20):
+        for i, s in enumerate(streams):
+            with torch.cuda.stream(s):
+                got[i].append(mods[i](xs[i]))
+    torch.cuda.synchronize()
+    for i in range(2):
+        assert all(torch.equal(y, want[i][0]) for y in got[i])
+        assert mods[i].dense_route_counters() == want[i][1]
+        mods[i].destroy()
