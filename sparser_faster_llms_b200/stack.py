@@ -13,9 +13,10 @@ This helper has no counterpart in the reference, whose benchmark launches eagerl
 from __future__ import annotations
 
 import torch
+from torch.nn.modules import module
 
 from . import _lib
-from .twell import _BaseTwELLMLP
+from .twell import TwELLGatedMLP, TwELLMLP
 
 
 class GraphedFFNStack:
@@ -70,11 +71,14 @@ class GraphedFFNStack:
 
     @staticmethod
     def _writes_into(mlp) -> bool:
-        """Whether the module can be given the tensor it writes: this package's own forward, not
-        in place, with nothing hooked to it."""
-        return (isinstance(mlp, _BaseTwELLMLP) and type(mlp).forward is _BaseTwELLMLP.forward
-                and "forward" not in vars(mlp) and not mlp.inplace
-                and not (mlp._forward_hooks or mlp._forward_pre_hooks))
+        """Whether the module can be given the tensor it writes: one of this package's own modules
+        (a subclass may change any part of the forward), not in place, with nothing replaced in
+        it and nothing hooked to it or to every module."""
+        return (type(mlp) in (TwELLMLP, TwELLGatedMLP) and not mlp.inplace
+                and not vars(mlp).keys() & {"forward", "_call_impl", "_compiled_call_impl",
+                                            "_call_args", "_entry", "_ensure_layer"}
+                and not (mlp._forward_hooks or mlp._forward_pre_hooks
+                         or module._global_forward_hooks or module._global_forward_pre_hooks))
 
     def _body(self) -> None:
         # The host -> device copies run on a second stream in chunks of a few layers, each
