@@ -236,9 +236,10 @@ def workspace(device: torch.device) -> tuple[int | None, int]:
 
 
 def call(fn_name: str, device: torch.device, *args) -> None:
-    """Invoke ``fn_name(*args, stream)`` on ``device``'s current stream and raise on error."""
+    """Invoke ``fn_name(*args, stream)`` on the current stream of ``device`` (a device, its name or
+    its ordinal) and raise on error."""
     fn = getattr(load_library(), fn_name)
-    if device.index == torch.cuda.current_device():
+    if getattr(device, "index", None) == torch.cuda.current_device():  # an ordinal has no index
         status = fn(*args, current_stream_handle(device))
     else:
         with torch.cuda.device(device):

@@ -1,10 +1,12 @@
 """C-ABI library: loads without a GPU, exports every declared symbol, validates arguments
 before touching CUDA."""
+import contextlib
 import ctypes
 import re
 from pathlib import Path
 
 import pytest
+import torch
 
 from sparser_faster_llms_b200 import _lib, build
 
@@ -64,3 +66,11 @@ def test_argument_validation_happens_before_any_cuda_call(lib):
 def test_missing_library_fails_loudly(tmp_path):
     with pytest.raises(RuntimeError, match="no CPU or PyTorch fallback"):
         _lib.load_library(tmp_path / "nope.so")
+
+
+@pytest.mark.parametrize("device", [torch.device("cuda:0"), torch.device("cuda"), "cuda:0", 0, 1])
+def test_call_takes_a_device_its_name_or_its_ordinal(lib, monkeypatch, device):
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 0)
+    monkeypatch.setattr(torch.cuda, "device", contextlib.nullcontext)
+    monkeypatch.setattr(_lib, "current_stream_handle", lambda device: None)
+    _lib.call("b200_twell_pack", device, None, None, None, None, 0, 256, 256, 8)
