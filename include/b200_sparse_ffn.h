@@ -269,6 +269,28 @@ int b200_hybrid_train_backward(const void* x, const void* g, const void* k, cons
                                size_t scratch_bytes, void* stream);
 
 /*
+ * The same three with the [M, H] intermediate matrices held for at most max_rows tokens at a time,
+ * rounded down to a multiple of 256 (at least 256); each never takes more than 1 GB, max_rows 0
+ * sets no other limit.  The weight gradients of several chunks add up in fp32.
+ */
+size_t b200_hybrid_train_scratch_bytes_chunked(int64_t M, int64_t D, int64_t H, int64_t tail_rows,
+                                               int backward, int64_t max_rows);
+
+int b200_hybrid_train_forward_chunked(const void* x, const void* g, const void* k, const void* v,
+                                      void* out, void* p_slab, void* r_slab, void* t_slab, float* l0,
+                                      float* l1, int* dropped, int* n_over, int64_t M, int64_t D,
+                                      int64_t H, int cf, int64_t tail_rows, void* workspace,
+                                      size_t workspace_bytes, void* scratch, size_t scratch_bytes,
+                                      int64_t max_rows, void* stream);
+
+int b200_hybrid_train_backward_chunked(const void* x, const void* g, const void* k, const void* v,
+                                       const void* p_slab, const void* r_slab, const void* g_out,
+                                       const float* l1_grad, void* dx, void* dg, void* dk, void* dv,
+                                       int64_t M, int64_t D, int64_t H, int cf, int64_t tail_rows,
+                                       void* workspace, size_t workspace_bytes, void* scratch,
+                                       size_t scratch_bytes, int64_t max_rows, void* stream);
+
+/*
  * Forward: R = (x k_w^T) sampled at P's pattern (bf16), T = R * P (bf16 multiply),
  * row_l1[r] = sum |T[r,:]| (fp32), row_nnz[r] = true positive count of the row,
  * row_drop[r] = entries of the row lost to slab overflow.  Replaces

@@ -385,10 +385,10 @@ tail_gather_kernel(uint32_t* __restrict__ P, const uint4* __restrict__ x,
 
 // l1 = inv_m * sum of n partial sums, in a fixed order.
 __global__ void __launch_bounds__(1024)
-l1_sum_kernel(const float* __restrict__ part, int n, float inv_m, float* __restrict__ l1) {
+l1_sum_kernel(const float* __restrict__ part, int64_t n, float inv_m, float* __restrict__ l1) {
   __shared__ float warp_s[32];
   float s = 0.f;
-  for (int i = threadIdx.x; i < n; i += 1024) s += part[i];
+  for (int64_t i = threadIdx.x; i < n; i += 1024) s += part[i];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   if ((threadIdx.x & 31) == 0) warp_s[threadIdx.x >> 5] = s;
@@ -401,18 +401,21 @@ l1_sum_kernel(const float* __restrict__ part, int n, float inv_m, float* __restr
   }
 }
 
-// Scratch of a training call; `tail` rows at most leave the slabs.
+// Scratch of a training call; `tail` rows at most leave the slabs.  The [M, H] matrices are held for
+// one chunk of rows; the weight gradients of several chunks add up in fp32 (carry).
 struct TrainWs {
   RowState* state;
   unsigned char* flags;
   int *row_slot, *row_drop, *rows;
   __nv_bfloat16 *xt, *pt, *rt;   // tail rows: x, gate values, up products
-  __nv_bfloat16 *t, *dru;        // [M, H] and (backward) [M, 2 H]
-  float *l1_part, *part;
+  __nv_bfloat16 *t, *dru;        // [chunk, H] and (backward) [chunk, 2 H]
+  float *l1_part, *part, *carry;
+  int64_t chunk;
   size_t part_bytes, total;
 };
 
-TrainWs train_ws(void* base, int64_t M, int64_t D, int64_t H, int64_t tail, bool bwd) {
+TrainWs train_ws(void* base, int64_t M, int64_t D, int64_t H, int64_t tail, bool bwd,
+                 int64_t max_rows) {
   unsigned char* p = static_cast<unsigned char*>(base);
   size_t off = 0;
   auto take = [&](size_t bytes) {
@@ -421,6 +424,7 @@ TrainWs train_ws(void* base, int64_t M, int64_t D, int64_t H, int64_t tail, bool
     return q;
   };
   TrainWs w = {};
+  w.chunk = chunk_rows(M, H, 1, max_rows);
   w.state = reinterpret_cast<RowState*>(take(sizeof(RowState)));
   w.flags = take((size_t)M);
   w.row_slot = reinterpret_cast<int*>(take((size_t)M * 4));
@@ -429,17 +433,27 @@ TrainWs train_ws(void* base, int64_t M, int64_t D, int64_t H, int64_t tail, bool
   w.xt = reinterpret_cast<__nv_bfloat16*>(take((size_t)tail * D * 2));
   w.pt = reinterpret_cast<__nv_bfloat16*>(take((size_t)tail * H * 2));
   if (bwd) w.rt = reinterpret_cast<__nv_bfloat16*>(take((size_t)tail * H * 2));
-  w.t = reinterpret_cast<__nv_bfloat16*>(take((size_t)M * H * 2));
-  if (bwd) w.dru = reinterpret_cast<__nv_bfloat16*>(take((size_t)M * H * 4));
-  const int64_t mt = (M + pg::kTile - 1) / pg::kTile, nt = H / pg::kTile, slots = sm_count() / 2;
-  if (!bwd) w.l1_part = reinterpret_cast<float*>(take((size_t)mt * nt * 16 * 4));
-  size_t part = pg::part_bytes(mt * nt, (int)(D / kStageK), slots, false);
+  w.t = reinterpret_cast<__nv_bfloat16*>(take((size_t)w.chunk * H * 2));
+  if (bwd) w.dru = reinterpret_cast<__nv_bfloat16*>(take((size_t)w.chunk * H * 4));
+  const int64_t nt = H / pg::kTile, slots = sm_count() / 2;
+  auto row_tiles = [](int64_t rows) { return (rows + pg::kTile - 1) / pg::kTile; };
+  if (!bwd) w.l1_part = reinterpret_cast<float*>(take((size_t)row_tiles(M) * nt * 16 * 4));
+  size_t part = 0;
   auto more = [&](size_t b) { part = b > part ? b : part; };
-  more(pg::part_bytes(mt * (D / pg::kTile), (int)((bwd ? 2 : 1) * H / kStageK), slots, true));
-  if (bwd)
-    more(pg::part_bytes(3 * nt * (D / pg::kTile), (int)((M + kStageK - 1) / kStageK), slots, false));
+  if (!bwd) more(pg::part_bytes(row_tiles(M) * nt, (int)(D / kStageK), slots, false));
+  const int64_t sizes[2] = {w.chunk, w.chunk > 0 ? M % w.chunk : 0};
+  for (int64_t rows : sizes) {  // which tiles are cut depends on their number
+    if (rows <= 0) continue;
+    more(pg::part_bytes(row_tiles(rows) * nt, (int)(D / kStageK), slots, false));
+    more(pg::part_bytes(row_tiles(rows) * (D / pg::kTile), (int)((bwd ? 2 : 1) * H / kStageK), slots,
+                        true));
+    if (bwd)
+      more(pg::part_bytes(3 * nt * (D / pg::kTile), (int)((rows + kStageK - 1) / kStageK), slots,
+                          false));
+  }
   w.part = reinterpret_cast<float*>(take(part));
   w.part_bytes = part;
+  if (bwd && w.chunk < M) w.carry = reinterpret_cast<float*>(take((size_t)3 * H * D * 4));
   w.total = off;
   return w;
 }
@@ -459,12 +473,9 @@ int tail_product(const TrainWs& w, const void* weight, __nv_bfloat16* out, bool 
 }
 
 int train_check(const char* fn, int64_t M, int64_t D, int64_t H, int cf, int64_t tail,
-                std::initializer_list<const void*> ptrs, const void* scratch, size_t scratch_bytes,
-                size_t need) {
+                std::initializer_list<const void*> ptrs, const void* scratch) {
   if (int rc = check_dims(fn, M, D, H, cf)) return rc;
   if (M == 0) return fail(B200_EINVAL, "%s: M must be > 0", fn);
-  // row numbers, tiles and the sums of |T| (16 per tile of 256 x 256, H <= 65536) are 32-bit
-  if (M > (int64_t)1 << 26) return fail(B200_EUNSUPPORTED, "%s: M > 2^26 rows", fn);
   if (tail < 0 || tail > M) return fail(B200_EINVAL, "%s: need 0 <= tail_rows <= M", fn);
   for (const void* p : ptrs) {
     if (p == nullptr) return fail(B200_ENULL, "%s: NULL pointer", fn);
@@ -473,8 +484,12 @@ int train_check(const char* fn, int64_t M, int64_t D, int64_t H, int cf, int64_t
   if (scratch == nullptr) return fail(B200_ENULL, "%s: scratch is NULL", fn);
   if (reinterpret_cast<uintptr_t>(scratch) & 255u)
     return fail(B200_EALIGN, "%s: scratch is not 256-byte aligned", fn);
-  if (scratch_bytes < need)
-    return fail(B200_EWORKSPACE, "%s: scratch holds %zu bytes, %zu needed", fn, scratch_bytes, need);
+  return B200_OK;
+}
+
+int train_room(const char* fn, size_t have, size_t need) {
+  if (have < need)
+    return fail(B200_EWORKSPACE, "%s: scratch holds %zu bytes, %zu needed", fn, have, need);
   return B200_OK;
 }
 
@@ -484,24 +499,29 @@ int train_check(const char* fn, int64_t M, int64_t D, int64_t H, int cf, int64_t
 
 using namespace b200;
 
-extern "C" size_t b200_hybrid_train_scratch_bytes(int64_t M, int64_t D, int64_t H, int64_t tail_rows,
-                                                  int backward) {
-  if (M <= 0 || D < 256 || H < 256 || D % 256 || H % 256 || tail_rows < 0) return 0;
-  return train_ws(nullptr, M, D, H, tail_rows, backward != 0).total;
+extern "C" size_t b200_hybrid_train_scratch_bytes_chunked(int64_t M, int64_t D, int64_t H,
+                                                          int64_t tail_rows, int backward,
+                                                          int64_t max_rows) {
+  if (M <= 0 || D < 256 || H < 256 || H > 65536 || D % 256 || H % 256 || tail_rows < 0) return 0;
+  return train_ws(nullptr, M, D, H, tail_rows, backward != 0, max_rows).total;
 }
 
-extern "C" int b200_hybrid_train_forward(const void* x, const void* g, const void* k, const void* v,
-                                         void* out, void* p_slab, void* r_slab, void* t_slab,
-                                         float* l0, float* l1, int* dropped, int* n_over, int64_t M,
-                                         int64_t D, int64_t H, int cf, int64_t tail_rows,
-                                         void* workspace, size_t workspace_bytes, void* scratch,
-                                         size_t scratch_bytes, void* stream) {
+extern "C" size_t b200_hybrid_train_scratch_bytes(int64_t M, int64_t D, int64_t H, int64_t tail_rows,
+                                                  int backward) {
+  return b200_hybrid_train_scratch_bytes_chunked(M, D, H, tail_rows, backward, 0);
+}
+
+extern "C" int b200_hybrid_train_forward_chunked(
+    const void* x, const void* g, const void* k, const void* v, void* out, void* p_slab,
+    void* r_slab, void* t_slab, float* l0, float* l1, int* dropped, int* n_over, int64_t M,
+    int64_t D, int64_t H, int cf, int64_t tail_rows, void* workspace, size_t workspace_bytes,
+    void* scratch, size_t scratch_bytes, int64_t max_rows, void* stream) {
   const char* fn = "b200_hybrid_train_forward";
-  const TrainWs w = train_ws(scratch, M, D, H, tail_rows, false);
-  if (int rc = train_check(fn, M, D, H, cf, tail_rows,
-                           {x, g, k, v, out, p_slab, r_slab, t_slab}, scratch, scratch_bytes,
-                           w.total))
+  if (int rc = train_check(fn, M, D, H, cf, tail_rows, {x, g, k, v, out, p_slab, r_slab, t_slab},
+                           scratch))
     return rc;
+  const TrainWs w = train_ws(scratch, M, D, H, tail_rows, false, max_rows);
+  if (int rc = train_room(fn, scratch_bytes, w.total)) return rc;
   if (l0 == nullptr || l1 == nullptr || dropped == nullptr || n_over == nullptr)
     return fail(B200_ENULL, "%s: NULL result pointer", fn);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -512,8 +532,7 @@ extern "C" int b200_hybrid_train_forward(const void* x, const void* g, const voi
     return fail(B200_ECUDA, "%s: cudaMemsetAsync failed", fn);
   // the gate pattern
   pdl_suppressed() = true;  // its predecessor is the memset
-  int rc = M > 128 ? pair_pack(x, g, nullptr, p_slab, nullptr, M, D, H, cf, nullptr, room,
-                               st)
+  int rc = M > 128 ? pair_pack(x, g, nullptr, p_slab, nullptr, M, D, H, cf, nullptr, room, st)
                    : b200_twell_pack(x, g, nullptr, p_slab, M, D, H, cf, stream);
   pdl_suppressed() = false;
   if (rc) return rc;
@@ -528,38 +547,53 @@ extern "C" int b200_hybrid_train_forward(const void* x, const void* g, const voi
     if (int e = check_launch(fn)) return e;
     if (int e = tail_product(w, g, w.pt, true, tail_rows, D, H, st)) return e;
   }
-  // R, T
-  pg::Args a = base_args(M, H, D);
-  a.slab_p = static_cast<uint32_t*>(p_slab);
-  a.slab_r = static_cast<uint32_t*>(r_slab);
-  a.slab_t = static_cast<uint32_t*>(t_slab);
-  a.slab_w = W;
-  a.row_words = tiles * W;
-  a.row_slot = tail_rows > 0 ? w.row_slot : nullptr;
-  a.tail_p = w.pt;
-  a.l1_part = w.l1_part;
-  pg::give_room(a, room);
-  const pg::Operand ox = {x, M, D}, ok = {k, H, D}, ot = {w.t, M, H};
-  if (int e = pg::launch<pg::kFwd, false, false>(fn, ox, ot, ok, ot, a, M, sm_count(), st)) return e;
-  if (int e = pair_down(w.t, 1, v, out, M, D, H, {nullptr, 0u}, room, st)) return e;
-  l1_sum_kernel<<<1, 1024, 0, st>>>(w.l1_part, (int)((M + pg::kTile - 1) / pg::kTile) * tiles * 16,
-                                    inv_m, l1);
+  // R, T and T v, chunk by chunk
+  for (int64_t r0 = 0; r0 < M; r0 += w.chunk) {
+    const int64_t m = M - r0 < w.chunk ? M - r0 : w.chunk;
+    const void* xc = static_cast<const __nv_bfloat16*>(x) + r0 * D;
+    pg::Args a = base_args(m, H, D);
+    a.slab_w = W;
+    a.row_words = tiles * W;
+    a.slab_p = static_cast<uint32_t*>(p_slab) + r0 * a.row_words;
+    a.slab_r = static_cast<uint32_t*>(r_slab) + r0 * a.row_words;
+    a.slab_t = static_cast<uint32_t*>(t_slab) + r0 * a.row_words;
+    a.row_slot = tail_rows > 0 ? w.row_slot + r0 : nullptr;
+    a.tail_p = w.pt;
+    a.l1_part = w.l1_part + r0 / pg::kTile * tiles * 16;  // chunks are whole row tiles
+    pg::give_room(a, room);
+    const pg::Operand ox = {xc, m, D}, ok = {k, H, D}, ot = {w.t, m, H};
+    if (int e = pg::launch<pg::kFwd, false, false>(fn, ox, ot, ok, ot, a, m, sm_count(), st)) return e;
+    if (int e = pair_down(w.t, 1, v, static_cast<__nv_bfloat16*>(out) + r0 * D, m, D, H,
+                          {nullptr, 0u}, room, st))
+      return e;
+  }
+  l1_sum_kernel<<<1, 1024, 0, st>>>(w.l1_part, (M + pg::kTile - 1) / pg::kTile * tiles * 16, inv_m,
+                                    l1);
   return check_launch(fn);
 }
 
-extern "C" int b200_hybrid_train_backward(const void* x, const void* g, const void* k, const void* v,
-                                          const void* p_slab, const void* r_slab,
-                                          const void* g_out, const float* l1_grad, void* dx,
-                                          void* dg, void* dk, void* dv, int64_t M, int64_t D,
-                                          int64_t H, int cf, int64_t tail_rows, void* workspace,
-                                          size_t workspace_bytes, void* scratch,
-                                          size_t scratch_bytes, void* stream) {
+extern "C" int b200_hybrid_train_forward(const void* x, const void* g, const void* k, const void* v,
+                                         void* out, void* p_slab, void* r_slab, void* t_slab,
+                                         float* l0, float* l1, int* dropped, int* n_over, int64_t M,
+                                         int64_t D, int64_t H, int cf, int64_t tail_rows,
+                                         void* workspace, size_t workspace_bytes, void* scratch,
+                                         size_t scratch_bytes, void* stream) {
+  return b200_hybrid_train_forward_chunked(x, g, k, v, out, p_slab, r_slab, t_slab, l0, l1, dropped,
+                                           n_over, M, D, H, cf, tail_rows, workspace,
+                                           workspace_bytes, scratch, scratch_bytes, 0, stream);
+}
+
+extern "C" int b200_hybrid_train_backward_chunked(
+    const void* x, const void* g, const void* k, const void* v, const void* p_slab,
+    const void* r_slab, const void* g_out, const float* l1_grad, void* dx, void* dg, void* dk,
+    void* dv, int64_t M, int64_t D, int64_t H, int cf, int64_t tail_rows, void* workspace,
+    size_t workspace_bytes, void* scratch, size_t scratch_bytes, int64_t max_rows, void* stream) {
   const char* fn = "b200_hybrid_train_backward";
-  const TrainWs w = train_ws(scratch, M, D, H, tail_rows, true);
   if (int rc = train_check(fn, M, D, H, cf, tail_rows,
-                           {x, g, k, v, p_slab, r_slab, g_out, dx, dg, dk, dv}, scratch,
-                           scratch_bytes, w.total))
+                           {x, g, k, v, p_slab, r_slab, g_out, dx, dg, dk, dv}, scratch))
     return rc;
+  const TrainWs w = train_ws(scratch, M, D, H, tail_rows, true, max_rows);
+  if (int rc = train_room(fn, scratch_bytes, w.total)) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const SplitRoom room = {w.part, w.part_bytes, split_counters(workspace, workspace_bytes)};
   const int tiles = (int)(H / kTileN), W = kTileN / cf;
@@ -576,42 +610,68 @@ extern "C" int b200_hybrid_train_backward(const void* x, const void* g, const vo
     if (int e = tail_product(w, g, w.pt, true, tail_rows, D, H, st)) return e;
     if (int e = tail_product(w, k, w.rt, false, tail_rows, D, H, st)) return e;
   }
-  // dT = g_out V^T on the pattern; dR = dT P, dU = dT R, T = R P
-  pg::Args a = base_args(M, H, D);
-  a.slab_p = const_cast<uint32_t*>(static_cast<const uint32_t*>(p_slab));
-  a.slab_r = const_cast<uint32_t*>(static_cast<const uint32_t*>(r_slab));
-  a.slab_w = W;
-  a.row_words = tiles * W;
-  a.row_slot = tail_rows > 0 ? w.row_slot : nullptr;
-  a.tail_p = w.pt;
-  a.tail_r = w.rt;
-  a.l1_grad = l1_grad;
-  a.inv_m = 1.f / (float)M;
-  pg::give_room(a, room);
-  const pg::Operand og = {g_out, M, D}, ov = {v, H, D}, odu = {w.dru, M, 2 * H}, ot = {w.t, M, H};
-  if (int e = pg::launch<pg::kBwd, false, false>(fn, og, odu, ov, ot, a, M, sm_count(), st)) return e;
-  // dX = [dR | dU] [K; G]
-  pg::Args b = base_args(M, D, 2 * H);
-  b.seg_ksteps = (int)(H / kStageK);
-  b.out = static_cast<__nv_bfloat16*>(dx);
-  b.ld = D;
-  b.wide = aligned32(dx);
-  pg::give_room(b, room);
-  const pg::Operand odru = {w.dru, M, 2 * H}, okd = {k, D, H}, ogd = {g, D, H};
-  if (int e = pg::launch<pg::kStore, false, true>(fn, odru, odru, okd, ogd, b, M, sm_count(), st))
-    return e;
-  // [dK; dG] = [dR | dU]^T X and dV = T^T g_out in one launch
-  pg::Args c = base_args(3 * H, D, M);
-  c.second_mt = (int)(2 * H / pg::kTile);
-  c.out = static_cast<__nv_bfloat16*>(dk);
-  c.out_more[0] = static_cast<__nv_bfloat16*>(dg);
-  c.out_more[1] = static_cast<__nv_bfloat16*>(dv);
-  c.out_mt = (int)(H / pg::kTile);
-  c.ld = D;
-  c.wide = aligned32(dk) && aligned32(dg) && aligned32(dv);
-  pg::give_room(c, room);
-  const pg::Operand a0 = {w.dru, 2 * H, M}, a1 = {w.t, H, M}, b0 = {x, D, M}, b1 = {g_out, D, M};
-  return pg::launch<pg::kStore, true, true>(fn, a0, a1, b0, b1, c, 3 * H, sm_count(), st);
+  for (int64_t r0 = 0; r0 < M; r0 += w.chunk) {
+    const int64_t m = M - r0 < w.chunk ? M - r0 : w.chunk;
+    const void* xc = static_cast<const __nv_bfloat16*>(x) + r0 * D;
+    const void* gc = static_cast<const __nv_bfloat16*>(g_out) + r0 * D;
+    void* dxc = static_cast<__nv_bfloat16*>(dx) + r0 * D;
+    // dT = g_out V^T on the pattern; dR = dT P, dU = dT R, T = R P
+    pg::Args a = base_args(m, H, D);
+    a.slab_w = W;
+    a.row_words = tiles * W;
+    a.slab_p = const_cast<uint32_t*>(static_cast<const uint32_t*>(p_slab)) + r0 * a.row_words;
+    a.slab_r = const_cast<uint32_t*>(static_cast<const uint32_t*>(r_slab)) + r0 * a.row_words;
+    a.row_slot = tail_rows > 0 ? w.row_slot + r0 : nullptr;
+    a.tail_p = w.pt;
+    a.tail_r = w.rt;
+    a.l1_grad = l1_grad;
+    a.inv_m = 1.f / (float)M;
+    pg::give_room(a, room);
+    const pg::Operand og = {gc, m, D}, ov = {v, H, D}, odu = {w.dru, m, 2 * H}, ot = {w.t, m, H};
+    if (int e = pg::launch<pg::kBwd, false, false>(fn, og, odu, ov, ot, a, m, sm_count(), st)) return e;
+    // dX = [dR | dU] [K; G]
+    pg::Args b = base_args(m, D, 2 * H);
+    b.seg_ksteps = (int)(H / kStageK);
+    b.out = static_cast<__nv_bfloat16*>(dxc);
+    b.ld = D;
+    b.wide = aligned32(dxc);
+    pg::give_room(b, room);
+    const pg::Operand odru = {w.dru, m, 2 * H}, okd = {k, D, H}, ogd = {g, D, H};
+    if (int e = pg::launch<pg::kStore, false, true>(fn, odru, odru, okd, ogd, b, m, sm_count(), st))
+      return e;
+    // [dK; dG] = [dR | dU]^T X and dV = T^T g_out in one launch
+    pg::Args c = base_args(3 * H, D, m);
+    c.second_mt = (int)(2 * H / pg::kTile);
+    c.out = static_cast<__nv_bfloat16*>(dk);
+    c.out_more[0] = static_cast<__nv_bfloat16*>(dg);
+    c.out_more[1] = static_cast<__nv_bfloat16*>(dv);
+    c.out_mt = (int)(H / pg::kTile);
+    c.ld = D;
+    c.wide = aligned32(dk) && aligned32(dg) && aligned32(dv);
+    c.carry = w.carry;
+    c.carry_in = r0 > 0;
+    c.carry_out = r0 + m < M;
+    pg::give_room(c, room);
+    const pg::Operand a0 = {w.dru, 2 * H, m}, a1 = {w.t, H, m}, b0 = {xc, D, m}, b1 = {gc, D, m};
+    const int e = w.carry == nullptr
+                      ? pg::launch<pg::kStore, true, true>(fn, a0, a1, b0, b1, c, 3 * H, sm_count(), st)
+                      : pg::launch<pg::kStoreCarry, true, true>(fn, a0, a1, b0, b1, c, 3 * H,
+                                                                sm_count(), st);
+    if (e) return e;
+  }
+  return B200_OK;
+}
+
+extern "C" int b200_hybrid_train_backward(const void* x, const void* g, const void* k, const void* v,
+                                          const void* p_slab, const void* r_slab,
+                                          const void* g_out, const float* l1_grad, void* dx,
+                                          void* dg, void* dk, void* dv, int64_t M, int64_t D,
+                                          int64_t H, int cf, int64_t tail_rows, void* workspace,
+                                          size_t workspace_bytes, void* scratch,
+                                          size_t scratch_bytes, void* stream) {
+  return b200_hybrid_train_backward_chunked(x, g, k, v, p_slab, r_slab, g_out, l1_grad, dx, dg, dk,
+                                            dv, M, D, H, cf, tail_rows, workspace, workspace_bytes,
+                                            scratch, scratch_bytes, 0, stream);
 }
 
 namespace b200 {

@@ -51,6 +51,7 @@ enum Epilogue {
   kGateUpHp = 8, // kPack and kMulHp likewise
   kMul = 2,      // out = bf16(g * bf16(acc)) on the slab pattern, 0 elsewhere
   kMulHp = 3,    // g * acc in fp32, as three bf16 terms side by side (out row = [hi | mid | lo])
+  kStoreCarry = 9,  // kStore on a product whose k comes in several launches: fp32 sums carried between
   kFwd = 4,      // training forward: R = bf16(acc) and T = R * P as slabs, T dense, l1 partial sums
   kBwd = 5       // training backward: dense [dR | dU] and T from acc = dT
 };
@@ -58,7 +59,7 @@ enum Epilogue {
 // Shared memory of the eight epilogue warps: 32 rows x 256 bytes of pattern each, or the blocks of
 // the training epilogues.
 __host__ __device__ constexpr int buf_bytes(int epi) {
-  return epi == kStore ? 0 : epi == kBwd ? 8 * 3 * 4096 : 8 * 32 * 256;
+  return epi == kStore || epi == kStoreCarry ? 0 : epi == kBwd ? 8 * 3 * 4096 : 8 * 32 * 256;
 }
 
 struct Args {
@@ -76,6 +77,8 @@ struct Args {
   int relu;                  // kStore
   __nv_bfloat16* out_more[2];  // kStore: results of the row tiles from out_mt and 2 out_mt on
   int out_mt;                // 0: all rows in out
+  float* carry;              // kStoreCarry: [tiles][2][8 warps][128 columns][32 rows] sums so far
+  int carry_in, carry_out;   //   whether it is added, and whether it takes the sums instead of out
   const float* bias;         // packs; bias16: 16-byte aligned
   int bias16;
   // slab operands [rows][row_words], slab_w words per 256 columns
@@ -594,6 +597,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap map_a0,
   constexpr bool kGate2 = EPI == kGateUp || EPI == kGateUpHp;
   constexpr bool kIsPack = EPI == kPack || EPI == kPackDense || kGate2;
   constexpr bool kTrain = EPI == kFwd || EPI == kBwd;
+  constexpr bool kPlain = EPI == kStore || EPI == kStoreCarry;
   constexpr int kBufBytes = buf_bytes(EPI) / 8;  // of one epilogue warp
   constexpr int kPhases = kGate2 ? 2 : 1;  // accumulators per item
 
@@ -782,7 +786,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap map_a0,
       const int row = row0 + lane;
       const bool live = row < rows;
       __nv_bfloat16* out = a.out + (size_t)row * a.ld + nt * kTile + half * 128;
-      if (EPI == kStore && a.out_mt > 0 && mt >= a.out_mt) {
+      if (kPlain && a.out_mt > 0 && mt >= a.out_mt) {
         const int o = mt / a.out_mt;
         out = a.out_more[o - 1] + (size_t)(row - o * a.out_mt * kTile) * a.ld + nt * kTile + half * 128;
       }
@@ -965,7 +969,20 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap map_a0,
         for (int cb = 0; cb < 4; ++cb) {
           float v[32];
           fetch32(src, cb, v);
-          if (EPI == kStore) {
+          if (EPI == kStoreCarry) {
+            float* carry = a.carry + (((size_t)im.tile * 2 + crank) * 8 + q * 2 + half) * (128 * 32) +
+                           cb * 1024 + lane;
+            if (a.carry_in) {
+#pragma unroll
+              for (int c = 0; c < 32; ++c) v[c] += __ldcg(carry + c * 32);
+            }
+            if (a.carry_out) {
+#pragma unroll
+              for (int c = 0; c < 32; ++c) __stcg(carry + c * 32, v[c]);
+              continue;
+            }
+          }
+          if (kPlain) {
             uint32_t w[16];
 #pragma unroll
             for (int p = 0; p < 16; ++p)
@@ -1087,7 +1104,7 @@ template <int EPI, bool A_MN, bool B_MN>
 int launch(const char* fn, const Operand& a0, const Operand& a1, const Operand& b0,
            const Operand& b1, Args args, int64_t row_capacity, int sm_count, cudaStream_t stream) {
   constexpr bool kTrain = EPI == kFwd || EPI == kBwd;
-  constexpr int STAGES = EPI == kStore ? 6 : EPI == kBwd ? 4 : 5;
+  constexpr int STAGES = EPI == kStore || EPI == kStoreCarry ? 6 : EPI == kBwd ? 4 : 5;
   constexpr size_t smem = (size_t)STAGES * kStageBytes + buf_bytes(EPI) + 1024;
   CUtensorMap ma0, ma1, mb0, mb1;
   if (int rc = operand_map(&ma0, a0, A_MN)) return rc;

@@ -1,6 +1,7 @@
 """Sizes of the scratch that calls on the paired tensor-core GEMM ask for, against what each of their
 launches writes.  A launch cuts its last wave of tiles along k, and how depends on the number of tiles,
 so every row chunk of a call is looked at by itself.  The library sizes for 148 SMs without a device."""
+import ctypes
 import random
 
 import pytest
@@ -71,3 +72,40 @@ def test_chunked_scratch_holds_every_chunk(lib, max_rows):
             got = lib.b200_twell_mlp_scratch_bytes_chunked(m, d, h, 1, 0, max_rows)
             assert got == 0 or got >= mlp_need(m, d, h, 1, max_rows), (m, d, h)
             assert got <= lib.b200_twell_mlp_scratch_bytes(m, d, h, 1, 0) + (1 << 26)
+
+
+def train_need(m, d, h, tail, bwd, max_rows):
+    sizes = chunks(m, h, 1, max_rows)
+    nt, mt = h // TILE, lambda rows: -(-rows // TILE)
+    cut = 0 if bwd else range_bytes(mt(m) * nt, d, False)
+    for rows in set(sizes):
+        cut = max(cut, range_bytes(mt(rows) * nt, d, False),
+                  range_bytes(mt(rows) * (d // TILE), (2 if bwd else 1) * h, True),
+                  range_bytes(3 * nt * (d // TILE), rows, False) if bwd else 0)
+    rows_out = tail * (4 + 2 * d + (4 if bwd else 2) * h) + m * 9
+    carry = 12 * h * d if bwd and len(sizes) > 1 else 0
+    return rows_out + sizes[0] * h * (6 if bwd else 2) + cut + carry + \
+        (0 if bwd else mt(m) * nt * 64)
+
+
+@pytest.mark.parametrize("d,h", SHAPES + [(256, 256)])
+@pytest.mark.parametrize("bwd", [0, 1])
+def test_training_scratch_holds_every_chunk_and_stays_bounded(lib, d, h, bwd):
+    for max_rows in (0, 256, 5000):
+        for m in token_counts(h, 1)[::3] + [1, 129, 5_000_000]:
+            for tail in (0, min(m, 2048)):
+                got = lib.b200_hybrid_train_scratch_bytes_chunked(m, d, h, tail, bwd, max_rows)
+                need = train_need(m, d, h, tail, bwd, max_rows)
+                assert need <= got <= need + (1 << 14)
+    # a step of five million tokens: bounded matrices and a few bytes per token
+    most = (3 if bwd else 1) * (1 << 30) + 12 * h * d + 5_000_000 * (9 + h / 4) + (1 << 28)
+    assert lib.b200_hybrid_train_scratch_bytes(5_000_000, d, h, 2048, bwd) < most
+
+
+def test_training_takes_as_many_tokens_as_the_other_entry_points(lib):
+    buf = (ctypes.c_char * 512)()
+    p = (ctypes.addressof(buf) + 255) & ~255
+    for m, status in ((1 << 27, -6), (1 << 30, -6), ((1 << 30) + 1, -4)):
+        # a valid call but for its scratch (no CUDA call is made), or one token too many
+        assert lib.b200_hybrid_train_forward(*[p] * 12, m, 256, 256, 8, 0, None, 0, p, 64, None) == status
+        assert lib.b200_hybrid_train_backward(*[p] * 12, m, 256, 256, 8, 0, None, 0, p, 64, None) == status
