@@ -291,6 +291,26 @@ int b200_hybrid_train_backward_chunked(const void* x, const void* g, const void*
                                        size_t scratch_bytes, int64_t max_rows, void* stream);
 
 /*
+ * The same two for a report of where the time goes: the device times (ms) of four parts are added
+ * to part_ms[4] (host), each part is waited for.  Forward: gate product and pack; rows taken out of
+ * the slabs; R and T; out.  Backward: rows taken out; dT, dR, dU; dX; the weight gradients.
+ */
+int b200_hybrid_train_forward_timed(const void* x, const void* g, const void* k, const void* v,
+                                    void* out, void* p_slab, void* r_slab, void* t_slab, float* l0,
+                                    float* l1, int* dropped, int* n_over, int64_t M, int64_t D,
+                                    int64_t H, int cf, int64_t tail_rows, void* workspace,
+                                    size_t workspace_bytes, void* scratch, size_t scratch_bytes,
+                                    int64_t max_rows, float* part_ms, void* stream);
+
+int b200_hybrid_train_backward_timed(const void* x, const void* g, const void* k, const void* v,
+                                     const void* p_slab, const void* r_slab, const void* g_out,
+                                     const float* l1_grad, void* dx, void* dg, void* dk, void* dv,
+                                     int64_t M, int64_t D, int64_t H, int cf, int64_t tail_rows,
+                                     void* workspace, size_t workspace_bytes, void* scratch,
+                                     size_t scratch_bytes, int64_t max_rows, float* part_ms,
+                                     void* stream);
+
+/*
  * Forward: R = (x k_w^T) sampled at P's pattern (bf16), T = R * P (bf16 multiply),
  * row_l1[r] = sum |T[r,:]| (fp32), row_nnz[r] = true positive count of the row,
  * row_drop[r] = entries of the row lost to slab overflow.  Replaces

@@ -62,6 +62,13 @@ _PROTOTYPES = {
     "b200_hybrid_train_backward_chunked": (c_int, [c_void_p] * 12 + [
         c_int64, c_int64, c_int64, c_int, c_int64, c_void_p, c_size_t, c_void_p, c_size_t, c_int64,
         c_void_p]),
+    # the same with max_rows, part_ms
+    "b200_hybrid_train_forward_timed": (c_int, [c_void_p] * 12 + [
+        c_int64, c_int64, c_int64, c_int, c_int64, c_void_p, c_size_t, c_void_p, c_size_t, c_int64,
+        c_void_p, c_void_p]),
+    "b200_hybrid_train_backward_timed": (c_int, [c_void_p] * 12 + [
+        c_int64, c_int64, c_int64, c_int, c_int64, c_void_p, c_size_t, c_void_p, c_size_t, c_int64,
+        c_void_p, c_void_p]),
     "b200_hybrid_sddmm_fwd": (c_int, [c_void_p] * 8 + [c_int64, c_int64, c_int64, c_int, c_void_p]),
     "b200_hybrid_sddmm_bwd": (c_int, [c_void_p] * 7 + [c_int64, c_int64, c_int64, c_int,
                                                        c_void_p]),

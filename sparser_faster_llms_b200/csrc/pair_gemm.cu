@@ -487,6 +487,43 @@ int train_check(const char* fn, int64_t M, int64_t D, int64_t H, int cf, int64_t
   return B200_OK;
 }
 
+// Device times of the parts of a call, added to ms[]; ms == nullptr: nothing is recorded.  Every part
+// is waited for.
+class Parts {
+ public:
+  Parts(float* ms, cudaStream_t stream) : ms_(ms), stream_(stream) {
+    if (ms_ == nullptr) return;
+    for (cudaEvent_t& e : event_) ok_ = cudaEventCreate(&e) == cudaSuccess && ok_;
+    ok_ = ok_ && cudaEventRecord(event_[0], stream_) == cudaSuccess;
+  }
+  ~Parts() {
+    for (cudaEvent_t e : event_)
+      if (e != nullptr) cudaEventDestroy(e);
+  }
+  // Ends part `i`; the next one begins.
+  void end(int i) {
+    if (ms_ == nullptr || !ok_) return;
+    float t = 0.f;
+    ok_ = cudaEventRecord(event_[1], stream_) == cudaSuccess &&
+          cudaEventSynchronize(event_[1]) == cudaSuccess &&
+          cudaEventElapsedTime(&t, event_[0], event_[1]) == cudaSuccess;
+    if (!ok_) return;
+    ms_[i] += t;
+    cudaEvent_t e = event_[0];
+    event_[0] = event_[1];
+    event_[1] = e;
+  }
+  int status(const char* fn) const {
+    return ok_ ? B200_OK : fail(B200_ECUDA, "%s: the parts of the call could not be timed", fn);
+  }
+
+ private:
+  float* ms_;
+  cudaStream_t stream_;
+  cudaEvent_t event_[2] = {nullptr, nullptr};
+  bool ok_ = true;
+};
+
 int train_room(const char* fn, size_t have, size_t need) {
   if (have < need)
     return fail(B200_EWORKSPACE, "%s: scratch holds %zu bytes, %zu needed", fn, have, need);
@@ -511,11 +548,11 @@ extern "C" size_t b200_hybrid_train_scratch_bytes(int64_t M, int64_t D, int64_t 
   return b200_hybrid_train_scratch_bytes_chunked(M, D, H, tail_rows, backward, 0);
 }
 
-extern "C" int b200_hybrid_train_forward_chunked(
+extern "C" int b200_hybrid_train_forward_timed(
     const void* x, const void* g, const void* k, const void* v, void* out, void* p_slab,
     void* r_slab, void* t_slab, float* l0, float* l1, int* dropped, int* n_over, int64_t M,
     int64_t D, int64_t H, int cf, int64_t tail_rows, void* workspace, size_t workspace_bytes,
-    void* scratch, size_t scratch_bytes, int64_t max_rows, void* stream) {
+    void* scratch, size_t scratch_bytes, int64_t max_rows, float* part_ms, void* stream) {
   const char* fn = "b200_hybrid_train_forward";
   if (int rc = train_check(fn, M, D, H, cf, tail_rows, {x, g, k, v, out, p_slab, r_slab, t_slab},
                            scratch))
@@ -528,6 +565,7 @@ extern "C" int b200_hybrid_train_forward_chunked(
   const SplitRoom room = {w.part, w.part_bytes, split_counters(workspace, workspace_bytes)};
   const int tiles = (int)(H / kTileN), W = kTileN / cf;
   const float inv_m = 1.f / (float)M;
+  Parts parts(part_ms, st);
   if (cudaMemsetAsync(w.state, 0, sizeof(RowState), st) != cudaSuccess)
     return fail(B200_ECUDA, "%s: cudaMemsetAsync failed", fn);
   // the gate pattern
@@ -536,6 +574,7 @@ extern "C" int b200_hybrid_train_forward_chunked(
                    : b200_twell_pack(x, g, nullptr, p_slab, M, D, H, cf, stream);
   pdl_suppressed() = false;
   if (rc) return rc;
+  parts.end(0);
   tail_rows_kernel<false><<<(unsigned)((M + 31) / 32), 256, 0, st>>>(
       static_cast<const uint32_t*>(p_slab), (int)M, tiles, W, (int)tail_rows, w.flags, w.row_slot,
       w.row_drop, w.rows, w.state, l0, dropped, n_over, inv_m);
@@ -547,6 +586,7 @@ extern "C" int b200_hybrid_train_forward_chunked(
     if (int e = check_launch(fn)) return e;
     if (int e = tail_product(w, g, w.pt, true, tail_rows, D, H, st)) return e;
   }
+  parts.end(1);
   // R, T and T v, chunk by chunk
   for (int64_t r0 = 0; r0 < M; r0 += w.chunk) {
     const int64_t m = M - r0 < w.chunk ? M - r0 : w.chunk;
@@ -563,13 +603,27 @@ extern "C" int b200_hybrid_train_forward_chunked(
     pg::give_room(a, room);
     const pg::Operand ox = {xc, m, D}, ok = {k, H, D}, ot = {w.t, m, H};
     if (int e = pg::launch<pg::kFwd, false, false>(fn, ox, ot, ok, ot, a, m, sm_count(), st)) return e;
+    parts.end(2);
     if (int e = pair_down(w.t, 1, v, static_cast<__nv_bfloat16*>(out) + r0 * D, m, D, H,
                           {nullptr, 0u}, room, st))
       return e;
+    parts.end(3);
   }
   l1_sum_kernel<<<1, 1024, 0, st>>>(w.l1_part, (M + pg::kTile - 1) / pg::kTile * tiles * 16, inv_m,
                                     l1);
+  parts.end(3);
+  if (int e = parts.status(fn)) return e;
   return check_launch(fn);
+}
+
+extern "C" int b200_hybrid_train_forward_chunked(
+    const void* x, const void* g, const void* k, const void* v, void* out, void* p_slab,
+    void* r_slab, void* t_slab, float* l0, float* l1, int* dropped, int* n_over, int64_t M,
+    int64_t D, int64_t H, int cf, int64_t tail_rows, void* workspace, size_t workspace_bytes,
+    void* scratch, size_t scratch_bytes, int64_t max_rows, void* stream) {
+  return b200_hybrid_train_forward_timed(x, g, k, v, out, p_slab, r_slab, t_slab, l0, l1, dropped,
+                                         n_over, M, D, H, cf, tail_rows, workspace, workspace_bytes,
+                                         scratch, scratch_bytes, max_rows, nullptr, stream);
 }
 
 extern "C" int b200_hybrid_train_forward(const void* x, const void* g, const void* k, const void* v,
@@ -583,11 +637,12 @@ extern "C" int b200_hybrid_train_forward(const void* x, const void* g, const voi
                                            workspace_bytes, scratch, scratch_bytes, 0, stream);
 }
 
-extern "C" int b200_hybrid_train_backward_chunked(
+extern "C" int b200_hybrid_train_backward_timed(
     const void* x, const void* g, const void* k, const void* v, const void* p_slab,
     const void* r_slab, const void* g_out, const float* l1_grad, void* dx, void* dg, void* dk,
     void* dv, int64_t M, int64_t D, int64_t H, int cf, int64_t tail_rows, void* workspace,
-    size_t workspace_bytes, void* scratch, size_t scratch_bytes, int64_t max_rows, void* stream) {
+    size_t workspace_bytes, void* scratch, size_t scratch_bytes, int64_t max_rows, float* part_ms,
+    void* stream) {
   const char* fn = "b200_hybrid_train_backward";
   if (int rc = train_check(fn, M, D, H, cf, tail_rows,
                            {x, g, k, v, p_slab, r_slab, g_out, dx, dg, dk, dv}, scratch))
@@ -597,6 +652,7 @@ extern "C" int b200_hybrid_train_backward_chunked(
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const SplitRoom room = {w.part, w.part_bytes, split_counters(workspace, workspace_bytes)};
   const int tiles = (int)(H / kTileN), W = kTileN / cf;
+  Parts parts(part_ms, st);
   if (tail_rows > 0) {
     if (cudaMemsetAsync(w.state, 0, sizeof(RowState), st) != cudaSuccess)
       return fail(B200_ECUDA, "%s: cudaMemsetAsync failed", fn);
@@ -609,6 +665,7 @@ extern "C" int b200_hybrid_train_backward_chunked(
     if (int e = check_launch(fn)) return e;
     if (int e = tail_product(w, g, w.pt, true, tail_rows, D, H, st)) return e;
     if (int e = tail_product(w, k, w.rt, false, tail_rows, D, H, st)) return e;
+    parts.end(0);
   }
   for (int64_t r0 = 0; r0 < M; r0 += w.chunk) {
     const int64_t m = M - r0 < w.chunk ? M - r0 : w.chunk;
@@ -629,6 +686,7 @@ extern "C" int b200_hybrid_train_backward_chunked(
     pg::give_room(a, room);
     const pg::Operand og = {gc, m, D}, ov = {v, H, D}, odu = {w.dru, m, 2 * H}, ot = {w.t, m, H};
     if (int e = pg::launch<pg::kBwd, false, false>(fn, og, odu, ov, ot, a, m, sm_count(), st)) return e;
+    parts.end(1);
     // dX = [dR | dU] [K; G]
     pg::Args b = base_args(m, D, 2 * H);
     b.seg_ksteps = (int)(H / kStageK);
@@ -639,6 +697,7 @@ extern "C" int b200_hybrid_train_backward_chunked(
     const pg::Operand odru = {w.dru, m, 2 * H}, okd = {k, D, H}, ogd = {g, D, H};
     if (int e = pg::launch<pg::kStore, false, true>(fn, odru, odru, okd, ogd, b, m, sm_count(), st))
       return e;
+    parts.end(2);
     // [dK; dG] = [dR | dU]^T X and dV = T^T g_out in one launch
     pg::Args c = base_args(3 * H, D, m);
     c.second_mt = (int)(2 * H / pg::kTile);
@@ -658,8 +717,19 @@ extern "C" int b200_hybrid_train_backward_chunked(
                       : pg::launch<pg::kStoreCarry, true, true>(fn, a0, a1, b0, b1, c, 3 * H,
                                                                 sm_count(), st);
     if (e) return e;
+    parts.end(3);
   }
-  return B200_OK;
+  return parts.status(fn);
+}
+
+extern "C" int b200_hybrid_train_backward_chunked(
+    const void* x, const void* g, const void* k, const void* v, const void* p_slab,
+    const void* r_slab, const void* g_out, const float* l1_grad, void* dx, void* dg, void* dk,
+    void* dv, int64_t M, int64_t D, int64_t H, int cf, int64_t tail_rows, void* workspace,
+    size_t workspace_bytes, void* scratch, size_t scratch_bytes, int64_t max_rows, void* stream) {
+  return b200_hybrid_train_backward_timed(x, g, k, v, p_slab, r_slab, g_out, l1_grad, dx, dg, dk, dv,
+                                          M, D, H, cf, tail_rows, workspace, workspace_bytes,
+                                          scratch, scratch_bytes, max_rows, nullptr, stream);
 }
 
 extern "C" int b200_hybrid_train_backward(const void* x, const void* g, const void* k, const void* v,

@@ -40,6 +40,7 @@ every row on the slabs: entries past a tile's capacity are dropped and counted.
 """
 from __future__ import annotations
 
+import ctypes
 import os
 import time
 from dataclasses import dataclass
@@ -254,7 +255,7 @@ def ff_forward_impl(X: torch.Tensor, G: torch.Tensor, K: torch.Tensor, V: torch.
     dropped, n_over = torch.empty((), **i32), torch.empty((), **i32)
     with _Timer("ff_forward_gated_total"):
         scratch = _train_scratch(dev, m, d, h, cap, 0)
-        _lib.call("b200_hybrid_train_forward", dev, Xf.data_ptr(), G.data_ptr(), K.data_ptr(),
+        _train_call("b200_hybrid_train_forward", _FORWARD_PARTS, dev, Xf.data_ptr(), G.data_ptr(), K.data_ptr(),
                   V.data_ptr(), out.data_ptr(), P.data_ptr(), R.data_ptr(), T.data_ptr(),
                   l0.data_ptr(), l1.data_ptr(), dropped.data_ptr(), n_over.data_ptr(), m, d, h, cf,
                   cap, *_lib.workspace(dev), scratch.data_ptr(), scratch.numel())
@@ -268,6 +269,22 @@ def _train_scratch(dev: torch.device, m: int, d: int, h: int, tail: int, bwd: in
     """Intermediate matrices of one call, from torch's allocator (never shared between calls)."""
     need = int(_lib.load_library().b200_hybrid_train_scratch_bytes(m, d, h, tail, bwd))
     return torch.empty(need, dtype=torch.uint8, device=dev)
+
+
+# Names of the timed parts of a call, in the library's order.
+_FORWARD_PARTS = ("gate_gemm_pack", "dense_tail_forward", "sddmm_R_T", "spmm_out")
+_BACKWARD_PARTS = ("dense_tail_backward", "sddmm_dT_dR_dU", "spmm_dX", "wgrad_dense_dK_dG_dV")
+
+
+def _train_call(fn: str, parts: tuple[str, ...], dev: torch.device, *args) -> None:
+    """``fn(*args)``; with profiling on, the times of its parts are kept for the report."""
+    if not _PERF_ENABLED:
+        _lib.call(fn, dev, *args)
+        return
+    ms = (ctypes.c_float * len(parts))()
+    _lib.call(fn + "_timed", dev, *args, 0, ctypes.addressof(ms))
+    for name, t in zip(parts, ms):
+        _PERF.setdefault(name, []).append(t)
 
 
 _CSC_SCRATCH: dict[tuple, dict[str, torch.Tensor]] = {}
@@ -315,7 +332,7 @@ def ff_backward_impl(X, G, K, V, P, R, T, gR, gl0, gl1):
         dG, dK, dV = torch.empty_like(G), torch.empty_like(K), torch.empty_like(V)
         with _Timer("ff_backward_gated_total"):
             scratch = _train_scratch(dev, m, d, h, cap, 1)
-            _lib.call("b200_hybrid_train_backward", dev, Xf.data_ptr(), G.data_ptr(),
+            _train_call("b200_hybrid_train_backward", _BACKWARD_PARTS, dev, Xf.data_ptr(), G.data_ptr(),
                       K.data_ptr(), V.data_ptr(), P.data_ptr(), R.data_ptr(), gRf.data_ptr(),
                       _lib.ptr(gl1_dev), dX.data_ptr(), dG.data_ptr(), dK.data_ptr(),
                       dV.data_ptr(), m, d, h, cf, cap, *_lib.workspace(dev), scratch.data_ptr(),

@@ -1,4 +1,6 @@
 """Hybrid operator registration: schemas, fake (meta) shapes, knobs, loader idempotence (CPU)."""
+import ctypes
+
 import pytest
 import torch
 
@@ -69,3 +71,25 @@ def test_dropin_registers_the_loader_name():
     from sparser_faster_llms_b200 import sparse_ops_loader
     assert sys.modules[dropin.LOADER_NAME] is sparse_ops_loader
     dropin.uninstall()
+
+
+def test_profiled_calls_keep_the_times_of_their_parts(monkeypatch):
+    calls = []
+
+    def call(fn, device, *args):
+        calls.append((fn, args[:-1]))
+        if fn.endswith("_timed"):
+            (ctypes.c_float * 4).from_address(args[-1])[:] = [1.0, 2.0, 3.0, 4.0]
+
+    monkeypatch.setattr(sparse_ops._lib, "call", call)
+    monkeypatch.setattr(sparse_ops, "_PERF", {})
+    for on in (False, True):
+        monkeypatch.setattr(sparse_ops, "_PERF_ENABLED", on)
+        sparse_ops._train_call("b200_hybrid_train_forward", sparse_ops._FORWARD_PARTS, None, 7, 8)
+        sparse_ops._train_call("b200_hybrid_train_backward", sparse_ops._BACKWARD_PARTS, None, 9)
+    assert [c[0] for c in calls] == ["b200_hybrid_train_forward", "b200_hybrid_train_backward",
+                                     "b200_hybrid_train_forward_timed",
+                                     "b200_hybrid_train_backward_timed"]
+    assert calls[2][1] == (7, 8, 0) and calls[3][1] == (9, 0)
+    assert sparse_ops._PERF == {n: [float(i % 4 + 1)] for i, n in enumerate(
+        sparse_ops._FORWARD_PARTS + sparse_ops._BACKWARD_PARTS)}
