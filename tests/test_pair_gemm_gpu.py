@@ -111,8 +111,9 @@ def test_gate_bias_of_any_alignment(offset):
     x, gate, up, down = synthetic.dyadic_case(m, d, h, seed=5)
     want = tf.pack_preactivations((fo.gate_preactivation(x, gate) + b).numpy(), 8)
     packed = twell.allocate_packed_output(m, h, device=DEV)
-    _lib.call("b200_twell_pack", torch.device(DEV), x.to(DEV).data_ptr(), gate.to(DEV).data_ptr(),
-              bias.data_ptr(), packed.data_ptr(), m, d, h, 8)
+    xg, gg = x.to(DEV), gate.to(DEV)  # held: a freed copy's memory would serve the next one
+    _lib.call("b200_twell_pack", torch.device(DEV), xg.data_ptr(), gg.data_ptr(), bias.data_ptr(),
+              packed.data_ptr(), m, d, h, 8)
     torch.cuda.synchronize()
     assert (packed.cpu().view(torch.int32).numpy().view("uint32") == want).all()
 
