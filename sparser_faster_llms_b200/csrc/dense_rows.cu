@@ -38,9 +38,9 @@ int sm_count();
 int pair_gemm_status();
 bool pair_mlp_serves(int64_t M, int64_t D, int64_t H, bool gated, bool hp);
 size_t pair_part_bytes(int64_t M, int64_t D, int64_t H);
-int pair_gate_up(bool hp, const void* x, const void* gate, const float* bias, const void* up,
-                 void* packed, void* hidden, int64_t M, int64_t D, int64_t H, int cf,
-                 bool keep_all, cudaStream_t stream);
+int pair_gate_up(const void* x, const void* gate, const float* bias, const void* up, void* packed,
+                 void* hidden, int64_t M, int64_t D, int64_t H, int cf, bool keep_all,
+                 cudaStream_t stream);
 int pair_down(const void* hidden, int terms, const void* down, void* out, int64_t M, int64_t D,
               int64_t H, const RunIf& run_if, const SplitRoom& room, cudaStream_t stream);
 
@@ -1318,7 +1318,7 @@ int b200_twell_gated_mlp_hybrid_counted(const void* x, const void* gate, const f
     if (counters != nullptr) w.counters = counters;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int tiles = (int)(H / kTileN), slab_w = kTileN / cf;
-    if (int rc = pair_gate_up(false, x, gate, gate_bias, up, packed, w.h_all, M, D, H, cf, true, st))
+    if (int rc = pair_gate_up(x, gate, gate_bias, up, packed, w.h_all, M, D, H, cf, true, st))
       return rc;
     const unsigned row_blocks = (unsigned)((M + 7) / 8);
     route_flags_kernel<<<row_blocks, 256, 0, st>>>(

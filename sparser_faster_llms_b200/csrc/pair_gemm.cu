@@ -79,17 +79,13 @@ int pair_pack(const void* x, const void* w, const float* bias, void* packed, voi
 }
 
 // hidden[M, H] (hp: [M, 3 H]) = gate values of the slabs times x up^T on their pattern.
-// row_slot / tail_p: rows whose gate values come from a dense matrix instead (may be null).
 int pair_up(bool hp, const void* x, const void* packed, const void* up, void* hidden, int64_t M,
-            int64_t D, int64_t H, int cf, const int* row_slot, const void* tail_p,
-            const RunIf& run_if, const SplitRoom& room, cudaStream_t stream) {
+            int64_t D, int64_t H, int cf, const RunIf& run_if, const SplitRoom& room, cudaStream_t stream) {
   pg::Args a = base_args(M, H, D);
   a.run_if = run_if;
   a.slab_p = const_cast<uint32_t*>(static_cast<const uint32_t*>(packed));
   a.slab_w = kTileN / cf;
   a.row_words = (int)(H / kTileN) * a.slab_w;
-  a.row_slot = row_slot;
-  a.tail_p = static_cast<const __nv_bfloat16*>(tail_p);
   a.out = static_cast<__nv_bfloat16*>(hidden);
   a.ld = hp ? 3 * H : H;
   a.wide = aligned32(hidden);
@@ -119,9 +115,9 @@ int pair_down(const void* hidden, int terms, const void* down, void* out, int64_
 // Slabs and hidden matrix in one launch: the gate and up products of a tile follow one another in
 // the two accumulators, and the pack epilogue of the first runs under the MMAs of the second.
 // keep_all: hidden values are computed from every gate positive, not only from the stored ones.
-int pair_gate_up(bool hp, const void* x, const void* gate, const float* bias, const void* up,
-                 void* packed, void* hidden, int64_t M, int64_t D, int64_t H, int cf,
-                 bool keep_all, cudaStream_t stream) {
+int pair_gate_up(const void* x, const void* gate, const float* bias, const void* up, void* packed,
+                 void* hidden, int64_t M, int64_t D, int64_t H, int cf, bool keep_all,
+                 cudaStream_t stream) {
   pg::Args a = base_args(M, H, D);
   a.bias = bias;
   a.bias16 = aligned16(bias);
@@ -130,13 +126,11 @@ int pair_gate_up(bool hp, const void* x, const void* gate, const float* bias, co
   a.slab_w = kTileN / cf;
   a.row_words = (int)(H / kTileN) * a.slab_w;
   a.out = static_cast<__nv_bfloat16*>(hidden);
-  a.ld = hp ? 3 * H : H;
+  a.ld = H;
   a.wide = aligned32(hidden);
   const pg::Operand ox = {x, M, D}, og = {gate, H, D}, ou = {up, H, D};
-  return hp ? pg::launch<pg::kGateUpHp, false, false>("gate and up products", ox, ox, og, ou, a, M,
-                                                      sm_count(), stream)
-            : pg::launch<pg::kGateUp, false, false>("gate and up products", ox, ox, og, ou, a, M,
-                                                    sm_count(), stream);
+  return pg::launch<pg::kGateUp, false, false>("gate and up products", ox, ox, og, ou, a, M,
+                                               sm_count(), stream);
 }
 
 namespace {
@@ -229,7 +223,7 @@ int pair_mlp(bool gated, bool hp, const void* x, const void* gate, const float* 
         return fail(B200_ECUDA, "fused MLP: cudaMemsetAsync failed");
     }
     if (gated && !choose) {
-      if (int rc = pair_gate_up(hp, xc, gate, bias, up, pc, scratch, m, D, H, cf, false, stream))
+      if (int rc = pair_gate_up(xc, gate, bias, up, pc, scratch, m, D, H, cf, false, stream))
         return rc;
     } else {
       pdl_suppressed() = choose;  // its predecessor is the memset
@@ -238,8 +232,7 @@ int pair_mlp(bool gated, bool hp, const void* x, const void* gate, const float* 
       pdl_suppressed() = false;
       if (rc) return rc;
       if (gated)
-        if (int rc = pair_up(hp, xc, pc, up, scratch, m, D, H, cf, nullptr, nullptr, run_if, room,
-                             stream))
+        if (int rc = pair_up(hp, xc, pc, up, scratch, m, D, H, cf, run_if, room, stream))
           return rc;
     }
     if (int rc = pair_down(scratch, terms, down, oc, m, D, H, run_if, room, stream))

@@ -48,7 +48,6 @@ enum Epilogue {
   kPack = 1,     // TwELL slabs of relu(acc + bias)
   kPackDense = 6,  // the same, and the stored values as a dense matrix
   kGateUp = 7,   // kPack on a first accumulator (B0) and kMul with its values on a second (B1)
-  kGateUpHp = 8, // kPack and kMulHp likewise
   kMul = 2,      // out = bf16(g * bf16(acc)) on the slab pattern, 0 elsewhere
   kMulHp = 3,    // g * acc in fp32, as three bf16 terms side by side (out row = [hi | mid | lo])
   kStoreCarry = 9,  // kStore on a product whose k comes in several launches: fp32 sums carried between
@@ -86,7 +85,7 @@ struct Args {
   uint32_t* slab_r;          // kFwd: output, kBwd: input
   uint32_t* slab_t;          // kFwd: output
   int slab_w, row_words;
-  // rows taken out of the slabs: row_slot[row] >= 0 is the row of tail_p / tail_r
+  // kFwd, kBwd, rows taken out of the slabs: row_slot[row] >= 0 is the row of tail_p / tail_r
   const int* row_slot;
   const __nv_bfloat16* tail_p;
   const __nv_bfloat16* tail_r;
@@ -213,8 +212,7 @@ __device__ __forceinline__ unsigned char* at(unsigned char* buf, int row, int of
 }
 
 // Pattern buffer of one warp: 32 rows x 128 columns of bf16 values (zero where nothing is stored),
-// filled from the slabs of tile `nt`, columns [128 half, +128); rows with a tail slot get their
-// dense values.
+// filled from the slabs of tile `nt`, columns [128 half, +128).
 __device__ __forceinline__ void load_values(const Args& a, unsigned char* buf, int row0, int rows,
                                             int nt, int half, int lane) {
 #pragma unroll
@@ -244,20 +242,6 @@ __device__ __forceinline__ void load_values(const Args& a, unsigned char* buf, i
               (uint16_t)(w[j] >> 16);
       }
       if (most < w0 + 32) break;
-    }
-  }
-  if (a.row_slot != nullptr) {
-    const int mine = row0 + lane < rows ? a.row_slot[row0 + lane] : -1;
-    uint32_t todo = __ballot_sync(0xffffffffu, mine >= 0);
-    __syncwarp();
-    while (todo != 0u) {
-      const int t = __ffs(todo) - 1;
-      todo &= todo - 1;
-      const int slot = __shfl_sync(0xffffffffu, mine, t);
-      const __nv_bfloat16* src =
-          a.tail_p + (size_t)slot * a.n_tiles * kTile + nt * kTile + half * 128 + lane * 4;
-      *reinterpret_cast<uint2*>(at(buf, t, lane * 8)) =
-          *reinterpret_cast<const uint2*>(src);
     }
   }
   __syncwarp();
@@ -594,7 +578,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap map_a0,
                  const __grid_constant__ CUtensorMap map_b0,
                  const __grid_constant__ CUtensorMap map_b1, const __grid_constant__ Args a) {
   constexpr uint32_t kIdesc = umma_idesc(256, 256) | (A_MN ? 1u << 15 : 0u) | (B_MN ? 1u << 16 : 0u);
-  constexpr bool kGate2 = EPI == kGateUp || EPI == kGateUpHp;
+  constexpr bool kGate2 = EPI == kGateUp;
   constexpr bool kIsPack = EPI == kPack || EPI == kPackDense || kGate2;
   constexpr bool kTrain = EPI == kFwd || EPI == kBwd;
   constexpr bool kPlain = EPI == kStore || EPI == kStoreCarry;
@@ -1003,7 +987,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap map_a0,
               }
             }
             if (live) store64(out + cb * 32, w, a.wide);
-          } else if (EPI == kMulHp || EPI == kGateUpHp) {
+          } else if (EPI == kMulHp) {
             uint4 g4[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j)
@@ -1123,7 +1107,8 @@ int launch(const char* fn, const Operand& a0, const Operand& a1, const Operand& 
   const int64_t slots = sm_count / 2;
   const bool can_sum = EPI == kStore && args.out_mt == 0 && !args.relu &&
                        args.ld == (long long)args.n_tiles * kTile;
-  Split sp = EPI != kGateUp && EPI != kGateUpHp && args.part != nullptr && args.counters != nullptr && args.rows_ptr == nullptr
+  Split sp = EPI != kGateUp && args.part != nullptr && args.counters != nullptr &&
+                     args.rows_ptr == nullptr
                  ? choose_split(tiles, args.ksteps, slots, can_sum)
                  : Split{tiles, 1};
   if (split_bytes(sp, tiles) > args.part_bytes) sp = {tiles, 1};
