@@ -93,9 +93,10 @@ def set_tail_rows_adaptive(on: bool) -> None:
     gate matrix (read back asynchronously, never waited for): twice the last count rounded up
     to 128 rows, at most ``tail_rows_regular`` - and no tail at all while the last count is
     zero (the call then only counts its overflow rows, so that the next one has a tail).  Off
-    (the default) the tail always spans ``min(tail_rows_regular, tokens)`` rows, which is what
-    the reference's forward computes (custom_op.cpp:125-127 sets the active rows to the
-    capacity).  The price of the adaptive form: the first call in which overflow rows appear,
+    (the default) the tail has room for ``min(tail_rows_regular, tokens)`` rows; its products
+    stop at the rows that overflowed, whose number the device knows (the reference's forward
+    computes the whole capacity, custom_op.cpp:125-127).  What the adaptive form saves is the
+    room.  The price of the adaptive form: the first call in which overflow rows appear,
     or more than doubles, leaves the excess rows on their slab prefix for that one call
     (counted in ``dropped``).  No reference counterpart."""
     _CONFIG["tail_rows_adaptive"] = 1 if on else 0

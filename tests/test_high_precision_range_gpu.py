@@ -4,7 +4,8 @@ infinite ones and finite ones above the largest bf16 must come out as from an fp
 A few tokens activate a neuron of their own whose gate and up values are powers of two: one hidden
 value of 2^128 - 2^117 (finite in fp32, rounds to infinity in bf16) with a down row scaled by 2^-100,
 one that overflows fp32 with a down row of +-1.  Reference: the oracle's slabs with fp64 products.
-Bound: one rounding of y to bf16, 2^-9.
+Bound: one rounding of y to bf16 (8 significant bits: half an ulp is at most 2^-8 of the value), and
+1e-3 for fp32 sums of some 180 terms of order 1.
 """
 import pytest
 import torch
@@ -48,5 +49,5 @@ def test_hidden_values_outside_the_range_of_bf16(m):
         else:
             ref = hr @ down.double()
             err = (y[r].double() - ref).abs()
-            assert bool((err <= 2.0 ** -9 * ref.abs() + 1e-3).all()), (r, float(err.max()))
+            assert bool((err <= 2.0 ** -8 * ref.abs() + 1e-3).all()), (r, float(err.max()))
     mod.destroy()

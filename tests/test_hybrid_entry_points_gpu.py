@@ -1,7 +1,8 @@
 """Hybrid entry points of the C ABI that the training operator itself no longer calls: sampled up product
 and dense-form weight gradients, against 64-bit products on the stored pattern.
 
-Bounds: a stored R is one bf16 rounding of an fp32 sum, 2^-9 of the value plus 1e-5 of the sum of magnitudes;
+Bounds: a stored R is one bf16 rounding of an fp32 sum, at most 2^-8 of the value (half an ulp of 8
+significant bits) plus 1e-5 of the sum of magnitudes;
 T is the exact bf16 product of stored values.  A weight gradient is one bf16 rounding of an fp32 sum:
 1.7e-3 in the 2-norm, with the order of summation below that.
 """
@@ -43,7 +44,7 @@ def test_sampled_up_product(m, d, h, cf):
     xr, kr = x.double()[rows], ffn.up.double()[cols]
     ref, size = (xr * kr).sum(1), (xr * kr).abs().sum(1)
     got = values(r, stored)
-    assert bool(((got.double() - ref).abs() <= 2.0 ** -9 * ref.abs() + 1e-5 * size).all())
+    assert bool(((got.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-5 * size).all())
     assert torch.equal(values(t, stored), got * values(p, stored))
     counts = p.view(*stored.shape[:2], -1)[:, :, 0]
     assert torch.equal(nnz, counts.sum(1).int())

@@ -46,8 +46,8 @@ def ops():
 
 @pytest.fixture(params=["sparse", "dense"])
 def wgrad_mode(request):
-    """Both forms of the weight-gradient products: column lists + transposed SpMM, and
-    scatter + tcgen05 GEMM (the automatic choice depends on the token count)."""
+    """Both forms of the backward: gathers along slabs and column lists, and dense products on
+    paired-SM tiles (the automatic choice)."""
     sparse_ops.set_weight_gradient_mode(request.param)
     yield request.param
     sparse_ops.set_weight_gradient_mode("auto")
