@@ -271,7 +271,7 @@ def pack_kernel_name(B: int, d: int, hl: int) -> str:
         return "twell_pack_kernel"
     if B <= 32:
         return "twell_pack_tc_splitk_wide_kernel"
-    if B <= 128 and tiles * 4 <= 148:
+    if (B <= 128 and tiles * 4 <= 148) or (B <= 256 and tiles <= 16):
         return "twell_pack_tc_splitk_mid_kernel"
     return "pair_gemm_kernel"
 

@@ -70,7 +70,7 @@ int b200_twell_pack(const void* x, const void* w, const float* bias, void* packe
 /*
  * Same as b200_twell_pack with the kernel family chosen by the caller:
  *   kernel 0 = automatic (M == 1: kernel 6 where it serves; M <= 16: kernel 1; 17..32: kernel 3
- *              or 5; 33..128: kernel 8 while its grid is one wave; beyond: kernel 7),
+ *              or 5; 33..256: kernel 8 while its grid is one wave; beyond: kernel 7),
  *   kernel 1 = mma.sync split-k cluster kernel (any M),
  *   kernel 3 = tcgen05 split-k cluster kernel (32 tokens per tile, D split 4 ways),
  *   kernel 5 = tcgen05 split-k cluster kernel with D split 8 ways (D % 512 == 0; chosen
@@ -81,7 +81,7 @@ int b200_twell_pack(const void* x, const void* w, const float* bias, void* packe
  *   kernel 7 = persistent tcgen05 kernel on pairs of SMs, 256 tokens x 256 neurons per pair, two
  *              accumulators (2 and 4 are other names of it),
  *   kernel 8 / 9 = tcgen05 split-k cluster kernel with 128-token tiles, D split 4 / 2 ways
- *              (8 is chosen automatically for 33..128 tokens while its grid is a single wave).
+ *              (8 is chosen automatically for 33..256 tokens while its grid is a single wave).
  * All produce identical slab bytes on exact-arithmetic inputs.  No reference
  * counterpart (the reference has one WGMMA kernel, matmul_d2t.cu:287-709).
  */

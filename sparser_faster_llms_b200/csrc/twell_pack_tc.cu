@@ -1,7 +1,7 @@
 // Gate projection + ReLU + TwELL pack on the 5th-generation tensor cores.
 //
 // Kernels of this file, by token count: twell_pack_tc_splitk_(wide_)kernel (17..32 tokens) and
-// twell_pack_tc_splitk_mid_kernel (33..128, 128-token tiles), both with D split over a cluster.
+// twell_pack_tc_splitk_mid_kernel (33..256, 128-token tiles), both with D split over a cluster.
 // Larger calls run on pairs of SMs (pair_gemm.cuh).
 //
 // CTA tile: one 256-neuron TwELL tile x NTOK tokens x a slice of D.
@@ -441,7 +441,7 @@ twell_pack_tc_splitk_wide_kernel(const __grid_constant__ CUtensorMap tmap_w,
 }
 
 // ---------------------------------------------------------------------------
-// Split-k kernel for 33..128 tokens (up to 256 on request): the decode kernel above with 128-token tiles.  A tile of
+// Split-k kernel for 33..256 tokens: the decode kernel above with 128-token tiles.  A tile of
 // 256 neurons x 128 tokens has only H / 256 CTAs to itself when d_model is not split (32 at
 // d_ff 8192: 32 SMs walking 32 latency-bound k-steps, 31-36 us per call whatever the token
 // count); split four ways over a cluster every SM streams a quarter of the weight rows.
@@ -756,15 +756,17 @@ int twell_pack_tc_splitk_mid(const void* x, const void* w, const float* bias, vo
   return launch_tc_splitk_mid<4, 4>(x, w, bias, packed, M, D, H, cf, stream);
 }
 
-// Cluster size for the 128-token split-k kernel: the largest of 4 and 2 whose grid is one
-// wave (one CTA per SM); 0 when neither is.  Measured on B200 (D 2048, d_ff 8192): 17.0 us
-// at 33..128 tokens against 27.4-29.5 us for unsplit tiles; at D 4096, d_ff 16384 and 128
-// tokens the four-way split needs two waves (45.6 against 50.2 us).
-int twell_pack_mid_split(int64_t M, int64_t H, int sm_count) {
-  const int64_t tiles = H / kTileN, blocks = (M + kTokMid - 1) / kTokMid;
-  if (tiles * 4 * blocks <= sm_count) return 4;
-  if (tiles * 2 * blocks <= sm_count) return 2;
-  return 0;
+// Whether 33..256 tokens take the 128-token kernel with D split four ways instead of 256-token tiles
+// on pairs of SMs: while its grid is one wave (one CTA per SM).  One block of tokens, D 2048,
+// H 8192: 15.9 against 19.4 us.  Two blocks double the clusters, and of clusters of four 33 are
+// resident at once (the rest of a GPC's SMs is no multiple of four), so the line lies at 16 tiles.
+// Measured on B200, 256 tokens, us, split-k / pairs: D 1024, H 4096 12.9 / 13.7; D 2048, H 1024
+// 13.8 / 18.4; D 2048, H 4096 15.0 / 19.0; D 4096, H 4096 19.5 / 29.7; 18 tiles (36 clusters),
+// D 2048, H 4608 27.0 / 19.1.
+bool twell_pack_mid_serves(int64_t M, int64_t H, int sm_count) {
+  const int64_t clusters = H / kTileN * ((M + kTokMid - 1) / kTokMid);
+  if (M <= 32 || M > 2 * kTokMid) return false;
+  return M <= kTokMid ? 4 * clusters <= sm_count : clusters <= sm_count / 4 - 4;
 }
 
 // Error word raised by a bounded wait that gave up (0 = none).  Reads and clears it;

@@ -532,3 +532,13 @@ def test_automatic_kernel_choice_at_every_token_count_boundary(m, d, h):
     got = out[:rows].float().cpu()
     assert fo.max_abs_and_rel_l2(got, ref)[1] < 2e-3
     assert _lib.load_library().b200_twell_pack_tc_status() == 0
+
+
+@pytest.mark.parametrize("m", [128, 129, 200, 256, 257])
+@pytest.mark.parametrize("d,h", [(1024, 4096), (1024, 4352), (512, 8448), (256, 9472)])
+def test_pack_on_both_sides_of_the_one_wave_line(m, d, h):
+    """Clusters of four with one or two blocks of 128 tokens up to the number that is resident at
+    once, pairs of SMs beyond: slab bit-exact on exact-arithmetic inputs."""
+    x, gate, _, _ = synthetic.dyadic_case(m, d, h, seed=m + d + h)
+    want = tf.pack_preactivations(fo.gate_preactivation(x, gate).numpy(), 8)
+    assert np.array_equal(to_np_u32(twell.matmul_sparse(x.to(DEV), gate.to(DEV))), want)
