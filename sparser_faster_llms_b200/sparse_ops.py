@@ -79,9 +79,9 @@ _PERF_ENABLED = os.environ.get("SPARSE_ENABLE_PERF_PROFILING", "0") not in ("0",
 def set_weight_gradient_mode(mode: str) -> None:
     """``"dense"`` and ``"auto"`` (the default): the backward runs as dense tensor-core products
     whose epilogues apply the slab pattern (``csrc/pair_gemm.cu``); deterministic.  ``"sparse"``:
-    gathers along the slabs and along column lists, whose order follows atomic arrival.  Measured
-    on B200 (16384 tokens, D = 1024, H = 4096, 41 positives per token), forward + backward: see
-    ``csrc/pair_gemm.cu``.  No reference counterpart: the reference always transposes the hybrid
+    gathers along the slabs and along column lists for all four gradients, whose order follows
+    atomic arrival.  Measured on B200 (D = 1024, H = 4096, 41 positives per token), forward +
+    backward, dense / sparse: 16384 tokens 1.0 / 2.0 ms, 999 tokens 0.33 / 0.92 ms.  No reference counterpart: the reference always transposes the hybrid
     container and runs its SpMM (custom_op.cpp:247-269)."""
     if mode not in ("sparse", "dense", "auto"):
         raise ValueError("mode must be 'sparse', 'dense' or 'auto'")
