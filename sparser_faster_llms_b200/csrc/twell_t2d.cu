@@ -213,10 +213,6 @@ twell_t2d_kernel(const __nv_bfloat16* x, const uint32_t* __restrict__ packed,
   for (int e = 0; e < 8; ++e) acc[e] = 0.f;
   int buf = 0;
 
-  // Up to 16 tokens the successor is usually the mma.sync pack kernel, whose small CTAs would become
-  // resident beside this kernel's and slow its row loads (D 4096, H 16384, eager layers: 2 tokens
-  // 45.2 -> 48.8 us, 4 tokens 51.3 -> 56.2, 16 tokens 69.7 -> 71.7).
-  if (M > 16) pdl_trigger();
   const __nv_bfloat16* up_lane = up + warp * 256 + lane * 8;
   const __nv_bfloat16* down_lane = down + warp * 256 + lane * 8;
   const __nv_bfloat162* x2 = reinterpret_cast<const __nv_bfloat162*>(&xv);
@@ -333,6 +329,13 @@ twell_t2d_kernel(const __nv_bfloat16* x, const uint32_t* __restrict__ packed,
     __syncthreads();  // entries are rewritten by the next chunk
   }
 
+  // The successor may become resident once every CTA has gathered its rows.  Not before the loop, whose
+  // code the trigger's memory clobber changes: fp32 products then took 3-5 % longer (D 2048, H 8192, 2 %,
+  // 777 tokens 171 against 162 us; D 4096, H 16384, 300 tokens 396 against 373), the others were level
+  // (32 tokens, H 8192 24.2 either way, 28 layers 716).  Up to 16 tokens the successor is usually the
+  // mma.sync pack kernel, whose small CTAs would become resident beside this kernel's and slow its
+  // row loads (D 4096, H 16384, eager layers: 2 tokens 45.2 -> 48.8 us, 16 tokens 69.7 -> 71.7).
+  if (M > 16) pdl_trigger();
   // Push this CTA's column sums to the owners: CTA r owns columns [r*cols, (r+1)*cols)
   // and receives rank q's contribution in inbox[q*cols .. (q+1)*cols).
   const int cols = D / cs;
