@@ -1057,8 +1057,12 @@ sum_ranges_kernel(const float4* __restrict__ sums, uint2* __restrict__ out, int 
 
 // How the tiles of the last wave are cut along k: as many equal ranges as still fit the wave, at
 // least 4 k-steps each.  A product of less than one wave whose sums go to memory (`all`) takes up
-// to 8 ranges, added by a kernel of their own on all SMs; the last wave of a larger one up to 4,
-// added by the warps that arrive last.
+// to 8 ranges, added by a kernel of their own on all SMs; the last wave of another one up to 4,
+// added by the warps that arrive last.  Those warps read the sums back in eight dependent rounds, so
+// short products are left whole: non-gated MLP, 2 %, us, cut / whole: 16 k-steps (D 1024, H 4096)
+// 1200 tokens 59.7 / 51.9; 32 (D 2048, H 8192) 1200 tokens 110 / 106, 3000 tokens 174 / 171;
+// 64 (D 4096, H 16384) 640 tokens 181 / 184, 1200 tokens 266 / 270.
+constexpr int kCutKsteps = 64;
 struct Split {
   int64_t full_tiles;
   int splits;
@@ -1066,9 +1070,11 @@ struct Split {
 inline Split choose_split(int64_t tiles, int ksteps, int64_t slots, bool all) {
   const int64_t tail = tiles % slots;
   if (tail == 0) return {tiles, 1};
+  const bool own_kernel = all && tiles < slots;
+  if (!own_kernel && ksteps < kCutKsteps) return {tiles, 1};
   int64_t s = slots / tail;
   if (s > ksteps / 4) s = ksteps / 4;
-  if (s > (all && tiles < slots ? 8 : 4)) s = all && tiles < slots ? 8 : 4;
+  if (s > (own_kernel ? 8 : 4)) s = own_kernel ? 8 : 4;
   if (s < 2) return {tiles, 1};
   return {tiles - tail, (int)s};
 }

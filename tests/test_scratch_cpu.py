@@ -8,7 +8,7 @@ import pytest
 
 from sparser_faster_llms_b200 import _lib, build
 
-PAIRS, TILE, STAGE_K = 74, 256, 64
+PAIRS, TILE, STAGE_K, CUT_KSTEPS = 74, 256, 64, 64
 SHAPES = [(1024, 4096), (2048, 5632), (2048, 8192), (2048, 11008), (4096, 11008), (4096, 16384)]
 
 
@@ -21,9 +21,10 @@ def lib():
 def range_bytes(tiles, k, own_kernel):
     """fp32 sums of the ranges that a product of `tiles` tiles is cut into."""
     ksteps, tail = -(-k // STAGE_K), tiles % PAIRS
-    if tail == 0:
+    own_kernel = own_kernel and tiles < PAIRS
+    if tail == 0 or (not own_kernel and ksteps < CUT_KSTEPS):
         return 0
-    most = 8 if own_kernel and tiles < PAIRS else 4
+    most = 8 if own_kernel else 4
     splits = min(PAIRS // tail, ksteps // 4, most)
     return 0 if splits < 2 else tail * splits * TILE * TILE * 4
 
