@@ -432,7 +432,9 @@ int b200_twell_gated_t2d_hybrid(const void* x, const void* packed, const void* g
                                 void* hybrid_ws, size_t hybrid_ws_bytes, void* workspace,
                                 size_t workspace_bytes, void* stream);
 
-/* b200_twell_pack followed by b200_twell_gated_t2d_hybrid. */
+/* b200_twell_pack followed by b200_twell_gated_t2d_hybrid; where the call is large enough for the
+ * dense form of b200_twell_gated_mlp_scratch and hybrid_ws holds the hidden matrix of all rows, every
+ * row runs in that form and routing decides which overflowed rows keep all their positives. */
 int b200_twell_gated_mlp_hybrid(const void* x, const void* gate, const float* gate_bias,
                                 const void* up, const void* down, const void* down_t,
                                 void* packed, void* out, int64_t M, int64_t D, int64_t H, int cf,

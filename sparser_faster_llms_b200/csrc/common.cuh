@@ -63,12 +63,12 @@ inline int ensure_dynamic_smem(Kernel kern, size_t bytes, size_t (&granted)[64],
 // (the wait returns once the predecessor grid has completed and its memory is visible).
 // pdl_wait() is a no-op in a kernel launched without the attribute.
 //
-// The contraction of more than 16 tokens and the one-token layer kernel also issue pdl_trigger(): their successor's CTAs
-// become resident as their own CTAs leave, and use the time until pdl_wait() returns to set up
-// and to ask L2 for the first part of their weights (a quarter: asking for all of it, or from
-// inside the predecessor, fetches rows that are gone from L2 again when they are read).  Neither
-// alone gains much; together, 28 layers of D 2048, H 8192: one token 370 -> 342 us, 32 tokens
-// 757 -> 700 us.  The pack kernels do not: a contraction that is resident early has nothing to
+// The contraction of more than 16 tokens and the one-token layer kernel also issue pdl_trigger(),
+// behind their row loads: their successor's CTAs become resident as their own CTAs leave, and use
+// the time until pdl_wait() returns to set up and to ask L2 for the first part of their weights (a
+// quarter: asking for all of it, or from inside the predecessor, fetches rows that are gone from L2
+// again when they are read).  Neither alone gains much; together, 28 layers of D 2048, H 8192: one
+// token 370 -> 342 us, 32 tokens 757 -> 700 us.  The pack kernels do not: a contraction that is resident early has nothing to
 // fetch and takes shared memory and L1 from them (832 us at 32 tokens).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

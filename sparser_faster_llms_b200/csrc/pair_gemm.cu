@@ -140,10 +140,16 @@ namespace {
 bool rows_in_l2(int64_t D, int64_t H) { return 4 * H * D <= (int64_t)100 << 20; }
 
 // From this many tokens on the products are dense.  Measured under graph replay with weights from
-// HBM, us per layer, gather form at 0.5 % / 2 % density -> dense form (any density):
-//   D 1024, H 4096:   256 tokens 27 / 37 -> 34;  512 tokens 35 / 53 -> 35;  1024 tokens 41 / 73 -> 39
-//   D 2048, H 8192:   128 tokens 32 / 48 -> 50;  256 tokens 48 / 84 -> 51;  512 tokens 69 / 140 -> 58
-//   D 4096, H 16384:  64 tokens 91 (1 %) -> 93;  128 tokens 123 (1 %) -> 98
+// HBM, us per layer, gather form at 0.5 % / 1 % / 2 % density -> dense form (any density):
+//   D 1024, H 4096:   256 tokens 25 / 29 / 36 -> 34;  320 tokens 33 / 38 / 48 -> 35;
+//                     800 tokens 37 / 46 / 63 -> 39;  1200 tokens 43 / 55 / 77 -> 54
+//   D 2048, H 8192:   128 tokens 30 / 37 / 49 -> 50;  160 tokens 46 / 57 / 80 -> 50;
+//                     512 tokens 68 / 92 / 135 -> 57;  800 tokens 77 / 109 / 169 -> 92
+//   D 2048, H 11008:  256 tokens 61 / 77 / 107 -> 54;  300 tokens 63 / 82 / 123 -> 82
+//   D 4096, H 16384:  64 tokens - / 91 / - -> 93;  96 tokens 88 / 122 / 182 -> 95
+// The call cannot know its density: the lines lie where the dense form is level or ahead at 1 %.  At
+// 0.5 % it is up to 1.3 times slower where the tiles just exceed a wave (300 tokens at H 11008,
+// 800 at H 8192, 1200 at H 4096), and level or ahead elsewhere.
 int64_t dense_from(int64_t D, int64_t H) {
   return D * H <= (int64_t)1 << 23 ? 320 : rows_in_l2(D, H) ? 160 : 96;
 }
@@ -160,11 +166,13 @@ bool pair_mlp_serves(int64_t M, int64_t D, int64_t H, bool gated, bool hp) {
 
 // Whether the device chooses between the dense and the gather form of the up and down products by
 // the stored entries of the call (two launches that return at once and a 4-byte memset, about
-// 10 us); otherwise gate and up run in one launch and the dense form always.  At 0.5 % density
-// the always-dense form is level with the gather form up to 4096 tokens (D 2048, H 8192: 305
-// against 301 us) and ahead of it at D 1024 (88 against 96 us) and D 4096 (1152 against 1407 us).
-// At 16384 tokens, D 2048, H 8192: gather 1070 us at 0.5 %, dense 1280 at any density, gather
-// 2650 at 2 %.
+// 10 us); otherwise gate and up run in one launch and the dense form always.  At 0.5 % density, us,
+// always dense / gather: D 2048, H 8192, 1600 tokens 171 / 141, 2048 tokens 173 / 160, 4096 tokens
+// 295 / 302; D 1024, H 4096, 2048 tokens 60 / 54, 4096 tokens 89 / 97; D 4096, H 16384, 2048 tokens
+// 572 / 745.  At 16384 tokens, D 2048, H 8192: gather 1103 us at 0.5 %, dense 1217 at any density,
+// gather 2659 at 2 %.  The non-gated MLP, whose dense form saves less, always asks; what asking costs
+// at low density: D 1024, H 4096, 1200 tokens 45 against 35 us at 0.5 %, 52 / 52 at 2 %, 53 / 84 at
+// 5 %; D 2048, H 8192, 800 tokens 69 / 58, 79 / 105, 80 / 193.
 static bool choose_on_device(int64_t M, int64_t D, int64_t H, bool gated, bool hp) {
   if (hp || !gated) return true;
   return M > 4096 && rows_in_l2(D, H) && 4 * H * D > (int64_t)32 << 20;
