@@ -329,10 +329,10 @@ twell_t2d_kernel(const __nv_bfloat16* x, const uint32_t* __restrict__ packed,
     __syncthreads();  // entries are rewritten by the next chunk
   }
 
-  // The successor may become resident once every CTA has gathered its rows.  Not before the loop, whose
-  // code the trigger's memory clobber changes: fp32 products then took 3-5 % longer (D 2048, H 8192, 2 %,
-  // 777 tokens 171 against 162 us; D 4096, H 16384, 300 tokens 396 against 373), the others were level
-  // (32 tokens, H 8192 24.2 either way, 28 layers 716).  Up to 16 tokens the successor is usually the
+  // The successor may become resident once every CTA has gathered its rows.  Not before the loop: a
+  // trigger there changes the loop's code, also where it is not reached, and fp32 products then took 3-5 %
+  // longer (D 2048, H 8192, 2 %, 777 tokens 171 against 162 us; D 4096, H 16384, 300 tokens 396 against
+  // 373); the others were level (32 tokens, H 8192 24.2 either way, 28 layers 716).  Up to 16 tokens the successor is usually the
   // mma.sync pack kernel, whose small CTAs would become resident beside this kernel's and slow its
   // row loads (D 4096, H 16384, eager layers: 2 tokens 45.2 -> 48.8 us, 16 tokens 69.7 -> 71.7).
   if (M > 16) pdl_trigger();

@@ -256,10 +256,11 @@ def ff_forward_impl(X: torch.Tensor, G: torch.Tensor, K: torch.Tensor, V: torch.
     dropped, n_over = torch.empty((), **i32), torch.empty((), **i32)
     with _Timer("ff_forward_gated_total"):
         scratch = _train_scratch(dev, m, d, h, cap, 0)
-        _train_call("b200_hybrid_train_forward", _FORWARD_PARTS, dev, Xf.data_ptr(), G.data_ptr(), K.data_ptr(),
-                  V.data_ptr(), out.data_ptr(), P.data_ptr(), R.data_ptr(), T.data_ptr(),
-                  l0.data_ptr(), l1.data_ptr(), dropped.data_ptr(), n_over.data_ptr(), m, d, h, cf,
-                  cap, *_lib.workspace(dev), scratch.data_ptr(), scratch.numel())
+        _train_call("b200_hybrid_train_forward", _FORWARD_PARTS, dev, Xf.data_ptr(), G.data_ptr(),
+                    K.data_ptr(), V.data_ptr(), out.data_ptr(), P.data_ptr(), R.data_ptr(),
+                    T.data_ptr(), l0.data_ptr(), l1.data_ptr(), dropped.data_ptr(),
+                    n_over.data_ptr(), m, d, h, cf, cap, *_lib.workspace(dev), scratch.data_ptr(),
+                    scratch.numel())
     if _CONFIG["tail_rows_adaptive"] and not _CONFIG["discard_overflow"] \
             and _CONFIG["tail_rows_regular"] > 0:
         _tail_observe(tail_key, n_over)
@@ -333,11 +334,11 @@ def ff_backward_impl(X, G, K, V, P, R, T, gR, gl0, gl1):
         dG, dK, dV = torch.empty_like(G), torch.empty_like(K), torch.empty_like(V)
         with _Timer("ff_backward_gated_total"):
             scratch = _train_scratch(dev, m, d, h, cap, 1)
-            _train_call("b200_hybrid_train_backward", _BACKWARD_PARTS, dev, Xf.data_ptr(), G.data_ptr(),
-                      K.data_ptr(), V.data_ptr(), P.data_ptr(), R.data_ptr(), gRf.data_ptr(),
-                      _lib.ptr(gl1_dev), dX.data_ptr(), dG.data_ptr(), dK.data_ptr(),
-                      dV.data_ptr(), m, d, h, cf, cap, *_lib.workspace(dev), scratch.data_ptr(),
-                      scratch.numel())
+            _train_call("b200_hybrid_train_backward", _BACKWARD_PARTS, dev, Xf.data_ptr(),
+                        G.data_ptr(), K.data_ptr(), V.data_ptr(), P.data_ptr(), R.data_ptr(),
+                        gRf.data_ptr(), _lib.ptr(gl1_dev), dX.data_ptr(), dG.data_ptr(),
+                        dK.data_ptr(), dV.data_ptr(), m, d, h, cf, cap, *_lib.workspace(dev),
+                        scratch.data_ptr(), scratch.numel())
         _LAST_TRANSPOSE_OVERFLOW = dev  # no column lists: nothing can overflow
         return dX.reshape(X.shape), dG, dK, dV
     # "sparse": gathers along the slabs and along column lists

@@ -138,3 +138,12 @@ def test_rows_beyond_the_dense_capacity_stay_lossy():
     assert err[taken].max() < 1.5e-2 and err[hot & ~taken].max() > 0.1
     plain.destroy()
     routed.destroy()
+
+
+@pytest.mark.parametrize("m,h,hp,gated", [(400, 2304, False, False), (1000, 2048, False, False),
+                                          (8192, 2048, True, True)])
+@pytest.mark.parametrize("kind", ["plain", "dense"])
+def test_last_wave_cut_along_k(m, h, hp, gated, kind):
+    """64 k-steps: the tiles of the last wave are cut in four (18 tiles) or two (32 and 34) ranges, whose sums
+    the warps that arrive last add; gate values and the dense operand come out of the sums."""
+    assert run_case(m, 4096, h, hp=hp, gated=gated, dense=kind == "dense") > 0

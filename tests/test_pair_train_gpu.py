@@ -107,3 +107,10 @@ def test_entry_counts_around_the_words_fetched_ahead(width, density):
     """Means of 26 / 51 / 13 / 90 entries per 256-neuron tile: more than the 16 slab words that
     are fetched ahead, a few of them only, and (first two) full slabs with overflowed rows."""
     run_case(97, 256, 768, density, width=width)
+
+
+@pytest.mark.parametrize("m", [300, 1100])
+def test_last_wave_cut_along_k(m):
+    """64 k-steps and more: 16 tiles of gate, R / T and dT in four ranges each; 80 tiles of dX, the last
+    six in four."""
+    run_case(m, 4096, 2048, 0.03)

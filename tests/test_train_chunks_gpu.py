@@ -34,7 +34,7 @@ def chunked(monkeypatch):
 
 @pytest.mark.parametrize("m,d,h,max_rows,hot", [
     (999, 1024, 4096, 256, 0), (1300, 256, 2048, 512, 0), (300, 768, 1280, 1, 0),
-    (700, 512, 2048, 256, 9)])
+    (700, 512, 2048, 256, 9), (9000, 512, 1280, 4096, 0)])  # the last: carried sums of tiles cut along k
 def test_chunks_of_a_step(chunked, m, d, h, max_rows, hot):
     seen = chunked(max_rows)
     taken, left = run_case(m, d, h, 0.03, hot=hot)
