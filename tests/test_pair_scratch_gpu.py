@@ -68,3 +68,31 @@ def test_scratch_of_any_16_byte_alignment(m, hp, offset):
     assert _lib.load_library().b200_twell_hybrid_status() == 0
     assert torch.equal(outs[0], outs[1])
     assert bool((scratch[need + offset:] == 0x5A).all())
+
+
+@pytest.mark.parametrize("m,d,h,gated,hp", [(160, 2048, 8192, True, False), (400, 4096, 2304, False, False),
+                                            (4096, 2048, 8192, True, True)])
+def test_without_a_workspace_no_tile_is_cut(m, d, h, gated, hp):
+    """Calls whose tiles are cut along k when there are counters for it, here without a workspace."""
+    flags = _lib.FLAG_HIGH_PRECISION if hp else 0
+    need = _lib.load_library().b200_twell_mlp_scratch_bytes(m, d, h, int(gated), flags)
+    assert need > 0
+    x, gate, up, down = synthetic.dyadic_case(m, d, h, seed=m + h)
+    want = tf.pack_preactivations(fo.gate_preactivation(x, gate).numpy(), 8)
+    xg, gg, ug, dg = (t.to(DEV) for t in (x, gate, up, down))
+    packed = twell.allocate_packed_output(m, h, device=DEV)
+    out = torch.empty_like(xg)
+    scratch = torch.empty(need, dtype=torch.uint8, device=DEV)
+    if gated:
+        _lib.call("b200_twell_gated_mlp_scratch", DEV, xg.data_ptr(), gg.data_ptr(), None,
+                  ug.data_ptr(), dg.data_ptr(), packed.data_ptr(), out.data_ptr(), m, d, h, 8,
+                  flags, None, 0, scratch.data_ptr(), need)
+    else:
+        _lib.call("b200_twell_mlp_scratch", DEV, xg.data_ptr(), gg.data_ptr(), dg.data_ptr(),
+                  packed.data_ptr(), out.data_ptr(), m, d, h, 8, 2, None, 0, scratch.data_ptr(), need)
+    torch.cuda.synchronize()
+    assert _lib.load_library().b200_twell_hybrid_status() == 0
+    assert (packed.cpu().view(torch.int32).numpy().view("uint32") == want).all()
+    rows = [0, 127, 128, m // 2, m - 1]
+    ref = hidden_of(x[rows], up if gated else None, want[rows], h, 8, hp) @ down.double()
+    assert ((out[rows].double().cpu() - ref).norm() / ref.norm()).item() < REL
