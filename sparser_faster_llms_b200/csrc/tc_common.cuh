@@ -21,6 +21,14 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return (uint32_t)__cvta_generic_to_shared(p);
 }
 
+// True for one lane of a converged warp.  Unlike a test of the lane number it tells the compiler that
+// exactly one thread goes on, so operands of TMA and tcgen05 instructions need no per-lane handling.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n.reg .pred q;\nelect.sync _|q, 0xffffffff;\nselp.u32 %0, 1, 0, q;\n}" : "=r"(p));
+  return p != 0;
+}
+
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
 }
@@ -157,6 +165,51 @@ __device__ __forceinline__ bool epi_barrier_and(bool v) {
       : "r"((uint32_t)v)
       : "memory");
   return r != 0;
+}
+
+// Producer and MMA threads of a ring of STAGES shared-memory stages, `ksteps` steps through it.  Both are
+// bound by the instructions of their one thread (a step of four MMAs is 128 to 512 clocks), so they are
+// entered through elect_one(), the stage and phase are counted instead of computed and nothing is polled
+// but the step's own barrier: a wait that gives up ends the role (false), and the other roles' waits on it
+// run out in turn.  Pack of 32 tokens, D 2048, H 8192: 28 layers of pack + contraction 713 -> 702 us.
+template <int STAGES, typename Load>
+__device__ __forceinline__ bool ring_produce(uint64_t* full, uint64_t* empty, int ksteps, uint32_t bytes,
+                                             Load load) {
+  int s = 0, k = 0;
+  uint32_t phase = 1;
+#pragma unroll 1
+  for (; k < ksteps; ++k) {
+    if (!mbar_wait(&empty[s], phase)) break;
+    mbar_expect_tx(&full[s], bytes);
+    load(k, s);
+    if (++s == STAGES) {
+      s = 0;
+      phase ^= 1u;
+    }
+  }
+  if (k == ksteps) return true;
+  for (int j = k > STAGES ? k - STAGES : 0; j < k; ++j)  // copies in flight land before the CTA leaves
+    mbar_wait(&full[j % STAGES], (uint32_t)(j / STAGES) & 1u);
+  return false;
+}
+
+// step(first, stage) issues the MMAs of a k-step.
+template <int STAGES, typename Step>
+__device__ __forceinline__ bool ring_issue(uint64_t* full, uint64_t* empty, int ksteps, Step step) {
+  int s = 0;
+  uint32_t phase = 0;
+#pragma unroll 1
+  for (int k = 0; k < ksteps; ++k) {
+    if (!mbar_wait(&full[s], phase)) return false;
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    step(k == 0, s);
+    umma_commit(&empty[s]);
+    if (++s == STAGES) {
+      s = 0;
+      phase ^= 1u;
+    }
+  }
+  return true;
 }
 
 // Named barrier `id` (1..15) for `count` threads (a multiple of 32).

@@ -115,47 +115,36 @@ twell_pack_tc_splitk_kernel(const __grid_constant__ CUtensorMap tmap_w,
   pdl_wait();
 
   if (warp == 0) {
-    if (lane == 0) {
-      for (int k = 0; k < ksteps && !abort_s; ++k) {
-        const int s = k % STAGES;
-        const uint32_t phase = (uint32_t)(k / STAGES) & 1u;
-        if (!mbar_wait(&empty_bar[s], phase ^ 1u)) {
-          abort_s = 1;
-          atomicExch(&g_tc_error, 1);
-          break;
-        }
-        unsigned char* st = smem + (size_t)s * kStageBytes;
-        mbar_expect_tx(&full_bar[s], (uint32_t)kStageBytes);
-        const int kcoord = k_base + k * kStageK;
-        // one copy for the tile's 256 weight rows (A0 | A1 are contiguous): a copy costs the
-        // producer thread about 160 ns whatever its size
-        tma_load_2d(st, &tmap_w, kcoord, tile * kTileN, &full_bar[s]);
-        tma_load_2d(st + 2 * kATileBytes, &tmap_x, kcoord, m0, &full_bar[s]);
-      }
+    if (elect_one() &&
+        !ring_produce<STAGES>(full_bar, empty_bar, ksteps, kStageBytes, [&](int k, int s) {
+          unsigned char* st = smem + (size_t)s * kStageBytes;
+          const int kcoord = k_base + k * kStageK;
+          // one copy for the tile's 256 weight rows (A0 | A1 are contiguous)
+          tma_load_2d(st, &tmap_w, kcoord, tile * kTileN, &full_bar[s]);
+          tma_load_2d(st + 2 * kATileBytes, &tmap_x, kcoord, m0, &full_bar[s]);
+        })) {
+      abort_s = 1;
+      atomicExch(&g_tc_error, 1);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      for (int k = 0; k < ksteps && !abort_s; ++k) {
-        const int s = k % STAGES;
-        const uint32_t phase = (uint32_t)(k / STAGES) & 1u;
-        if (!mbar_wait(&full_bar[s], phase)) {
-          abort_s = 1;
-          atomicExch(&g_tc_error, 2);
-          break;
-        }
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t a0 = smem_u32(smem + (size_t)s * kStageBytes);
-        const uint64_t da0 = umma_desc(a0), da1 = umma_desc(a0 + kATileBytes),
-                       db = umma_desc(a0 + 2 * kATileBytes);
+    const uint64_t d0 = umma_desc(smem_u32(smem));
+    if (elect_one()) {
+      const bool done = ring_issue<STAGES>(full_bar, empty_bar, ksteps, [&](bool first, int s) {
+        const uint64_t da0 = d0 + (uint32_t)s * (kStageBytes >> 4), da1 = da0 + (kATileBytes >> 4),
+                       db = da0 + (2 * kATileBytes >> 4);
 #pragma unroll
         for (int kk = 0; kk < kStageK / 16; ++kk) {
-          const uint32_t acc = (k > 0 || kk > 0) ? 1u : 0u;
+          const uint32_t acc = !first || kk > 0 ? 1u : 0u;
           umma_bf16(tmem_base, da0 + 2 * kk, db + 2 * kk, kIdesc, acc);
           umma_bf16(tmem_base + NTOK, da1 + 2 * kk, db + 2 * kk, kIdesc, acc);
         }
-        umma_commit(&empty_bar[s]);
+      });
+      if (done) {
+        umma_commit(&acc_bar);
+      } else {
+        abort_s = 1;
+        atomicExch(&g_tc_error, 2);
       }
-      if (!abort_s) umma_commit(&acc_bar);
     }
   } else {
     // ---- epilogue part 1: TMEM -> registers -> owner CTA's shared memory ----
@@ -313,47 +302,36 @@ twell_pack_tc_splitk_wide_kernel(const __grid_constant__ CUtensorMap tmap_w,
   pdl_wait();
 
   if (warp == 0) {
-    if (lane == 0) {
-      for (int k = 0; k < ksteps && !abort_s; ++k) {
-        const int s = k % STAGES;
-        const uint32_t phase = (uint32_t)(k / STAGES) & 1u;
-        if (!mbar_wait(&empty_bar[s], phase ^ 1u)) {
-          abort_s = 1;
-          atomicExch(&g_tc_error, 1);
-          break;
-        }
-        unsigned char* st = smem + (size_t)s * kStageBytes;
-        mbar_expect_tx(&full_bar[s], (uint32_t)kStageBytes);
-        const int kcoord = k_base + k * kStageK;
-        // one copy for the tile's 256 weight rows (A0 | A1 are contiguous): a copy costs the
-        // producer thread about 160 ns whatever its size
-        tma_load_2d(st, &tmap_w, kcoord, tile * kTileN, &full_bar[s]);
-        tma_load_2d(st + 2 * kATileBytes, &tmap_x, kcoord, m0, &full_bar[s]);
-      }
+    if (elect_one() &&
+        !ring_produce<STAGES>(full_bar, empty_bar, ksteps, kStageBytes, [&](int k, int s) {
+          unsigned char* st = smem + (size_t)s * kStageBytes;
+          const int kcoord = k_base + k * kStageK;
+          // one copy for the tile's 256 weight rows (A0 | A1 are contiguous)
+          tma_load_2d(st, &tmap_w, kcoord, tile * kTileN, &full_bar[s]);
+          tma_load_2d(st + 2 * kATileBytes, &tmap_x, kcoord, m0, &full_bar[s]);
+        })) {
+      abort_s = 1;
+      atomicExch(&g_tc_error, 1);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      for (int k = 0; k < ksteps && !abort_s; ++k) {
-        const int s = k % STAGES;
-        const uint32_t phase = (uint32_t)(k / STAGES) & 1u;
-        if (!mbar_wait(&full_bar[s], phase)) {
-          abort_s = 1;
-          atomicExch(&g_tc_error, 2);
-          break;
-        }
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t a0 = smem_u32(smem + (size_t)s * kStageBytes);
-        const uint64_t da0 = umma_desc(a0), da1 = umma_desc(a0 + kATileBytes),
-                       db = umma_desc(a0 + 2 * kATileBytes);
+    const uint64_t d0 = umma_desc(smem_u32(smem));
+    if (elect_one()) {
+      const bool done = ring_issue<STAGES>(full_bar, empty_bar, ksteps, [&](bool first, int s) {
+        const uint64_t da0 = d0 + (uint32_t)s * (kStageBytes >> 4), da1 = da0 + (kATileBytes >> 4),
+                       db = da0 + (2 * kATileBytes >> 4);
 #pragma unroll
         for (int kk = 0; kk < kStageK / 16; ++kk) {
-          const uint32_t acc = (k > 0 || kk > 0) ? 1u : 0u;
+          const uint32_t acc = !first || kk > 0 ? 1u : 0u;
           umma_bf16(tmem_base, da0 + 2 * kk, db + 2 * kk, kIdesc, acc);
           umma_bf16(tmem_base + NTOK, da1 + 2 * kk, db + 2 * kk, kIdesc, acc);
         }
-        umma_commit(&empty_bar[s]);
+      });
+      if (done) {
+        umma_commit(&acc_bar);
+      } else {
+        abort_s = 1;
+        atomicExch(&g_tc_error, 2);
       }
-      if (!abort_s) umma_commit(&acc_bar);
     }
   } else {
     // ---- epilogue part 1: TMEM -> registers -> owner CTA's shared memory ----
@@ -516,45 +494,35 @@ twell_pack_tc_splitk_mid_kernel(const __grid_constant__ CUtensorMap tmap_w,
 
   bool ok = true;
   if (warp == 0) {
-    if (lane == 0) {
-      for (int k = 0; k < ksteps && !abort_s; ++k) {
-        const int s = k % STAGES;
-        const uint32_t phase = (uint32_t)(k / STAGES) & 1u;
-        if (!mbar_wait(&empty_bar[s], phase ^ 1u)) {
-          abort_s = 1;
-          atomicExch(&g_tc_error, 1);
-          break;
-        }
-        unsigned char* st = smem + (size_t)s * kStageBytes;
-        mbar_expect_tx(&full_bar[s], (uint32_t)kStageBytes);
-        const int kcoord = k_base + k * kStageK;
-        tma_load_2d(st, &tmap_w, kcoord, tile * kTileN, &full_bar[s]);  // 256 rows: A0 | A1
-        tma_load_2d(st + 2 * kATileBytes, &tmap_x, kcoord, m0, &full_bar[s]);
-      }
+    if (elect_one() &&
+        !ring_produce<STAGES>(full_bar, empty_bar, ksteps, kStageBytes, [&](int k, int s) {
+          unsigned char* st = smem + (size_t)s * kStageBytes;
+          const int kcoord = k_base + k * kStageK;
+          tma_load_2d(st, &tmap_w, kcoord, tile * kTileN, &full_bar[s]);  // 256 rows: A0 | A1
+          tma_load_2d(st + 2 * kATileBytes, &tmap_x, kcoord, m0, &full_bar[s]);
+        })) {
+      abort_s = 1;
+      atomicExch(&g_tc_error, 1);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      for (int k = 0; k < ksteps && !abort_s; ++k) {
-        const int s = k % STAGES;
-        const uint32_t phase = (uint32_t)(k / STAGES) & 1u;
-        if (!mbar_wait(&full_bar[s], phase)) {
-          abort_s = 1;
-          atomicExch(&g_tc_error, 2);
-          break;
-        }
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t a0 = smem_u32(smem + (size_t)s * kStageBytes);
-        const uint64_t da0 = umma_desc(a0), da1 = umma_desc(a0 + kATileBytes),
-                       db = umma_desc(a0 + 2 * kATileBytes);
+    const uint64_t d0 = umma_desc(smem_u32(smem));
+    if (elect_one()) {
+      const bool done = ring_issue<STAGES>(full_bar, empty_bar, ksteps, [&](bool first, int s) {
+        const uint64_t da0 = d0 + (uint32_t)s * (kStageBytes >> 4), da1 = da0 + (kATileBytes >> 4),
+                       db = da0 + (2 * kATileBytes >> 4);
 #pragma unroll
         for (int kk = 0; kk < kStageK / 16; ++kk) {
-          const uint32_t acc = (k > 0 || kk > 0) ? 1u : 0u;
+          const uint32_t acc = !first || kk > 0 ? 1u : 0u;
           umma_bf16(tmem_base, da0 + 2 * kk, db + 2 * kk, kIdesc, acc);
           umma_bf16(tmem_base + NTOK, da1 + 2 * kk, db + 2 * kk, kIdesc, acc);
         }
-        umma_commit(&empty_bar[s]);
+      });
+      if (done) {
+        umma_commit(&acc_bar);
+      } else {
+        abort_s = 1;
+        atomicExch(&g_tc_error, 2);
       }
-      if (!abort_s) umma_commit(&acc_bar);
     }
   } else {
     // every MMA of this CTA has read its operands once the accumulators are published
