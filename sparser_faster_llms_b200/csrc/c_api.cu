@@ -72,6 +72,10 @@ int pair_mlp(bool gated, bool hp, const void* x, const void* gate, const float* 
              const void* up, const void* down, void* packed, void* out, int64_t M, int64_t D,
              int64_t H, int cf, void* workspace, size_t workspace_bytes, void* scratch,
              int64_t max_rows, cudaStream_t stream);
+bool tile_mlp_serves(int64_t M, int64_t D, int64_t H, bool hp);
+int tile_mlp(bool gated, const void* x, const void* gate, const float* bias, const void* up,
+             const void* down, void* packed, void* out, int64_t M, int64_t D, int64_t H, int cf,
+             void* hidden, cudaStream_t stream);
 int twell_decode_status();
 #ifdef B200_TRACE
 void twell_decode_trace(unsigned long long* out16);
@@ -401,13 +405,28 @@ bool pair_wanted(int64_t M, int64_t D, int64_t H, bool gated, bool hp, const voi
   const size_t need = pair_mlp_scratch_bytes(M, D, H, gated, hp, max_rows);
   return need != 0 && scratch_bytes >= need;
 }
+
+// Scratch of a call on one-SM tiles: its hidden matrix.  0: the call does not run on them.
+size_t tile_scratch_bytes(int64_t M, int64_t D, int64_t H, bool hp, int64_t max_rows) {
+  if (max_rows > 0 && max_rows < M) return 0;
+  return tile_mlp_serves(M, D, H, hp) ? (size_t)M * H * 2 : 0;
+}
+
+bool tile_wanted(int64_t M, int64_t D, int64_t H, bool hp, const void* scratch, size_t scratch_bytes,
+                 int64_t max_rows) {
+  if (scratch == nullptr || M < 1 || D % 256 || H % 256 || D < 256 || H < 256) return false;
+  const size_t need = tile_scratch_bytes(M, D, H, hp, max_rows);
+  return need != 0 && scratch_bytes >= need;
+}
 }  // namespace
 
 size_t b200_twell_mlp_scratch_bytes_chunked(int64_t M, int64_t D, int64_t H, int gated,
                                             uint32_t flags, int64_t max_rows) {
   if (M <= 0 || D < 256 || D > 4096 || D % 256 || H < 256 || H > 65536 || H % 256) return 0;
-  return pair_mlp_scratch_bytes(M, D, H, gated != 0, (flags & B200_FLAG_HIGH_PRECISION) != 0,
-                                max_rows);
+  const bool hp = (flags & B200_FLAG_HIGH_PRECISION) != 0;
+  const size_t pair = pair_mlp_scratch_bytes(M, D, H, gated != 0, hp, max_rows);
+  const size_t tile = tile_scratch_bytes(M, D, H, hp, max_rows);
+  return pair > tile ? pair : tile;
 }
 
 size_t b200_twell_mlp_scratch_bytes(int64_t M, int64_t D, int64_t H, int gated, uint32_t flags) {
@@ -420,6 +439,13 @@ int b200_twell_gated_mlp_chunked(const void* x, const void* gate, const float* g
                                  void* workspace, size_t workspace_bytes, void* scratch,
                                  size_t scratch_bytes, int64_t max_rows, void* stream) {
   const bool hp = (flags & B200_FLAG_HIGH_PRECISION) != 0;
+  if (tile_wanted(M, D, H, hp, scratch, scratch_bytes, max_rows)) {
+    B200_TRY(check_decode_args("b200_twell_gated_mlp", x, gate, gate_bias, up, down, packed, out,
+                               M, D, H, cf, flags, workspace, true));
+    B200_TRY(check_ptr("b200_twell_gated_mlp", "scratch", scratch));
+    return tile_mlp(true, x, gate, gate_bias, up, down, packed, out, M, D, H, cf, scratch,
+                    static_cast<cudaStream_t>(stream));
+  }
   if (pair_wanted(M, D, H, true, hp, scratch, scratch_bytes, max_rows)) {
     B200_TRY(check_decode_args("b200_twell_gated_mlp", x, gate, gate_bias, up, down, packed, out,
                                M, D, H, cf, flags, workspace, true));
@@ -535,6 +561,14 @@ int b200_twell_mlp_chunked(const void* x, const void* up, const void* down, void
                            int64_t M, int64_t D, int64_t H, int cf, int num_splits,
                            void* workspace, size_t workspace_bytes, void* scratch,
                            size_t scratch_bytes, int64_t max_rows, void* stream) {
+  if ((num_splits == 1 || num_splits == 2 || num_splits == 4 || num_splits == 8) &&
+      tile_wanted(M, D, H, false, scratch, scratch_bytes, max_rows)) {
+    B200_TRY(check_decode_args("b200_twell_mlp", x, up, nullptr, nullptr, down, packed, out, M, D,
+                               H, cf, 0, workspace, false));
+    B200_TRY(check_ptr("b200_twell_mlp", "scratch", scratch));
+    return tile_mlp(false, x, up, nullptr, nullptr, down, packed, out, M, D, H, cf, scratch,
+                    static_cast<cudaStream_t>(stream));
+  }
   if ((num_splits == 1 || num_splits == 2 || num_splits == 4 || num_splits == 8) &&
       pair_wanted(M, D, H, false, false, scratch, scratch_bytes, max_rows)) {
     B200_TRY(check_decode_args("b200_twell_mlp", x, up, nullptr, nullptr, down, packed, out, M, D,

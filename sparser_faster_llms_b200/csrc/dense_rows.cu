@@ -43,6 +43,13 @@ int pair_gate_up(const void* x, const void* gate, const float* bias, const void*
                  cudaStream_t stream);
 int pair_down(const void* hidden, int terms, const void* down, void* out, int64_t M, int64_t D,
               int64_t H, const RunIf& run_if, const SplitRoom& room, cudaStream_t stream);
+int tile_mlp_status();
+bool tile_mlp_serves(int64_t M, int64_t D, int64_t H, bool hp);
+int tile_first(bool gated, const void* x, const void* gate, const float* bias, const void* up,
+               void* packed, void* hidden, int64_t M, int64_t D, int64_t H, int cf, bool keep_all,
+               cudaStream_t stream);
+int tile_second(const void* hidden, const void* down, void* out, int64_t M, int64_t D, int64_t H,
+                cudaStream_t stream);
 
 namespace {
 
@@ -881,11 +888,12 @@ struct DenseWs {
 
 size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
 
-// Whether a routed call takes every row through the paired tensor-core tiles: that needs the whole
-// [M, H] hidden matrix, so not where it is above 1 GB and above what the dense rows take anyway.
-bool pair_rows(int64_t M, int64_t D, int64_t H, int64_t cap) {
+// Whether a routed call takes every row through the tensor-core tiles of the plain call of its size: that
+// needs the whole [M, H] hidden matrix, so not where it is above 1 GB and above what the dense rows take
+// anyway.
+bool tile_rows(int64_t M, int64_t D, int64_t H, int64_t cap) {
   const int64_t hidden = M * H * 2, rows = cap * (D + H) * 2;
-  return pair_mlp_serves(M, D, H, true, false) &&
+  return (tile_mlp_serves(M, D, H, false) || pair_mlp_serves(M, D, H, true, false)) &&
          hidden <= (rows > ((int64_t)1 << 30) ? rows : (int64_t)1 << 30);
 }
 
@@ -905,7 +913,7 @@ DenseWs dense_ws_layout(void* base, int64_t M, int64_t D, int64_t H, int64_t cap
   w.hd = reinterpret_cast<__nv_bfloat16*>(p + off);
   off += align256((size_t)cap_pad * H * 2);
   w.total = w.routed = off;
-  if (pair_rows(M, D, H, cap)) {
+  if (tile_rows(M, D, H, cap)) {
     off = (size_t)(reinterpret_cast<unsigned char*>(w.xd) - p);
     w.h_all = w.xd;
     off += align256((size_t)M * H * 2);
@@ -1299,11 +1307,11 @@ int b200_twell_gated_mlp_hybrid_counted(const void* x, const void* gate, const f
   if (reinterpret_cast<uintptr_t>(counters) & 3u)
     return fail(B200_EALIGN, "%s: counters is not 4-byte aligned", fn);
   if (M > 0 && flags == 0 && D <= 4096 && dense_cap > 0 &&
-      pair_rows(M, D, H, dense_cap < M ? dense_cap : M) &&
+      tile_rows(M, D, H, dense_cap < M ? dense_cap : M) &&
       hybrid_ws_bytes >= dense_ws_layout(nullptr, M, D, H, dense_cap < M ? dense_cap : M).total &&
       nnz_threshold >= 0 && M <= (int64_t)1 << 20 && hybrid_ws != nullptr && x && gate && up &&
       down && down_t && packed && out) {
-    // Large calls: every row on the paired tensor-core tiles.  The hidden values of a routed row
+    // Large calls: every row on the tensor-core tiles.  The hidden values of a routed row
     // are those of the dense formula as long as no positive is dropped, so routing only decides
     // which overflowed rows stay lossy (beyond dense_cap); nothing is computed twice.
     if (int rc = check_dims(fn, M, D, H, cf)) return rc;
@@ -1318,7 +1326,9 @@ int b200_twell_gated_mlp_hybrid_counted(const void* x, const void* gate, const f
     if (counters != nullptr) w.counters = counters;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int tiles = (int)(H / kTileN), slab_w = kTileN / cf;
-    if (int rc = pair_gate_up(x, gate, gate_bias, up, packed, w.h_all, M, D, H, cf, true, st))
+    const bool small = tile_mlp_serves(M, D, H, false);
+    if (int rc = small ? tile_first(true, x, gate, gate_bias, up, packed, w.h_all, M, D, H, cf, true, st)
+                       : pair_gate_up(x, gate, gate_bias, up, packed, w.h_all, M, D, H, cf, true, st))
       return rc;
     const unsigned row_blocks = (unsigned)((M + 7) / 8);
     route_flags_kernel<<<row_blocks, 256, 0, st>>>(
@@ -1329,6 +1339,7 @@ int b200_twell_gated_mlp_hybrid_counted(const void* x, const void* gate, const f
       truncate_rows_kernel<<<row_blocks, 256, 0, st>>>(static_cast<const uint32_t*>(packed), w.flags,
                                                       w.counters, (int)M, tiles, slab_w, w.h_all);
     if (int rc = check_launch(fn)) return rc;
+    if (small) return tile_second(w.h_all, down, out, M, D, H, st);
     const SplitRoom room = {w.part, pair_part_bytes(M, D, H),
                             workspace != nullptr && workspace_bytes >= 16384
                                 ? static_cast<unsigned int*>(workspace) : nullptr};
@@ -1395,8 +1406,8 @@ int b200_twell_hybrid_status(void) {
   int v = 0, zero = 0;
   if (cudaMemcpyFromSymbol(&v, g_dense_error, sizeof(int)) != cudaSuccess) return -1;
   if (v != 0) cudaMemcpyToSymbol(g_dense_error, &zero, sizeof(int));
-  const int pair = pair_gemm_status();
-  return v != 0 ? v : pair;
+  const int pair = pair_gemm_status(), tile = tile_mlp_status();
+  return v != 0 ? v : pair != 0 ? pair : tile;
 }
 
 }  // extern "C"

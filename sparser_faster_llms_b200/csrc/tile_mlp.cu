@@ -1,0 +1,510 @@
+// The fused MLPs for some dozens to some hundreds of tokens: two launches of one-SM tensor-core tiles
+// that fill the GPU where the 256 x 256 tiles of the paired GEMM (pair_gemm.cuh) would leave most of it
+// idle.
+//
+//   first    CTA = 128 tokens x NB neurons (64 or 128) of the gate and of the up product, both in one
+//            accumulator of 2 NB columns; the CTAs of a 256-neuron slab tile form a cluster and
+//            exchange their stored counts, so every CTA knows the slots of its entries.  Writes the
+//            slabs and hidden = relu(gate) * up on the stored pattern.
+//   second   CTA = 128 tokens x ND output columns x a slice of the neurons; a cluster of CL CTAs holds
+//            all slices.  Every CTA hands each owner its 128 x ND / CL fp32 sums through distributed
+//            shared memory, the owner adds them in rank order and stores.
+//
+// What bounds both: the weights' stream and, per SM, the 64 bytes a clock that TMA brings into shared
+// memory, so the split is the one that puts the weights on as many SMs as fit one wave.  The gather form
+// has two latency chains of four to six round trips behind the same stream, and its rows come through
+// L2 once per token.
+//
+// Threads (352): warp 0 loads weights, warp 1 tokens, warp 2 issues the MMAs, warps 3..10 epilogue, two
+// per TMEM lane quarter (lane = token).  Every wait is bounded; one that gives up sets the error word,
+// and the CTA goes on to the common cluster barriers, which frees TMEM.
+#include "pair_gemm.cuh"
+
+namespace cg = cooperative_groups;
+
+namespace b200 {
+
+int sm_count();
+
+namespace {
+
+namespace tm {
+
+constexpr int kThreads = 352;
+constexpr int kRows = 128;                 // tokens per CTA
+constexpr int kRowBytes = kRows * 128;     // their 64-k stage
+constexpr int kRing = 192 * 1024;          // shared memory of the stages
+
+__device__ int g_error = 0;
+
+__device__ __forceinline__ void give_up(int* abort_s, int code) {
+  *(volatile int*)abort_s = 1;
+  atomicExch(&g_error, code);
+}
+
+template <int STAGES>
+struct Ring {
+  uint64_t full[STAGES], empty[STAGES], done;
+  uint32_t tmem;
+  int abort;
+};
+
+// Barriers and TMEM; every thread of the cluster takes part in the cluster barrier that the caller
+// waits for before it touches another CTA's shared memory.
+template <int STAGES, int COLS>
+__device__ __forceinline__ void set_up(Ring<STAGES>& r, int warp) {
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(&r.full[s], 2);  // both producers
+      mbar_init(&r.empty[s], 1);
+    }
+    mbar_init(&r.done, 1);
+    r.abort = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 2) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+                 ::"r"(smem_u32(&r.tmem)), "r"(COLS)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+}
+
+// One producer thread: `load(k, stage)` issues its copies of a k-step, `bytes` in all.
+template <int STAGES, typename Load>
+__device__ __forceinline__ void produce(Ring<STAGES>& r, int ksteps, uint32_t bytes, int code, Load load) {
+  if (!ring_produce<STAGES>(r.full, r.empty, ksteps, bytes, load)) give_up(&r.abort, code);
+}
+
+// The MMA thread.
+template <int STAGES, typename Step>
+__device__ __forceinline__ void issue(Ring<STAGES>& r, int ksteps, int code, Step step) {
+  if (ring_issue<STAGES>(r.full, r.empty, ksteps, step)) umma_commit(&r.done);
+  else give_up(&r.abort, code);
+}
+
+template <int STAGES, int COLS>
+__device__ __forceinline__ void free_tmem(Ring<STAGES>& r, int warp) {
+  if (warp != 2) return;
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(r.tmem), "r"(COLS)
+               : "memory");
+}
+
+struct FirstArgs {
+  const float* bias;      // bias16: 16-byte aligned
+  int bias16;
+  uint32_t* packed;
+  int slab_w, row_words;
+  __nv_bfloat16* hidden;  // [M][H]
+  long long H;
+  int wide;               // hidden rows are 32-byte aligned
+  int M, ksteps, box;     // box: token rows per copy
+  int keep_all;           // values past a slab's capacity still count in the product
+};
+
+// grid = (H / NB, ceil(M / 128)), cluster = 256 / NB along the neurons.
+template <bool GATED, int NB>
+__global__ void __launch_bounds__(kThreads, 1)
+first_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_g,
+             const __grid_constant__ CUtensorMap map_u, const __grid_constant__ FirstArgs a) {
+  constexpr int CL = kTileN / NB;
+  constexpr int COLS = (GATED ? 2 : 1) * NB;
+  constexpr int kStage = kRowBytes + COLS * 128;
+  constexpr int STAGES = kRing / kStage > 8 ? 8 : kRing / kStage;
+  constexpr int BLKS = NB / 64;  // 32-column blocks per epilogue warp
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>(
+      (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  __shared__ __align__(8) Ring<STAGES> ring;
+  __shared__ int count[2 * CL][kRows];  // stored entries by (rank, column half) and token
+
+  cg::cluster_group cluster = cg::this_cluster();
+  const int crank = (int)blockIdx.x % CL;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int n0 = (int)blockIdx.x * NB, m0 = (int)blockIdx.y * kRows;
+  cluster.barrier_arrive();
+  set_up<STAGES, COLS>(ring, warp);
+  if (threadIdx.x == 0)
+    for (int k = 0; k < 2 && k < a.ksteps; ++k) {
+      tma_prefetch_2d(&map_g, k * kStageK, n0);
+      if (GATED) tma_prefetch_2d(&map_u, k * kStageK, n0);
+    }
+  pdl_wait();
+
+  uint32_t gw[BLKS][16];  // gate values as bf16 pairs, zero where nothing is stored
+  uint32_t mask[BLKS];
+  int cnt = 0;
+  bool ok = false;
+  const int q = warp & 3, half = (warp - 3) >> 2;
+  const int rl = q * 32 + lane, row = m0 + rl;
+  const bool live = row < a.M;
+  const uint32_t acc = ring.tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(half * (NB / 2));
+  if (warp == 0) {
+    if (elect_one())
+      produce(ring, a.ksteps, COLS * 128, 1, [&](int k, int s) {
+        unsigned char* b = smem + (size_t)s * kStage + kRowBytes;
+        tma_load_2d(b, &map_g, k * kStageK, n0, &ring.full[s]);
+        if (GATED) tma_load_2d(b + NB * 128, &map_u, k * kStageK, n0, &ring.full[s]);
+      });
+  } else if (warp == 1) {
+    if (elect_one())
+      produce(ring, a.ksteps, a.box * 128, 2, [&](int k, int s) {
+        tma_load_2d(smem + (size_t)s * kStage, &map_x, k * kStageK, m0, &ring.full[s]);
+      });
+  } else if (warp == 2) {
+    const uint64_t da0 = umma_desc(smem_u32(smem));
+    const uint32_t tmem = ring.tmem;
+    if (elect_one())
+      issue(ring, a.ksteps, 3, [&](bool first, int s) {
+        const uint64_t da = da0 + (uint32_t)s * (kStage >> 4), db = da + (kRowBytes >> 4);
+#pragma unroll
+        for (int kk = 0; kk < kStageK / 16; ++kk)
+          umma_bf16(tmem, da + 2 * kk, db + 2 * kk, umma_idesc(kRows, COLS),
+                    !first || kk > 0 ? 1u : 0u);
+      });
+  } else {
+    ok = mbar_wait(&ring.done, 0u);
+    ok = __all_sync(0xffffffffu, ok);
+    if (!ok) give_up(&ring.abort, 4);
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+    for (int b = 0; b < BLKS; ++b) {
+      float v[32];
+      tmem_ld32(acc + (uint32_t)(b * 32), v);
+      if (a.bias != nullptr) {
+        const float* bp = a.bias + n0 + half * (NB / 2) + b * 32;
+        if (a.bias16) {
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+            const float4 bv = __ldg(reinterpret_cast<const float4*>(bp) + c);
+            v[4 * c] += bv.x;
+            v[4 * c + 1] += bv.y;
+            v[4 * c + 2] += bv.z;
+            v[4 * c + 3] += bv.w;
+          }
+        } else {
+#pragma unroll
+          for (int c = 0; c < 32; ++c) v[c] += __ldg(bp + c);
+        }
+      }
+      uint32_t m = 0;
+#pragma unroll
+      for (int c = 0; c < 32; ++c) m |= v[c] > 0.f ? 1u << c : 0u;
+      mask[b] = live ? m : 0u;
+      cnt += __popc(mask[b]);
+#pragma unroll
+      for (int p = 0; p < 16; ++p) gw[b][p] = pg::pack2(fmaxf(v[2 * p], 0.f), fmaxf(v[2 * p + 1], 0.f));
+    }
+  }
+  if (warp == 0) pdl_trigger();
+  cluster.barrier_wait();  // every CTA of the cluster runs
+  if (warp >= 3) {
+#pragma unroll
+    for (int r = 0; r < CL; ++r) *cluster.map_shared_rank(&count[2 * crank + half][rl], r) = cnt;
+  }
+  cluster.sync();
+  if (warp >= 3 && ok) {
+    int slot = 0, total = 0;
+#pragma unroll
+    for (int i = 0; i < 2 * CL; ++i) {
+      const int c = count[i][rl];
+      if (i < 2 * crank + half) slot += c;
+      total += c;
+    }
+    const int cap = a.slab_w - 1, tile = (int)blockIdx.x / CL;
+    uint32_t* slab = a.packed + (size_t)row * a.row_words + (size_t)tile * a.slab_w;
+    if (crank == 0 && half == 0 && live) slab[0] = (uint32_t)total;
+    __nv_bfloat16* out = a.hidden + (size_t)row * a.H + n0 + half * (NB / 2);
+#pragma unroll
+    for (int b = 0; b < BLKS; ++b) {
+      if (total > cap) {  // values past the slab's capacity are not stored and leave the product too
+        uint32_t m = mask[b];
+        while (__popc(m) > max(cap - slot, 0)) m &= ~(0x80000000u >> __clz(m));
+        mask[b] = m;
+#pragma unroll
+        for (int p = 0; p < 16 && !a.keep_all; ++p)
+          gw[b][p] &= ((m >> (2 * p)) & 1u ? 0xFFFFu : 0u) | ((m >> (2 * p + 1)) & 1u ? 0xFFFF0000u : 0u);
+      }
+      const uint32_t col0 = (uint32_t)(n0 + half * (NB / 2) + b * 32), m = mask[b];
+#pragma unroll
+      for (int c = 0; c < 32; ++c)
+        if ((m >> c) & 1u) {
+          ++slot;
+          slab[slot] = (col0 + c) | (c & 1 ? gw[b][c / 2] & 0xFFFF0000u : gw[b][c / 2] << 16);
+        }
+      if (!GATED) {
+        if (live) pg::store64(out + b * 32, gw[b], a.wide);
+      } else {
+        float v[32];
+        __syncwarp();
+        tmem_ld32(acc + (uint32_t)(NB + b * 32), v);
+        uint32_t w[16];
+#pragma unroll
+        for (int p = 0; p < 16; ++p) {
+          const uint32_t nz = pg::nonzero2(gw[b][p]);  // never touch u where nothing is stored
+          w[p] = pg::mul2(gw[b][p], pg::pack2(v[2 * p], v[2 * p + 1]) & nz) & nz;
+        }
+        if (live) pg::store64(out + b * 32, w, a.wide);
+      }
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  free_tmem<STAGES, COLS>(ring, warp);
+}
+
+// Owner's place of a 16-byte piece (0..3) of a token's 16 sums: pieces rotate with the row pair, so
+// that eight lanes on eight rows reach all banks.
+__device__ __forceinline__ float* sum_at(float* sums, int src, int row, int piece) {
+  return sums + ((size_t)src * kRows + row) * 16 + ((piece ^ ((row >> 1) & 3)) << 2);
+}
+
+// grid = (D / ND * CL, ceil(M / 128)), cluster = CL along k.  map_d: the weights as they are stored, [H][D].
+template <int ND, int CL>
+__global__ void __launch_bounds__(kThreads, 1)
+second_kernel(const __grid_constant__ CUtensorMap map_h, const __grid_constant__ CUtensorMap map_d,
+              __nv_bfloat16* __restrict__ out, int M, int D, int ksteps, int box) {
+  constexpr int PER = ND / CL / 16;             // 16-column groups per owner (1 or 2 or 4)
+  constexpr int kSums = PER * CL * kRows * 64;  // bytes received: ND x 128 fp32
+  constexpr int kStage = kRowBytes + ND * 128;
+  constexpr int STAGES = (224 * 1024 - kSums) / kStage > 8 ? 8 : (224 * 1024 - kSums) / kStage;
+  constexpr uint32_t kIdesc = umma_idesc(kRows, ND) | 1u << 16;
+  static_assert(ND % (16 * CL) == 0, "an owner's columns are whole 16-column groups");
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>(
+      (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  float* sums = reinterpret_cast<float*>(smem + (size_t)STAGES * kStage);  // [PER][CL][128][16]
+  __shared__ __align__(8) Ring<STAGES> ring;
+
+  cg::cluster_group cluster = cg::this_cluster();
+  const int crank = (int)blockIdx.x % CL;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int c0 = (int)blockIdx.x / CL * ND, m0 = (int)blockIdx.y * kRows;
+  const int k0 = crank * ksteps / CL, k1 = (crank + 1) * ksteps / CL;
+  cluster.barrier_arrive();
+  set_up<STAGES, ND>(ring, warp);
+  pdl_wait();
+
+  bool ok = false;
+  const int q = warp & 3, half = (warp - 3) >> 2;
+  if (warp == 0) {
+    if (elect_one())
+      produce(ring, k1 - k0, ND * 128, 5, [&](int k, int s) {
+        unsigned char* b = smem + (size_t)s * kStage + kRowBytes;
+#pragma unroll
+        for (int i = 0; i < ND / 64; ++i)
+          tma_load_2d(b + i * 8192, &map_d, c0 + i * 64, (k0 + k) * kStageK, &ring.full[s]);
+      });
+  } else if (warp == 1) {
+    if (elect_one())
+      produce(ring, k1 - k0, box * 128, 6, [&](int k, int s) {
+        tma_load_2d(smem + (size_t)s * kStage, &map_h, (k0 + k) * kStageK, m0, &ring.full[s]);
+      });
+  } else if (warp == 2) {
+    const uint64_t da0 = umma_desc(smem_u32(smem)), db0 = pg::desc_mn(smem_u32(smem) + kRowBytes);
+    const uint32_t tmem = ring.tmem;
+    if (elect_one())
+      issue(ring, k1 - k0, 7, [&](bool first, int s) {
+        const uint64_t da = da0 + (uint32_t)s * (kStage >> 4), db = db0 + (uint32_t)s * (kStage >> 4);
+#pragma unroll
+        for (int kk = 0; kk < kStageK / 16; ++kk)
+          umma_bf16(tmem, da + 2 * kk, db + 128 * kk, kIdesc, !first || kk > 0 ? 1u : 0u);
+      });
+  } else {
+    ok = mbar_wait(&ring.done, 0u);
+    ok = __all_sync(0xffffffffu, ok);
+    if (!ok) give_up(&ring.abort, 8);
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  }
+  if (warp == 0) pdl_trigger();
+  cluster.barrier_wait();  // every CTA of the cluster runs
+  if (warp >= 3 && ok && m0 + q * 32 < M) {
+    const int rl = q * 32 + lane;
+    const uint32_t acc = ring.tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(half * (ND / 2));
+#pragma unroll
+    for (int b = 0; b < ND / 64; ++b) {
+      float v[32];
+      __syncwarp();
+      tmem_ld32(acc + (uint32_t)(b * 32), v);
+#pragma unroll
+      for (int g = 0; g < 2 && m0 + rl < M; ++g) {
+        const int group = half * (ND / 32) + b * 2 + g;  // of 16 columns
+        float* dst = cluster.map_shared_rank(sums, group / PER) + (size_t)(group % PER) * CL * kRows * 16;
+#pragma unroll
+        for (int p = 0; p < 4; ++p)
+          *reinterpret_cast<float4*>(sum_at(dst, crank, rl, p)) =
+              make_float4(v[16 * g + 4 * p], v[16 * g + 4 * p + 1], v[16 * g + 4 * p + 2],
+                          v[16 * g + 4 * p + 3]);
+      }
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  cluster.sync();
+  free_tmem<STAGES, ND>(ring, warp);
+  if (warp < 3 || ring.abort) return;
+  const int et = threadIdx.x - 96, rl = et >> 1, row = m0 + rl;
+  if (row >= M) return;
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    float* mine = sums + (size_t)i * CL * kRows * 16;
+    float v[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) v[c] = 0.f;
+#pragma unroll
+    for (int r = 0; r < CL; ++r)
+#pragma unroll
+      for (int p = 0; p < 2; ++p) {
+        const float4 u = *reinterpret_cast<const float4*>(sum_at(mine, r, rl, 2 * (et & 1) + p));
+        v[4 * p] += u.x;
+        v[4 * p + 1] += u.y;
+        v[4 * p + 2] += u.z;
+        v[4 * p + 3] += u.w;
+      }
+    *reinterpret_cast<uint4*>(out + (size_t)row * D + c0 + (crank * PER + i) * 16 + 8 * (et & 1)) =
+        make_uint4(pg::pack2(v[0], v[1]), pg::pack2(v[2], v[3]), pg::pack2(v[4], v[5]),
+                   pg::pack2(v[6], v[7]));
+  }
+}
+
+template <typename Kernel, typename... Args>
+int launch_cluster(const char* fn, Kernel kern, dim3 grid, int cluster, size_t smem, size_t (&granted)[64],
+                   cudaStream_t stream, Args... args) {
+  if (int rc = ensure_dynamic_smem(kern, smem, granted, fn)) return rc;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(kThreads, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)cluster;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = add_pdl_attribute(attr, 1);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, args...);
+  if (e != cudaSuccess) return fail(B200_ECUDA, "%s: launch: %s", fn, cudaGetErrorString(e));
+  return B200_OK;
+}
+
+template <bool GATED, int NB>
+int launch_first(const void* x, const void* g, const void* u, FirstArgs a, int64_t D, cudaStream_t stream) {
+  constexpr int kStage = kRowBytes + (GATED ? 2 : 1) * NB * 128;
+  constexpr int STAGES = kRing / kStage > 8 ? 8 : kRing / kStage;
+  CUtensorMap mx, mg, mu;
+  if (int rc = make_map(&mx, x, a.M, D, a.box)) return rc;
+  if (int rc = make_map(&mg, g, a.H, D, NB)) return rc;
+  if (int rc = make_map(&mu, u, a.H, D, NB)) return rc;
+  static size_t granted[64] = {0};
+  return launch_cluster("gate and up tiles", first_kernel<GATED, NB>,
+                        dim3((unsigned)(a.H / NB), (unsigned)((a.M + kRows - 1) / kRows), 1), kTileN / NB,
+                        (size_t)STAGES * kStage + 1024, granted, stream, mx, mg, mu, a);
+}
+
+template <int ND, int CL>
+int launch_second(const void* hidden, const void* down, void* out, int64_t M, int64_t D, int64_t H,
+                  int box, cudaStream_t stream) {
+  constexpr int kSums = ND * kRows * 4;
+  constexpr int kStage = kRowBytes + ND * 128;
+  constexpr int STAGES = (224 * 1024 - kSums) / kStage > 8 ? 8 : (224 * 1024 - kSums) / kStage;
+  CUtensorMap mh, md;
+  if (int rc = make_map(&mh, hidden, M, H, box)) return rc;
+  if (int rc = make_map(&md, down, H, D, 64)) return rc;
+  static size_t granted[64] = {0};
+  return launch_cluster("down tiles", second_kernel<ND, CL>,
+                        dim3((unsigned)(D / ND * CL), (unsigned)((M + kRows - 1) / kRows), 1), CL,
+                        (size_t)STAGES * kStage + kSums + 1024, granted, stream, mh, md,
+                        static_cast<__nv_bfloat16*>(out), (int)M, (int)D, (int)(H / kStageK),
+                        box);
+}
+
+}  // namespace tm
+
+}  // namespace
+
+// Which calls of the fused MLPs run here: from 33 tokens on, while the first launch fits one wave.  us per
+// layer under graph replay, weights from HBM, forms before (gathers, or pairs of SMs) -> now:
+//   gated    D 1024, H 4096:   64 tokens, 2 % 22 -> 14;  256 tokens 35 -> 16;  512 tokens 32 -> 23
+//            D 2048, H 5632:   37 tokens 27 -> 20;  128 tokens 38 -> 23;  384 tokens 47 -> 34
+//            D 2048, H 8192:   40 tokens, 0.5 % / 2 % 24 / 35 -> 24;  128 tokens 30 / 48 -> 27;
+//                              256 tokens 48 -> 38
+//            D 2048, H 11008:  64 tokens, 0.5 % / 2 % 30 / 44 -> 33;  128 tokens 60 -> 40
+//            D 4096, H 16384:  64 tokens, 0.5 % / 2 % 64 / 115 -> 73;  128 tokens 91 -> 77
+//   plain    D 2048, H 8192:   33 tokens, 0.5 % / 2 % 21 / 25 -> 20;  256 tokens 32 / 46 -> 30
+// Up to 32 tokens the gathers touch few rows (D 2048, H 8192, 32 tokens, 0.5 % / 2 % 17 / 24 -> 24).  In
+// two waves the form is level with the pairs at best (H 11008, 200 tokens 49 -> 54).
+bool tile_mlp_serves(int64_t M, int64_t D, int64_t H, bool hp) {
+  if (hp || M < 33 || M > 512 || D > 4096 || H < 2048) return false;
+  return (M + tm::kRows - 1) / tm::kRows * (H / 128) <= sm_count();
+}
+
+namespace {
+
+// CTAs in clusters of four that are resident at once (a GPC's SMs are no multiple of four).
+int64_t fours() { return (sm_count() / 4 - 4) * 4; }
+int64_t row_tiles(int64_t M) { return (M + tm::kRows - 1) / tm::kRows; }
+int token_box(int64_t M) { return M < tm::kRows ? (int)((M + 7) / 8 * 8) : tm::kRows; }
+
+}  // namespace
+
+// Slabs and hidden values ([M, H] bf16, 16-byte aligned); keep_all: of every gate positive, not only of
+// the stored ones.
+int tile_first(bool gated, const void* x, const void* gate, const float* bias, const void* up,
+               void* packed, void* hidden, int64_t M, int64_t D, int64_t H, int cf, bool keep_all,
+               cudaStream_t stream) {
+  tm::FirstArgs a = {};
+  a.bias = bias;
+  a.bias16 = aligned16(bias);
+  a.packed = static_cast<uint32_t*>(packed);
+  a.slab_w = kTileN / cf;
+  a.row_words = (int)(H / kTileN) * a.slab_w;
+  a.hidden = static_cast<__nv_bfloat16*>(hidden);
+  a.H = H;
+  a.wide = (reinterpret_cast<uintptr_t>(hidden) & 31u) == 0;
+  a.M = (int)M;
+  a.ksteps = (int)(D / kStageK);
+  a.box = token_box(M);
+  a.keep_all = keep_all;
+  // 64 neurons per CTA while that is one wave: 128 tokens, D 2048, H 8192 16.5 against 21 us; the
+  // accumulators of 128 neurons cost twice the MMAs per step.
+  if (row_tiles(M) * (H / 64) <= fours())
+    return gated ? tm::launch_first<true, 64>(x, gate, up, a, D, stream)
+                 : tm::launch_first<false, 64>(x, gate, gate, a, D, stream);
+  return gated ? tm::launch_first<true, 128>(x, gate, up, a, D, stream)
+               : tm::launch_first<false, 128>(x, gate, gate, a, D, stream);
+}
+
+// out[M, D] = hidden[M, H] down with down [H, D] as it is stored.
+int tile_second(const void* hidden, const void* down, void* out, int64_t M, int64_t D, int64_t H,
+                cudaStream_t stream) {
+  const int box = token_box(M);
+  // As with the neurons, and k in four slices: 128 tokens, D 2048 12.5 (64 columns) against
+  // 16 us (128); 256 tokens 35 against 21.  Clusters of eight fit half the GPU at once (21 us).
+  if (row_tiles(M) * (D / 64) * 4 <= fours())
+    return tm::launch_second<64, 4>(hidden, down, out, M, D, H, box, stream);
+  if (row_tiles(M) * (D / 128) * 4 <= fours())
+    return tm::launch_second<128, 4>(hidden, down, out, M, D, H, box, stream);
+  return tm::launch_second<128, 2>(hidden, down, out, M, D, H, box, stream);
+}
+
+int tile_mlp(bool gated, const void* x, const void* gate, const float* bias, const void* up,
+             const void* down, void* packed, void* out, int64_t M, int64_t D, int64_t H, int cf,
+             void* hidden, cudaStream_t stream) {
+  if (int rc = tile_first(gated, x, gate, bias, up, packed, hidden, M, D, H, cf, false, stream)) return rc;
+  return tile_second(hidden, down, out, M, D, H, stream);
+}
+
+// Error word raised by a bounded wait that gave up (0 = none).  Reads and clears it; synchronises.
+int tile_mlp_status() {
+  int v = 0, zero = 0;
+  if (cudaMemcpyFromSymbol(&v, tm::g_error, sizeof(int)) != cudaSuccess) return -1;
+  if (v != 0) cudaMemcpyToSymbol(tm::g_error, &zero, sizeof(int));
+  return v;
+}
+
+}  // namespace b200

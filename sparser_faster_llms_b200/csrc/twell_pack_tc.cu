@@ -38,6 +38,7 @@ namespace cg = cooperative_groups;
 namespace b200 {
 
 int pair_gemm_status();
+int tile_mlp_status();
 
 namespace {
 
@@ -743,8 +744,8 @@ int twell_pack_tc_status() {
   int v = 0, zero = 0;
   if (cudaMemcpyFromSymbol(&v, g_tc_error, sizeof(int)) != cudaSuccess) return -1;
   if (v != 0) cudaMemcpyToSymbol(g_tc_error, &zero, sizeof(int));
-  const int pair = pair_gemm_status();
-  return v != 0 ? v : pair;
+  const int pair = pair_gemm_status(), tile = tile_mlp_status();
+  return v != 0 ? v : pair != 0 ? pair : tile;
 }
 
 }  // namespace b200

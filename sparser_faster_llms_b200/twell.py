@@ -478,7 +478,7 @@ def _gated_mlp(layer_number, A, UP, DOWN, C_packed, OUT, highest_precision, cf) 
     entry["m"] = m
 
 
-_DENSE_FROM_TOKENS = 64  # no shape has a use for scratch below this many tokens
+_DENSE_FROM_TOKENS = 33  # no shape has a use for scratch below this many tokens
 
 
 def _mlp_scratch(dev, m, d, h, gated, flags) -> tuple[torch.Tensor | None, int]:

@@ -1,0 +1,60 @@
+"""Fused MLPs on one-SM tiles: edges of the 128-token tiles and of their copies' boxes, both neuron and column
+widths, every split of the second product, overflowed slabs, a gate bias, the result over the input.  Inputs,
+oracle and bounds of ``test_pair_gemm_gpu`` (the products are dense: y is rounded once)."""
+import pytest
+import torch
+
+from sparser_faster_llms_b200 import _lib, synthetic, twell
+from test_pair_gemm_gpu import DEV, run_case
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("m,d,h", [(33, 2048, 8192), (37, 256, 2048), (127, 768, 2304), (128, 4096, 4352),
+                                   (129, 1024, 8192), (256, 4096, 2048), (257, 2048, 5632),
+                                   (511, 512, 4096), (512, 1024, 4608), (64, 2048, 16384)])
+@pytest.mark.parametrize("cf,gated", [(8, True), (2, True), (8, False)])
+def test_tile_form(m, d, h, cf, gated):
+    assert run_case(m, d, h, cf=cf, gated=gated) > 0
+
+
+@pytest.mark.parametrize("m,h", [(40, 2048), (300, 4096), (130, 16384)])
+@pytest.mark.parametrize("gated", [True, False])
+def test_values_past_a_slab_leave_the_product(m, h, gated):
+    run_case(m, 512, h, gated=gated, dense=True)
+
+
+@pytest.mark.parametrize("h", [4096, 11008])
+def test_bias_and_result_over_the_input(h):
+    m, d = 100, 1024
+    x, gate, up, down = synthetic.dyadic_case(m, d, h, seed=3)
+    bias = torch.randint(-2, 3, (h,)).float() / 4
+    run_case(m, d, h, bias=bias)
+    args = [t.to(DEV) for t in (gate, up, down)]
+    y = twell.TwELLGatedMLP(9400, *args)(x.to(DEV))
+    z = x.to(DEV)
+    assert twell.TwELLGatedMLP(9401, *args, inplace=True)(z) is z
+    assert torch.equal(y, z)
+    assert _lib.load_library().b200_twell_hybrid_status() == 0
+
+
+@pytest.mark.parametrize("m,h", [(130, 2304), (300, 4096)])
+def test_routed_rows_keep_their_positives(m, h):
+    """A routed call of this size: rows with an overflowed slab up to the capacity equal the dense formula,
+    all others the plain call, bit for bit."""
+    d, cap = 512, 16
+    x, gate, up, down = synthetic.dyadic_case(m, d, h, seed=9)
+    x[::5, 0] = -0.5
+    args = [t.to(DEV) for t in (gate, up, down)]
+    plain, routed = twell.TwELLGatedMLP(9402, *args), twell.TwELLGatedMLP(9403, *args)
+    routed.enable_dense_route(nnz_threshold=h, dense_cap=cap, min_tokens=128)
+    y0, y1 = plain(x.to(DEV)).cpu(), routed(x.to(DEV)).cpu()
+    hot = torch.nonzero(torch.arange(m) % 5 == 0).flatten()
+    assert routed.dense_route_counters()["dense_rows"] == cap
+    taken = torch.zeros(m, dtype=torch.bool)
+    taken[hot[:cap]] = True
+    assert torch.equal(y0[~taken], y1[~taken])
+    p = torch.relu(x.double() @ gate.double().T).bfloat16().double()
+    u = (x.double() @ up.double().T).bfloat16().double()
+    ref = ((p * u).bfloat16().double() @ down.double())[taken]
+    assert ((y1.double()[taken] - ref).norm() / ref.norm()).item() < 2e-3  # y rounded once
