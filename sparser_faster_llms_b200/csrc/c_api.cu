@@ -66,13 +66,16 @@ int pair_pack(const void* x, const void* w, const float* bias, void* packed, voi
               int64_t D, int64_t H, int cf, unsigned int* entries, const SplitRoom& room,
               cudaStream_t stream);
 bool pair_mlp_serves(int64_t M, int64_t D, int64_t H, bool gated, bool hp);
-size_t pair_mlp_scratch_bytes(int64_t M, int64_t D, int64_t H, bool gated, bool hp,
-                              int64_t max_rows);
+size_t pair_mlp_scratch_bytes(int64_t M, int64_t D, int64_t H, bool hp, int64_t max_rows);
 int pair_mlp(bool gated, bool hp, const void* x, const void* gate, const float* bias,
              const void* up, const void* down, void* packed, void* out, int64_t M, int64_t D,
              int64_t H, int cf, void* workspace, size_t workspace_bytes, void* scratch,
              int64_t max_rows, cudaStream_t stream);
-bool tile_mlp_serves(int64_t M, int64_t D, int64_t H, bool hp);
+bool tile_mlp_serves(int64_t M, int64_t D, int64_t H);
+bool values_mlp_serves(int64_t M, int64_t D, int64_t H);
+int values_mlp(const void* x, const void* gate, const float* bias, const void* up, const void* down,
+               void* packed, void* out, int64_t M, int64_t D, int64_t H, int cf, void* workspace,
+               size_t workspace_bytes, float* values, cudaStream_t stream);
 int tile_mlp(bool gated, const void* x, const void* gate, const float* bias, const void* up,
              const void* down, void* packed, void* out, int64_t M, int64_t D, int64_t H, int cf,
              void* hidden, cudaStream_t stream);
@@ -398,35 +401,37 @@ int b200_twell_gated_mlp(const void* x, const void* gate, const float* gate_bias
 }
 
 namespace {
-// Whether a fused-MLP call runs on the paired tensor-core GEMM with the given scratch.
-bool pair_wanted(int64_t M, int64_t D, int64_t H, bool gated, bool hp, const void* scratch,
-                 size_t scratch_bytes, int64_t max_rows) {
-  if (scratch == nullptr || M < 1 || D % 256 || H % 256 || D < 256 || D > 4096) return false;
-  const size_t need = pair_mlp_scratch_bytes(M, D, H, gated, hp, max_rows);
-  return need != 0 && scratch_bytes >= need;
+// Forms of the fused MLPs that run on the tensor cores throughout, given room for what stands between
+// their launches.
+enum MlpForm { kGather, kTiles, kValues, kPairs };
+
+MlpForm mlp_form(int64_t M, int64_t D, int64_t H, bool gated, bool hp, int64_t max_rows) {
+  if (M < 1 || D < 256 || D > 4096 || D % 256 || H < 256 || H > 65536 || H % 256) return kGather;
+  const bool whole = max_rows <= 0 || max_rows >= M;  // only the pairs work in row chunks
+  if (whole && hp && values_mlp_serves(M, D, H)) return kValues;
+  if (whole && !hp && tile_mlp_serves(M, D, H)) return kTiles;
+  return pair_mlp_serves(M, D, H, gated, hp) ? kPairs : kGather;
 }
 
-// Scratch of a call on one-SM tiles: its hidden matrix.  0: the call does not run on them.
-size_t tile_scratch_bytes(int64_t M, int64_t D, int64_t H, bool hp, int64_t max_rows) {
-  if (max_rows > 0 && max_rows < M) return 0;
-  return tile_mlp_serves(M, D, H, hp) ? (size_t)M * H * 2 : 0;
-}
-
-bool tile_wanted(int64_t M, int64_t D, int64_t H, bool hp, const void* scratch, size_t scratch_bytes,
-                 int64_t max_rows) {
-  if (scratch == nullptr || M < 1 || D % 256 || H % 256 || D < 256 || H < 256) return false;
-  const size_t need = tile_scratch_bytes(M, D, H, hp, max_rows);
-  return need != 0 && scratch_bytes >= need;
+size_t mlp_scratch(MlpForm form, int64_t M, int64_t D, int64_t H, bool hp, int64_t max_rows) {
+  switch (form) {
+    case kTiles: return (size_t)M * H * 2;        // hidden values in bf16
+    case kValues: return (size_t)M * (H / 2) * 4;  // in fp32, in slots of the widest slab
+    case kPairs: return pair_mlp_scratch_bytes(M, D, H, hp, max_rows);
+    default: return 0;
+  }
 }
 }  // namespace
 
 size_t b200_twell_mlp_scratch_bytes_chunked(int64_t M, int64_t D, int64_t H, int gated,
                                             uint32_t flags, int64_t max_rows) {
-  if (M <= 0 || D < 256 || D > 4096 || D % 256 || H < 256 || H > 65536 || H % 256) return 0;
   const bool hp = (flags & B200_FLAG_HIGH_PRECISION) != 0;
-  const size_t pair = pair_mlp_scratch_bytes(M, D, H, gated != 0, hp, max_rows);
-  const size_t tile = tile_scratch_bytes(M, D, H, hp, max_rows);
-  return pair > tile ? pair : tile;
+  const MlpForm form = mlp_form(M, D, H, gated != 0, hp, max_rows);
+  if (form == kGather) return 0;
+  // never less than the pairs take, whichever form the call's size selects
+  const size_t own = mlp_scratch(form, M, D, H, hp, max_rows);
+  const size_t pair = pair_mlp_scratch_bytes(M, D, H, hp, max_rows);
+  return own > pair ? own : pair;
 }
 
 size_t b200_twell_mlp_scratch_bytes(int64_t M, int64_t D, int64_t H, int gated, uint32_t flags) {
@@ -439,20 +444,20 @@ int b200_twell_gated_mlp_chunked(const void* x, const void* gate, const float* g
                                  void* workspace, size_t workspace_bytes, void* scratch,
                                  size_t scratch_bytes, int64_t max_rows, void* stream) {
   const bool hp = (flags & B200_FLAG_HIGH_PRECISION) != 0;
-  if (tile_wanted(M, D, H, hp, scratch, scratch_bytes, max_rows)) {
+  const MlpForm form = mlp_form(M, D, H, true, hp, max_rows);
+  if (form != kGather && scratch != nullptr &&
+      scratch_bytes >= mlp_scratch(form, M, D, H, hp, max_rows)) {
     B200_TRY(check_decode_args("b200_twell_gated_mlp", x, gate, gate_bias, up, down, packed, out,
                                M, D, H, cf, flags, workspace, true));
     B200_TRY(check_ptr("b200_twell_gated_mlp", "scratch", scratch));
-    return tile_mlp(true, x, gate, gate_bias, up, down, packed, out, M, D, H, cf, scratch,
-                    static_cast<cudaStream_t>(stream));
-  }
-  if (pair_wanted(M, D, H, true, hp, scratch, scratch_bytes, max_rows)) {
-    B200_TRY(check_decode_args("b200_twell_gated_mlp", x, gate, gate_bias, up, down, packed, out,
-                               M, D, H, cf, flags, workspace, true));
-    B200_TRY(check_ptr("b200_twell_gated_mlp", "scratch", scratch));
-    return pair_mlp(true, hp, x, gate, gate_bias, up, down, packed, out, M, D, H, cf,
-                    workspace, workspace_bytes, scratch, max_rows,
-                    static_cast<cudaStream_t>(stream));
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (form == kTiles)
+      return tile_mlp(true, x, gate, gate_bias, up, down, packed, out, M, D, H, cf, scratch, st);
+    if (form == kValues)
+      return values_mlp(x, gate, gate_bias, up, down, packed, out, M, D, H, cf, workspace,
+                        workspace_bytes, static_cast<float*>(scratch), st);
+    return pair_mlp(true, hp, x, gate, gate_bias, up, down, packed, out, M, D, H, cf, workspace,
+                    workspace_bytes, scratch, max_rows, st);
   }
   return b200_twell_gated_mlp(x, gate, gate_bias, up, down, packed, out, M, D, H, cf, flags,
                               workspace, workspace_bytes, stream);
@@ -561,22 +566,17 @@ int b200_twell_mlp_chunked(const void* x, const void* up, const void* down, void
                            int64_t M, int64_t D, int64_t H, int cf, int num_splits,
                            void* workspace, size_t workspace_bytes, void* scratch,
                            size_t scratch_bytes, int64_t max_rows, void* stream) {
-  if ((num_splits == 1 || num_splits == 2 || num_splits == 4 || num_splits == 8) &&
-      tile_wanted(M, D, H, false, scratch, scratch_bytes, max_rows)) {
+  const MlpForm form = mlp_form(M, D, H, false, false, max_rows);
+  if ((num_splits == 1 || num_splits == 2 || num_splits == 4 || num_splits == 8) && form != kGather &&
+      scratch != nullptr && scratch_bytes >= mlp_scratch(form, M, D, H, false, max_rows)) {
     B200_TRY(check_decode_args("b200_twell_mlp", x, up, nullptr, nullptr, down, packed, out, M, D,
                                H, cf, 0, workspace, false));
     B200_TRY(check_ptr("b200_twell_mlp", "scratch", scratch));
-    return tile_mlp(false, x, up, nullptr, nullptr, down, packed, out, M, D, H, cf, scratch,
-                    static_cast<cudaStream_t>(stream));
-  }
-  if ((num_splits == 1 || num_splits == 2 || num_splits == 4 || num_splits == 8) &&
-      pair_wanted(M, D, H, false, false, scratch, scratch_bytes, max_rows)) {
-    B200_TRY(check_decode_args("b200_twell_mlp", x, up, nullptr, nullptr, down, packed, out, M, D,
-                               H, cf, 0, workspace, false));
-    B200_TRY(check_ptr("b200_twell_mlp", "scratch", scratch));
-    return pair_mlp(false, false, x, up, nullptr, nullptr, down, packed, out, M, D, H, cf,
-                    workspace, workspace_bytes, scratch, max_rows,
-                    static_cast<cudaStream_t>(stream));
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (form == kTiles)
+      return tile_mlp(false, x, up, nullptr, nullptr, down, packed, out, M, D, H, cf, scratch, st);
+    return pair_mlp(false, false, x, up, nullptr, nullptr, down, packed, out, M, D, H, cf, workspace,
+                    workspace_bytes, scratch, max_rows, st);
   }
   return b200_twell_mlp(x, up, down, packed, out, M, D, H, cf, num_splits, workspace,
                         workspace_bytes, stream);

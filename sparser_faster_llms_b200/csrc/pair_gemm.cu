@@ -134,6 +134,21 @@ int pair_gate_up(const void* x, const void* gate, const float* bias, const void*
                                                sm_count(), stream);
 }
 
+// The same in high precision: fp32 hidden values in the slots of the slabs (values: [M][H / cf]).
+int pair_gate_up_values(const void* x, const void* gate, const float* bias, const void* up, void* packed,
+                        float* values, int64_t M, int64_t D, int64_t H, int cf, cudaStream_t stream) {
+  pg::Args a = base_args(M, H, D);
+  a.bias = bias;
+  a.bias16 = aligned16(bias);
+  a.slab_p = static_cast<uint32_t*>(packed);
+  a.slab_w = kTileN / cf;
+  a.row_words = (int)(H / kTileN) * a.slab_w;
+  a.values = values;
+  const pg::Operand ox = {x, M, D}, og = {gate, H, D}, ou = {up, H, D};
+  return pg::launch<pg::kGateUpHp, false, false>("gate and up products", ox, ox, og, ou, a, M,
+                                                 sm_count(), stream);
+}
+
 namespace {
 
 // Up and down rows together stay in L2, where a gathered entry is cheaper.
@@ -197,9 +212,7 @@ static size_t chunks_part_bytes(int64_t M, int64_t rows, int64_t D, int64_t H, i
 
 // 240 bytes of it take a 16-byte aligned scratch to the 256 bytes at which its parts begin (rows of
 // sums are written 32 bytes at a time).
-size_t pair_mlp_scratch_bytes(int64_t M, int64_t D, int64_t H, bool gated, bool hp,
-                              int64_t max_rows) {
-  if (!pair_mlp_serves(M, D, H, gated, hp)) return 0;
+size_t pair_mlp_scratch_bytes(int64_t M, int64_t D, int64_t H, bool hp, int64_t max_rows) {
   const int terms = hp ? 3 : 1;
   const int64_t rows = chunk_rows(M, H, terms, max_rows);
   return 240 + align256((size_t)rows * H * 2 * terms) + 256 + chunks_part_bytes(M, rows, D, H, terms);

@@ -48,6 +48,7 @@ enum Epilogue {
   kPack = 1,     // TwELL slabs of relu(acc + bias)
   kPackDense = 6,  // the same, and the stored values as a dense matrix
   kGateUp = 7,   // kPack on a first accumulator (B0) and kMul with its values on a second (B1)
+  kGateUpHp = 8,  // kPack on B0, and its values times the sums on B1 in fp32, in the slots of the slab
   kMul = 2,      // out = bf16(g * bf16(acc)) on the slab pattern, 0 elsewhere
   kMulHp = 3,    // g * acc in fp32, as three bf16 terms side by side (out row = [hi | mid | lo])
   kStoreCarry = 9,  // kStore on a product whose k comes in several launches: fp32 sums carried between
@@ -92,6 +93,7 @@ struct Args {
   float* l1_part;            // kFwd: [tiles][16] sums of |T|
   const float* l1_grad;      // kBwd: device scalar or null
   float inv_m;
+  float* values;             // kGateUpHp: [rows][row_words], hidden values of the stored entries
   int keep_all;              // kGateUp: values past a slab's capacity still count in the product
   unsigned int* entries;     // packs: stored entries are added here (may be null)
   RunIf run_if;
@@ -578,7 +580,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap map_a0,
                  const __grid_constant__ CUtensorMap map_b0,
                  const __grid_constant__ CUtensorMap map_b1, const __grid_constant__ Args a) {
   constexpr uint32_t kIdesc = umma_idesc(256, 256) | (A_MN ? 1u << 15 : 0u) | (B_MN ? 1u << 16 : 0u);
-  constexpr bool kGate2 = EPI == kGateUp;
+  constexpr bool kGate2 = EPI == kGateUp || EPI == kGateUpHp;
   constexpr bool kIsPack = EPI == kPack || EPI == kPackDense || kGate2;
   constexpr bool kTrain = EPI == kFwd || EPI == kBwd;
   constexpr bool kPlain = EPI == kStore || EPI == kStoreCarry;
@@ -875,9 +877,10 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap map_a0,
         load_pattern();
       }
 
+      uint32_t mask[4];
+      int slot = 0, first_slot = 0;
       if (kIsPack) {
         // pass 1: positives of each 32-column block as a mask, bf16 values into the buffer
-        uint32_t mask[4];
         int cnt = 0;
 #pragma unroll
         for (int cb = 0; cb < 4; ++cb) {
@@ -916,11 +919,12 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap map_a0,
         }
         if (src.part == nullptr) release();
         // the second half's slots follow the first half's
-        int slot = 0;
+        slot = 0;
         if (half == 0) half_count[parity][q * 32 + lane] = cnt;
         named_barrier(1 + q, 64);
         if (half == 1) slot = half_count[parity][q * 32 + lane];
         parity ^= 1;
+        first_slot = slot;
         const int cap = a.slab_w - 1;
         uint32_t* slab = a.slab_p + (size_t)row * a.row_words + (size_t)nt * a.slab_w;
         if (half == 1 && live) slab[0] = (uint32_t)(slot + cnt);
@@ -979,7 +983,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap map_a0,
                         shift, done);
         }
       } else if (!kIsPack || kGate2) {
-#pragma unroll 1
+#pragma unroll(EPI == kGateUpHp ? 4 : 1)
         for (int cb = 0; cb < 4; ++cb) {
           float v[32];
           fetch32(src, cb, v);
@@ -1017,6 +1021,23 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap map_a0,
               }
             }
             if (live) store64(out + cb * 32, w, a.wide);
+          } else if (EPI == kGateUpHp) {
+            const int cap = a.slab_w - 1;
+            float* h = a.values + (size_t)row * a.row_words + (size_t)nt * a.slab_w + 1;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const uint4 g4 = *reinterpret_cast<const uint4*>(at(buf, lane, cb * 64 + j * 16));
+              const uint32_t g[4] = {g4.x, g4.y, g4.z, g4.w};
+#pragma unroll
+              for (int e = 0; e < 8; ++e) {
+                const int c = 8 * j + e;
+                if ((mask[cb] >> c) & 1u) {
+                  if (first_slot < cap) h[first_slot] = (e & 1 ? hi_f(g[e >> 1]) : lo_f(g[e >> 1])) * v[c];
+                  ++first_slot;
+                }
+              }
+            }
+            __syncwarp();
           } else if (EPI == kMulHp) {
             uint4 g4[4];
 #pragma unroll
@@ -1143,7 +1164,7 @@ int launch(const char* fn, const Operand& a0, const Operand& a1, const Operand& 
   const int64_t slots = sm_count / 2;
   const bool can_sum = EPI == kStore && args.out_mt == 0 && !args.relu &&
                        args.ld == (long long)args.n_tiles * kTile;
-  Split sp = EPI != kGateUp && args.part != nullptr && args.counters != nullptr &&
+  Split sp = EPI != kGateUp && EPI != kGateUpHp && args.part != nullptr && args.counters != nullptr &&
                      args.rows_ptr == nullptr
                  ? choose_split(tiles, args.ksteps, slots, can_sum)
                  : Split{tiles, 1};

@@ -25,6 +25,11 @@ namespace cg = cooperative_groups;
 namespace b200 {
 
 int sm_count();
+int pair_gate_up_values(const void* x, const void* gate, const float* bias, const void* up, void* packed,
+                        float* values, int64_t M, int64_t D, int64_t H, int cf, cudaStream_t stream);
+int twell_values_t2d(const void* packed, const float* values, const void* down, void* out, int64_t M,
+                     int64_t D, int64_t H, int cf, void* workspace, size_t workspace_bytes,
+                     cudaStream_t stream);
 
 namespace {
 
@@ -95,12 +100,26 @@ __device__ __forceinline__ void free_tmem(Ring<STAGES>& r, int warp) {
                : "memory");
 }
 
+// 32 columns of sums, added over the ranges in their order.
+template <int RANGES, int COLS>
+__device__ __forceinline__ void load_sums(uint32_t addr, float (&v)[32]) {
+  tmem_ld32(addr, v);
+#pragma unroll
+  for (int r = 1; r < RANGES; ++r) {
+    float w[32];
+    tmem_ld32(addr + (uint32_t)(r * COLS), w);
+#pragma unroll
+    for (int c = 0; c < 32; ++c) v[c] += w[c];
+  }
+}
+
 struct FirstArgs {
   const float* bias;      // bias16: 16-byte aligned
   int bias16;
   uint32_t* packed;
   int slab_w, row_words;
   __nv_bfloat16* hidden;  // [M][H]
+  float* values;          // VALUES: instead of hidden, fp32 values in the slots of the slab [M][row_words]
   long long H;
   int wide;               // hidden rows are 32-byte aligned
   int M, ksteps, box;     // box: token rows per copy
@@ -108,7 +127,7 @@ struct FirstArgs {
 };
 
 // grid = (H / NB, ceil(M / 128)), cluster = 256 / NB along the neurons.
-template <bool GATED, int NB>
+template <bool GATED, bool VALUES, int NB>
 __global__ void __launch_bounds__(kThreads, 1)
 first_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_g,
              const __grid_constant__ CUtensorMap map_u, const __grid_constant__ FirstArgs a) {
@@ -117,6 +136,10 @@ first_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ 
   constexpr int kStage = kRowBytes + COLS * 128;
   constexpr int STAGES = kRing / kStage > 8 ? 8 : kRing / kStage;
   constexpr int BLKS = NB / 64;  // 32-column blocks per epilogue warp
+  // High precision keeps the sums of two or four ranges of k apart in TMEM and adds them in fp32: a tensor
+  // core's running sum loses bits with its length (64 tokens, D 2048, 5 %: error against 64 bits
+  // 1.6712e-3 with one range, 1.6593e-3 where D was split four ways before).
+  constexpr int RANGES = VALUES ? 512 / COLS : 1;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -128,7 +151,7 @@ first_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n0 = (int)blockIdx.x * NB, m0 = (int)blockIdx.y * kRows;
   cluster.barrier_arrive();
-  set_up<STAGES, COLS>(ring, warp);
+  set_up<STAGES, RANGES * COLS>(ring, warp);
   if (threadIdx.x == 0)
     for (int k = 0; k < 2 && k < a.ksteps; ++k) {
       tma_prefetch_2d(&map_g, k * kStageK, n0);
@@ -160,11 +183,13 @@ first_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ 
     const uint64_t da0 = umma_desc(smem_u32(smem));
     const uint32_t tmem = ring.tmem;
     if (elect_one())
-      issue(ring, a.ksteps, 3, [&](bool first, int s) {
+      issue(ring, a.ksteps, 3, [&, k = 0, range = -1, next = 0](bool, int s) mutable {
+        const bool first = k++ == next;
+        if (first) next = (++range + 1) * a.ksteps / RANGES;
         const uint64_t da = da0 + (uint32_t)s * (kStage >> 4), db = da + (kRowBytes >> 4);
 #pragma unroll
         for (int kk = 0; kk < kStageK / 16; ++kk)
-          umma_bf16(tmem, da + 2 * kk, db + 2 * kk, umma_idesc(kRows, COLS),
+          umma_bf16(tmem + (uint32_t)(range * COLS), da + 2 * kk, db + 2 * kk, umma_idesc(kRows, COLS),
                     !first || kk > 0 ? 1u : 0u);
       });
   } else {
@@ -175,7 +200,7 @@ first_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ 
 #pragma unroll
     for (int b = 0; b < BLKS; ++b) {
       float v[32];
-      tmem_ld32(acc + (uint32_t)(b * 32), v);
+      load_sums<RANGES, COLS>(acc + (uint32_t)(b * 32), v);
       if (a.bias != nullptr) {
         const float* bp = a.bias + n0 + half * (NB / 2) + b * 32;
         if (a.bias16) {
@@ -218,6 +243,7 @@ first_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ 
     }
     const int cap = a.slab_w - 1, tile = (int)blockIdx.x / CL;
     uint32_t* slab = a.packed + (size_t)row * a.row_words + (size_t)tile * a.slab_w;
+    float* values = VALUES ? a.values + (size_t)row * a.row_words + (size_t)tile * a.slab_w : nullptr;
     if (crank == 0 && half == 0 && live) slab[0] = (uint32_t)total;
     __nv_bfloat16* out = a.hidden + (size_t)row * a.H + n0 + half * (NB / 2);
 #pragma unroll
@@ -231,16 +257,22 @@ first_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ 
           gw[b][p] &= ((m >> (2 * p)) & 1u ? 0xFFFFu : 0u) | ((m >> (2 * p + 1)) & 1u ? 0xFFFF0000u : 0u);
       }
       const uint32_t col0 = (uint32_t)(n0 + half * (NB / 2) + b * 32), m = mask[b];
+      float v[32];
+      if (VALUES) {
+        __syncwarp();
+        load_sums<RANGES, COLS>(acc + (uint32_t)(NB + b * 32), v);
+      }
 #pragma unroll
       for (int c = 0; c < 32; ++c)
         if ((m >> c) & 1u) {
           ++slot;
           slab[slot] = (col0 + c) | (c & 1 ? gw[b][c / 2] & 0xFFFF0000u : gw[b][c / 2] << 16);
+          if (VALUES) values[slot] = (c & 1 ? pg::hi_f(gw[b][c / 2]) : pg::lo_f(gw[b][c / 2])) * v[c];
         }
-      if (!GATED) {
+      if (VALUES) {
+      } else if (!GATED) {
         if (live) pg::store64(out + b * 32, gw[b], a.wide);
       } else {
-        float v[32];
         __syncwarp();
         tmem_ld32(acc + (uint32_t)(NB + b * 32), v);
         uint32_t w[16];
@@ -255,7 +287,7 @@ first_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ 
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  free_tmem<STAGES, COLS>(ring, warp);
+  free_tmem<STAGES, RANGES * COLS>(ring, warp);
 }
 
 // Owner's place of a 16-byte piece (0..3) of a token's 16 sums: pieces rotate with the row pair, so
@@ -392,7 +424,7 @@ int launch_cluster(const char* fn, Kernel kern, dim3 grid, int cluster, size_t s
   return B200_OK;
 }
 
-template <bool GATED, int NB>
+template <bool GATED, bool VALUES, int NB>
 int launch_first(const void* x, const void* g, const void* u, FirstArgs a, int64_t D, cudaStream_t stream) {
   constexpr int kStage = kRowBytes + (GATED ? 2 : 1) * NB * 128;
   constexpr int STAGES = kRing / kStage > 8 ? 8 : kRing / kStage;
@@ -401,7 +433,7 @@ int launch_first(const void* x, const void* g, const void* u, FirstArgs a, int64
   if (int rc = make_map(&mg, g, a.H, D, NB)) return rc;
   if (int rc = make_map(&mu, u, a.H, D, NB)) return rc;
   static size_t granted[64] = {0};
-  return launch_cluster("gate and up tiles", first_kernel<GATED, NB>,
+  return launch_cluster("gate and up tiles", first_kernel<GATED, VALUES, NB>,
                         dim3((unsigned)(a.H / NB), (unsigned)((a.M + kRows - 1) / kRows), 1), kTileN / NB,
                         (size_t)STAGES * kStage + 1024, granted, stream, mx, mg, mu, a);
 }
@@ -438,8 +470,8 @@ int launch_second(const void* hidden, const void* down, void* out, int64_t M, in
 //   plain    D 2048, H 8192:   33 tokens, 0.5 % / 2 % 21 / 25 -> 20;  256 tokens 32 / 46 -> 30
 // Up to 32 tokens the gathers touch few rows (D 2048, H 8192, 32 tokens, 0.5 % / 2 % 17 / 24 -> 24).  In
 // two waves the form is level with the pairs at best (H 11008, 200 tokens 49 -> 54).
-bool tile_mlp_serves(int64_t M, int64_t D, int64_t H, bool hp) {
-  if (hp || M < 33 || M > 512 || D > 4096 || H < 2048) return false;
+bool tile_mlp_serves(int64_t M, int64_t D, int64_t H) {
+  if (M < 33 || M > 512 || D > 4096 || H < 2048) return false;
   return (M + tm::kRows - 1) / tm::kRows * (H / 128) <= sm_count();
 }
 
@@ -453,10 +485,10 @@ int token_box(int64_t M) { return M < tm::kRows ? (int)((M + 7) / 8 * 8) : tm::k
 }  // namespace
 
 // Slabs and hidden values ([M, H] bf16, 16-byte aligned); keep_all: of every gate positive, not only of
-// the stored ones.
+// the stored ones.  values (gated): instead of hidden, their fp32 hidden values in the slots of the slabs.
 int tile_first(bool gated, const void* x, const void* gate, const float* bias, const void* up,
-               void* packed, void* hidden, int64_t M, int64_t D, int64_t H, int cf, bool keep_all,
-               cudaStream_t stream) {
+               void* packed, void* hidden, float* values, int64_t M, int64_t D, int64_t H, int cf,
+               bool keep_all, cudaStream_t stream) {
   tm::FirstArgs a = {};
   a.bias = bias;
   a.bias16 = aligned16(bias);
@@ -464,6 +496,7 @@ int tile_first(bool gated, const void* x, const void* gate, const float* bias, c
   a.slab_w = kTileN / cf;
   a.row_words = (int)(H / kTileN) * a.slab_w;
   a.hidden = static_cast<__nv_bfloat16*>(hidden);
+  a.values = values;
   a.H = H;
   a.wide = (reinterpret_cast<uintptr_t>(hidden) & 31u) == 0;
   a.M = (int)M;
@@ -473,10 +506,12 @@ int tile_first(bool gated, const void* x, const void* gate, const float* bias, c
   // 64 neurons per CTA while that is one wave: 128 tokens, D 2048, H 8192 16.5 against 21 us; the
   // accumulators of 128 neurons cost twice the MMAs per step.
   if (row_tiles(M) * (H / 64) <= fours())
-    return gated ? tm::launch_first<true, 64>(x, gate, up, a, D, stream)
-                 : tm::launch_first<false, 64>(x, gate, gate, a, D, stream);
-  return gated ? tm::launch_first<true, 128>(x, gate, up, a, D, stream)
-               : tm::launch_first<false, 128>(x, gate, gate, a, D, stream);
+    return values != nullptr ? tm::launch_first<true, true, 64>(x, gate, up, a, D, stream)
+           : gated           ? tm::launch_first<true, false, 64>(x, gate, up, a, D, stream)
+                             : tm::launch_first<false, false, 64>(x, gate, gate, a, D, stream);
+  return values != nullptr ? tm::launch_first<true, true, 128>(x, gate, up, a, D, stream)
+         : gated           ? tm::launch_first<true, false, 128>(x, gate, up, a, D, stream)
+                           : tm::launch_first<false, false, 128>(x, gate, gate, a, D, stream);
 }
 
 // out[M, D] = hidden[M, H] down with down [H, D] as it is stored.
@@ -492,10 +527,37 @@ int tile_second(const void* hidden, const void* down, void* out, int64_t M, int6
   return tm::launch_second<128, 2>(hidden, down, out, M, D, H, box, stream);
 }
 
+// High precision below the sizes of pair_mlp_serves: gate and up as tensor-core products, here or on pairs
+// of SMs, and the down product gathered along the stored entries with fp32 hidden values (half the rows
+// that gathering both reads, and no partial sums of the up product).  us per layer under graph replay, pack
+// + gathers -> now, at 0.5 % / 2 % density:
+//   D 1024, H 4096   33 tokens 17.7 / 18.9 -> 13.0 / 14.7;  256 tokens 22.9 / 32.7 -> 16.2 / 19.4;
+//                    6000 tokens 123 / 240 -> 118 / 175
+//   D 2048, H 8192   33 tokens 21.8 / 28.0 -> 23.4 / 28.5 (not taken);  48 tokens 23.5 / 33.3 -> 23.9 / 29.2;
+//                    257 tokens 39.0 / 71.1 -> 42.8 / 56.2;  777 tokens 78 / 162 -> 73 / 110;
+//                    4000 tokens 287 / 661 -> 242 / 385
+//   D 2048, H 11008  129 tokens, pairs 35.7 / 57.7 -> 42.8 / 53.0 (not taken);  160 tokens 43 / 86 -> 45 / 58
+//   D 4096, H 16384  at 1 %: 48 tokens 73 -> 70;  200 tokens 158 -> 104;  1000 tokens 517 -> 326
+bool values_mlp_serves(int64_t M, int64_t D, int64_t H) {
+  if (D > 4096 || H < 2048 || M * D * H >= (int64_t)1 << 36) return false;
+  return M >= 160 || (tile_mlp_serves(M, D, H) && M >= (D * H <= (int64_t)1 << 23 ? 33 : 48));
+}
+
+// values: [M, H / cf] fp32, 16-byte aligned.
+int values_mlp(const void* x, const void* gate, const float* bias, const void* up, const void* down,
+               void* packed, void* out, int64_t M, int64_t D, int64_t H, int cf, void* workspace,
+               size_t workspace_bytes, float* values, cudaStream_t stream) {
+  const int rc = tile_mlp_serves(M, D, H)
+                     ? tile_first(true, x, gate, bias, up, packed, nullptr, values, M, D, H, cf, false, stream)
+                     : pair_gate_up_values(x, gate, bias, up, packed, values, M, D, H, cf, stream);
+  if (rc) return rc;
+  return twell_values_t2d(packed, values, down, out, M, D, H, cf, workspace, workspace_bytes, stream);
+}
+
 int tile_mlp(bool gated, const void* x, const void* gate, const float* bias, const void* up,
              const void* down, void* packed, void* out, int64_t M, int64_t D, int64_t H, int cf,
              void* hidden, cudaStream_t stream) {
-  if (int rc = tile_first(gated, x, gate, bias, up, packed, hidden, M, D, H, cf, false, stream)) return rc;
+  if (int rc = tile_first(gated, x, gate, bias, up, packed, hidden, nullptr, M, D, H, cf, false, stream)) return rc;
   return tile_second(hidden, down, out, M, D, H, stream);
 }
 

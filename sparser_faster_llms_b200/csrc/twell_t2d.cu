@@ -8,6 +8,8 @@
 //   pass A (gated only): warp s dots its slice of the token's x row (8 values per
 //           lane, in registers) with the same slice of up[j, :];
 //           slice sums meet in shared memory and give u, then h = g * u;
+//           (VALUES: h comes as an fp32 array aligned with the slab, computed by the caller's
+//           tensor-core products; only pass B runs and half the rows are read)
 //   pass B: warp s adds h * down[j, slice s] into 8 accumulators per lane - each
 //           warp owns its output columns, so no reduction inside the CTA.
 // The CTA pushes its column sums into the owning CTA of its cluster through
@@ -115,9 +117,10 @@ __device__ __forceinline__ float2 far_gather(const FusedAr& ar, const unsigned c
 
 // NI = D / 256 = warps per CTA.
 // grid.x = M * nc * cs, cluster = cs.  ws_partial: [M][nc][D] fp32, ws_counter: [M][8] (nc > 1).
-template <int NI, bool GATED, bool HP>
+template <int NI, bool GATED, bool HP, bool VALUES>
 __global__ void __launch_bounds__(NI * 32)
 twell_t2d_kernel(const __nv_bfloat16* x, const uint32_t* __restrict__ packed,
+                 const float* __restrict__ values,
                  const __nv_bfloat16* __restrict__ up, const __nv_bfloat16* __restrict__ down,
                  __nv_bfloat16* out, int M, int tiles, int slab_w, int cs, int nc,
                  float* ws_partial, unsigned int* ws_counter,
@@ -127,6 +130,7 @@ twell_t2d_kernel(const __nv_bfloat16* x, const uint32_t* __restrict__ packed,
   constexpr int NTHREADS = NI * 32;
   __shared__ int tile_off[kMaxTiles + 1];
   __shared__ uint32_t entries[kChunk];
+  __shared__ float hidden_s[VALUES ? kChunk : 1];  // their hidden values
   __shared__ float usum[2][GATED ? kDepth : 1][GATED ? NI : 1];  // double-buffered per batch
   __shared__ __align__(16) float inbox[D];  // [cs][D / cs]: column sums pushed by the cluster
   __shared__ int is_last;
@@ -227,8 +231,9 @@ twell_t2d_kernel(const __nv_bfloat16* x, const uint32_t* __restrict__ packed,
         const int mid = (a + b) >> 1;
         if (tile_off[mid] <= k) a = mid; else b = mid;
       }
-      const uint32_t word = src[(size_t)a * slab_w + 1 + (k - tile_off[a])];
-      entries[i] = word;
+      const size_t at = (size_t)a * slab_w + 1 + (k - tile_off[a]);
+      entries[i] = src[at];
+      if (VALUES) hidden_s[i] = __ldg(values + (size_t)row * row_words + at);
     }
     __syncthreads();
 
@@ -290,7 +295,7 @@ twell_t2d_kernel(const __nv_bfloat16* x, const uint32_t* __restrict__ packed,
           h_lane = HP ? __bfloat162float(gval) * s
                       : __bfloat162float(__hmul(gval, __float2bfloat16_rn(s)));
         } else {
-          h_lane = __bfloat162float(gval);
+          h_lane = VALUES ? hidden_s[e0 + lane] : __bfloat162float(gval);
         }
       }
       // pass B: column-sliced down projection (padding entries have h = 0, row = 0)
@@ -444,14 +449,14 @@ twell_t2d_kernel(const __nv_bfloat16* x, const uint32_t* __restrict__ packed,
   collect();
 }
 
-template <int NI, bool GATED, bool HP>
-int launch_t2d(const void* x, const void* packed, const void* up, const void* down, void* out,
+template <int NI, bool GATED, bool HP, bool VALUES>
+int launch_t2d(const void* x, const void* packed, const float* values, const void* up, const void* down, void* out,
                int64_t M, int64_t H, int cf, int cs, int nc, float* ws_partial,
                unsigned int* ws_counter, const unsigned char* skip_rows, const FusedAr& ar,
                const RunIf& run_if, cudaStream_t stream) {
   const int slab_w = kTileN / cf;
   const int tiles = (int)(H / kTileN);
-  auto kern = twell_t2d_kernel<NI, GATED, HP>;
+  auto kern = twell_t2d_kernel<NI, GATED, HP, VALUES>;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(M * nc * cs), 1, 1);
   cfg.blockDim = dim3(NI * 32, 1, 1);
@@ -493,7 +498,7 @@ int launch_t2d(const void* x, const void* packed, const void* up, const void* do
   cfg.numAttrs = add_pdl_attribute(attr, 1, 2);
   cudaError_t e = cudaLaunchKernelEx(
       &cfg, kern, reinterpret_cast<const __nv_bfloat16*>(x),
-      reinterpret_cast<const uint32_t*>(packed), reinterpret_cast<const __nv_bfloat16*>(up),
+      reinterpret_cast<const uint32_t*>(packed), values, reinterpret_cast<const __nv_bfloat16*>(up),
       reinterpret_cast<const __nv_bfloat16*>(down), reinterpret_cast<__nv_bfloat16*>(out), (int)M,
       tiles, slab_w, cs, nc, ws_partial, ws_counter, skip_rows, ar,
       run_if);
@@ -501,16 +506,16 @@ int launch_t2d(const void* x, const void* packed, const void* up, const void* do
   return B200_OK;
 }
 
-template <bool GATED, bool HP>
-int dispatch_ni(int ni, const void* x, const void* packed, const void* up, const void* down,
+template <bool GATED, bool HP, bool VALUES = false>
+int dispatch_ni(int ni, const void* x, const void* packed, const float* values, const void* up, const void* down,
                 void* out, int64_t M, int64_t H, int cf, int cs, int nc, float* ws_partial,
                 unsigned int* ws_counter, const unsigned char* skip_rows, const FusedAr& ar,
                 const RunIf& run_if, cudaStream_t stream) {
   switch (ni) {
 #define B200_CASE(N)                                                                           \
   case N:                                                                                      \
-    return launch_t2d<N, GATED, HP>(x, packed, up, down, out, M, H, cf, cs, nc, ws_partial,   \
-                                    ws_counter, skip_rows, ar, run_if, stream);
+    return launch_t2d<N, GATED, HP, VALUES>(x, packed, values, up, down, out, M, H, cf, cs, nc, ws_partial,   \
+                                            ws_counter, skip_rows, ar, run_if, stream);
     B200_CASE(1) B200_CASE(2) B200_CASE(3) B200_CASE(4) B200_CASE(5) B200_CASE(6) B200_CASE(7)
     B200_CASE(8) B200_CASE(9) B200_CASE(10) B200_CASE(11) B200_CASE(12) B200_CASE(13)
     B200_CASE(14) B200_CASE(15) B200_CASE(16)
@@ -531,11 +536,14 @@ constexpr size_t kT2dCounterWords = kCounterWords - 64;
 
 // Launch shape.  cs: CTAs per cluster (D / cs must stay a multiple of 8 columns).
 // nc: clusters per token - more than one only when there are few tokens and the
-// caller's workspace can hold the partial sums.
+// caller's workspace can hold the partial sums.  ctas_per_sm: how far a token is spread while the grid
+// grows; the values form holds half the rows in flight and takes 1024 threads per SM (2 % density, us, two
+// CTAs / 1024 threads per SM: D 2048, H 8192, 128 tokens 44.2 / 34.7, 256 tokens 68.9 / 49.2; D 1024,
+// H 4096, 256 tokens 30.7 / 19.3, 512 tokens 33.8 / 26.0; more threads: 128 tokens 38.3).
 void t2d_shape(int64_t M, int64_t D, int sm_count, size_t workspace_bytes, int* cs_out,
-               int* nc_out) {
+               int* nc_out, int64_t ctas_per_sm = 2) {
   int cs = 1;
-  while (cs < 8 && M * cs * 2 <= (int64_t)sm_count * 2 && (D / (cs * 2)) % 8 == 0) cs *= 2;
+  while (cs < 8 && M * cs * 2 <= (int64_t)sm_count * ctas_per_sm && (D / (cs * 2)) % 8 == 0) cs *= 2;
   int nc = 1;
   if (workspace_bytes > kCounterWords * 4 && M * 8 <= (int64_t)kT2dCounterWords) {
     const int64_t cap_floats = (int64_t)((workspace_bytes - kCounterWords * 4) / 4);
@@ -556,13 +564,15 @@ void t2d_shape(int64_t M, int64_t D, int sm_count, size_t workspace_bytes, int* 
   *nc_out = nc;
 }
 
-int twell_t2d_launch(bool gated, bool hp, const void* x, const void* packed, const void* up,
-                     const void* down, void* out, int64_t M, int64_t D, int64_t H, int cf,
-                     void* workspace, size_t workspace_bytes, int sm_count, cudaStream_t stream,
-                     const unsigned char* skip_rows = nullptr,
-                     const FusedAr* fused_ar = nullptr, const RunIf& run_if = {nullptr, 0u}) {
+namespace {
+
+int t2d_launch(bool gated, bool hp, const void* x, const void* packed, const float* values,
+               const void* up, const void* down, void* out, int64_t M, int64_t D, int64_t H, int cf,
+               void* workspace, size_t workspace_bytes, int sm_count, cudaStream_t stream,
+               const unsigned char* skip_rows, const FusedAr* fused_ar, const RunIf& run_if) {
   int cs = 1, nc = 1;
-  t2d_shape(M, D, sm_count, workspace != nullptr ? workspace_bytes : 0, &cs, &nc);
+  t2d_shape(M, D, sm_count, workspace != nullptr ? workspace_bytes : 0, &cs, &nc,
+            values != nullptr ? 8192 / D : 2);
   FusedAr far = {};
   if (fused_ar != nullptr && fused_ar->world > 1) {
     // Every CTA must be resident while it waits for the peers (the exact residency check
@@ -580,18 +590,21 @@ int twell_t2d_launch(bool gated, bool hp, const void* x, const void* packed, con
   float* partial = workspace ? reinterpret_cast<float*>(counters + kCounterWords) : nullptr;
   const int ni = (int)(D / 256);
   auto run = [&](int cs_, int nc_) {
+    if (values != nullptr)
+      return dispatch_ni<false, true, true>(ni, x, packed, values, up, down, out, M, H, cf, cs_, nc_,
+                                            partial, counters, skip_rows, far, run_if, stream);
     if (gated) {
-      return hp ? dispatch_ni<true, true>(ni, x, packed, up, down, out, M, H, cf, cs_, nc_, partial,
+      return hp ? dispatch_ni<true, true>(ni, x, packed, nullptr, up, down, out, M, H, cf, cs_, nc_, partial,
                                           counters, skip_rows, far, run_if,
                                          stream)
-                : dispatch_ni<true, false>(ni, x, packed, up, down, out, M, H, cf, cs_, nc_,
+                : dispatch_ni<true, false>(ni, x, packed, nullptr, up, down, out, M, H, cf, cs_, nc_,
                                            partial, counters, skip_rows, far, run_if,
                                          stream);
     }
-    return hp ? dispatch_ni<false, true>(ni, x, packed, up, down, out, M, H, cf, cs_, nc_, partial,
+    return hp ? dispatch_ni<false, true>(ni, x, packed, nullptr, up, down, out, M, H, cf, cs_, nc_, partial,
                                          counters, skip_rows, far, run_if,
                                          stream)
-              : dispatch_ni<false, false>(ni, x, packed, up, down, out, M, H, cf, cs_, nc_,
+              : dispatch_ni<false, false>(ni, x, packed, nullptr, up, down, out, M, H, cf, cs_, nc_,
                                           partial, counters, skip_rows, far, run_if,
                                          stream);
   };
@@ -605,7 +618,26 @@ int twell_t2d_launch(bool gated, bool hp, const void* x, const void* packed, con
   return rc;
 }
 
+}  // namespace
+
+int twell_t2d_launch(bool gated, bool hp, const void* x, const void* packed, const void* up,
+                     const void* down, void* out, int64_t M, int64_t D, int64_t H, int cf,
+                     void* workspace, size_t workspace_bytes, int sm_count, cudaStream_t stream,
+                     const unsigned char* skip_rows = nullptr,
+                     const FusedAr* fused_ar = nullptr, const RunIf& run_if = {nullptr, 0u}) {
+  return t2d_launch(gated, hp, x, packed, nullptr, up, down, out, M, D, H, cf, workspace,
+                    workspace_bytes, sm_count, stream, skip_rows, fused_ar, run_if);
+}
+
 int sm_count();  // c_api.cu
+
+// out = h down over the stored entries, h given in fp32 in the slots of the slab ([M][H / cf] floats).
+int twell_values_t2d(const void* packed, const float* values, const void* down, void* out, int64_t M,
+                     int64_t D, int64_t H, int cf, void* workspace, size_t workspace_bytes,
+                     cudaStream_t stream) {
+  return t2d_launch(false, true, nullptr, packed, values, nullptr, down, out, M, D, H, cf, workspace,
+                    workspace_bytes, sm_count(), stream, nullptr, nullptr, {nullptr, 0u});
+}
 
 }  // namespace b200
 

@@ -58,3 +58,11 @@ def test_routed_rows_keep_their_positives(m, h):
     u = (x.double() @ up.double().T).bfloat16().double()
     ref = ((p * u).bfloat16().double() @ down.double())[taken]
     assert ((y1.double()[taken] - ref).norm() / ref.norm()).item() < 2e-3  # y rounded once
+
+
+@pytest.mark.parametrize("m,d,h", [(33, 1024, 2048), (48, 2048, 5632), (128, 4096, 16384), (257, 1024, 8192),
+                                   (160, 512, 11008), (777, 256, 4352), (4095, 2048, 2304)])
+@pytest.mark.parametrize("cf,dense", [(8, False), (2, False), (8, True)])
+def test_high_precision_with_gathered_down_product(m, d, h, cf, dense):
+    """fp32 hidden values in the slots of the slabs, from one-SM tiles and from pairs of SMs."""
+    assert run_case(m, d, h, cf=cf, hp=True, dense=dense) > 0
