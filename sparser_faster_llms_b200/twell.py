@@ -20,6 +20,7 @@ pybind extension.  Differences a caller can observe:
 """
 from __future__ import annotations
 
+import ctypes
 import os
 from pathlib import Path
 from types import SimpleNamespace
@@ -29,6 +30,11 @@ import torch
 from torch import nn
 
 from . import _lib
+
+try:  # native host side of eager calls; without it the Python path below serves them
+    from . import _host_call
+except ImportError:
+    _host_call = None
 
 # Attributes the reference module exposes and the reference benchmark pokes at
 # (benchmark_inference.py:55-117).  There is no JIT build here; they exist so that
@@ -421,6 +427,27 @@ def ensure_d2t_layer_shape(layer_number: int, M: int, ext=None) -> None:
     _layer(layer_number)["m"] = int(M)
 
 
+_HOST_FNS: tuple | None = None  # the library and the addresses of its entry points
+
+
+def _host_served(gated, A, first, bias, UP, DOWN, C_packed, OUT, cf, option) -> bool:
+    """The whole call in native code (``csrc_host/host_call.cpp``); False: not the plain case."""
+    global _HOST_FNS
+    if _host_call is None or not (isinstance(A, torch.Tensor) and A.is_cuda):
+        return False
+    lib = _lib.load_library()
+    if _HOST_FNS is None or _HOST_FNS[0] is not lib:
+        _HOST_FNS = (lib, *(ctypes.cast(getattr(lib, name), ctypes.c_void_p).value for name in (
+            "b200_twell_mlp_scratch", "b200_twell_gated_mlp_scratch", "b200_twell_mlp_scratch_bytes")))
+    status = _host_call.call(_HOST_FNS[2 if gated else 1], _HOST_FNS[3], A, first, bias, UP, DOWN,
+                             C_packed, OUT, cf, option, *_lib.workspace(A.device), _DENSE_FROM_TOKENS)
+    if status is None:
+        return False
+    if status != _lib.OK:
+        _lib.check("b200_twell_gated_mlp_scratch" if gated else "b200_twell_mlp_scratch", status)
+    return True
+
+
 def _gated_mlp(layer_number, A, UP, DOWN, C_packed, OUT, highest_precision, cf) -> None:
     entry = _layer(layer_number)
     if entry["cf"] != cf:
@@ -428,6 +455,11 @@ def _gated_mlp(layer_number, A, UP, DOWN, C_packed, OUT, highest_precision, cf) 
             f"layer {int(layer_number)} was created with compression_factor={entry['cf']}, "
             f"called with {cf}")
     GATE = entry["B"]
+    if ("dense_route" not in entry and "fused_allreduce" not in entry
+            and _host_served(True, A, GATE, entry["bias"], UP, DOWN, C_packed, OUT, cf,
+                             _lib.FLAG_HIGH_PRECISION if highest_precision else 0)):
+        entry["m"] = A.shape[0]
+        return
     _need(A, "A", torch.bfloat16)
     _need(UP, "UP", torch.bfloat16)
     _need(DOWN, "DOWN", torch.bfloat16)
@@ -556,6 +588,9 @@ def d2t_layer_dense_route_counters(layer_number: int) -> dict | None:
 def _plain_mlp(layer_number, A, DOWN, C_packed, OUT, num_splits) -> None:
     entry = _layer(layer_number)
     UP = entry["B"]
+    if _host_served(False, A, UP, None, None, DOWN, C_packed, OUT, entry["cf"], int(num_splits)):
+        entry["m"] = A.shape[0]
+        return
     _need(A, "A", torch.bfloat16)
     _need(DOWN, "DOWN", torch.bfloat16)
     m, d = A.shape
