@@ -33,8 +33,10 @@ int twell_pack_tc_splitk8(const void* x, const void* w, const float* bias, void*
 int twell_pack_tc_splitk_mid(const void* x, const void* w, const float* bias, void* packed,
                              int64_t M, int64_t D, int64_t H, int cf, int split,
                              cudaStream_t stream);
-bool twell_pack_mid_serves(int64_t M, int64_t H, int sm_count);
 int twell_pack_tc_status();
+bool tile_pack_serves(int64_t M, int64_t H);
+int tile_pack(const void* x, const void* w, const float* bias, void* packed, int64_t M, int64_t D,
+              int64_t H, int cf, cudaStream_t stream);
 int twell_t2d_launch(bool gated, bool hp, const void* x, const void* packed, const void* up,
                      const void* down, void* out, int64_t M, int64_t D, int64_t H, int cf,
                      void* workspace, size_t workspace_bytes, int sm_count, cudaStream_t stream,
@@ -209,19 +211,15 @@ int b200_twell_pack_select(const void* x, const void* w, const float* bias, void
   }
   if (kernel == 0 && M > 16 && M <= 32 && H <= 8 * kTileN && D % 512 == 0)
     return twell_pack_tc_splitk8(x, w, bias, packed, M, D, H, cf, st);
+  if (kernel == 0 && tile_pack_serves(M, H)) return tile_pack(x, w, bias, packed, M, D, H, cf, st);
   if (kernel == 3 || (kernel == 0 && M > 16 && M <= 32))
     return twell_pack_tc_splitk(x, w, bias, packed, M, D, H, cf, st);
   if (kernel == 5) return twell_pack_tc_splitk8(x, w, bias, packed, M, D, H, cf, st);
   if (kernel == 8) return twell_pack_tc_splitk_mid(x, w, bias, packed, M, D, H, cf, 4, st);
   if (kernel == 9) return twell_pack_tc_splitk_mid(x, w, bias, packed, M, D, H, cf, 2, st);
-  // 33..256 tokens: 128-token tiles with d_model split four ways over a cluster while that grid is
-  // one wave; beyond, 256-token tiles on pairs of SMs.  Where the four-way grid does not fit, us,
-  // two-way split / pairs: D 2048, H 8192, 256 tokens 24.9 / 19.5; H 11008, 64 tokens 24.7 / 19.5;
-  // D 4096, H 16384, 64 tokens 40.3 / 35.0.  Against one-SM tiles of 256 tokens from 257 tokens on:
-  // D 2048, H 8192: 512 tokens 32.8 / 20.3, 2048 tokens 65.8 / 56.2, 16384 tokens 576 / 397; level
-  // at D 4096 up to 512 tokens (H 16384: 57.5 / 58.4).
-  if (kernel == 0 && twell_pack_mid_serves(M, H, sm_count()))
-    return twell_pack_tc_splitk_mid(x, w, bias, packed, M, D, H, cf, 4, st);
+  // Beyond the one-SM tiles, 256-token tiles on pairs of SMs.  Against one-SM tiles of 256 tokens from
+  // 257 tokens on: D 2048, H 8192: 512 tokens 32.8 / 20.3, 2048 tokens 65.8 / 56.2, 16384 tokens
+  // 576 / 397; level at D 4096 up to 512 tokens (H 16384: 57.5 / 58.4).
   if (kernel == 2 || kernel == 4 || kernel == 7 || (kernel == 0 && M > 32))
     return pair_pack(x, w, bias, packed, nullptr, M, D, H, cf, nullptr, {nullptr, 0, nullptr}, st);
   return twell_pack_small(x, w, bias, packed, M, D, H, cf, st);

@@ -8,7 +8,7 @@
 namespace b200 {
 
 int sm_count();
-bool twell_pack_mid_serves(int64_t M, int64_t H, int sm_count);
+bool tile_pack_serves(int64_t M, int64_t H);
 int twell_t2d_launch(bool gated, bool hp, const void* x, const void* packed, const void* up,
                      const void* down, void* out, int64_t M, int64_t D, int64_t H, int cf,
                      void* workspace, size_t workspace_bytes, int sm_count, cudaStream_t stream,
@@ -585,7 +585,7 @@ extern "C" int b200_hybrid_train_forward_timed(
     return fail(B200_ECUDA, "%s: cudaMemsetAsync failed", fn);
   // the gate pattern
   pdl_suppressed() = true;  // its predecessor is the memset
-  int rc = M > 128 && !twell_pack_mid_serves(M, H, sm_count())
+  int rc = M > 128 && !tile_pack_serves(M, H)
                ? pair_pack(x, g, nullptr, p_slab, nullptr, M, D, H, cf, nullptr, room, st)
                : b200_twell_pack(x, g, nullptr, p_slab, M, D, H, cf, stream);
   pdl_suppressed() = false;

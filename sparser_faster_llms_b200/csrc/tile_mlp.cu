@@ -127,7 +127,7 @@ struct FirstArgs {
 };
 
 // grid = (H / NB, ceil(M / 128)), cluster = 256 / NB along the neurons.
-template <bool GATED, bool VALUES, int NB>
+template <bool GATED, bool VALUES, int NB, int RANGES>
 __global__ void __launch_bounds__(kThreads, 1)
 first_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_g,
              const __grid_constant__ CUtensorMap map_u, const __grid_constant__ FirstArgs a) {
@@ -136,10 +136,10 @@ first_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ 
   constexpr int kStage = kRowBytes + COLS * 128;
   constexpr int STAGES = kRing / kStage > 8 ? 8 : kRing / kStage;
   constexpr int BLKS = NB / 64;  // 32-column blocks per epilogue warp
-  // High precision keeps the sums of two or four ranges of k apart in TMEM and adds them in fp32: a tensor
-  // core's running sum loses bits with its length (64 tokens, D 2048, 5 %: error against 64 bits
-  // 1.6712e-3 with one range, 1.6593e-3 where D was split four ways before).
-  constexpr int RANGES = VALUES ? 512 / COLS : 1;
+  // High precision and the pack keep the sums of two or four ranges of k apart in TMEM and add them in
+  // fp32: a tensor core's running sum loses bits with its length (64 tokens, D 2048, 5 %: error against
+  // 64 bits 1.6712e-3 with one range, 1.6593e-3 where D was split four ways before).
+  static_assert(RANGES * COLS <= 512, "TMEM columns");
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -226,7 +226,7 @@ first_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ 
       for (int p = 0; p < 16; ++p) gw[b][p] = pg::pack2(fmaxf(v[2 * p], 0.f), fmaxf(v[2 * p + 1], 0.f));
     }
   }
-  if (warp == 0) pdl_trigger();
+  if (warp == 0 && (VALUES || a.hidden != nullptr)) pdl_trigger();  // not for a contraction after a pack
   cluster.barrier_wait();  // every CTA of the cluster runs
   if (warp >= 3) {
 #pragma unroll
@@ -271,7 +271,7 @@ first_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ 
         }
       if (VALUES) {
       } else if (!GATED) {
-        if (live) pg::store64(out + b * 32, gw[b], a.wide);
+        if (live && a.hidden != nullptr) pg::store64(out + b * 32, gw[b], a.wide);
       } else {
         __syncwarp();
         tmem_ld32(acc + (uint32_t)(NB + b * 32), v);
@@ -424,7 +424,7 @@ int launch_cluster(const char* fn, Kernel kern, dim3 grid, int cluster, size_t s
   return B200_OK;
 }
 
-template <bool GATED, bool VALUES, int NB>
+template <bool GATED, bool VALUES, int NB, int RANGES = VALUES ? 256 / NB : 1>
 int launch_first(const void* x, const void* g, const void* u, FirstArgs a, int64_t D, cudaStream_t stream) {
   constexpr int kStage = kRowBytes + (GATED ? 2 : 1) * NB * 128;
   constexpr int STAGES = kRing / kStage > 8 ? 8 : kRing / kStage;
@@ -433,7 +433,7 @@ int launch_first(const void* x, const void* g, const void* u, FirstArgs a, int64
   if (int rc = make_map(&mg, g, a.H, D, NB)) return rc;
   if (int rc = make_map(&mu, u, a.H, D, NB)) return rc;
   static size_t granted[64] = {0};
-  return launch_cluster("gate and up tiles", first_kernel<GATED, VALUES, NB>,
+  return launch_cluster("gate and up tiles", first_kernel<GATED, VALUES, NB, RANGES>,
                         dim3((unsigned)(a.H / NB), (unsigned)((a.M + kRows - 1) / kRows), 1), kTileN / NB,
                         (size_t)STAGES * kStage + 1024, granted, stream, mx, mg, mu, a);
 }
@@ -512,6 +512,37 @@ int tile_first(bool gated, const void* x, const void* gate, const float* bias, c
   return values != nullptr ? tm::launch_first<true, true, 128>(x, gate, up, a, D, stream)
          : gated           ? tm::launch_first<true, false, 128>(x, gate, up, a, D, stream)
                            : tm::launch_first<false, false, 128>(x, gate, gate, a, D, stream);
+}
+
+// Whether a pack runs here: 33 to 256 tokens while the grid is one wave, and 17 to 32 tokens where the
+// four-way split over a cluster is more than one.  us, split-k (or pairs of SMs) / here, weights from HBM:
+//   33 to 128 tokens   D 1024, H 4096 10.9 / 7.4;  D 2048, H 2048 12.5 / 10.5;  H 5632 13.9 / 11.1;
+//                      H 8192 15.5 / 11.6;  H 11008 18.6 / 14.7;  D 4096, H 4096 16.9 / 16.8;  H 16384 34.5 / 29.5
+//   256 tokens         D 1024, H 4096 12.3 / 7.9;  D 2048, H 4096 14.0 / 11.0;  H 8192 17.7 / 13.8;
+//                      two waves: H 11008 18.7 / 25.3
+//   32 tokens          D 2048, H 5632 8.8 / 10.9;  H 8192 10.5 / 11.5;  two waves of the split: H 11008
+//                      17.8 / 14.5;  D 4096, H 16384 32.7 / 29.4
+bool tile_pack_serves(int64_t M, int64_t H) {
+  if (M <= 32) return M > 16 && H / 64 > fours() && H / 128 <= sm_count();
+  return M <= 256 && row_tiles(M) * (H / 128) <= sm_count();
+}
+
+// Slabs only.
+int tile_pack(const void* x, const void* w, const float* bias, void* packed, int64_t M, int64_t D,
+              int64_t H, int cf, cudaStream_t stream) {
+  tm::FirstArgs a = {};
+  a.bias = bias;
+  a.bias16 = aligned16(bias);
+  a.packed = static_cast<uint32_t*>(packed);
+  a.slab_w = kTileN / cf;
+  a.row_words = (int)(H / kTileN) * a.slab_w;
+  a.H = H;
+  a.M = (int)M;
+  a.ksteps = (int)(D / kStageK);
+  a.box = token_box(M);
+  if (row_tiles(M) * (H / 64) <= fours())
+    return tm::launch_first<false, false, 64, 4>(x, w, w, a, D, stream);
+  return tm::launch_first<false, false, 128, 4>(x, w, w, a, D, stream);
 }
 
 // out[M, D] = hidden[M, H] down with down [H, D] as it is stored.

@@ -1,8 +1,8 @@
 // Gate projection + ReLU + TwELL pack on the 5th-generation tensor cores.
 //
-// Kernels of this file, by token count: twell_pack_tc_splitk_(wide_)kernel (17..32 tokens) and
-// twell_pack_tc_splitk_mid_kernel (33..256, 128-token tiles), both with D split over a cluster.
-// Larger calls run on pairs of SMs (pair_gemm.cuh).
+// Kernels of this file: twell_pack_tc_splitk_(wide_)kernel (17..32 tokens) and, only where a caller asks for it,
+// twell_pack_tc_splitk_mid_kernel (128-token tiles), both with D split over a cluster.
+// Larger calls run on one-SM tiles (tile_mlp.cu) and on pairs of SMs (pair_gemm.cuh).
 //
 // CTA tile: one 256-neuron TwELL tile x NTOK tokens x a slice of D.
 // Neurons ride the MMA M axis as two 128-row accumulators, tokens the N axis:
@@ -717,25 +717,13 @@ int twell_pack_tc_splitk8(const void* x, const void* w, const float* bias, void*
 // 12.8 us for the 4-way split: one SM pulls about 64 GB/s through TMA, so the weight stream
 // needs well over 100 CTAs to reach the HBM rate.)
 
-// 33..256 tokens: split-k over a cluster of `split` (4 or 2) CTAs with 128-token tiles.
+// 33..256 tokens: split-k over a cluster of `split` (4 or 2) CTAs with 128-token tiles.  Only by choice of the
+// caller: the one-SM tiles of tile_mlp.cu are level or ahead at every size.
 int twell_pack_tc_splitk_mid(const void* x, const void* w, const float* bias, void* packed,
                              int64_t M, int64_t D, int64_t H, int cf, int split,
                              cudaStream_t stream) {
   if (split == 2) return launch_tc_splitk_mid<2, 4>(x, w, bias, packed, M, D, H, cf, stream);
   return launch_tc_splitk_mid<4, 4>(x, w, bias, packed, M, D, H, cf, stream);
-}
-
-// Whether 33..256 tokens take the 128-token kernel with D split four ways instead of 256-token tiles
-// on pairs of SMs: while its grid is one wave (one CTA per SM).  One block of tokens, D 2048,
-// H 8192: 15.9 against 19.4 us.  Two blocks double the clusters, and of clusters of four 33 are
-// resident at once (the rest of a GPC's SMs is no multiple of four), so the line lies at 16 tiles.
-// Measured on B200, 256 tokens, us, split-k / pairs: D 1024, H 4096 12.9 / 13.7; D 2048, H 1024
-// 13.8 / 18.4; D 2048, H 4096 15.0 / 19.0; D 4096, H 4096 19.5 / 29.7; 18 tiles (36 clusters),
-// D 2048, H 4608 27.0 / 19.1.
-bool twell_pack_mid_serves(int64_t M, int64_t H, int sm_count) {
-  const int64_t clusters = H / kTileN * ((M + kTokMid - 1) / kTokMid);
-  if (M <= 32 || M > 2 * kTokMid) return false;
-  return M <= kTokMid ? 4 * clusters <= sm_count : clusters <= sm_count / 4 - 4;
 }
 
 // Error word raised by a bounded wait that gave up (0 = none).  Reads and clears it;

@@ -4,6 +4,7 @@ oracle and bounds of ``test_pair_gemm_gpu`` (the products are dense: y is rounde
 import pytest
 import torch
 
+from oracle import ffn_oracle as fo, twell_format as tf
 from sparser_faster_llms_b200 import _lib, synthetic, twell
 from test_pair_gemm_gpu import DEV, run_case
 
@@ -66,3 +67,21 @@ def test_routed_rows_keep_their_positives(m, h):
 def test_high_precision_with_gathered_down_product(m, d, h, cf, dense):
     """fp32 hidden values in the slots of the slabs, from one-SM tiles and from pairs of SMs."""
     assert run_case(m, d, h, cf=cf, hp=True, dense=dense) > 0
+
+
+@pytest.mark.parametrize("m,d,h", [(17, 256, 8960), (32, 1024, 16384), (33, 256, 256), (64, 2048, 8192),
+                                   (128, 768, 2304), (129, 512, 4352), (256, 4096, 8192)])
+@pytest.mark.parametrize("cf", [8, 4])
+def test_pack_form(m, d, h, cf):
+    """Slabs alone, both neuron widths, bit for bit on the exact inputs; a row past the slab's capacity keeps
+    its true count."""
+    x, gate, _, _ = synthetic.dyadic_case(m, d, h, seed=m)
+    x[::7, 0] = -0.5
+    want = tf.pack_preactivations(fo.gate_preactivation(x, gate).numpy(), cf)
+    packed = twell.allocate_packed_output(m, h, device=DEV, compression_factor=cf)
+    xg, gg = x.to(DEV), gate.to(DEV)
+    _lib.call("b200_twell_pack", torch.device(DEV), xg.data_ptr(), gg.data_ptr(), None, packed.data_ptr(),
+              m, d, h, cf)
+    torch.cuda.synchronize()
+    assert (packed.cpu().view(torch.int32).numpy().view("uint32") == want).all()
+    assert _lib.load_library().b200_twell_pack_tc_status() == 0
