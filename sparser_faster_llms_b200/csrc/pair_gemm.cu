@@ -79,23 +79,20 @@ int pair_pack(const void* x, const void* w, const float* bias, void* packed, voi
                                                   sm_count(), stream);
 }
 
-// hidden[M, H] (hp: [M, 3 H]) = gate values of the slabs times x up^T on their pattern.
-int pair_up(bool hp, const void* x, const void* packed, const void* up, void* hidden, int64_t M,
-            int64_t D, int64_t H, int cf, const RunIf& run_if, const SplitRoom& room, cudaStream_t stream) {
+// hidden[M, 3 H] = gate values of the slabs times x up^T on their pattern, as three bf16 terms.
+int pair_up(const void* x, const void* packed, const void* up, void* hidden, int64_t M, int64_t D,
+            int64_t H, int cf, const RunIf& run_if, const SplitRoom& room, cudaStream_t stream) {
   pg::Args a = base_args(M, H, D);
   a.run_if = run_if;
   a.slab_p = const_cast<uint32_t*>(static_cast<const uint32_t*>(packed));
   a.slab_w = kTileN / cf;
   a.row_words = (int)(H / kTileN) * a.slab_w;
   a.out = static_cast<__nv_bfloat16*>(hidden);
-  a.ld = hp ? 3 * H : H;
+  a.ld = 3 * H;
   a.wide = aligned32(hidden);
   pg::give_room(a, room);
   const pg::Operand ox = {x, M, D}, ou = {up, H, D};
-  return hp ? pg::launch<pg::kMulHp, false, false>("up product", ox, ox, ou, ou, a, M, sm_count(),
-                                                   stream)
-            : pg::launch<pg::kMul, false, false>("up product", ox, ox, ou, ou, a, M, sm_count(),
-                                                 stream);
+  return pg::launch<pg::kMulHp, false, false>("up product", ox, ox, ou, ou, a, M, sm_count(), stream);
 }
 
 // out[M, D] = hidden[M, terms * H] [down; down; ...] with down [H, D] as it is stored.
@@ -172,33 +169,26 @@ int64_t dense_from(int64_t D, int64_t H) {
 }  // namespace
 
 // Which calls of the fused MLPs take this form.  High precision pays three down products, so it
-// needs a larger call; the non-gated MLP saves only half as much.
+// needs a larger call; the non-gated MLP saves only half as much (600 tokens, D 1024, H 4096, gathers at
+// 0.5 % / 2 % -> dense 21 / 30 -> 31; 300 tokens, D 2048, H 8192 33 / 53 -> 44).
 bool pair_mlp_serves(int64_t M, int64_t D, int64_t H, bool gated, bool hp) {
   if (H < 2048) return false;  // few entries per token: nothing to gain
   if (hp) return M * D * H >= (int64_t)1 << 36;
   return M >= (gated ? 1 : 2) * dense_from(D, H);
 }
 
-// Whether the device chooses between the dense and the gather form of the up and down products by
-// the stored entries of the call (two launches that return at once and a 4-byte memset, about
-// 10 us); otherwise gate and up run in one launch and the dense form always.  At 0.5 % density, us,
-// always dense / gather: D 2048, H 8192, 1600 tokens 171 / 141, 2048 tokens 173 / 160, 4096 tokens
-// 295 / 302; D 1024, H 4096, 2048 tokens 60 / 54, 4096 tokens 89 / 97; D 4096, H 16384, 2048 tokens
-// 572 / 745.  At 16384 tokens, D 2048, H 8192: gather 1103 us at 0.5 %, dense 1217 at any density,
-// gather 2659 at 2 %.  The non-gated MLP, whose dense form saves less, always asks; what asking costs
-// at low density: D 1024, H 4096, 1200 tokens 45 against 35 us at 0.5 %, 52 / 52 at 2 %, 53 / 84 at
-// 5 %; D 2048, H 8192, 800 tokens 69 / 58, 79 / 105, 80 / 193.
-static bool choose_on_device(int64_t M, int64_t D, int64_t H, bool gated, bool hp) {
-  if (hp || !gated) return true;
-  return M > 4096 && rows_in_l2(D, H) && 4 * H * D > (int64_t)32 << 20;
-}
+// Only high precision lets the device choose between the dense and the gather form of the up and down
+// products by the stored entries of the call (two launches that return at once and a 4-byte memset, some
+// 9 us); bf16 products run dense always, gate and up in one launch.  us, asking / always dense, at 0.5 %,
+// 1 %, 2 %: D 2048, H 8192, 9000 tokens 591 / 569, 611 / 571, 655 / 586; 16384 tokens 1051 / 1047, 1065 /
+// 1049, 1085 / 1003; non-gated, D 1024, H 4096, 3000 tokens 61 / 54, 65 / 55, 66 / 55; D 2048, H 8192,
+// 1300 tokens 80 / 82, 91 / 83, 91 / 83, 3000 tokens 144 / 145, 151 / 145, 153 / 146; H 11008, 6000
+// tokens 330 / 356, 366 / 361; D 4096, H 16384 at 1 % 4000 tokens 680 / 670.
 
-// Stored entries per token up to which the gather form is the faster one.  Measured (D 2048,
-// H 8192): up + down 49 ns per token dense and 0.8 ns per entry gathered; high precision 104 ns;
-// D 4096, H 16384 (rows from HBM as well): 176 ns against 2.7 ns, high precision 382 ns.
-static int64_t gather_entries(int64_t D, int64_t H, bool hp) {
-  return H * (hp ? 2 : 1) / (rows_in_l2(D, H) ? 128 : 224);
-}
+// Stored entries per token up to which the gather form is the faster one in high precision.  Measured
+// (D 2048, H 8192): up + down 104 ns per token dense and 0.8 ns per entry gathered; D 4096, H 16384
+// (rows from HBM as well): 382 ns against 2.7 ns.
+static int64_t gather_entries(int64_t D, int64_t H) { return H / (rows_in_l2(D, H) ? 64 : 112); }
 
 size_t pair_part_bytes(int64_t M, int64_t D, int64_t H) { return mlp_part_bytes(M, D, H, 1); }
 
@@ -236,33 +226,26 @@ int pair_mlp(bool gated, bool hp, const void* x, const void* gate, const float* 
     const void* xc = static_cast<const __nv_bfloat16*>(x) + r0 * D;
     void* pc = static_cast<uint32_t*>(packed) + r0 * row_words;
     void* oc = static_cast<__nv_bfloat16*>(out) + r0 * D;
-    RunIf run_if = {nullptr, 0u};
-    const bool choose = choose_on_device(m, D, H, gated, hp);
-    if (choose) {
-      const int64_t limit = m * gather_entries(D, H, hp);
-      run_if = {entries, (unsigned int)(limit < 0x7fffffff ? limit : 0x7fffffff)};
-      if (cudaMemsetAsync(entries, 0, sizeof(unsigned int), stream) != cudaSuccess)
-        return fail(B200_ECUDA, "fused MLP: cudaMemsetAsync failed");
-    }
-    if (gated && !choose) {
-      if (int rc = pair_gate_up(xc, gate, bias, up, pc, scratch, m, D, H, cf, false, stream))
+    if (!hp) {
+      if (int rc = gated ? pair_gate_up(xc, gate, bias, up, pc, scratch, m, D, H, cf, false, stream)
+                         : pair_pack(xc, gate, bias, pc, scratch, m, D, H, cf, nullptr, room, stream))
         return rc;
-    } else {
-      pdl_suppressed() = choose;  // its predecessor is the memset
-      const int rc = pair_pack(xc, gate, bias, pc, gated ? nullptr : scratch, m, D, H, cf,
-                               choose ? entries : nullptr, room, stream);
-      pdl_suppressed() = false;
-      if (rc) return rc;
-      if (gated)
-        if (int rc = pair_up(hp, xc, pc, up, scratch, m, D, H, cf, run_if, room, stream))
-          return rc;
+      if (int rc = pair_down(scratch, 1, down, oc, m, D, H, {nullptr, 0u}, room, stream)) return rc;
+      continue;
     }
-    if (int rc = pair_down(scratch, terms, down, oc, m, D, H, run_if, room, stream))
+    const int64_t limit = m * gather_entries(D, H);
+    const RunIf run_if = {entries, (unsigned int)(limit < 0x7fffffff ? limit : 0x7fffffff)};
+    if (cudaMemsetAsync(entries, 0, sizeof(unsigned int), stream) != cudaSuccess)
+      return fail(B200_ECUDA, "fused MLP: cudaMemsetAsync failed");
+    pdl_suppressed() = true;  // its predecessor is the memset
+    const int rc = pair_pack(xc, gate, bias, pc, nullptr, m, D, H, cf, entries, room, stream);
+    pdl_suppressed() = false;
+    if (rc) return rc;
+    if (int rc = pair_up(xc, pc, up, scratch, m, D, H, cf, run_if, room, stream)) return rc;
+    if (int rc = pair_down(scratch, terms, down, oc, m, D, H, run_if, room, stream)) return rc;
+    if (int rc = twell_t2d_launch(true, true, xc, pc, up, down, oc, m, D, H, cf, workspace,
+                                  workspace_bytes, sm_count(), stream, nullptr, nullptr, run_if))
       return rc;
-    if (run_if.entries != nullptr)
-      if (int rc = twell_t2d_launch(gated, hp, xc, pc, up, down, oc, m, D, H, cf, workspace,
-                                    workspace_bytes, sm_count(), stream, nullptr, nullptr, run_if))
-        return rc;
   }
   return B200_OK;
 }

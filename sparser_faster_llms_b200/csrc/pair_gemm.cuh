@@ -47,9 +47,9 @@ enum Epilogue {
   kStore = 0,    // out[row, col] = bf16(acc)
   kPack = 1,     // TwELL slabs of relu(acc + bias)
   kPackDense = 6,  // the same, and the stored values as a dense matrix
-  kGateUp = 7,   // kPack on a first accumulator (B0) and kMul with its values on a second (B1)
+  kGateUp = 7,   // kPack on a first accumulator (B0) and kMul with its values on a second (B1):
+                 //   out = bf16(g * bf16(acc)) on the slab pattern, 0 elsewhere
   kGateUpHp = 8,  // kPack on B0, and its values times the sums on B1 in fp32, in the slots of the slab
-  kMul = 2,      // out = bf16(g * bf16(acc)) on the slab pattern, 0 elsewhere
   kMulHp = 3,    // g * acc in fp32, as three bf16 terms side by side (out row = [hi | mid | lo])
   kStoreCarry = 9,  // kStore on a product whose k comes in several launches: fp32 sums carried between
   kFwd = 4,      // training forward: R = bf16(acc) and T = R * P as slabs, T dense, l1 partial sums
@@ -809,7 +809,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap map_a0,
       uint2 pw[kTrain ? 8 : 1], rw[EPI == kBwd ? 8 : 1];  // the rows' first slab words
       int tail_slot = -1;
       auto load_pattern = [&]() {
-        if constexpr (EPI == kMul || EPI == kMulHp) load_values(a, buf, row0, rows, nt, half, lane);
+        if constexpr (EPI == kMulHp) load_values(a, buf, row0, rows, nt, half, lane);
         if constexpr (kTrain) {
           load_words(a.slab_p, a, row0, rows, nt, 0, lane, pw);
           if (a.row_slot != nullptr && live) tail_slot = a.row_slot[row];
@@ -1007,7 +1007,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap map_a0,
               w[p] = a.relu ? pack2(fmaxf(v[2 * p], 0.f), fmaxf(v[2 * p + 1], 0.f))
                             : pack2(v[2 * p], v[2 * p + 1]);
             if (live) store64(out + cb * 32, w, a.wide);
-          } else if (EPI == kMul || EPI == kGateUp) {
+          } else if (EPI == kGateUp) {
             uint32_t w[16];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
