@@ -150,7 +150,8 @@ twell_t2d_kernel(const __nv_bfloat16* x, const uint32_t* __restrict__ packed,
   if (run_if.entries != nullptr && *run_if.entries > run_if.limit) return;
   // Fused all-reduce: every CTA reads the call epoch now (the round trip hides under the slab
   // load).  It is advanced by the last (token, slice) group to finish, which cannot happen
-  // before every CTA of the grid has contributed its partial sums, i.e. has started.
+  // before every CTA that has entries has contributed its partial sums, i.e. has started (the others
+  // leave without using it).
   const bool fused = ar.world > 1;
   unsigned char* my_block = nullptr;
 #pragma unroll
@@ -207,7 +208,16 @@ twell_t2d_kernel(const __nv_bfloat16* x, const uint32_t* __restrict__ packed,
   }
   __syncthreads();
   const int n_total = tile_off[tiles];
-  const int parts = cs * nc;
+  // Clusters that this token's entries are worth: another one shortens the gather loop and costs the
+  // partial sums' trip through memory.  us per layer, one cluster / four / eight: D 2048, H 8192, 2
+  // tokens with 41 entries 14.9 / 16.2 / 16.9, 82 entries 16.1 / 16.6 / 16.6, 164 entries 17.6 / 16.5 /
+  // 17.2, 410 entries 22.7 / 18.1 / 17.1; 12 tokens with 41 entries 16.5 / 19.9 (three), 410 30.4 / 28.1.
+  const int used = n_total <= 16 * cs ? 1 : n_total <= 40 * cs ? min(nc, 4) : nc;
+  if (cidx >= used) {  // the same for the whole cluster
+    cluster.barrier_wait();
+    return;
+  }
+  const int parts = cs * used;
   const int per = (n_total + parts - 1) / parts;
   const int lo = (cidx * cs + crank) * per;
   const int hi = min(n_total, lo + per);
@@ -395,7 +405,7 @@ twell_t2d_kernel(const __nv_bfloat16* x, const uint32_t* __restrict__ packed,
       }
     }
   };
-  if (nc == 1) {
+  if (used == 1) {
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const int c = 2 * (tid + k * NTHREADS);
@@ -427,7 +437,7 @@ twell_t2d_kernel(const __nv_bfloat16* x, const uint32_t* __restrict__ packed,
   __syncthreads();
   if (tid == 0) {
     const unsigned int old = atomicAdd(&ws_counter[row * 8 + crank], 1u);
-    is_last = (old == (unsigned int)(nc - 1));
+    is_last = (old == (unsigned int)(used - 1));
   }
   __syncthreads();
   if (!is_last) return;
@@ -438,7 +448,7 @@ twell_t2d_kernel(const __nv_bfloat16* x, const uint32_t* __restrict__ packed,
     const int c = 2 * (tid + k * NTHREADS);
     if (c >= cols) break;
     float s0 = 0.f, s1 = 0.f;
-    for (int q = 0; q < nc; ++q) {
+    for (int q = 0; q < used; ++q) {
       const float2 v = __ldcg(reinterpret_cast<const float2*>(tok_part + (size_t)q * D + c));
       s0 += v.x;
       s1 += v.y;
@@ -547,7 +557,13 @@ void t2d_shape(int64_t M, int64_t D, int sm_count, size_t workspace_bytes, int* 
   int nc = 1;
   if (workspace_bytes > kCounterWords * 4 && M * 8 <= (int64_t)kT2dCounterWords) {
     const int64_t cap_floats = (int64_t)((workspace_bytes - kCounterWords * 4) / 4);
-    int64_t want = ((int64_t)sm_count * 2) / (M * cs);  // about two CTAs per SM in total
+    // About two CTAs per SM of up to 256 threads (us, D 2048, H 8192: 6 tokens, 2 %, six clusters 20.2,
+    // four 18.0; 10 tokens, 5 %, two 27.7, three 26.1; 18 tokens, 5 %, one 31.8, two 29.6), and 98 of the
+    // wider ones, whose rows also share HBM (4 tokens, D 4096, H 16384, 1 %: 256 CTAs 51.0, 64 42.7; 8
+    // tokens 56.6 / 46.3).
+    const bool wide = D > 2048;
+    int64_t want = (int64_t)sm_count * (wide ? 2 : 6) / 3 / (M * cs);
+    if (want > 4 && (wide || want < 8)) want = 4;
     // Clusters per token are capped: every extra cluster adds a partial sum to the final
     // reduction.  Measured at one token (D 2048, H 8192, 28 layers): 0.479 ms per step with a
     // cap of 4..8, 0.483 with 16, 0.515 with 32, 0.514 with 1.  B200_T2D_MAX_NC overrides.
