@@ -70,7 +70,8 @@ int b200_twell_pack(const void* x, const void* w, const float* bias, void* packe
 /*
  * Same as b200_twell_pack with the kernel family chosen by the caller:
  *   kernel 0 = automatic (M == 1: kernel 6 where it serves; M <= 16: kernel 1; 17..32: kernel 3
- *              or 5; 33..256: kernel 8 while its grid is one wave; beyond: kernel 7),
+ *              or 5, one-SM tiles where the split of kernel 3 is two waves; 33..256: one-SM tiles (128
+ *              tokens x 64 or 128 neurons) while their grid is one wave; beyond: kernel 7),
  *   kernel 1 = mma.sync split-k cluster kernel (any M),
  *   kernel 3 = tcgen05 split-k cluster kernel (32 tokens per tile, D split 4 ways),
  *   kernel 5 = tcgen05 split-k cluster kernel with D split 8 ways (D % 512 == 0; chosen
@@ -80,8 +81,7 @@ int b200_twell_pack(const void* x, const void* w, const float* bias, void* packe
  *              automatically for such calls unless B200_ONE_TOKEN=0,
  *   kernel 7 = persistent tcgen05 kernel on pairs of SMs, 256 tokens x 256 neurons per pair, two
  *              accumulators (2 and 4 are other names of it),
- *   kernel 8 / 9 = tcgen05 split-k cluster kernel with 128-token tiles, D split 4 / 2 ways
- *              (8 is chosen automatically for 33..256 tokens while its grid is a single wave).
+ *   kernel 8 / 9 = tcgen05 split-k cluster kernel with 128-token tiles, D split 4 / 2 ways.
  * All produce identical slab bytes on exact-arithmetic inputs.  No reference
  * counterpart (the reference has one WGMMA kernel, matmul_d2t.cu:287-709).
  */
@@ -131,10 +131,11 @@ int b200_twell_gated_mlp(const void* x, const void* gate, const float* gate_bias
 
 /*
  * The same two functions with room for the hidden matrix: a call of more than a few dozen tokens
- * then runs as three tensor-core GEMMs (gate + pack, up times the slab pattern, down) instead of
+ * then runs as tensor-core products (gate + up with the pack in their epilogue, down) instead of
  * pack + per-entry gathers.  Same slab words; the products of the mixed mode are not rounded to
- * bf16 one by one (fp32 sums of exact products), the high-precision mode keeps its hidden values
- * to 24 bits as three bf16 terms.
+ * bf16 one by one (fp32 sums of exact products).  The high-precision mode gathers the down product
+ * with fp32 hidden values below 2^36 multiply-adds per product, and keeps them to 24 bits as three
+ * bf16 terms of a dense product above.
  *   scratch: b200_twell_mlp_scratch_bytes(M, D, H, gated, flags) bytes (0 = such a call has no
  *     use for it), 16-byte aligned, uninitialised.  NULL or too small: the functions above.
  *   workspace: as above; its zero-filled counters are also used to finish the last wave of
