@@ -132,7 +132,8 @@ int b200_twell_gated_mlp(const void* x, const void* gate, const float* gate_bias
 /*
  * The same two functions with room for the hidden matrix: a call of more than a few dozen tokens
  * then runs as tensor-core products (gate + up with the pack in their epilogue, down) instead of
- * pack + per-entry gathers.  Same slab words; the products of the mixed mode are not rounded to
+ * pack + per-entry gathers.  Same slab words on exact-arithmetic inputs (elsewhere last bits may differ,
+ * where D is split otherwise than in b200_twell_pack); the products of the mixed mode are not rounded to
  * bf16 one by one (fp32 sums of exact products).  The high-precision mode gathers the down product
  * with fp32 hidden values below 2^36 multiply-adds per product, and keeps them to 24 bits as three
  * bf16 terms of a dense product above.

@@ -73,7 +73,7 @@ int pair_mlp(bool gated, bool hp, const void* x, const void* gate, const float* 
              const void* up, const void* down, void* packed, void* out, int64_t M, int64_t D,
              int64_t H, int cf, void* workspace, size_t workspace_bytes, void* scratch,
              int64_t max_rows, cudaStream_t stream);
-bool tile_mlp_serves(int64_t M, int64_t D, int64_t H);
+bool tile_mlp_serves(int64_t M, int64_t D, int64_t H, bool gated);
 bool values_mlp_serves(int64_t M, int64_t D, int64_t H);
 int values_mlp(const void* x, const void* gate, const float* bias, const void* up, const void* down,
                void* packed, void* out, int64_t M, int64_t D, int64_t H, int cf, void* workspace,
@@ -407,7 +407,7 @@ MlpForm mlp_form(int64_t M, int64_t D, int64_t H, bool gated, bool hp, int64_t m
   if (M < 1 || D < 256 || D > 4096 || D % 256 || H < 256 || H > 65536 || H % 256) return kGather;
   const bool whole = max_rows <= 0 || max_rows >= M;  // only the pairs work in row chunks
   if (whole && hp && values_mlp_serves(M, D, H)) return kValues;
-  if (whole && !hp && tile_mlp_serves(M, D, H)) return kTiles;
+  if (whole && !hp && tile_mlp_serves(M, D, H, gated)) return kTiles;
   return pair_mlp_serves(M, D, H, gated, hp) ? kPairs : kGather;
 }
 

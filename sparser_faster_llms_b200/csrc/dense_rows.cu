@@ -44,7 +44,7 @@ int pair_gate_up(const void* x, const void* gate, const float* bias, const void*
 int pair_down(const void* hidden, int terms, const void* down, void* out, int64_t M, int64_t D,
               int64_t H, const RunIf& run_if, const SplitRoom& room, cudaStream_t stream);
 int tile_mlp_status();
-bool tile_mlp_serves(int64_t M, int64_t D, int64_t H);
+bool tile_mlp_serves(int64_t M, int64_t D, int64_t H, bool gated);
 int tile_first(bool gated, const void* x, const void* gate, const float* bias, const void* up,
                void* packed, void* hidden, float* values, int64_t M, int64_t D, int64_t H, int cf,
                bool keep_all, cudaStream_t stream);
@@ -893,7 +893,7 @@ size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
 // anyway.
 bool tile_rows(int64_t M, int64_t D, int64_t H, int64_t cap) {
   const int64_t hidden = M * H * 2, rows = cap * (D + H) * 2;
-  return (tile_mlp_serves(M, D, H) || pair_mlp_serves(M, D, H, true, false)) &&
+  return (tile_mlp_serves(M, D, H, true) || pair_mlp_serves(M, D, H, true, false)) &&
          hidden <= (rows > ((int64_t)1 << 30) ? rows : (int64_t)1 << 30);
 }
 
@@ -1326,7 +1326,7 @@ int b200_twell_gated_mlp_hybrid_counted(const void* x, const void* gate, const f
     if (counters != nullptr) w.counters = counters;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int tiles = (int)(H / kTileN), slab_w = kTileN / cf;
-    const bool small = tile_mlp_serves(M, D, H);
+    const bool small = tile_mlp_serves(M, D, H, true);
     if (int rc = small ? tile_first(true, x, gate, gate_bias, up, packed, w.h_all, nullptr, M, D, H, cf,
                                              true, st)
                        : pair_gate_up(x, gate, gate_bias, up, packed, w.h_all, M, D, H, cf, true, st))

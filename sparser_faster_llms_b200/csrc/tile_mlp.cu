@@ -136,9 +136,10 @@ first_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ 
   constexpr int kStage = kRowBytes + COLS * 128;
   constexpr int STAGES = kRing / kStage > 8 ? 8 : kRing / kStage;
   constexpr int BLKS = NB / 64;  // 32-column blocks per epilogue warp
-  // High precision and the pack keep the sums of two or four ranges of k apart in TMEM and add them in
-  // fp32: a tensor core's running sum loses bits with its length (64 tokens, D 2048, 5 %: error against
-  // 64 bits 1.6712e-3 with one range, 1.6593e-3 where D was split four ways before).
+  // Four ranges of k (two where TMEM holds no more) stay apart and are added in fp32: a tensor core's
+  // running sum loses bits with its length.  Stored gate values of N(0, 1) tokens that are not the rounded
+  // 64-bit value, one range / four: D 1024 0.55 / 0.16 %, D 2048 1.07 / 0.33 %, D 4096 1.81 / 0.71 %.  The
+  // pack of the same size splits D the same way, so its slab words are the same.
   static_assert(RANGES * COLS <= 512, "TMEM columns");
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>(
@@ -274,7 +275,7 @@ first_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ 
         if (live && a.hidden != nullptr) pg::store64(out + b * 32, gw[b], a.wide);
       } else {
         __syncwarp();
-        tmem_ld32(acc + (uint32_t)(NB + b * 32), v);
+        load_sums<RANGES, COLS>(acc + (uint32_t)(NB + b * 32), v);
         uint32_t w[16];
 #pragma unroll
         for (int p = 0; p < 16; ++p) {
@@ -424,7 +425,7 @@ int launch_cluster(const char* fn, Kernel kern, dim3 grid, int cluster, size_t s
   return B200_OK;
 }
 
-template <bool GATED, bool VALUES, int NB, int RANGES = VALUES ? 256 / NB : 1>
+template <bool GATED, bool VALUES, int NB, int RANGES = GATED ? 256 / NB : 4>
 int launch_first(const void* x, const void* g, const void* u, FirstArgs a, int64_t D, cudaStream_t stream) {
   constexpr int kStage = kRowBytes + (GATED ? 2 : 1) * NB * 128;
   constexpr int STAGES = kRing / kStage > 8 ? 8 : kRing / kStage;
@@ -459,6 +460,15 @@ int launch_second(const void* hidden, const void* down, void* out, int64_t M, in
 
 }  // namespace
 
+namespace {
+
+// CTAs in clusters of four that are resident at once (a GPC's SMs are no multiple of four).
+int64_t fours() { return (sm_count() / 4 - 4) * 4; }
+int64_t row_tiles(int64_t M) { return (M + tm::kRows - 1) / tm::kRows; }
+int token_box(int64_t M) { return M < tm::kRows ? (int)((M + 7) / 8 * 8) : tm::kRows; }
+
+}  // namespace
+
 // Which calls of the fused MLPs run here: from 33 tokens on, while the first launch fits one wave.  us per
 // layer under graph replay, weights from HBM, forms before (gathers, or pairs of SMs) -> now:
 //   gated    D 1024, H 4096:   64 tokens, 2 % 22 -> 14;  256 tokens 35 -> 16;  512 tokens 32 -> 23
@@ -470,19 +480,14 @@ int launch_second(const void* hidden, const void* down, void* out, int64_t M, in
 //   plain    D 2048, H 8192:   33 tokens, 0.5 % / 2 % 21 / 25 -> 20;  256 tokens 32 / 46 -> 30
 // Up to 32 tokens the gathers touch few rows (D 2048, H 8192, 32 tokens, 0.5 % / 2 % 17 / 24 -> 24).  In
 // two waves the form is level with the pairs at best (H 11008, 200 tokens 49 -> 54).
-bool tile_mlp_serves(int64_t M, int64_t D, int64_t H) {
+//
+// One row tile at H 8704 to 9472 stays with the gathers (or the pairs): its pack adds four ranges of D, of
+// which the accumulators of 128 neurons hold two.
+bool tile_mlp_serves(int64_t M, int64_t D, int64_t H, bool gated) {
   if (M < 33 || M > 512 || D > 4096 || H < 2048) return false;
-  return (M + tm::kRows - 1) / tm::kRows * (H / 128) <= sm_count();
+  if (gated && M <= tm::kRows && H / 64 > fours() && H / 64 <= sm_count()) return false;
+  return row_tiles(M) * (H / 128) <= sm_count();
 }
-
-namespace {
-
-// CTAs in clusters of four that are resident at once (a GPC's SMs are no multiple of four).
-int64_t fours() { return (sm_count() / 4 - 4) * 4; }
-int64_t row_tiles(int64_t M) { return (M + tm::kRows - 1) / tm::kRows; }
-int token_box(int64_t M) { return M < tm::kRows ? (int)((M + 7) / 8 * 8) : tm::kRows; }
-
-}  // namespace
 
 // Slabs and hidden values ([M, H] bf16, 16-byte aligned); keep_all: of every gate positive, not only of
 // the stored ones.  values (gated): instead of hidden, their fp32 hidden values in the slots of the slabs.
@@ -541,8 +546,8 @@ int tile_pack(const void* x, const void* w, const float* bias, void* packed, int
   a.ksteps = (int)(D / kStageK);
   a.box = token_box(M);
   if (row_tiles(M) * (H / 64) <= fours())
-    return tm::launch_first<false, false, 64, 4>(x, w, w, a, D, stream);
-  return tm::launch_first<false, false, 128, 4>(x, w, w, a, D, stream);
+    return tm::launch_first<false, false, 64>(x, w, w, a, D, stream);
+  return tm::launch_first<false, false, 128>(x, w, w, a, D, stream);
 }
 
 // out[M, D] = hidden[M, H] down with down [H, D] as it is stored.
@@ -571,14 +576,14 @@ int tile_second(const void* hidden, const void* down, void* out, int64_t M, int6
 //   D 4096, H 16384  at 1 %: 48 tokens 73 -> 70;  200 tokens 158 -> 104;  1000 tokens 517 -> 326
 bool values_mlp_serves(int64_t M, int64_t D, int64_t H) {
   if (D > 4096 || H < 2048 || M * D * H >= (int64_t)1 << 36) return false;
-  return M >= 160 || (tile_mlp_serves(M, D, H) && M >= (D * H <= (int64_t)1 << 23 ? 33 : 48));
+  return M >= 160 || (tile_mlp_serves(M, D, H, true) && M >= (D * H <= (int64_t)1 << 23 ? 33 : 48));
 }
 
 // values: [M, H / cf] fp32, 16-byte aligned.
 int values_mlp(const void* x, const void* gate, const float* bias, const void* up, const void* down,
                void* packed, void* out, int64_t M, int64_t D, int64_t H, int cf, void* workspace,
                size_t workspace_bytes, float* values, cudaStream_t stream) {
-  const int rc = tile_mlp_serves(M, D, H)
+  const int rc = tile_mlp_serves(M, D, H, true)
                      ? tile_first(true, x, gate, bias, up, packed, nullptr, values, M, D, H, cf, false, stream)
                      : pair_gate_up_values(x, gate, bias, up, packed, values, M, D, H, cf, stream);
   if (rc) return rc;
