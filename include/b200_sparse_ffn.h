@@ -36,7 +36,10 @@ extern "C" {
 #define B200_EWORKSPACE (-6)  /* caller-provided workspace is too small        */
 
 /* flags for the contraction entry points */
-#define B200_FLAG_HIGH_PRECISION 1u /* fp32 fma everywhere, h kept in fp32     */
+/* No product rounded to bf16, sums in fp32, h kept in fp32.  Contractions gather with fp32 fma; where a fused
+ * MLP takes the up product from the tensor cores below 2^36 multiply-adds, its sums are over at most 512
+ * k-values each, added in fp32 (error of h against 64 bits 5e-7 of its norm; fp32 fma chains 1e-7). */
+#define B200_FLAG_HIGH_PRECISION 1u
 
 /* Library version (major*10000 + minor*100 + patch) and the sm arch it was built for. */
 int b200_version(void);

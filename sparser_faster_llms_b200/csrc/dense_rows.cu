@@ -674,10 +674,6 @@ dense_rows_gemm_splitk_kernel(const __grid_constant__ CUtensorMap tmap_a0,
   }
 }
 
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-
 // Persistent form of the same GEMM: one CTA per SM walks the (feature tile, token tile) list
 // with a stride of the grid, feature tile fastest, so the CTAs of a wave share one token tile.
 // TMEM holds two accumulator pairs (4 x NTOK columns): while the epilogue warps drain pair a

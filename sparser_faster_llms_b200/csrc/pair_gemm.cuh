@@ -42,6 +42,12 @@ constexpr int kTile = 256;                   // rows and columns per pair
 constexpr int kOperandBytes = 128 * 128;     // one CTA's half of A or B per 64-k stage
 constexpr int kStageBytes = 2 * kOperandBytes;
 constexpr int kBatch = 16;                   // slab rows whose words are in flight at a time
+// k-steps per range of the up product in high precision; the ranges are added in fp32.  Error of the hidden
+// values against 64 bits, N(0, 1) tokens: one range over D 2048 / 4096 2.1e-6 / 4.4e-6; ranges of 8 k-steps
+// 4.8e-7, of 4 2.4e-7, of 1 1.3e-7 / 1.6e-7 (fp32 FMA chains 0.8e-7 / 0.9e-7).  y is off by 1.66e-3 with
+// any of them.  A range costs the epilogue about 1.2 us: 777 tokens, D 2048, H 8192, 2 %, one range 110 us,
+// of 8 k-steps 117, of 4 124, of 1 185; gathers 161.
+constexpr int kDrain = 8;
 
 enum Epilogue {
   kStore = 0,    // out[row, col] = bf16(acc)
@@ -727,37 +733,42 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap map_a0,
       for (int t = pair; t < total && !failed; t += pairs) {
         const Item im = item_of(t, a);
 #pragma unroll 1
-        for (int ph = 0; ph < kPhases; ++ph, ++i) {
-          const int b = i & 1;
-          if (!mbar_wait(&tempty_bar[b], ((uint32_t)(i >> 1) & 1u) ^ 1u)) {
-            failed = 4;
-            break;
-          }
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t acc = tmem_base + (uint32_t)(b * 256);
-          uint32_t add = 0;
+        for (int ph = 0; ph < kPhases && !failed; ++ph) {
+          // the up product of the high-precision form comes in ranges of kDrain k-steps
+          const int range = EPI == kGateUpHp && ph == 1 ? kDrain : im.k1 - im.k0;
 #pragma unroll 1
-          for (int k = im.k0; k < im.k1; ++k) {
-            if (!mbar_wait(&full_bar[s], phase)) {
-              failed = 2;
+          for (int k0 = im.k0; k0 < im.k1; k0 += range, ++i) {
+            const int b = i & 1, k1 = min(k0 + range, im.k1);
+            if (!mbar_wait(&tempty_bar[b], ((uint32_t)(i >> 1) & 1u) ^ 1u)) {
+              failed = 4;
               break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint64_t da = da0 + (uint32_t)s * (kStageBytes >> 4);
-            const uint64_t db = db0 + (uint32_t)s * (kStageBytes >> 4);
+            const uint32_t acc = tmem_base + (uint32_t)(b * 256);
+            uint32_t add = 0;
+#pragma unroll 1
+            for (int k = k0; k < k1; ++k) {
+              if (!mbar_wait(&full_bar[s], phase)) {
+                failed = 2;
+                break;
+              }
+              asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+              const uint64_t da = da0 + (uint32_t)s * (kStageBytes >> 4);
+              const uint64_t db = db0 + (uint32_t)s * (kStageBytes >> 4);
 #pragma unroll
-            for (int kk = 0; kk < kStageK / 16; ++kk) {
-              mma(acc, da + (A_MN ? 128 : 2) * kk, db + (B_MN ? 128 : 2) * kk, kIdesc, add);
-              add = 1;
+              for (int kk = 0; kk < kStageK / 16; ++kk) {
+                mma(acc, da + (A_MN ? 128 : 2) * kk, db + (B_MN ? 128 : 2) * kk, kIdesc, add);
+                add = 1;
+              }
+              commit(&empty_bar[s]);
+              if (++s == STAGES) {
+                s = 0;
+                phase ^= 1u;
+              }
             }
-            commit(&empty_bar[s]);
-            if (++s == STAGES) {
-              s = 0;
-              phase ^= 1u;
-            }
+            if (failed) break;
+            commit(&tfull_bar[b]);
           }
-          if (failed) break;
-          commit(&tfull_bar[b]);
         }
       }
       if (failed) {
@@ -964,6 +975,44 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap map_a0,
           }
         }
         if (!kGate2) continue;
+        if constexpr (EPI == kGateUpHp) {  // the up product of the same tile, range by range
+          float u[4][32] = {};
+          bool ok = true;
+#pragma unroll 1
+          for (int k = 0; k < a.ksteps; k += kDrain) {
+            ok = take();
+            if (!ok) break;
+            const uint32_t acc = lane_addr + (uint32_t)((i & 1) * 256);
+#pragma unroll
+            for (int cb = 0; cb < 4; ++cb) {
+              float v[32];
+              tmem_ld32(acc + (uint32_t)(cb * 32), v);
+#pragma unroll
+              for (int c = 0; c < 32; ++c) u[cb][c] += v[c];
+            }
+            release();
+          }
+          if (!ok) break;
+          float* h = a.values + (size_t)row * a.row_words + (size_t)nt * a.slab_w + 1;
+#pragma unroll
+          for (int cb = 0; cb < 4; ++cb) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const uint4 g4 = *reinterpret_cast<const uint4*>(at(buf, lane, cb * 64 + j * 16));
+              const uint32_t g[4] = {g4.x, g4.y, g4.z, g4.w};
+#pragma unroll
+              for (int e = 0; e < 8; ++e) {
+                const int c = 8 * j + e;
+                if ((mask[cb] >> c) & 1u) {
+                  if (first_slot < cap) h[first_slot] = (e & 1 ? hi_f(g[e >> 1]) : lo_f(g[e >> 1])) * u[cb][c];
+                  ++first_slot;
+                }
+              }
+            }
+            __syncwarp();
+          }
+          continue;
+        }
         if (!take()) break;  // the up product of the same tile
         src = Source{lane_addr + (uint32_t)((i & 1) * 256), nullptr, 1};
       }
@@ -982,8 +1031,8 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap map_a0,
           backward_tile(a, &map_a1, &map_b1, src, buf, row0, rows, nt, half, lane, pw, rw, tail_slot,
                         shift, done);
         }
-      } else if (!kIsPack || kGate2) {
-#pragma unroll(EPI == kGateUpHp ? 4 : 1)
+      } else if (!kIsPack || EPI == kGateUp) {
+#pragma unroll 1
         for (int cb = 0; cb < 4; ++cb) {
           float v[32];
           fetch32(src, cb, v);
@@ -1021,23 +1070,6 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap map_a0,
               }
             }
             if (live) store64(out + cb * 32, w, a.wide);
-          } else if (EPI == kGateUpHp) {
-            const int cap = a.slab_w - 1;
-            float* h = a.values + (size_t)row * a.row_words + (size_t)nt * a.slab_w + 1;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const uint4 g4 = *reinterpret_cast<const uint4*>(at(buf, lane, cb * 64 + j * 16));
-              const uint32_t g[4] = {g4.x, g4.y, g4.z, g4.w};
-#pragma unroll
-              for (int e = 0; e < 8; ++e) {
-                const int c = 8 * j + e;
-                if ((mask[cb] >> c) & 1u) {
-                  if (first_slot < cap) h[first_slot] = (e & 1 ? hi_f(g[e >> 1]) : lo_f(g[e >> 1])) * v[c];
-                  ++first_slot;
-                }
-              }
-            }
-            __syncwarp();
           } else if (EPI == kMulHp) {
             uint4 g4[4];
 #pragma unroll

@@ -50,6 +50,7 @@ __device__ __forceinline__ void give_up(int* abort_s, int code) {
 template <int STAGES>
 struct Ring {
   uint64_t full[STAGES], empty[STAGES], done;
+  uint64_t up_full[2], up_empty[2];  // VALUES: ranges of the up product
   uint32_t tmem;
   int abort;
 };
@@ -65,6 +66,11 @@ __device__ __forceinline__ void set_up(Ring<STAGES>& r, int warp) {
       mbar_init(&r.empty[s], 1);
     }
     mbar_init(&r.done, 1);
+#pragma unroll
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&r.up_full[b], 1);
+      mbar_init(&r.up_empty[b], 8);  // the epilogue warps
+    }
     r.abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -113,6 +119,42 @@ __device__ __forceinline__ void load_sums(uint32_t addr, float (&v)[32]) {
   }
 }
 
+// The MMA thread of the form with fp32 hidden values where a quarter of D is more than kDrain k-steps or TMEM
+// does not hold four ranges of both products: the gate product in RANGES ranges of k at TMEM column 0,
+// the up product in ranges of kDrain k-steps that alternate between two accumulators at column 256, which the
+// epilogue warps empty.
+template <int STAGES, int NB, int RANGES>
+__device__ __forceinline__ bool issue_values(Ring<STAGES>& r, int ksteps, uint64_t da0) {
+  constexpr uint32_t kStage = kRowBytes + 2 * NB * 128, kIdesc = umma_idesc(kRows, NB);
+  int s = 0, range = -1, next = 0;
+  uint32_t phase = 0;
+#pragma unroll 1
+  for (int k = 0; k < ksteps; ++k) {
+    const int up = k / pg::kDrain, b = up & 1;
+    const bool up_first = k % pg::kDrain == 0;
+    if (!mbar_wait(&r.full[s], phase)) return false;
+    if (up_first && !mbar_wait(&r.up_empty[b], ((uint32_t)(up >> 1) & 1u) ^ 1u)) return false;
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const bool first = k == next;
+    if (first) next = (++range + 1) * ksteps / RANGES;
+    const uint64_t da = da0 + (uint32_t)s * (kStage >> 4), db = da + (kRowBytes >> 4);
+#pragma unroll
+    for (int kk = 0; kk < kStageK / 16; ++kk) {
+      umma_bf16(r.tmem + (uint32_t)(range * NB), da + 2 * kk, db + 2 * kk, kIdesc, !first || kk > 0 ? 1u : 0u);
+      umma_bf16(r.tmem + (uint32_t)(256 + b * NB), da + 2 * kk, db + (NB * 128 >> 4) + 2 * kk, kIdesc,
+                !up_first || kk > 0 ? 1u : 0u);
+    }
+    umma_commit(&r.empty[s]);
+    if ((k + 1) % pg::kDrain == 0 || k + 1 == ksteps) umma_commit(&r.up_full[b]);
+    if (++s == STAGES) {
+      s = 0;
+      phase ^= 1u;
+    }
+  }
+  umma_commit(&r.done);
+  return true;
+}
+
 struct FirstArgs {
   const float* bias;      // bias16: 16-byte aligned
   int bias16;
@@ -127,7 +169,7 @@ struct FirstArgs {
 };
 
 // grid = (H / NB, ceil(M / 128)), cluster = 256 / NB along the neurons.
-template <bool GATED, bool VALUES, int NB, int RANGES>
+template <bool GATED, bool VALUES, bool DRAIN, int NB, int RANGES>
 __global__ void __launch_bounds__(kThreads, 1)
 first_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_g,
              const __grid_constant__ CUtensorMap map_u, const __grid_constant__ FirstArgs a) {
@@ -136,11 +178,12 @@ first_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ 
   constexpr int kStage = kRowBytes + COLS * 128;
   constexpr int STAGES = kRing / kStage > 8 ? 8 : kRing / kStage;
   constexpr int BLKS = NB / 64;  // 32-column blocks per epilogue warp
+  constexpr int kTmem = DRAIN ? 512 : RANGES * COLS;
   // Four ranges of k (two where TMEM holds no more) stay apart and are added in fp32: a tensor core's
   // running sum loses bits with its length.  Stored gate values of N(0, 1) tokens that are not the rounded
   // 64-bit value, one range / four: D 1024 0.55 / 0.16 %, D 2048 1.07 / 0.33 %, D 4096 1.81 / 0.71 %.  The
   // pack of the same size splits D the same way, so its slab words are the same.
-  static_assert(RANGES * COLS <= 512, "TMEM columns");
+  static_assert(RANGES * (DRAIN ? 2 * NB : COLS) <= 512, "TMEM columns");
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -152,7 +195,7 @@ first_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n0 = (int)blockIdx.x * NB, m0 = (int)blockIdx.y * kRows;
   cluster.barrier_arrive();
-  set_up<STAGES, RANGES * COLS>(ring, warp);
+  set_up<STAGES, kTmem>(ring, warp);
   if (threadIdx.x == 0)
     for (int k = 0; k < 2 && k < a.ksteps; ++k) {
       tma_prefetch_2d(&map_g, k * kStageK, n0);
@@ -162,6 +205,7 @@ first_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ 
 
   uint32_t gw[BLKS][16];  // gate values as bf16 pairs, zero where nothing is stored
   uint32_t mask[BLKS];
+  float u[DRAIN ? BLKS : 1][32] = {};
   int cnt = 0;
   bool ok = false;
   const int q = warp & 3, half = (warp - 3) >> 2;
@@ -183,25 +227,48 @@ first_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ 
   } else if (warp == 2) {
     const uint64_t da0 = umma_desc(smem_u32(smem));
     const uint32_t tmem = ring.tmem;
-    if (elect_one())
-      issue(ring, a.ksteps, 3, [&, k = 0, range = -1, next = 0](bool, int s) mutable {
-        const bool first = k++ == next;
-        if (first) next = (++range + 1) * a.ksteps / RANGES;
-        const uint64_t da = da0 + (uint32_t)s * (kStage >> 4), db = da + (kRowBytes >> 4);
+    if (elect_one()) {
+      if constexpr (DRAIN) {
+        if (!issue_values<STAGES, NB, RANGES>(ring, a.ksteps, da0)) give_up(&ring.abort, 3);
+      } else {
+        issue(ring, a.ksteps, 3, [&, k = 0, range = -1, next = 0](bool, int s) mutable {
+          const bool first = k++ == next;
+          if (first) next = (++range + 1) * a.ksteps / RANGES;
+          const uint64_t da = da0 + (uint32_t)s * (kStage >> 4), db = da + (kRowBytes >> 4);
 #pragma unroll
-        for (int kk = 0; kk < kStageK / 16; ++kk)
-          umma_bf16(tmem + (uint32_t)(range * COLS), da + 2 * kk, db + 2 * kk, umma_idesc(kRows, COLS),
-                    !first || kk > 0 ? 1u : 0u);
-      });
+          for (int kk = 0; kk < kStageK / 16; ++kk)
+            umma_bf16(tmem + (uint32_t)(range * COLS), da + 2 * kk, db + 2 * kk, umma_idesc(kRows, COLS),
+                      !first || kk > 0 ? 1u : 0u);
+        });
+      }
+    }
   } else {
-    ok = mbar_wait(&ring.done, 0u);
+    if (DRAIN) {  // the up product, range by range
+      ok = true;
+      for (int r = 0; r * pg::kDrain < a.ksteps && ok; ++r) {
+        ok = mbar_wait(&ring.up_full[r & 1], (uint32_t)(r >> 1) & 1u);
+        ok = __all_sync(0xffffffffu, ok);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+        for (int b = 0; b < BLKS && ok; ++b) {
+          float w[32];
+          tmem_ld32(acc + (uint32_t)(256 + (r & 1) * NB + b * 32), w);
+#pragma unroll
+          for (int c = 0; c < 32; ++c) u[b][c] += w[c];
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&ring.up_empty[r & 1]);
+      }
+    }
+    ok = mbar_wait(&ring.done, 0u) && (ok || !DRAIN);
     ok = __all_sync(0xffffffffu, ok);
     if (!ok) give_up(&ring.abort, 4);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
     for (int b = 0; b < BLKS; ++b) {
       float v[32];
-      load_sums<RANGES, COLS>(acc + (uint32_t)(b * 32), v);
+      load_sums<RANGES, DRAIN ? NB : COLS>(acc + (uint32_t)(b * 32), v);
       if (a.bias != nullptr) {
         const float* bp = a.bias + n0 + half * (NB / 2) + b * 32;
         if (a.bias16) {
@@ -258,22 +325,22 @@ first_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ 
           gw[b][p] &= ((m >> (2 * p)) & 1u ? 0xFFFFu : 0u) | ((m >> (2 * p + 1)) & 1u ? 0xFFFF0000u : 0u);
       }
       const uint32_t col0 = (uint32_t)(n0 + half * (NB / 2) + b * 32), m = mask[b];
-      float v[32];
-      if (VALUES) {
+      if (VALUES && !DRAIN) {
         __syncwarp();
-        load_sums<RANGES, COLS>(acc + (uint32_t)(NB + b * 32), v);
+        load_sums<RANGES, COLS>(acc + (uint32_t)(NB + b * 32), u[0]);
       }
 #pragma unroll
       for (int c = 0; c < 32; ++c)
         if ((m >> c) & 1u) {
           ++slot;
           slab[slot] = (col0 + c) | (c & 1 ? gw[b][c / 2] & 0xFFFF0000u : gw[b][c / 2] << 16);
-          if (VALUES) values[slot] = (c & 1 ? pg::hi_f(gw[b][c / 2]) : pg::lo_f(gw[b][c / 2])) * v[c];
+          if (VALUES) values[slot] = (c & 1 ? pg::hi_f(gw[b][c / 2]) : pg::lo_f(gw[b][c / 2])) * u[DRAIN ? b : 0][c];
         }
       if (VALUES) {
       } else if (!GATED) {
         if (live && a.hidden != nullptr) pg::store64(out + b * 32, gw[b], a.wide);
       } else {
+        float v[32];
         __syncwarp();
         load_sums<RANGES, COLS>(acc + (uint32_t)(NB + b * 32), v);
         uint32_t w[16];
@@ -288,7 +355,7 @@ first_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ 
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  free_tmem<STAGES, RANGES * COLS>(ring, warp);
+  free_tmem<STAGES, kTmem>(ring, warp);
 }
 
 // Owner's place of a 16-byte piece (0..3) of a token's 16 sums: pieces rotate with the row pair, so
@@ -425,8 +492,9 @@ int launch_cluster(const char* fn, Kernel kern, dim3 grid, int cluster, size_t s
   return B200_OK;
 }
 
-template <bool GATED, bool VALUES, int NB, int RANGES = GATED ? 256 / NB : 4>
+template <bool GATED, bool VALUES, int NB, bool DRAIN = VALUES && NB == 128>
 int launch_first(const void* x, const void* g, const void* u, FirstArgs a, int64_t D, cudaStream_t stream) {
+  constexpr int RANGES = GATED ? 256 / NB : 4;
   constexpr int kStage = kRowBytes + (GATED ? 2 : 1) * NB * 128;
   constexpr int STAGES = kRing / kStage > 8 ? 8 : kRing / kStage;
   CUtensorMap mx, mg, mu;
@@ -434,7 +502,7 @@ int launch_first(const void* x, const void* g, const void* u, FirstArgs a, int64
   if (int rc = make_map(&mg, g, a.H, D, NB)) return rc;
   if (int rc = make_map(&mu, u, a.H, D, NB)) return rc;
   static size_t granted[64] = {0};
-  return launch_cluster("gate and up tiles", first_kernel<GATED, VALUES, NB, RANGES>,
+  return launch_cluster("gate and up tiles", first_kernel<GATED, VALUES, DRAIN, NB, RANGES>,
                         dim3((unsigned)(a.H / NB), (unsigned)((a.M + kRows - 1) / kRows), 1), kTileN / NB,
                         (size_t)STAGES * kStage + 1024, granted, stream, mx, mg, mu, a);
 }
@@ -511,7 +579,8 @@ int tile_first(bool gated, const void* x, const void* gate, const float* bias, c
   // 64 neurons per CTA while that is one wave: 128 tokens, D 2048, H 8192 16.5 against 21 us; the
   // accumulators of 128 neurons cost twice the MMAs per step.
   if (row_tiles(M) * (H / 64) <= fours())
-    return values != nullptr ? tm::launch_first<true, true, 64>(x, gate, up, a, D, stream)
+    return values != nullptr ? (D <= 2048 ? tm::launch_first<true, true, 64>(x, gate, up, a, D, stream)
+                                          : tm::launch_first<true, true, 64, true>(x, gate, up, a, D, stream))
            : gated           ? tm::launch_first<true, false, 64>(x, gate, up, a, D, stream)
                              : tm::launch_first<false, false, 64>(x, gate, gate, a, D, stream);
   return values != nullptr ? tm::launch_first<true, true, 128>(x, gate, up, a, D, stream)

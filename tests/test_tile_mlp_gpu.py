@@ -128,3 +128,34 @@ def test_gate_sums_are_those_of_the_pack(m, d, h, gated):
     value = (word[..., 1:] & -65536)[live].view(torch.float32)
     off = (value != z[rows, col].bfloat16().float()).float().mean().item()
     assert off < d / 2 ** 18, off
+
+
+@pytest.mark.parametrize("m,d,h", [(100, 2048, 8192), (100, 4096, 4096), (250, 2048, 8192), (128, 4096, 16384),
+                                   (250, 768, 8192), (400, 2048, 11008), (600, 4096, 8192), (777, 2048, 8192)])
+def test_high_precision_hidden_values_against_64_bits(m, d, h):
+    """N(0, 1) tokens and N(0, 0.02) weights, one-SM tiles and pairs of SMs.  A tensor core's running sum loses
+    some 2^-26 of itself with every 16 k-values, so ranges of at most 512 of them keep the fp32 hidden values
+    within 32 x 2^-26 = 4.8e-7 (measured 2.4e-7 to 4.8e-7); one range over D 2048 is off by 2.1e-6, two by
+    1.0e-6."""
+    f = synthetic.make_ffn(d, h, seed=m, density=0.02, device=DEV, generate_on_device=True)
+    gen = torch.Generator(device=DEV).manual_seed(m)
+    x = torch.randn(m, d, generator=gen, device=DEV)
+    x[:, 0] = 1.0
+    x = x.bfloat16()
+    packed, out = torch.zeros(m, h // 8, dtype=torch.uint32, device=DEV), torch.empty_like(x)
+    need = _lib.load_library().b200_twell_mlp_scratch_bytes(m, d, h, 1, _lib.FLAG_HIGH_PRECISION)
+    assert need > 0
+    scratch = torch.empty(need, dtype=torch.uint8, device=DEV)
+    _lib.call("b200_twell_gated_mlp_scratch", torch.device(DEV), x.data_ptr(), f.gate.data_ptr(), None,
+              f.up.data_ptr(), f.down.data_ptr(), packed.data_ptr(), out.data_ptr(), m, d, h, 8,
+              _lib.FLAG_HIGH_PRECISION, *_lib.workspace(torch.device(DEV)), scratch.data_ptr(), need)
+    torch.cuda.synchronize()
+    word = packed.view(torch.int32).view(m, h // 256, 32)
+    live = torch.arange(1, 32, device=DEV) <= word[..., :1].clamp(max=31)
+    rows = torch.arange(m, device=DEV)[:, None, None].expand_as(live)[live]
+    col = (word[..., 1:] & 0xFFFF)[live].long()
+    g = (word[..., 1:] & -65536)[live].view(torch.float32).double()
+    got = scratch[:m * h // 8 * 4].view(torch.float32).view(m, h // 256, 32)[..., 1:][live].double()
+    want = g * (x.double() @ f.up.double().T)[rows, col]
+    rel = ((got - want).norm() / want.norm()).item()
+    assert rel < 7e-7, rel
