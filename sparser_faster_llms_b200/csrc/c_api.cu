@@ -41,7 +41,7 @@ int twell_t2d_launch(bool gated, bool hp, const void* x, const void* packed, con
                      const void* down, void* out, int64_t M, int64_t D, int64_t H, int cf,
                      void* workspace, size_t workspace_bytes, int sm_count, cudaStream_t stream,
                      const unsigned char* skip_rows = nullptr, const FusedAr* fused_ar = nullptr,
-                     const RunIf& run_if = {nullptr, 0u});
+                     const RunIf& run_if = {nullptr, 0u, 0, nullptr});
 
 size_t twell_decode_workspace_bytes(int64_t M, int64_t D, int64_t H);
 int twell_decode_launch(bool gated, bool hp, const void* x, const void* gate, const float* bias,

@@ -122,12 +122,28 @@ constexpr size_t kFarControlBytes = 1024;   // control words, padding; the inbox
 constexpr int kFarMaxTokens = 256;
 
 // A choice between two forms of one product that the device makes itself: the gather form runs
-// when *entries <= limit (stored gate entries of the call), the dense form when it is larger.
-// The form that does not run returns at once.  entries == nullptr: the launched form runs.
+// when the stored gate entries that were counted are at most `limit`, the dense form when they are
+// more.  The form that does not run returns at once.  entries == nullptr: the launched form runs.
 struct RunIf {
   const unsigned int* entries;
   unsigned int limit;
+  int words;              // the count is the sum of this many words (0: of one)
+  unsigned int* verdict;  // or null: the launch leaves 1 (dense form) or 0 here for those behind it
 };
+
+// A sample of a call's tokens, whose stored entries are counted per 256 neurons.
+constexpr int kSampleTokens = 128;
+constexpr int kSampleWords = 63;
+
+// Every lane of the calling warps takes part.
+__device__ __forceinline__ bool stored_more(const RunIf& r) {
+  if (r.words == 0) return __ldcg(r.entries) > r.limit;
+  unsigned int n = 0;
+  for (int i = (int)(threadIdx.x & 31); i < r.words; i += 32) n += __ldcg(r.entries + i);
+  const bool more = __reduce_add_sync(0xffffffffu, n) > r.limit;
+  if (r.verdict != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *r.verdict = more;
+  return more;
+}
 
 // Room for a last wave of tiles that is cut along k: fp32 sums of the ranges, and counters that are
 // zero at rest.  A launch whose cut does not fit `bytes`, or that gets no room, runs uncut.

@@ -33,14 +33,14 @@ int twell_t2d_launch(bool gated, bool hp, const void* x, const void* packed, con
                      const void* down, void* out, int64_t M, int64_t D, int64_t H, int cf,
                      void* workspace, size_t workspace_bytes, int sm_count, cudaStream_t stream,
                      const unsigned char* skip_rows, const FusedAr* fused_ar,
-                     const RunIf& run_if = {nullptr, 0u});
+                     const RunIf& run_if = {nullptr, 0u, 0, nullptr});
 int sm_count();
 int pair_gemm_status();
 bool pair_mlp_serves(int64_t M, int64_t D, int64_t H, bool gated, bool hp);
 size_t pair_part_bytes(int64_t M, int64_t D, int64_t H);
 int pair_gate_up(const void* x, const void* gate, const float* bias, const void* up, void* packed,
                  void* hidden, int64_t M, int64_t D, int64_t H, int cf, bool keep_all,
-                 cudaStream_t stream);
+                 cudaStream_t stream, const RunIf& run_if = {nullptr, 0u, 0, nullptr});
 int pair_down(const void* hidden, int terms, const void* down, void* out, int64_t M, int64_t D,
               int64_t H, const RunIf& run_if, const SplitRoom& room, cudaStream_t stream);
 int tile_mlp_status();
@@ -1340,7 +1340,7 @@ int b200_twell_gated_mlp_hybrid_counted(const void* x, const void* gate, const f
     const SplitRoom room = {w.part, pair_part_bytes(M, D, H),
                             workspace != nullptr && workspace_bytes >= 16384
                                 ? static_cast<unsigned int*>(workspace) : nullptr};
-    return pair_down(w.h_all, 1, down, out, M, D, H, {nullptr, 0u}, room, st);
+    return pair_down(w.h_all, 1, down, out, M, D, H, {nullptr, 0u, 0, nullptr}, room, st);
   }
   if (int rc = b200_twell_pack(x, gate, gate_bias, packed, M, D, H, cf, stream)) return rc;
   return t2d_hybrid(x, packed, gate, gate_bias, up, down, down_t, out, M, D, H, cf, flags,

@@ -9,6 +9,8 @@ namespace b200 {
 
 int sm_count();
 bool tile_pack_serves(int64_t M, int64_t H);
+int tile_sample(const void* x, const void* w, const float* bias, void* packed, unsigned int* counts,
+                int64_t M, int64_t D, int64_t H, int cf, cudaStream_t stream);
 int twell_t2d_launch(bool gated, bool hp, const void* x, const void* packed, const void* up,
                      const void* down, void* out, int64_t M, int64_t D, int64_t H, int cf,
                      void* workspace, size_t workspace_bytes, int sm_count, cudaStream_t stream,
@@ -113,10 +115,12 @@ int pair_down(const void* hidden, int terms, const void* down, void* out, int64_
 // Slabs and hidden matrix in one launch: the gate and up products of a tile follow one another in
 // the two accumulators, and the pack epilogue of the first runs under the MMAs of the second.
 // keep_all: hidden values are computed from every gate positive, not only from the stored ones.
+// run_if: slabs in any case, the hidden matrix where the dense form runs.
 int pair_gate_up(const void* x, const void* gate, const float* bias, const void* up, void* packed,
                  void* hidden, int64_t M, int64_t D, int64_t H, int cf, bool keep_all,
-                 cudaStream_t stream) {
+                 cudaStream_t stream, const RunIf& run_if = {nullptr, 0u, 0, nullptr}) {
   pg::Args a = base_args(M, H, D);
+  a.run_if = run_if;
   a.bias = bias;
   a.bias16 = aligned16(bias);
   a.keep_all = keep_all;
@@ -177,18 +181,33 @@ bool pair_mlp_serves(int64_t M, int64_t D, int64_t H, bool gated, bool hp) {
   return M >= (gated ? 1 : 2) * dense_from(D, H);
 }
 
-// Only high precision lets the device choose between the dense and the gather form of the up and down
-// products by the stored entries of the call (two launches that return at once and a 4-byte memset, some
-// 9 us); bf16 products run dense always, gate and up in one launch.  us, asking / always dense, at 0.5 %,
-// 1 %, 2 %: D 2048, H 8192, 9000 tokens 591 / 569, 611 / 571, 655 / 586; 16384 tokens 1051 / 1047, 1065 /
-// 1049, 1085 / 1003; non-gated, D 1024, H 4096, 3000 tokens 61 / 54, 65 / 55, 66 / 55; D 2048, H 8192,
-// 1300 tokens 80 / 82, 91 / 83, 91 / 83, 3000 tokens 144 / 145, 151 / 145, 153 / 146; H 11008, 6000
-// tokens 330 / 356, 366 / 361; D 4096, H 16384 at 1 % 4000 tokens 680 / 670.
+// Which bf16 calls let the device choose between the dense and the gather form of the up and down products
+// by their stored entries.  A gated call asks a sample, 128 tokens spread over it (13 us of one-SM tiles
+// before the others, and contraction CTAs that return at once, 3 us); a non-gated one has its gate product
+// count (a 4-byte memset and the contraction, some 9 us).  us at 0.1 / 0.2 / 0.5 / 1 / 2 % density, dense
+// always -> asking:
+//   gated      D 2048, H 8192,   9000 tokens 685 / 685 / 682 / 708 / 704 -> 420 / 486 / 646 / 699 / 718;
+//                               16384 tokens 1216 / 1218 / 1220 / 1226 / 1236 -> 723 / 869 / 1134 / 1216 / 1237
+//              D 2048, H 11008,  6000 tokens 606 / 633 / 617 / 582 / 664 -> 342 / 533 / 590 / 644 / 645
+//   non-gated  D 2048, H 8192,  12000 tokens 598 / 613 / 606 / 653 / 629 -> 453 / 467 / 575 / 609 / 617
+// Below 1.5 x 2^36 multiply-adds asking costs 5 to 10 % from 0.7 % on and saves at 0.2 % and less only (gated,
+// H 8192, 4500 tokens 337 / 320 / 339 / 330 / 327 -> 240 / 272 / 365 / 360 / 368): dense always.
+static bool asks(int64_t m, int64_t D, int64_t H, bool gated) {
+  if (m * D * H < (int64_t)3 << 35) return false;
+  return !gated || (m > 4096 && rows_in_l2(D, H) && H / kTileN <= kSampleWords);
+}
 
-// Stored entries per token up to which the gather form is the faster one in high precision.  Measured
-// (D 2048, H 8192): up + down 104 ns per token dense and 0.8 ns per entry gathered; D 4096, H 16384
-// (rows from HBM as well): 382 ns against 2.7 ns.
-static int64_t gather_entries(int64_t D, int64_t H) { return H / (rows_in_l2(D, H) ? 64 : 112); }
+// Stored entries per token up to which the gather form is the faster one.  Measured (D 2048, H 8192) in high
+// precision: up + down 104 ns per token dense and 0.8 ns per entry gathered; D 4096, H 16384 (rows from HBM
+// as well): 382 ns against 2.7 ns.  bf16: see asks().
+static int64_t gather_entries(int64_t D, int64_t H, bool gated, bool hp) {
+  if (hp) return H / (rows_in_l2(D, H) ? 64 : 112);
+  return H / (gated ? 180 : rows_in_l2(D, H) ? 160 : 224);
+}
+
+static unsigned int clamp_limit(int64_t limit) {
+  return (unsigned int)(limit < 0x7fffffff ? limit : 0x7fffffff);
+}
 
 size_t pair_part_bytes(int64_t M, int64_t D, int64_t H) { return mlp_part_bytes(M, D, H, 1); }
 
@@ -226,24 +245,38 @@ int pair_mlp(bool gated, bool hp, const void* x, const void* gate, const float* 
     const void* xc = static_cast<const __nv_bfloat16*>(x) + r0 * D;
     void* pc = static_cast<uint32_t*>(packed) + r0 * row_words;
     void* oc = static_cast<__nv_bfloat16*>(out) + r0 * D;
-    if (!hp) {
+    if (!hp && !asks(m, D, H, gated)) {
       if (int rc = gated ? pair_gate_up(xc, gate, bias, up, pc, scratch, m, D, H, cf, false, stream)
                          : pair_pack(xc, gate, bias, pc, scratch, m, D, H, cf, nullptr, room, stream))
         return rc;
-      if (int rc = pair_down(scratch, 1, down, oc, m, D, H, {nullptr, 0u}, room, stream)) return rc;
+      if (int rc = pair_down(scratch, 1, down, oc, m, D, H, {nullptr, 0u, 0, nullptr}, room, stream)) return rc;
       continue;
     }
-    const int64_t limit = m * gather_entries(D, H);
-    const RunIf run_if = {entries, (unsigned int)(limit < 0x7fffffff ? limit : 0x7fffffff)};
+    const int64_t per_token = gather_entries(D, H, gated, hp);
+    if (!hp && gated) {
+      // the sample's slabs lie where the hidden values will be
+      const RunIf ask = {entries, clamp_limit(kSampleTokens * per_token), (int)(H / kTileN), entries + kSampleWords};
+      const RunIf run_if = {ask.verdict, 0u, 0, nullptr};
+      if (int rc = tile_sample(xc, gate, bias, scratch, entries, m, D, H, cf, stream)) return rc;
+      if (int rc = pair_gate_up(xc, gate, bias, up, pc, scratch, m, D, H, cf, false, stream, ask)) return rc;
+      if (int rc = pair_down(scratch, 1, down, oc, m, D, H, run_if, room, stream)) return rc;
+      if (int rc = twell_t2d_launch(true, true, xc, pc, up, down, oc, m, D, H, cf, workspace,
+                                    workspace_bytes, sm_count(), stream, nullptr, nullptr, run_if))
+        return rc;
+      continue;
+    }
+    const RunIf run_if = {entries, clamp_limit(m * per_token), 0, nullptr};
     if (cudaMemsetAsync(entries, 0, sizeof(unsigned int), stream) != cudaSuccess)
       return fail(B200_ECUDA, "fused MLP: cudaMemsetAsync failed");
     pdl_suppressed() = true;  // its predecessor is the memset
-    const int rc = pair_pack(xc, gate, bias, pc, nullptr, m, D, H, cf, entries, room, stream);
+    const int rc = pair_pack(xc, gate, bias, pc, gated ? nullptr : scratch, m, D, H, cf, entries, room, stream);
     pdl_suppressed() = false;
     if (rc) return rc;
-    if (int rc = pair_up(xc, pc, up, scratch, m, D, H, cf, run_if, room, stream)) return rc;
+    if (gated)
+      if (int rc = pair_up(xc, pc, up, scratch, m, D, H, cf, run_if, room, stream)) return rc;
     if (int rc = pair_down(scratch, terms, down, oc, m, D, H, run_if, room, stream)) return rc;
-    if (int rc = twell_t2d_launch(true, true, xc, pc, up, down, oc, m, D, H, cf, workspace,
+    // fp32 products, as the dense form does not round them one by one either
+    if (int rc = twell_t2d_launch(gated, true, xc, pc, up, down, oc, m, D, H, cf, workspace,
                                   workspace_bytes, sm_count(), stream, nullptr, nullptr, run_if))
       return rc;
   }
@@ -604,7 +637,7 @@ extern "C" int b200_hybrid_train_forward_timed(
     if (int e = pg::launch<pg::kFwd, false, false>(fn, ox, ot, ok, ot, a, m, sm_count(), st)) return e;
     parts.end(2);
     if (int e = pair_down(w.t, 1, v, static_cast<__nv_bfloat16*>(out) + r0 * D, m, D, H,
-                          {nullptr, 0u}, room, st))
+                          {nullptr, 0u, 0, nullptr}, room, st))
       return e;
     parts.end(3);
   }

@@ -596,7 +596,12 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap map_a0,
   // Without a device-side choice or row count the set-up below runs while the predecessor drains.
   const bool early_wait = a.run_if.entries != nullptr || a.rows_ptr != nullptr;
   if (early_wait) pdl_wait();
-  if (a.run_if.entries != nullptr && *a.run_if.entries <= a.run_if.limit) return;
+  bool gate_only = false;  // kGateUp: the gather form follows, slabs are all that it needs
+  if (a.run_if.entries != nullptr && !stored_more(a.run_if)) {
+    if (EPI != kGateUp) return;
+    gate_only = true;
+  }
+  const int phases = gate_only ? 1 : kPhases;
   const int rows = a.rows_ptr != nullptr ? *a.rows_ptr : a.rows;
   const int m_tiles = (rows + kTile - 1) / kTile;
   const int tiles = m_tiles * a.n_tiles;
@@ -669,7 +674,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap map_a0,
         const int ra = (second ? mt - a.second_mt : mt) * kTile + crank * 128;
         const int rb = nt * kTile + crank * 128;
 #pragma unroll 1
-        for (int ph = 0; ph < kPhases && ok; ++ph) {
+        for (int ph = 0; ph < phases && ok; ++ph) {
           int kb = im.k0 % a.seg_ksteps;
           const CUtensorMap* mb =
               ph == 1 || second || im.k0 >= a.seg_ksteps ? &map_b1 : &map_b0;
@@ -733,7 +738,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap map_a0,
       for (int t = pair; t < total && !failed; t += pairs) {
         const Item im = item_of(t, a);
 #pragma unroll 1
-        for (int ph = 0; ph < kPhases && !failed; ++ph) {
+        for (int ph = 0; ph < phases && !failed; ++ph) {
           // the up product of the high-precision form comes in ranges of kDrain k-steps
           const int range = EPI == kGateUpHp && ph == 1 ? kDrain : im.k1 - im.k0;
 #pragma unroll 1
@@ -974,7 +979,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap map_a0,
             if (live) store64(out + cb * 32, w, a.wide);
           }
         }
-        if (!kGate2) continue;
+        if (!kGate2 || gate_only) continue;
         if constexpr (EPI == kGateUpHp) {  // the up product of the same tile, range by range
           float u[4][32] = {};
           bool ok = true;
@@ -1119,7 +1124,7 @@ __global__ void __launch_bounds__(256)
 sum_ranges_kernel(const float4* __restrict__ sums, uint2* __restrict__ out, int splits, size_t n4,
                   const RunIf run_if) {
   pdl_wait();
-  if (run_if.entries != nullptr && *run_if.entries <= run_if.limit) return;
+  if (run_if.entries != nullptr && !stored_more(run_if)) return;
   const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
   if (i >= n4) return;
   float4 v[8];

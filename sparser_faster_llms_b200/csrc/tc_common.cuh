@@ -289,11 +289,11 @@ inline EncodeTiledFn encode_fn() {
 // [rows, K] bf16 row-major; box = box_k (64 or 32) k-values x box_rows rows with the 128- or
 // 64-byte swizzle that matches the row length, zero fill.
 inline int make_map(CUtensorMap* map, const void* base, int64_t rows, int64_t K, int box_rows,
-                    int box_k = kStageK) {
+                    int box_k = kStageK, int64_t row_step = 1) {
   EncodeTiledFn fn = encode_fn();
   if (fn == nullptr) return fail(B200_ECUDA, "tensor map: cuTensorMapEncodeTiled unavailable");
   const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
-  const cuuint64_t strides[1] = {(cuuint64_t)K * 2};
+  const cuuint64_t strides[1] = {(cuuint64_t)(K * row_step) * 2};
   const cuuint32_t box[2] = {(cuuint32_t)box_k, (cuuint32_t)box_rows};
   const cuuint32_t estr[2] = {1, 1};
   CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides,

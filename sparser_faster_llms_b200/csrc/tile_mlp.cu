@@ -166,6 +166,8 @@ struct FirstArgs {
   int wide;               // hidden rows are 32-byte aligned
   int M, ksteps, box;     // box: token rows per copy
   int keep_all;           // values past a slab's capacity still count in the product
+  unsigned int* counts;   // stored entries of each 256 neurons, all tokens (one row tile), or null
+  int64_t row_step;       // host: rows of x are every row_step-th token
 };
 
 // grid = (H / NB, ceil(M / 128)), cluster = 256 / NB along the neurons.
@@ -301,6 +303,17 @@ first_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ 
     for (int r = 0; r < CL; ++r) *cluster.map_shared_rank(&count[2 * crank + half][rl], r) = cnt;
   }
   cluster.sync();
+  if (a.counts != nullptr && warp == 3 && crank == 0) {
+    int n = 0;
+    for (int r = lane; r < a.M; r += 32) {
+      int total = 0;
+#pragma unroll
+      for (int i = 0; i < 2 * CL; ++i) total += count[i][r];
+      n += min(total, a.slab_w - 1);
+    }
+    n = __reduce_add_sync(0xffffffffu, n);
+    if (lane == 0) a.counts[blockIdx.x / CL] = (unsigned int)n;
+  }
   if (warp >= 3 && ok) {
     int slot = 0, total = 0;
 #pragma unroll
@@ -498,7 +511,7 @@ int launch_first(const void* x, const void* g, const void* u, FirstArgs a, int64
   constexpr int kStage = kRowBytes + (GATED ? 2 : 1) * NB * 128;
   constexpr int STAGES = kRing / kStage > 8 ? 8 : kRing / kStage;
   CUtensorMap mx, mg, mu;
-  if (int rc = make_map(&mx, x, a.M, D, a.box)) return rc;
+  if (int rc = make_map(&mx, x, a.M, D, a.box, kStageK, a.row_step)) return rc;
   if (int rc = make_map(&mg, g, a.H, D, NB)) return rc;
   if (int rc = make_map(&mu, u, a.H, D, NB)) return rc;
   static size_t granted[64] = {0};
@@ -575,6 +588,7 @@ int tile_first(bool gated, const void* x, const void* gate, const float* bias, c
   a.M = (int)M;
   a.ksteps = (int)(D / kStageK);
   a.box = token_box(M);
+  a.row_step = 1;
   a.keep_all = keep_all;
   // 64 neurons per CTA while that is one wave: 128 tokens, D 2048, H 8192 16.5 against 21 us; the
   // accumulators of 128 neurons cost twice the MMAs per step.
@@ -614,8 +628,28 @@ int tile_pack(const void* x, const void* w, const float* bias, void* packed, int
   a.M = (int)M;
   a.ksteps = (int)(D / kStageK);
   a.box = token_box(M);
+  a.row_step = 1;
   if (row_tiles(M) * (H / 64) <= fours())
     return tm::launch_first<false, false, 64>(x, w, w, a, D, stream);
+  return tm::launch_first<false, false, 128>(x, w, w, a, D, stream);
+}
+
+// Slabs of kSampleTokens tokens spread evenly over the M of a call, and their stored entries by 256 neurons.
+int tile_sample(const void* x, const void* w, const float* bias, void* packed, unsigned int* counts,
+                int64_t M, int64_t D, int64_t H, int cf, cudaStream_t stream) {
+  tm::FirstArgs a = {};
+  a.bias = bias;
+  a.bias16 = aligned16(bias);
+  a.packed = static_cast<uint32_t*>(packed);
+  a.slab_w = kTileN / cf;
+  a.row_words = (int)(H / kTileN) * a.slab_w;
+  a.H = H;
+  a.M = kSampleTokens;
+  a.ksteps = (int)(D / kStageK);
+  a.box = token_box(a.M);
+  a.row_step = M / kSampleTokens;
+  a.counts = counts;
+  if (H / 64 <= fours()) return tm::launch_first<false, false, 64>(x, w, w, a, D, stream);
   return tm::launch_first<false, false, 128>(x, w, w, a, D, stream);
 }
 

@@ -39,6 +39,8 @@
 namespace cg = cooperative_groups;
 
 namespace b200 {
+
+int sm_count();  // c_api.cu
 namespace {
 
 constexpr int kMaxTiles = 256;  // H <= 65536
@@ -117,7 +119,11 @@ __device__ __forceinline__ float2 far_gather(const FusedAr& ar, const unsigned c
 
 // NI = D / 256 = warps per CTA.
 // grid.x = M * nc * cs, cluster = cs.  ws_partial: [M][nc][D] fp32, ws_counter: [M][8] (nc > 1).
-template <int NI, bool GATED, bool HP, bool VALUES>
+// ASKS: a launch that may have to return at once holds only the CTAs that are resident together, each of which
+// takes every gridDim.x-th token (nc = cs = 1).  9000 CTAs that read the choice and leave took 24 us (now 2.7),
+// and gathering with that read in every CTA 227 us instead of 205 (0.1 %, D 2048, H 8192).  A form of its own:
+// the loop costs the others registers (8 tokens 18.3 -> 19.5 us).
+template <int NI, bool GATED, bool HP, bool VALUES, bool ASKS>
 __global__ void __launch_bounds__(NI * 32)
 twell_t2d_kernel(const __nv_bfloat16* x, const uint32_t* __restrict__ packed,
                  const float* __restrict__ values,
@@ -141,13 +147,14 @@ twell_t2d_kernel(const __nv_bfloat16* x, const uint32_t* __restrict__ packed,
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int crank = blockIdx.x % cs;
   const int cidx = (blockIdx.x / cs) % nc;
-  const int row = blockIdx.x / (cs * nc);
+  int row = ASKS ? (int)blockIdx.x : blockIdx.x / (cs * nc);
   // Nothing of the predecessor's output (slab, routing flags) is read before it has completed.
   pdl_wait();
   // Rows routed to the dense tensor-core path: every CTA of every cluster of the row leaves
   // (the row is uniform per cluster, so no cluster barrier is left half-attended).
   if (skip_rows != nullptr && skip_rows[row]) return;
-  if (run_if.entries != nullptr && *run_if.entries > run_if.limit) return;
+  if (ASKS && stored_more(run_if)) return;
+  auto token = [&]() {
   // Fused all-reduce: every CTA reads the call epoch now (the round trip hides under the slab
   // load).  It is advanced by the last (token, slice) group to finish, which cannot happen
   // before every CTA that has entries has contributed its partial sums, i.e. has started (the others
@@ -457,16 +464,24 @@ twell_t2d_kernel(const __nv_bfloat16* x, const uint32_t* __restrict__ packed,
   }
   if (tid == 0) ws_counter[row * 8 + crank] = 0u;  // ready for the next launch
   collect();
+  };
+  token();
+  if constexpr (ASKS) {
+    for (row += (int)gridDim.x; row < M; row += (int)gridDim.x) {
+      __syncthreads();  // shared memory is used again
+      token();
+    }
+  }
 }
 
-template <int NI, bool GATED, bool HP, bool VALUES>
+template <int NI, bool GATED, bool HP, bool VALUES, bool ASKS>
 int launch_t2d(const void* x, const void* packed, const float* values, const void* up, const void* down, void* out,
                int64_t M, int64_t H, int cf, int cs, int nc, float* ws_partial,
                unsigned int* ws_counter, const unsigned char* skip_rows, const FusedAr& ar,
                const RunIf& run_if, cudaStream_t stream) {
   const int slab_w = kTileN / cf;
   const int tiles = (int)(H / kTileN);
-  auto kern = twell_t2d_kernel<NI, GATED, HP, VALUES>;
+  auto kern = twell_t2d_kernel<NI, GATED, HP, VALUES, ASKS>;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(M * nc * cs), 1, 1);
   cfg.blockDim = dim3(NI * 32, 1, 1);
@@ -505,6 +520,18 @@ int launch_t2d(const void* x, const void* packed, const float* values, const voi
       cfg.gridDim = dim3((unsigned)(M * nc * cs), 1, 1);
     }
   }
+  if (ASKS) {
+    if (cs != 1 || nc != 1) return fail(B200_EINVAL, "twell_t2d: a choice of the device needs one CTA per token");
+    static int resident[64] = {};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
+    if (resident[dev] == 0) {
+      int n = 0;
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, NI * 32, 0) != cudaSuccess || n < 1) n = 1;
+      resident[dev] = n * sm_count();
+    }
+    if (M > resident[dev]) cfg.gridDim = dim3((unsigned)resident[dev], 1, 1);
+  }
   cfg.numAttrs = add_pdl_attribute(attr, 1, 2);
   cudaError_t e = cudaLaunchKernelEx(
       &cfg, kern, reinterpret_cast<const __nv_bfloat16*>(x),
@@ -516,7 +543,7 @@ int launch_t2d(const void* x, const void* packed, const float* values, const voi
   return B200_OK;
 }
 
-template <bool GATED, bool HP, bool VALUES = false>
+template <bool GATED, bool HP, bool VALUES = false, bool ASKS = false>
 int dispatch_ni(int ni, const void* x, const void* packed, const float* values, const void* up, const void* down,
                 void* out, int64_t M, int64_t H, int cf, int cs, int nc, float* ws_partial,
                 unsigned int* ws_counter, const unsigned char* skip_rows, const FusedAr& ar,
@@ -524,8 +551,9 @@ int dispatch_ni(int ni, const void* x, const void* packed, const float* values, 
   switch (ni) {
 #define B200_CASE(N)                                                                           \
   case N:                                                                                      \
-    return launch_t2d<N, GATED, HP, VALUES>(x, packed, values, up, down, out, M, H, cf, cs, nc, ws_partial,   \
-                                            ws_counter, skip_rows, ar, run_if, stream);
+    return launch_t2d<N, GATED, HP, VALUES, ASKS>(x, packed, values, up, down, out, M, H, cf,  \
+                                                  cs, nc, ws_partial, ws_counter, skip_rows, ar, \
+                                                  run_if, stream);
     B200_CASE(1) B200_CASE(2) B200_CASE(3) B200_CASE(4) B200_CASE(5) B200_CASE(6) B200_CASE(7)
     B200_CASE(8) B200_CASE(9) B200_CASE(10) B200_CASE(11) B200_CASE(12) B200_CASE(13)
     B200_CASE(14) B200_CASE(15) B200_CASE(16)
@@ -606,6 +634,13 @@ int t2d_launch(bool gated, bool hp, const void* x, const void* packed, const flo
   float* partial = workspace ? reinterpret_cast<float*>(counters + kCounterWords) : nullptr;
   const int ni = (int)(D / 256);
   auto run = [&](int cs_, int nc_) {
+    if (run_if.entries != nullptr) {  // only in fp32 products
+      if (!hp || values != nullptr) return fail(B200_EINVAL, "twell_t2d: no choice of the device in this form");
+      return gated ? dispatch_ni<true, true, false, true>(ni, x, packed, nullptr, up, down, out, M, H, cf, cs_,
+                                                          nc_, partial, counters, skip_rows, far, run_if, stream)
+                   : dispatch_ni<false, true, false, true>(ni, x, packed, nullptr, up, down, out, M, H, cf, cs_,
+                                                           nc_, partial, counters, skip_rows, far, run_if, stream);
+    }
     if (values != nullptr)
       return dispatch_ni<false, true, true>(ni, x, packed, values, up, down, out, M, H, cf, cs_, nc_,
                                             partial, counters, skip_rows, far, run_if, stream);
@@ -640,19 +675,17 @@ int twell_t2d_launch(bool gated, bool hp, const void* x, const void* packed, con
                      const void* down, void* out, int64_t M, int64_t D, int64_t H, int cf,
                      void* workspace, size_t workspace_bytes, int sm_count, cudaStream_t stream,
                      const unsigned char* skip_rows = nullptr,
-                     const FusedAr* fused_ar = nullptr, const RunIf& run_if = {nullptr, 0u}) {
+                     const FusedAr* fused_ar = nullptr, const RunIf& run_if = {nullptr, 0u, 0, nullptr}) {
   return t2d_launch(gated, hp, x, packed, nullptr, up, down, out, M, D, H, cf, workspace,
                     workspace_bytes, sm_count, stream, skip_rows, fused_ar, run_if);
 }
-
-int sm_count();  // c_api.cu
 
 // out = h down over the stored entries, h given in fp32 in the slots of the slab ([M][H / cf] floats).
 int twell_values_t2d(const void* packed, const float* values, const void* down, void* out, int64_t M,
                      int64_t D, int64_t H, int cf, void* workspace, size_t workspace_bytes,
                      cudaStream_t stream) {
   return t2d_launch(false, true, nullptr, packed, values, nullptr, down, out, M, D, H, cf, workspace,
-                    workspace_bytes, sm_count(), stream, nullptr, nullptr, {nullptr, 0u});
+                    workspace_bytes, sm_count(), stream, nullptr, nullptr, {nullptr, 0u, 0, nullptr});
 }
 
 }  // namespace b200
