@@ -150,10 +150,10 @@ int pair_gate_up_values(const void* x, const void* gate, const float* bias, cons
                                                  sm_count(), stream);
 }
 
-namespace {
-
 // Up and down rows together stay in L2, where a gathered entry is cheaper.
 bool rows_in_l2(int64_t D, int64_t H) { return 4 * H * D <= (int64_t)100 << 20; }
+
+namespace {
 
 // From this many tokens on the products are dense.  Measured under graph replay with weights from
 // HBM, us per layer, gather form at 0.5 % / 1 % / 2 % density -> dense form (any density):

@@ -25,6 +25,7 @@ namespace cg = cooperative_groups;
 namespace b200 {
 
 int sm_count();
+bool rows_in_l2(int64_t D, int64_t H);
 int pair_gate_up_values(const void* x, const void* gate, const float* bias, const void* up, void* packed,
                         float* values, int64_t M, int64_t D, int64_t H, int cf, cudaStream_t stream);
 int twell_values_t2d(const void* packed, const float* values, const void* down, void* out, int64_t M,
@@ -550,24 +551,36 @@ int token_box(int64_t M) { return M < tm::kRows ? (int)((M + 7) / 8 * 8) : tm::k
 
 }  // namespace
 
-// Which calls of the fused MLPs run here: from 33 tokens on, while the first launch fits one wave.  us per
-// layer under graph replay, weights from HBM, forms before (gathers, or pairs of SMs) -> now:
-//   gated    D 1024, H 4096:   64 tokens, 2 % 22 -> 14;  256 tokens 35 -> 16;  512 tokens 32 -> 23
-//            D 2048, H 5632:   37 tokens 27 -> 20;  128 tokens 38 -> 23;  384 tokens 47 -> 34
-//            D 2048, H 8192:   40 tokens, 0.5 % / 2 % 24 / 35 -> 24;  128 tokens 30 / 48 -> 27;
-//                              256 tokens 48 -> 38
-//            D 2048, H 11008:  64 tokens, 0.5 % / 2 % 30 / 44 -> 33;  128 tokens 60 -> 40
-//            D 4096, H 16384:  64 tokens, 0.5 % / 2 % 64 / 115 -> 73;  128 tokens 91 -> 77
-//   plain    D 2048, H 8192:   33 tokens, 0.5 % / 2 % 21 / 25 -> 20;  256 tokens 32 / 46 -> 30
-// Up to 32 tokens the gathers touch few rows (D 2048, H 8192, 32 tokens, 0.5 % / 2 % 17 / 24 -> 24).  In
-// two waves the form is level with the pairs at best (H 11008, 200 tokens 49 -> 54).
+// Which calls of the fused MLPs run here.  Up to 32 tokens the gathers touch few rows (D 2048, H 8192, 32
+// tokens, 0.5 % / 2 % 17 / 24 us against 24).  Beyond, a call cannot know its density: the line lies where the
+// tiles are level with the gathers at 1 %, which for wide layers is later, as the tiles stream all of up and
+// down.  us per layer under graph replay, weights from HBM, gathers at 0.5 / 1 / 2 % -> tiles (any density):
+//   gated    D 1024, H 4096:   33 tokens 13.4 / 14.0 / 15.9 -> 13.3;  128 tokens 16.9 / 19.0 / 23.3 -> 15.1
+//            D 2048, H 5632:   33 tokens 17.7 / 19.9 / 22.0 -> 19.7;  128 tokens 22.4 / 26.6 / 35.0 -> 21.9
+//            D 2048, H 8192:   33 tokens 18.9 / 21.1 / 25.0 -> 24.4 (not taken);  40 tokens 20.5 / 23.6 / 29.7
+//                              -> 24.6;  128 tokens 25.5 / 31.9 / 43.8 -> 26.9
+//            D 2048, H 11008:  64 tokens 25.9 / 30.4 / 38.6 -> 33.4 (not taken);  80 tokens 29.7 / 37.7 / 52.3
+//                              -> 33.8
+//            D 4096, H 16384:  64 tokens 60.5 / 76.8 / 108 -> 75.3 (not taken);  80 tokens 72 / 102 / 163 -> 76
+//   plain    D 2048, H 11008:  33 tokens 21.4 / 23.2 / 25.8 -> 24.9;  64 tokens 23.0 / 26.0 / 30.3 -> 25.5
+//            D 4096, H 16384:  64 tokens 43.1 / 48.2 / 57.7 -> 54.1 (not taken);  96 tokens 49.0 / 58.4 / 76.1
+//                              -> 56.3
+// and while the first launch fits one wave: against the pairs of SMs, D 1024, H 4096, 256 tokens 35 -> 17, 512
+// tokens 32 -> 23; D 2048, H 5632, 384 tokens 47 -> 34; H 8192, 256 tokens 48 -> 36; D 4096, H 16384, 128
+// tokens 91 -> 80.  In two waves the form is level with the pairs at best (H 11008, 200 tokens 49 -> 54).
 //
 // One row tile at H 8704 to 9472 stays with the gathers (or the pairs): its pack adds four ranges of D, of
 // which the accumulators of 128 neurons hold two.
-bool tile_mlp_serves(int64_t M, int64_t D, int64_t H, bool gated) {
+static bool tiles_fit(int64_t M, int64_t D, int64_t H, bool gated) {
   if (M < 33 || M > 512 || D > 4096 || H < 2048) return false;
   if (gated && M <= tm::kRows && H / 64 > fours() && H / 64 <= sm_count()) return false;
   return row_tiles(M) * (H / 128) <= sm_count();
+}
+
+bool tile_mlp_serves(int64_t M, int64_t D, int64_t H, bool gated) {
+  const int64_t from = gated ? (D * H <= (int64_t)12 << 20 ? 33 : D * H <= (int64_t)1 << 24 ? 40 : 80)
+                             : (D * H <= (int64_t)1 << 25 ? 33 : 96);
+  return M >= from && tiles_fit(M, D, H, gated);
 }
 
 // Slabs and hidden values ([M, H] bf16, 16-byte aligned); keep_all: of every gate positive, not only of
@@ -668,25 +681,30 @@ int tile_second(const void* hidden, const void* down, void* out, int64_t M, int6
 
 // High precision below the sizes of pair_mlp_serves: gate and up as tensor-core products, here or on pairs
 // of SMs, and the down product gathered along the stored entries with fp32 hidden values (half the rows
-// that gathering both reads, and no partial sums of the up product).  us per layer under graph replay, pack
-// + gathers -> now, at 0.5 % / 2 % density:
-//   D 1024, H 4096   33 tokens 17.7 / 18.9 -> 13.0 / 14.7;  256 tokens 22.9 / 32.7 -> 16.2 / 19.4;
-//                    6000 tokens 123 / 240 -> 118 / 175
-//   D 2048, H 8192   33 tokens 21.8 / 28.0 -> 23.4 / 28.5 (not taken);  48 tokens 23.5 / 33.3 -> 23.9 / 29.2;
-//                    257 tokens 39.0 / 71.1 -> 42.8 / 56.2;  777 tokens 78 / 162 -> 73 / 110;
-//                    4000 tokens 287 / 661 -> 242 / 385
-//   D 2048, H 11008  129 tokens, pairs 35.7 / 57.7 -> 42.8 / 53.0 (not taken);  160 tokens 43 / 86 -> 45 / 58
-//   D 4096, H 16384  at 1 %: 48 tokens 73 -> 70;  200 tokens 158 -> 104;  1000 tokens 517 -> 326
+// that gathering both reads, and no partial sums of the up product).  The lines lie as above.  us per layer
+// under graph replay, pack + gathers -> this form, at 0.5 / 1 / 2 % density:
+//   D 1024, H 4096   33 tokens 13.3 / 13.9 / 15.5 -> 13.3 / 13.7 / 14.9;  257 tokens 23 / 28 / 35 -> 20 / 21 / 23;
+//                    1500 tokens 43 / 54 / 79 -> 50 / 56 / 67;  4000 tokens 82 / 110 / 166 -> 92 / 104 / 131
+//   D 2048, H 5632   48 tokens 19.3 / 21.3 / 25.0 -> 21.2 / 22.2 / 24.2;  160 tokens 28 / 35 / 49 -> 30 / 34 / 41
+//   D 2048, H 8192   64 tokens 20.9 / 24.2 / 29.8 -> 24.3 / 26.5 / 29.5 (not taken);  96 tokens 24.3 / 29.5 / 40.5
+//                    -> 26.6 / 29.7 / 35.2;  777 tokens 78 / 103 / 161 -> 80 / 90 / 118;  4000 tokens 298 / 411 /
+//                    660 -> 290 / 345 / 439
+//   D 2048, H 11008  160 tokens 43 / 57 / 85 -> 51 / 55 / 63;  257 tokens 53 / 67 / 95 -> 69 / 75 / 87 (not taken:
+//                    two waves of pairs that are mostly padding);  400 tokens 68 / 95 / 147 -> 73 / 82 / 98
+//   D 4096, H 16384  48 tokens 55 / 67 / 94 -> 64 / 70 / 78 (not taken);  64 tokens 57 / 70 / 97 -> 65 / 70 / 78;
+//                    200 tokens 105 / 157 / 256 -> 93 / 108 / 139
 bool values_mlp_serves(int64_t M, int64_t D, int64_t H) {
   if (D > 4096 || H < 2048 || M * D * H >= (int64_t)1 << 36) return false;
-  return M >= 160 || (tile_mlp_serves(M, D, H, true) && M >= (D * H <= (int64_t)1 << 23 ? 33 : 48));
+  if (M >= 160) return !(M > 256 && M < 320 && D * H > (int64_t)1 << 24 && rows_in_l2(D, H));
+  const int64_t from = D * H <= (int64_t)1 << 23 ? 33 : D * H <= (int64_t)12 << 20 ? 48 : rows_in_l2(D, H) ? 96 : 64;
+  return M >= from && tiles_fit(M, D, H, true);
 }
 
 // values: [M, H / cf] fp32, 16-byte aligned.
 int values_mlp(const void* x, const void* gate, const float* bias, const void* up, const void* down,
                void* packed, void* out, int64_t M, int64_t D, int64_t H, int cf, void* workspace,
                size_t workspace_bytes, float* values, cudaStream_t stream) {
-  const int rc = tile_mlp_serves(M, D, H, true)
+  const int rc = tiles_fit(M, D, H, true)
                      ? tile_first(true, x, gate, bias, up, packed, nullptr, values, M, D, H, cf, false, stream)
                      : pair_gate_up_values(x, gate, bias, up, packed, values, M, D, H, cf, stream);
   if (rc) return rc;

@@ -11,12 +11,20 @@ from test_pair_gemm_gpu import DEV, run_case
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("m,d,h", [(33, 2048, 8192), (37, 256, 2048), (127, 768, 2304), (128, 4096, 4352),
+@pytest.mark.parametrize("m,d,h", [(33, 2048, 5632), (40, 2048, 8192), (37, 256, 2048), (127, 768, 2304), (128, 4096, 4352),
                                    (129, 1024, 8192), (256, 4096, 2048), (257, 2048, 5632),
-                                   (511, 512, 4096), (512, 1024, 4608), (64, 2048, 16384)])
+                                   (511, 512, 4096), (512, 1024, 4608), (80, 2048, 16384)])
 @pytest.mark.parametrize("cf,gated", [(8, True), (2, True), (8, False)])
 def test_tile_form(m, d, h, cf, gated):
     assert run_case(m, d, h, cf=cf, gated=gated) > 0
+
+
+@pytest.mark.parametrize("m,d,h,gated,hp", [(39, 2048, 8192, True, False), (79, 2048, 11008, True, False),
+                                            (95, 4096, 16384, False, False), (95, 2048, 8192, True, True),
+                                            (63, 4096, 16384, True, True), (300, 2048, 11008, True, True)])
+def test_wide_layers_gather_below_their_lines(m, d, h, gated, hp):
+    """The tiles stream all of up and down, which a few dozen tokens of low density do not touch."""
+    assert run_case(m, d, h, gated=gated, hp=hp) == 0
 
 
 @pytest.mark.parametrize("m,h", [(40, 2048), (300, 4096), (130, 16384)])
