@@ -141,10 +141,14 @@ int b200_twell_gated_mlp(const void* x, const void* gate, const float* gate_bias
  * with fp32 hidden values below 2^36 multiply-adds per product, and keeps them to 24 bits as three
  * bf16 terms of a dense product above.
  *   scratch: b200_twell_mlp_scratch_bytes(M, D, H, gated, flags) bytes (0 = such a call has no
- *     use for it), 16-byte aligned, uninitialised.  NULL or too small: the functions above.
+ *     use for it), 16-byte aligned, uninitialised.  NULL or too small: the functions above.  The size is
+ *     for any compression factor; with B200_SCRATCH_CF(cf) added to flags it is for that one (high
+ *     precision holds fp32 values in the slots of the slabs).
  *   workspace: as above; its zero-filled counters are also used to finish the last wave of
  *     tiles in ranges of k (without a workspace that wave runs unsplit).
  */
+#define B200_SCRATCH_CF(cf) ((uint32_t)(cf) << 8)
+
 size_t b200_twell_mlp_scratch_bytes(int64_t M, int64_t D, int64_t H, int gated, uint32_t flags);
 
 int b200_twell_gated_mlp_scratch(const void* x, const void* gate, const float* gate_bias,

@@ -19,6 +19,12 @@ LIB_PATH = _PKG_DIR / "libb200_sparse_ffn.so"
 OK = 0
 FLAG_HIGH_PRECISION = 1
 
+
+def scratch_cf(cf: int) -> int:
+    """Added to the flags of the scratch queries: the size for this compression factor."""
+    return int(cf) << 8
+
+
 _ERRORS = {
     -1: "invalid argument",
     -2: "null pointer",

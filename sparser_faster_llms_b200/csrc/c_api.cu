@@ -411,10 +411,10 @@ MlpForm mlp_form(int64_t M, int64_t D, int64_t H, bool gated, bool hp, int64_t m
   return pair_mlp_serves(M, D, H, gated, hp) ? kPairs : kGather;
 }
 
-size_t mlp_scratch(MlpForm form, int64_t M, int64_t D, int64_t H, bool hp, int64_t max_rows) {
+size_t mlp_scratch(MlpForm form, int64_t M, int64_t D, int64_t H, int cf, bool hp, int64_t max_rows) {
   switch (form) {
-    case kTiles: return (size_t)M * H * 2;        // hidden values in bf16
-    case kValues: return (size_t)M * (H / 2) * 4;  // in fp32, in slots of the widest slab
+    case kTiles: return (size_t)M * H * 2;         // hidden values in bf16
+    case kValues: return (size_t)M * (H / cf) * 4;  // in fp32, in the slots of the slabs
     case kPairs: return pair_mlp_scratch_bytes(M, D, H, hp, max_rows);
     default: return 0;
   }
@@ -424,12 +424,9 @@ size_t mlp_scratch(MlpForm form, int64_t M, int64_t D, int64_t H, bool hp, int64
 size_t b200_twell_mlp_scratch_bytes_chunked(int64_t M, int64_t D, int64_t H, int gated,
                                             uint32_t flags, int64_t max_rows) {
   const bool hp = (flags & B200_FLAG_HIGH_PRECISION) != 0;
-  const MlpForm form = mlp_form(M, D, H, gated != 0, hp, max_rows);
-  if (form == kGather) return 0;
-  // never less than the pairs take, whichever form the call's size selects
-  const size_t own = mlp_scratch(form, M, D, H, hp, max_rows);
-  const size_t pair = pair_mlp_scratch_bytes(M, D, H, hp, max_rows);
-  return own > pair ? own : pair;
+  const int cf = (int)(flags >> 8) & 15;
+  return mlp_scratch(mlp_form(M, D, H, gated != 0, hp, max_rows), M, D, H, cf == 4 || cf == 8 ? cf : 2, hp,
+                     max_rows);
 }
 
 size_t b200_twell_mlp_scratch_bytes(int64_t M, int64_t D, int64_t H, int gated, uint32_t flags) {
@@ -443,8 +440,8 @@ int b200_twell_gated_mlp_chunked(const void* x, const void* gate, const float* g
                                  size_t scratch_bytes, int64_t max_rows, void* stream) {
   const bool hp = (flags & B200_FLAG_HIGH_PRECISION) != 0;
   const MlpForm form = mlp_form(M, D, H, true, hp, max_rows);
-  if (form != kGather && scratch != nullptr &&
-      scratch_bytes >= mlp_scratch(form, M, D, H, hp, max_rows)) {
+  if (form != kGather && scratch != nullptr && (cf == 2 || cf == 4 || cf == 8) &&
+      scratch_bytes >= mlp_scratch(form, M, D, H, cf, hp, max_rows)) {
     B200_TRY(check_decode_args("b200_twell_gated_mlp", x, gate, gate_bias, up, down, packed, out,
                                M, D, H, cf, flags, workspace, true));
     B200_TRY(check_ptr("b200_twell_gated_mlp", "scratch", scratch));
@@ -566,7 +563,7 @@ int b200_twell_mlp_chunked(const void* x, const void* up, const void* down, void
                            size_t scratch_bytes, int64_t max_rows, void* stream) {
   const MlpForm form = mlp_form(M, D, H, false, false, max_rows);
   if ((num_splits == 1 || num_splits == 2 || num_splits == 4 || num_splits == 8) && form != kGather &&
-      scratch != nullptr && scratch_bytes >= mlp_scratch(form, M, D, H, false, max_rows)) {
+      scratch != nullptr && scratch_bytes >= mlp_scratch(form, M, D, H, 2, false, max_rows)) {
     B200_TRY(check_decode_args("b200_twell_mlp", x, up, nullptr, nullptr, down, packed, out, M, D,
                                H, cf, 0, workspace, false));
     B200_TRY(check_ptr("b200_twell_mlp", "scratch", scratch));

@@ -85,7 +85,7 @@ PyObject* call(PyObject*, PyObject* const* v, Py_ssize_t n) {
   at::Tensor scratch;
   size_t scratch_bytes = 0;
   if (m >= scratch_from)
-    scratch_bytes = scratch_fn(m, d, h, gated, gated ? (uint32_t)option : 0u);
+    scratch_bytes = scratch_fn(m, d, h, gated, (gated ? (uint32_t)option : 0u) | (uint32_t)cf << 8);
   if (scratch_bytes != 0)
     scratch = at::empty({(int64_t)scratch_bytes}, at::TensorOptions().dtype(at::kByte).device(dev));
   void* scratch_ptr = scratch_bytes != 0 ? scratch.data_ptr() : nullptr;

@@ -502,7 +502,7 @@ def _gated_mlp(layer_number, A, UP, DOWN, C_packed, OUT, highest_precision, cf) 
                   counters.data_ptr())
         route["last"] = counters
     else:
-        scratch, scratch_bytes = _mlp_scratch(dev, m, d, h, True, flags)
+        scratch, scratch_bytes = _mlp_scratch(dev, m, d, h, cf, True, flags)
         _lib.call("b200_twell_gated_mlp_scratch", dev, A.data_ptr(), GATE.data_ptr(),
                   _lib.ptr(entry["bias"]), UP.data_ptr(), DOWN.data_ptr(), C_packed.data_ptr(),
                   OUT.data_ptr(), m, d, h, cf, flags, *_lib.workspace(dev), _lib.ptr(scratch),
@@ -513,12 +513,13 @@ def _gated_mlp(layer_number, A, UP, DOWN, C_packed, OUT, highest_precision, cf) 
 _DENSE_FROM_TOKENS = 33  # no shape has a use for scratch below this many tokens
 
 
-def _mlp_scratch(dev, m, d, h, gated, flags) -> tuple[torch.Tensor | None, int]:
+def _mlp_scratch(dev, m, d, h, cf, gated, flags) -> tuple[torch.Tensor | None, int]:
     """Hidden matrix and partial sums of a call that runs on the tensor cores (None: it does
     not).  From torch's allocator on every call, so calls on several streams never share it."""
     if m < _DENSE_FROM_TOKENS:
         return None, 0
-    need = int(_lib.load_library().b200_twell_mlp_scratch_bytes(m, d, h, int(gated), flags))
+    need = int(_lib.load_library().b200_twell_mlp_scratch_bytes(m, d, h, int(gated),
+                                                                flags | _lib.scratch_cf(cf)))
     if need == 0:
         return None, 0
     return torch.empty(need, dtype=torch.uint8, device=dev), need
@@ -599,7 +600,7 @@ def _plain_mlp(layer_number, A, DOWN, C_packed, OUT, num_splits) -> None:
         raise ValueError(f"UP/DOWN must both be [{h}, {d}]")
     _check_packed(C_packed, m, h, entry["cf"], "C_packed")
     dev = _same_device(A, UP, DOWN, C_packed, OUT)
-    scratch, scratch_bytes = _mlp_scratch(dev, m, d, h, False, 0)
+    scratch, scratch_bytes = _mlp_scratch(dev, m, d, h, entry["cf"], False, 0)
     _lib.call("b200_twell_mlp_scratch", dev, A.data_ptr(), UP.data_ptr(), DOWN.data_ptr(),
               C_packed.data_ptr(), OUT.data_ptr(), m, d, h, entry["cf"], int(num_splits),
               *_lib.workspace(dev), _lib.ptr(scratch), scratch_bytes)

@@ -96,3 +96,29 @@ def test_without_a_workspace_no_tile_is_cut(m, d, h, gated, hp):
     rows = [0, 127, 128, m // 2, m - 1]
     ref = hidden_of(x[rows], up if gated else None, want[rows], h, 8, hp) @ down.double()
     assert ((out[rows].double().cpu() - ref).norm() / ref.norm()).item() < REL
+
+
+@pytest.mark.parametrize("m,d,h,cf,hp", [(40, 2048, 8192, 8, False), (300, 1024, 4096, 4, False),
+                                         (100, 2048, 8192, 8, True), (100, 2048, 8192, 2, True),
+                                         (777, 2048, 8192, 8, True), (777, 1024, 4352, 4, True)])
+def test_scratch_of_one_compression_factor(m, d, h, cf, hp):
+    """One-SM tiles, and fp32 hidden values in the slots of the slabs: nothing is written past the size."""
+    flags = _lib.FLAG_HIGH_PRECISION if hp else 0
+    need = _lib.load_library().b200_twell_mlp_scratch_bytes(m, d, h, 1, flags | _lib.scratch_cf(cf))
+    assert need == (m * h // cf * 4 if hp else 2 * m * h)
+    x, *weights = synthetic.dyadic_case(m, d, h, seed=m)
+    x[::5, 0] = -0.5
+    gate, up, down = weights
+    want = tf.pack_preactivations(fo.gate_preactivation(x, gate).numpy(), cf)
+    xg, gg, ug, dg = (t.to(DEV) for t in (x, *weights))
+    packed = twell.allocate_packed_output(m, h, device=DEV, compression_factor=cf)
+    out = torch.empty_like(xg)
+    scratch = torch.full((need + GUARD,), 0x5A, dtype=torch.uint8, device=DEV)
+    _lib.call("b200_twell_gated_mlp_scratch", DEV, xg.data_ptr(), gg.data_ptr(), None, ug.data_ptr(),
+              dg.data_ptr(), packed.data_ptr(), out.data_ptr(), m, d, h, cf, flags, *_lib.workspace(DEV),
+              scratch.data_ptr(), need)
+    torch.cuda.synchronize()
+    assert (packed.cpu().view(torch.int32).numpy().view("uint32") == want).all()
+    assert bool((scratch[need:] == 0x5A).all())
+    ref = hidden_of(x, up, want, h, cf, hp) @ down.double()
+    assert ((out.double().cpu() - ref).norm() / ref.norm()).item() < REL

@@ -37,7 +37,17 @@ def chunks(m, h, terms, max_rows):
     return [min(rows, m - r) for r in range(0, m, rows)]
 
 
-def mlp_need(m, d, h, terms, max_rows):
+def one_sm_tiles(m, d, h):
+    """Whether a gated bf16 call runs on one-SM tiles: its line, and one wave of them."""
+    start = 33 if d * h <= 12 << 20 else 40 if d * h <= 1 << 24 else 80
+    return start <= m <= 512 and -(-m // 128) * h // 128 <= 148 and not (m <= 128 and 132 < h // 64 <= 148)
+
+
+def mlp_need(m, d, h, terms, max_rows, cf=2):
+    if terms == 3 and not 0 < max_rows < m and m * d * h < 1 << 36:
+        return m * h // cf * 4  # fp32 hidden values in the slots of the slabs
+    if terms == 1 and not 0 < max_rows < m and one_sm_tiles(m, d, h):
+        return m * h * 2
     sizes = chunks(m, h, terms, max_rows)
     cut = 0
     for rows in set(sizes):
@@ -61,9 +71,19 @@ def test_fused_mlp_scratch_holds_every_chunk(lib, d, h, gated, flags):
     seen = 0
     for m in token_counts(h, terms):
         got = lib.b200_twell_mlp_scratch_bytes(m, d, h, gated, flags)
-        assert got == 0 or got >= mlp_need(m, d, h, terms, 0), m
+        need = mlp_need(m, d, h, terms, 0)
+        assert got == 0 or need <= got <= need + 256, m
         seen += got > 0
     assert seen > 40
+
+
+@pytest.mark.parametrize("cf", [2, 4, 8])
+def test_high_precision_scratch_follows_the_compression_factor(lib, cf):
+    flags = _lib.FLAG_HIGH_PRECISION | _lib.scratch_cf(cf)
+    for m, d, h in ((777, 2048, 8192), (100, 1024, 4096), (16383, 1024, 4096)):
+        assert lib.b200_twell_mlp_scratch_bytes(m, d, h, 1, flags) == m * h // cf * 4
+    for m, d, h in ((40, 1024, 4096), (100, 2048, 8192)):  # bf16 on one-SM tiles: hidden values, no sums
+        assert lib.b200_twell_mlp_scratch_bytes(m, d, h, 1, _lib.scratch_cf(cf)) == 2 * m * h
 
 
 @pytest.mark.parametrize("max_rows", [1, 256, 600, 4096])
