@@ -3,9 +3,12 @@
 ``python -m sparser_faster_llms_b200.build`` compiles every ``csrc/*.cu`` into
 ``sparser_faster_llms_b200/libb200_sparse_ffn.so`` with plain nvcc: no torch
 headers, no pybind, static cudart, so the result is a stable C ABI that loads
-with ``ctypes`` on a machine without a GPU driver.  ``csrc_host/host_call.cpp`` becomes the extension
-module ``_host_call`` (Python and torch headers, no CUDA code); without it eager calls take their Python
-path.
+with ``ctypes`` on a machine without a GPU driver.
+
+``csrc_host/host_call.cpp`` becomes the extension module ``_host_call`` with the host compiler (Python and torch
+headers, no CUDA code).  It reads torch's tensors in place, so its file name carries the torch version, the C++
+ABI and Python's own tag, and only the file of the running pair is loaded.  It is optional: where torch, a
+compiler or the headers are missing the build warns, and eager calls take their Python path.
 """
 from __future__ import annotations
 
@@ -13,6 +16,8 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
+import warnings
 from pathlib import Path
 
 PKG_DIR = Path(__file__).resolve().parent
@@ -20,7 +25,6 @@ CSRC = PKG_DIR / "csrc"
 LIB_NAME = "libb200_sparse_ffn.so"
 LIB_PATH = PKG_DIR / LIB_NAME
 HOST_SOURCE = PKG_DIR / "csrc_host" / "host_call.cpp"
-HOST_PATH = PKG_DIR / "_host_call.so"
 GENCODE = "arch=compute_100a,code=sm_100a"
 
 
@@ -39,34 +43,50 @@ def sources() -> list[Path]:
     return sorted(CSRC.glob("*.cu"))
 
 
-def host_needs_build() -> bool:
-    return not HOST_PATH.exists() or HOST_SOURCE.stat().st_mtime > HOST_PATH.stat().st_mtime
-
-
-def start_host_build() -> tuple[Path, subprocess.Popen]:
-    """Starts the compiler on the extension module; it becomes visible when it is renamed."""
-    import sysconfig
-
+def host_path() -> Path:
+    """The extension module of the running Python and torch."""
     import torch
 
+    return PKG_DIR / (f"_host_call.torch-{torch.__version__}-abi{int(torch._C._GLIBCXX_USE_CXX11_ABI)}"
+                      f"{sysconfig.get_config_var('EXT_SUFFIX')}")
+
+
+def start_host_build(force: bool = False) -> tuple[Path, subprocess.Popen] | None:
+    """Starts the compiler on the extension module if it is missing or older than its source; None if there
+    is nothing to do or nothing to do it with."""
+    try:
+        import torch
+    except ImportError:
+        warnings.warn("no torch: the native host side of eager calls is not built")
+        return None
+    path = host_path()
+    if not force and path.exists() and HOST_SOURCE.stat().st_mtime <= path.stat().st_mtime:
+        return None
     root = Path(torch.__file__).parent
-    cuda = Path(find_nvcc()).resolve().parent.parent
-    tmp = HOST_PATH.with_suffix(".so.tmp")
-    include = [sysconfig.get_paths()["include"], root / "include",
-               root / "include" / "torch" / "csrc" / "api" / "include", cuda / "include"]
-    cmd = [shutil.which("g++") or "c++", "-O2", "-std=c++17", "-fPIC", "-shared",
-           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
-           *(f"-I{p}" for p in include), str(HOST_SOURCE), "-o", str(tmp), f"-L{root / 'lib'}",
-           "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
-    return tmp, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    tmp = path.with_name(path.name + ".tmp")
+    try:
+        cuda = Path(find_nvcc()).resolve().parent.parent
+        include = [sysconfig.get_paths()["include"], root / "include",
+                   root / "include" / "torch" / "csrc" / "api" / "include", cuda / "include"]
+        cmd = [shutil.which("g++") or "c++", "-O2", "-std=c++17", "-fPIC", "-shared",
+               f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+               *(f"-I{p}" for p in include), str(HOST_SOURCE), "-o", str(tmp), f"-L{root / 'lib'}",
+               "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+        return tmp, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    except (OSError, RuntimeError) as e:
+        warnings.warn(f"the native host side of eager calls is not built: {e}")
+        return None
 
 
 def finish_host_build(started: tuple[Path, subprocess.Popen]) -> None:
+    """The module becomes visible when it is renamed."""
     tmp, proc = started
     out, _ = proc.communicate()
-    if proc.returncode != 0:
-        raise RuntimeError(f"compiler failed on {HOST_SOURCE.name}:\n{out}")
-    os.replace(tmp, HOST_PATH)
+    if proc.returncode == 0:
+        os.replace(tmp, tmp.with_suffix(""))
+        return
+    tmp.unlink(missing_ok=True)
+    warnings.warn(f"the native host side of eager calls is not built, the compiler failed on {HOST_SOURCE.name}:\n{out}")
 
 
 def needs_build() -> bool:
@@ -80,7 +100,7 @@ def needs_build() -> bool:
 
 def build_library(force: bool = False, verbose: bool = False, extra_flags=()) -> Path:
     """Compile the library and the host module where missing or older than their sources."""
-    host = start_host_build() if force or host_needs_build() else None
+    host = start_host_build(force)
     try:
         return _build_library(force, verbose, extra_flags)
     finally:

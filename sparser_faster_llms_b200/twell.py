@@ -21,7 +21,9 @@ pybind extension.  Differences a caller can observe:
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 import os
+import warnings
 from pathlib import Path
 from types import SimpleNamespace
 from typing import Final
@@ -31,10 +33,25 @@ from torch import nn
 
 from . import _lib
 
-try:  # native host side of eager calls; without it the Python path below serves them
-    from . import _host_call
-except ImportError:
-    _host_call = None
+
+def _load_host_call():
+    """Native host side of eager calls, built for this Python and torch; without it (None) the Python path
+    below serves them."""
+    from .build import host_path
+    path = host_path()
+    if not path.exists():
+        return None
+    try:
+        spec = importlib.util.spec_from_file_location(f"{__package__}._host_call", path)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        return module
+    except ImportError as e:
+        warnings.warn(f"{path.name} does not load, eager calls take their Python path: {e}")
+        return None
+
+
+_host_call = _load_host_call()
 
 # Attributes the reference module exposes and the reference benchmark pokes at
 # (benchmark_inference.py:55-117).  There is no JIT build here; they exist so that
