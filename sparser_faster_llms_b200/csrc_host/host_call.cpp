@@ -65,6 +65,10 @@ PyObject* call(PyObject*, PyObject* const* v, Py_ssize_t n) {
   const at::Tensor* bias = v[4] == Py_None ? nullptr : plain(v[4], at::kFloat, 1);
   if (x == nullptr || first == nullptr || (v[4] != Py_None && bias == nullptr)) Py_RETURN_NONE;
   const long cf = PyLong_AsLong(v[9]), option = PyLong_AsLong(v[10]);
+  if (PyErr_Occurred()) {  // no number, or one beyond a long: the Python path decides
+    PyErr_Clear();
+    Py_RETURN_NONE;
+  }
   const int64_t m = x->size(0), d = x->size(1), h = first->size(0);
   if ((cf != 2 && cf != 4 && cf != 8) || h % 256 != 0) Py_RETURN_NONE;
   if (first->size(1) != d || !is_matrix(up, h, d) || !is_matrix(down, h, d) || !is_matrix(out, m, d) ||

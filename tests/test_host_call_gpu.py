@@ -60,3 +60,25 @@ def test_other_cases_take_the_python_path(served):
     mod.enable_dense_route(min_tokens=4)  # routed calls are not asked about
     mod(x)
     assert len(served) == 5
+
+
+@pytest.mark.parametrize("splits", [1 << 70, (1 << 70) + 2, -1])
+def test_numbers_beyond_a_long_are_left_to_the_python_path(served, monkeypatch, splits):
+    """ctypes passes the low 32 bits of a split count, and 0 and -1 are refused."""
+    _, u, dn = weights()
+    x = torch.zeros(40, 512, dtype=torch.bfloat16, device=DEV)
+    twell.create_d2t_layer(9502, u)
+
+    def outcome():
+        try:
+            return twell.run_mlp_layer(9502, x, dn, splits)
+        except ValueError as e:
+            return str(e)
+
+    native = outcome()
+    assert served == ([None] if splits > 1 << 62 else [-1])
+    monkeypatch.setattr(twell, "_host_call", None)
+    python = outcome()
+    assert type(native) is type(python)
+    assert torch.equal(native, python) if isinstance(python, torch.Tensor) else native == python
+    twell.destroy_d2t_layer(9502)
