@@ -264,16 +264,14 @@ def one_token_layer(B: int, d: int, hl: int, par) -> bool:
 
 def pack_kernel_name(B: int, d: int, hl: int) -> str:
     """The kernel b200_twell_pack launches for this call (csrc/c_api.cu)."""
-    tiles = hl // 256
     if B == 1 and d in (2048, 4096):
         return "twell_gemv_kernel"
     if B <= 16:
         return "twell_pack_kernel"
-    if B <= 32:
-        return "twell_pack_tc_splitk_wide_kernel"
-    if (B <= 128 and tiles * 4 <= 148) or (B <= 256 and tiles <= 16):
-        return "twell_pack_tc_splitk_mid_kernel"
-    return "pair_gemm_kernel"
+    one_wave = -(-B // 128) * (hl // 128) <= 148  # of one-SM tiles of 128 tokens x 128 neurons
+    if B <= 32:  # one-SM tiles where the split over a cluster would be two waves
+        return "first_kernel" if hl // 64 > 132 and one_wave else "twell_pack_tc_splitk_wide_kernel"
+    return "first_kernel" if B <= 256 and one_wave else "pair_gemm_kernel"
 
 
 def run_ours(args):

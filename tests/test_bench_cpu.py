@@ -33,3 +33,15 @@ def test_reference_arm_on_other_ranks_exits_quietly():
                          timeout=600, cwd=REPO, env=env)
     assert res.returncode == 0
     assert not [l for l in res.stdout.splitlines() if l.startswith("{")]
+
+
+def test_the_named_pack_kernel_is_the_one_that_the_library_selects():
+    """Token counts and layers on both sides of the selection in csrc/tile_mlp.cu (148 SMs)."""
+    sys.path.insert(0, str(REPO))
+    import bench
+    want = {(1, 2048, 8192): "twell_gemv_kernel", (8, 2048, 8192): "twell_pack_kernel",
+            (32, 2048, 8192): "twell_pack_tc_splitk_wide_kernel", (32, 2048, 11008): "first_kernel",
+            (33, 2048, 8192): "first_kernel", (128, 4096, 16384): "first_kernel",
+            (256, 2048, 8192): "first_kernel", (256, 2048, 11008): "pair_gemm_kernel",
+            (257, 1024, 4096): "pair_gemm_kernel"}
+    assert {k: bench.pack_kernel_name(*k) for k in want} == want
