@@ -711,6 +711,8 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap map_a0,
           }
         }
       }
+      const int next = s;
+      const uint32_t pass = phase;
       // the commits of the last stages must have arrived before this CTA may leave
 #pragma unroll 1
       for (int i = 0; i < STAGES && ok; ++i) {
@@ -723,6 +725,9 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap map_a0,
       if (!ok) {
         abort_s = 1;
         atomicExch(&g_error, 1);
+        // copies in flight land before the pair leaves: the leader's barriers count both CTAs'
+        if (crank == 0)
+          for (int j = 0; j < STAGES; ++j) mbar_wait(&full_bar[j], j < next ? pass ^ 1u : pass);
       }
     }
   } else if (warp == 1) {
