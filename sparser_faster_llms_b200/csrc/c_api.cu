@@ -423,7 +423,7 @@ size_t mlp_scratch(MlpForm form, int64_t M, int64_t D, int64_t H, int cf, bool h
 
 size_t b200_twell_mlp_scratch_bytes_chunked(int64_t M, int64_t D, int64_t H, int gated,
                                             uint32_t flags, int64_t max_rows) {
-  const bool hp = (flags & B200_FLAG_HIGH_PRECISION) != 0;
+  const bool hp = gated != 0 && (flags & B200_FLAG_HIGH_PRECISION) != 0;
   const int cf = (int)(flags >> 8) & 15;
   return mlp_scratch(mlp_form(M, D, H, gated != 0, hp, max_rows), M, D, H, cf == 4 || cf == 8 ? cf : 2, hp,
                      max_rows);

@@ -635,7 +635,7 @@ int t2d_launch(bool gated, bool hp, const void* x, const void* packed, const flo
   const int ni = (int)(D / 256);
   auto run = [&](int cs_, int nc_) {
     if (run_if.entries != nullptr) {  // only in fp32 products
-      if (!hp || values != nullptr) return fail(B200_EINVAL, "twell_t2d: no choice of the device in this form");
+      if (!hp || values != nullptr || skip_rows != nullptr) return fail(B200_EINVAL, "twell_t2d: no choice of the device in this form");
       return gated ? dispatch_ni<true, true, false, true>(ni, x, packed, nullptr, up, down, out, M, H, cf, cs_,
                                                           nc_, partial, counters, skip_rows, far, run_if, stream)
                    : dispatch_ni<false, true, false, true>(ni, x, packed, nullptr, up, down, out, M, H, cf, cs_,
