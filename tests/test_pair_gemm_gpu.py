@@ -157,3 +157,28 @@ def test_last_wave_cut_along_k(m, h, hp, gated, kind):
     """64 k-steps: the tiles of the last wave are cut in four (18 tiles) or two (32 and 34) ranges, whose sums
     the warps that arrive last add; gate values and the dense operand come out of the sums."""
     assert run_case(m, 4096, h, hp=hp, gated=gated, dense=kind == "dense") > 0
+
+
+@pytest.mark.parametrize("gated", [True, False])
+def test_a_captured_call_chooses_anew_at_every_replay(gated):
+    m, d, h = 6145, 2048, 8192
+    x, gate, up, down = synthetic.dyadic_case(m, d, h, seed=21)
+    g, u, dn = (t.to(DEV) for t in (gate, up, down))
+    mod = twell.TwELLGatedMLP(9310, g, u, dn) if gated else twell.TwELLMLP(9310, g, dn)
+    dense = x.to(DEV)
+    sparse = dense.clone()
+    sparse[:, 0] = 1.5
+    buf = sparse.clone()
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.no_grad(), torch.cuda.stream(stream):
+        want = [mod(sparse), mod(dense)]  # also the workspace of this stream
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            out = mod(buf)
+        for new, y in ((dense, want[1]), (sparse, want[0]), (dense, want[1])):
+            buf.copy_(new)
+            graph.replay()
+            stream.synchronize()
+            assert torch.equal(out, y)
+    mod.destroy()
