@@ -84,7 +84,8 @@ int b200_twell_pack(const void* x, const void* w, const float* bias, void* packe
  *              automatically for such calls unless B200_ONE_TOKEN=0,
  *   kernel 7 = persistent tcgen05 kernel on pairs of SMs, 256 tokens x 256 neurons per pair, two
  *              accumulators (2 and 4 are other names of it),
- *   kernel 8 / 9 = tcgen05 split-k cluster kernel with 128-token tiles, D split 4 / 2 ways.
+ *   kernel 8 / 9 = tcgen05 split-k cluster kernel with 128-token tiles, D split 4 / 2 ways (never
+ *              automatic; at 33..128 tokens kernel 8 adds the same sums as the one-SM tiles).
  * All produce identical slab bytes on exact-arithmetic inputs.  No reference
  * counterpart (the reference has one WGMMA kernel, matmul_d2t.cu:287-709).
  */
@@ -146,6 +147,10 @@ int b200_twell_gated_mlp(const void* x, const void* gate, const float* gate_bias
  *     precision holds fp32 values in the slots of the slabs).
  *   workspace: as above; its zero-filled counters are also used to finish the last wave of
  *     tiles in ranges of k (without a workspace that wave runs unsplit).
+ * From 1.5 * 2^36 multiply-adds per product on (high precision: 2^36) the device chooses between the
+ * dense products and the gathers by the stored entries, of the call or of a sample of its tokens.
+ * The dense down product reads every row of `down`: an infinite or NaN row that no token activates
+ * makes its column of every token NaN, where the gathers never touch it.
  */
 #define B200_SCRATCH_CF(cf) ((uint32_t)(cf) << 8)
 
