@@ -553,7 +553,8 @@ int token_box(int64_t M) { return M < tm::kRows ? (int)((M + 7) / 8 * 8) : tm::k
 
 // Which calls of the fused MLPs run here.  Up to 32 tokens the gathers touch few rows (D 2048, H 8192, 32
 // tokens, 0.5 % / 2 % 17 / 24 us against 24).  Beyond, a call cannot know its density: the line lies where the
-// tiles are level with the gathers at 1 %, which for wide layers is later, as the tiles stream all of up and
+// tiles are level with the gathers at 1 %, and gated layers whose rows come from HBM wait until they are level
+// at 0.5 %.  For wide layers that is later, as the tiles stream all of up and
 // down.  us per layer under graph replay, weights from HBM, gathers at 0.5 / 1 / 2 % -> tiles (any density):
 //   gated    D 1024, H 4096:   33 tokens 13.4 / 14.0 / 15.9 -> 13.3;  128 tokens 16.9 / 19.0 / 23.3 -> 15.1
 //            D 2048, H 5632:   33 tokens 17.7 / 19.9 / 22.0 -> 19.7;  128 tokens 22.4 / 26.6 / 35.0 -> 21.9
@@ -687,15 +688,15 @@ int tile_second(const void* hidden, const void* down, void* out, int64_t M, int6
 //                    1500 tokens 43 / 54 / 79 -> 50 / 56 / 67;  4000 tokens 82 / 110 / 166 -> 92 / 104 / 131
 //   D 2048, H 5632   48 tokens 19.3 / 21.3 / 25.0 -> 21.2 / 22.2 / 24.2;  160 tokens 28 / 35 / 49 -> 30 / 34 / 41
 //   D 2048, H 8192   64 tokens 20.9 / 24.2 / 29.8 -> 24.3 / 26.5 / 29.5 (not taken);  96 tokens 24.3 / 29.5 / 40.5
-//                    -> 26.6 / 29.7 / 35.2;  777 tokens 78 / 103 / 161 -> 80 / 90 / 118;  4000 tokens 298 / 411 /
+//                    -> 26.6 / 29.7 / 35.2;  257 tokens 39 / 51 / 70 -> 47 / 52 / 60 (not taken: pairs of SMs
+//                    that are mostly padding);  777 tokens 78 / 103 / 161 -> 80 / 90 / 118;  4000 tokens 298 / 411 /
 //                    660 -> 290 / 345 / 439
-//   D 2048, H 11008  160 tokens 43 / 57 / 85 -> 51 / 55 / 63;  257 tokens 53 / 67 / 95 -> 69 / 75 / 87 (not taken:
-//                    two waves of pairs that are mostly padding);  400 tokens 68 / 95 / 147 -> 73 / 82 / 98
+//   D 2048, H 11008  160 tokens 43 / 57 / 85 -> 51 / 55 / 63;  257 tokens 53 / 67 / 95 -> 69 / 75 / 87 (not taken);  400 tokens 68 / 95 / 147 -> 73 / 82 / 98
 //   D 4096, H 16384  48 tokens 55 / 67 / 94 -> 64 / 70 / 78 (not taken);  64 tokens 57 / 70 / 97 -> 65 / 70 / 78;
 //                    200 tokens 105 / 157 / 256 -> 93 / 108 / 139
 bool values_mlp_serves(int64_t M, int64_t D, int64_t H) {
   if (D > 4096 || H < 2048 || M * D * H >= (int64_t)1 << 36) return false;
-  if (M >= 160) return !(M > 256 && M < 320 && D * H > (int64_t)1 << 24 && rows_in_l2(D, H));
+  if (M >= 160) return !(M > 256 && M < 320 && D * H >= (int64_t)1 << 24 && rows_in_l2(D, H));
   const int64_t from = D * H <= (int64_t)1 << 23 ? 33 : D * H <= (int64_t)12 << 20 ? 48 : rows_in_l2(D, H) ? 96 : 64;
   return M >= from && tiles_fit(M, D, H, true);
 }

@@ -21,7 +21,8 @@ def test_tile_form(m, d, h, cf, gated):
 
 @pytest.mark.parametrize("m,d,h,gated,hp", [(39, 2048, 8192, True, False), (79, 2048, 11008, True, False),
                                             (95, 4096, 16384, False, False), (95, 2048, 8192, True, True),
-                                            (63, 4096, 16384, True, True), (300, 2048, 11008, True, True)])
+                                            (63, 4096, 16384, True, True), (257, 2048, 8192, True, True),
+                                            (300, 2048, 11008, True, True)])
 def test_wide_layers_gather_below_their_lines(m, d, h, gated, hp):
     """The tiles stream all of up and down, which a few dozen tokens of low density do not touch."""
     assert run_case(m, d, h, gated=gated, hp=hp) == 0
